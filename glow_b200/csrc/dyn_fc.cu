@@ -9,9 +9,10 @@
 // include/glow/Quantization/Base/Base.h:322-329), multiplied with the int8 weights into int32
 // sums, and the result is fp16(float(sum) * (row scale * weight scale[j]) + bias[j]).
 //
-// Two launches: a warp per input row finds the range, derives the parameters in the reference's
-// double arithmetic and writes the int8 row, its scale and (for weights with offsets) its sum;
-// then the tcgen05 contraction of qgemm.cu runs with its floating-point drain.
+// Two launches: a warp or a block per input row finds the range, derives the parameters in the
+// reference's double arithmetic and writes the int8 row (zero padded to whole 16-byte pieces), its
+// scale and (for weights with offsets) its sum; then the contraction runs with its floating-point
+// drain.  Weights off that grid, or given as [K, N], are copied first, in a launch of their own.
 #include "qgemm.cuh"
 #include "quant_math.cuh"
 
@@ -25,65 +26,6 @@ __device__ __forceinline__ int32_t quantize_i8(float x, float scale, float offse
   return (int32_t)(v < -128 ? -128 : (v > 127 ? 127 : v));
 }
 
-// in [M, K] fp16 -> q [M, K] int8, row_scales [M], row_sums [M] (may be nullptr).  A block per
-// row, element by element: the form for rows that are not 16-byte aligned multiples of 8.
-constexpr int kQuantThreads = 256;
-
-__global__ void __launch_bounds__(kQuantThreads) dyn_quantize_rows_kernel(const __half *__restrict__ in, int M, int K,
-                                                                          int8_t *__restrict__ q, float *__restrict__ row_scales,
-                                                                          int32_t *__restrict__ row_sums, int32_t *status) {
-  pdl_launch_dependents();  // a contraction that follows may set up now (it waits for this kernel before its loads)
-  __shared__ float s_mn[kQuantThreads / 32], s_mx[kQuantThreads / 32];
-  __shared__ int32_t s_sum[kQuantThreads / 32];
-  const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const __half *x = in + (size_t)row * K;
-  // minMaxArg over the row: NaNs never win a comparison
-  float mn = __half2float(x[0]), mx = mn;
-  for (int k = tid; k < K; k += kQuantThreads) {
-    const float v = __half2float(x[k]);
-    mn = v < mn ? v : mn;
-    mx = v > mx ? v : mx;
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    const float a = __shfl_xor_sync(0xffffffffu, mn, d), b = __shfl_xor_sync(0xffffffffu, mx, d);
-    mn = a < mn ? a : mn;
-    mx = b > mx ? b : mx;
-  }
-  if (lane == 0) { s_mn[warp] = mn; s_mx[warp] = mx; }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kQuantThreads / 32; i++) {
-    mn = s_mn[i] < mn ? s_mn[i] : mn;
-    mx = s_mx[i] > mx ? s_mx[i] : mx;
-  }
-  double scale_d;
-  int32_t offset;
-  choose_quantization_params_basic(mn, mx, /*Symmetric*/ 1, -128, 127, scale_d, offset);
-  const float scale = (float)scale_d, foffset = (float)offset;
-  // A symmetric range always nudges the zero point to 0; the contraction relies on it.
-  if (offset != 0 && tid == 0 && status != nullptr) atomicOr(status, GLOWB200_STATUS_UNSUPPORTED_TABLE);
-  int32_t sum = 0;
-  int8_t *o = q + (size_t)row * K;
-  for (int k = tid; k < K; k += kQuantThreads) {
-    const int32_t v = quantize_i8(__half2float(x[k]), scale, foffset);
-    o[k] = (int8_t)v;
-    sum += v;
-  }
-  if (row_sums != nullptr) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-    if (lane == 0) s_sum[warp] = sum;
-    __syncthreads();
-    if (tid == 0) {
-      int32_t total = 0;
-      for (int i = 0; i < kQuantThreads / 32; i++) total += s_sum[i];
-      row_sums[row] = total;
-    }
-  }
-  if (tid == 0) row_scales[row] = scale;
-}
-
 // fp16 bits -> float through the mixed-precision add (adding -0 keeps every value): conversion
 // instructions issue at an eighth of the rate.
 __device__ __forceinline__ float widen_f16(uint32_t h) {
@@ -92,29 +34,75 @@ __device__ __forceinline__ float widen_f16(uint32_t h) {
   return d;
 }
 
-// A WARP per row (K a multiple of 8, 16-byte aligned rows): the range is found on the fp16 pairs
-// themselves and reduced with shuffles, the second pass reads the row again (from L1 / L2) so
-// that few registers are held and many warps stay resident, and no block-wide barrier sits
-// between the load and the store.  Eight elements are quantized by reciprocal at a time; a tie
-// candidate among them sends the eight through the exact division.
-__global__ void __launch_bounds__(256) dyn_quantize_rows_warp_kernel(const __half *__restrict__ in, int M, int K,
-                                                                     int8_t *__restrict__ q, float *__restrict__ row_scales,
-                                                                     int32_t *__restrict__ row_sums, int32_t *status) {
+// Eight fp16 numbers from `p` on, positions from `valid` on replaced by `fill`.  VEC: rows are 16-byte
+// aligned multiples of 8; else only 4-byte words that hold a wanted number are touched.
+template <bool VEC>
+__device__ __forceinline__ void load8(const __half *p, int valid, uint32_t fill, uint32_t (&w)[4]) {
+  if constexpr (VEC) {
+    const uint4 v = valid > 0 ? *reinterpret_cast<const uint4 *>(p) : make_uint4(fill, fill, fill, fill);
+    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+  } else {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const int odd = (int)(a >> 1) & 1;
+    const uint32_t *x = reinterpret_cast<const uint32_t *>(a - 2 * odd);
+    uint32_t r[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) r[i] = (2 * i - odd < valid && (i < 4 || odd)) ? x[i] : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      w[i] = __funnelshift_r(r[i], r[i + 1], 16 * odd);
+      const int left = valid - 2 * i;
+      if (left == 1) w[i] = __byte_perm(w[i], fill, 0x5410);
+      else if (left <= 0) w[i] = fill;
+    }
+  }
+}
+
+// in [M, K] fp16 -> q [M, pitch] int8 (zero behind column K), row_scales [M], row_sums [M] (may be
+// nullptr).  WPR warps per row: one when the rows fill the SMs, else eight (a row of 4096 is then one
+// or two steps of its block instead of sixteen of a warp).  The range is found on the fp16 pairs
+// themselves; the second pass reads the row again (from L1 / L2) so that few registers are held and
+// many warps stay resident.  Eight elements are quantized by reciprocal at a time; a tie candidate
+// among them sends the eight through the exact division.
+// CH > 0: rows of at most CH steps, whose numbers stay in registers between the two passes.
+template <int WPR, bool VEC, int CH>
+__global__ void __launch_bounds__(256) dyn_quantize_rows_kernel(const __half *in, int M, int K, int pitch,
+                                                                int8_t *__restrict__ q, float *__restrict__ row_scales,
+                                                                int32_t *__restrict__ row_sums, int32_t *status) {
+  __shared__ float s_mn[8], s_mx[8];
+  __shared__ int32_t s_sum[8];
+  pdl_wait();
   pdl_launch_dependents();  // a contraction that follows may set up now (it waits for this kernel before its loads)
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = WPR == 1 ? blockIdx.x * 8 + warp : blockIdx.x;
   if (row >= M) return;
+  const int first = (WPR == 1 ? lane : (int)threadIdx.x) * 8;
+  constexpr int kStep = WPR * 256;
   const __half *x = in + (size_t)row * K;
   // minMaxArg over the row (NaNs never win a comparison; min / max of fp16 numbers is exact)
-  __half2 mn2 = __half2half2(x[0]), mx2 = mn2;
-#pragma unroll 4
-  for (int k = lane * 8; k < K; k += 256) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(x + k);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  const __half2 x00 = __half2half2(x[0]);
+  const uint32_t fill = *reinterpret_cast<const uint32_t *>(&x00);
+  __half2 mn2 = x00, mx2 = x00;
+  uint32_t kept[CH ? CH : 1][4];
+  auto range = [&](const uint32_t (&w)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const __half2 h = *reinterpret_cast<const __half2 *>(&w[i]);
       mn2 = __hmin2(mn2, h);
       mx2 = __hmax2(mx2, h);
+    }
+  };
+  if constexpr (CH > 0) {
+#pragma unroll
+    for (int c = 0; c < CH; c++) load8<VEC>(x + first + c * kStep, K - first - c * kStep, fill, kept[c]);
+#pragma unroll
+    for (int c = 0; c < CH; c++) range(kept[c]);
+  } else {
+#pragma unroll 4
+    for (int k = first; k < K; k += kStep) {
+      uint32_t w[4];
+      load8<VEC>(x + k, K - k, fill, w);
+      range(w);
     }
   }
   float mn = fminf(__low2float(mn2), __high2float(mn2)), mx = fmaxf(__low2float(mx2), __high2float(mx2));
@@ -123,10 +111,18 @@ __global__ void __launch_bounds__(256) dyn_quantize_rows_warp_kernel(const __hal
     mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, d));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
   }
+  if constexpr (WPR > 1) {
+    if (lane == 0) { s_mn[warp] = mn; s_mx[warp] = mx; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < WPR; i++) {
+      mn = fminf(mn, s_mn[i]);
+      mx = fmaxf(mx, s_mx[i]);
+    }
+  }
   // Handle::minMaxArg starts from element 0 and keeps what no later element beats: a NaN there
   // stays (every comparison with it is false), a NaN anywhere else never gets in.  The min / max
-  // instructions above drop NaNs wherever they are, so the first element is looked at again --
-  // the row then quantizes as it does in the kernel that compares with '<' and '>'.
+  // instructions above drop NaNs wherever they are, so the first element is looked at again.
   {
     const float x0 = __half2float(x[0]);
     if (x0 != x0) mn = mx = x0;
@@ -136,13 +132,11 @@ __global__ void __launch_bounds__(256) dyn_quantize_rows_warp_kernel(const __hal
   choose_quantization_params_basic(mn, mx, /*Symmetric*/ 1, -128, 127, scale_d, offset);
   const float scale = (float)scale_d, foffset = (float)offset;
   const float rcp = __frcp_rn(scale);
-  if (offset != 0 && lane == 0 && status != nullptr) atomicOr(status, GLOWB200_STATUS_UNSUPPORTED_TABLE);
+  // A symmetric range always nudges the zero point to 0; the contraction relies on it.
+  if (offset != 0 && first == 0 && status != nullptr) atomicOr(status, GLOWB200_STATUS_UNSUPPORTED_TABLE);
   int32_t sum = 0;
-  int8_t *o = q + (size_t)row * K;
-#pragma unroll 2
-  for (int k = lane * 8; k < K; k += 256) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(x + k);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  int8_t *o = q + (size_t)row * pitch;
+  auto quantize = [&](int k, const uint32_t (&w)[4]) {
     float f[8];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -167,6 +161,11 @@ __global__ void __launch_bounds__(256) dyn_quantize_rows_warp_kernel(const __hal
 #pragma unroll
       for (int i = 0; i < 8; i++) r[i] = quantize_i8(f[i], scale, foffset);
     }
+    if (k + 8 > K) {  // the padding
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (k + i >= K) r[i] = 0;
+    }
     uint32_t packed[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -175,13 +174,48 @@ __global__ void __launch_bounds__(256) dyn_quantize_rows_warp_kernel(const __hal
                   ((uint32_t)(r[4 * h + 3] & 0xff) << 24);
     }
     *reinterpret_cast<uint2 *>(o + k) = make_uint2(packed[0], packed[1]);
+  };
+  if constexpr (CH > 0) {
+#pragma unroll
+    for (int c = 0; c < CH; c++)
+      if (first + c * kStep < pitch) quantize(first + c * kStep, kept[c]);
+  } else {
+#pragma unroll 2
+    for (int k = first; k < pitch; k += kStep) {
+      uint32_t w[4];
+      load8<VEC>(x + k, K - k, fill, w);
+      quantize(k, w);
+    }
   }
   if (row_sums != nullptr) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-    if (lane == 0) row_sums[row] = sum;
+    if constexpr (WPR > 1) {
+      if (lane == 0) s_sum[warp] = sum;
+      __syncthreads();
+      sum = 0;
+#pragma unroll
+      for (int i = 0; i < WPR; i++) sum += s_sum[i];
+    }
+    if (first == 0) row_sums[row] = sum;
   }
-  if (lane == 0) row_scales[row] = scale;
+  if (first == 0) row_scales[row] = scale;
+}
+
+template <int WPR, int CH>
+cudaError_t launch_quantize_rows(bool vec, const __half *x, int M, int K, int pitch, int8_t *q, float *scales, int32_t *sums,
+                                 int32_t *status, cudaStream_t s) {
+  const dim3 grid((unsigned)(WPR == 1 ? (M + 7) / 8 : M));
+  return vec ? launch_pdl(dyn_quantize_rows_kernel<WPR, true, CH>, grid, 256, 0, s, x, M, K, pitch, q, scales, sums, status)
+             : launch_pdl(dyn_quantize_rows_kernel<WPR, false, CH>, grid, 256, 0, s, x, M, K, pitch, q, scales, sums, status);
+}
+
+cudaError_t quantize_rows(bool vec, const __half *x, int M, int K, int pitch, int8_t *q, float *scales, int32_t *sums,
+                          int32_t *status, cudaStream_t s) {
+  if (K <= 256 * 2) return launch_quantize_rows<1, 2>(vec, x, M, K, pitch, q, scales, sums, status, s);
+  if (M >= 8 * 2 * 148) return launch_quantize_rows<1, 0>(vec, x, M, K, pitch, q, scales, sums, status, s);
+  if (K <= 8 * 256 * 2) return launch_quantize_rows<8, 2>(vec, x, M, K, pitch, q, scales, sums, status, s);
+  return launch_quantize_rows<8, 0>(vec, x, M, K, pitch, q, scales, sums, status, s);
 }
 
 int run(void *out, const void *in, const int8_t *weights, const float *bias, const float *scales, const int32_t *offsets,
@@ -196,24 +230,18 @@ int run(void *out, const void *in, const int8_t *weights, const float *bias, con
     return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", workspace_bytes, need);
   GLOWB200_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
   uint8_t *w = reinterpret_cast<uint8_t *>(workspace);
+  const int pitch = (int)align_up((size_t)K, 16);
   int8_t *q = reinterpret_cast<int8_t *>(w);
-  w += align_up((size_t)M * K, 256);
+  w += align_up((size_t)M * pitch, 256);
   float *row_scales = reinterpret_cast<float *>(w);
   w += align_up((size_t)M * 4, 256);
   int32_t *row_sums = reinterpret_cast<int32_t *>(w);
   w += align_up((size_t)M * 4, 256);
-  int8_t *wt = reinterpret_cast<int8_t *>(w);
-  w += align_up((size_t)N * K, 256);
   const bool offsets_zero = (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) != 0 || (offsets == nullptr && u_offset == 0);
   const bool vec = (K % 8) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   int32_t *sums = offsets_zero ? nullptr : row_sums;
   const __half *x = reinterpret_cast<const __half *>(in);
-  if (vec)
-    dyn_quantize_rows_warp_kernel<<<(unsigned)((M + 7) / 8), 256, 0, s>>>(x, (int)M, (int)K, q, row_scales, sums, status);
-  else
-    dyn_quantize_rows_kernel<<<(unsigned)M, kQuantThreads, 0, s>>>(reinterpret_cast<const __half *>(in), (int)M, (int)K, q,
-                                                                           row_scales, offsets_zero ? nullptr : row_sums, status);
-  GLOWB200_CUDA_OK(cudaGetLastError());
+  GLOWB200_CUDA_OK(quantize_rows(vec, x, (int)M, (int)K, pitch, q, row_scales, sums, status, s));
   GemmParams p{};
   p.float_out = 1;
   p.out_f16 = reinterpret_cast<__half *>(out);
@@ -227,15 +255,11 @@ int run(void *out, const void *in, const int8_t *weights, const float *bias, con
   p.status = status;
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.k_corr = (int)K;
-  const bool tensor_cores = !(flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) && (K % 16) == 0;
-  if (!tensor_cores && weights != nullptr) return run_gemm_float_any(p, q, weights, s);
-  const int8_t *b = weights_transposed;
-  if (b == nullptr) {
-    if (int rc = transpose_i8(weights, wt, (int)K, (int)N, s)) return rc;
-    b = wt;
-  }
+  p.a_pitch = pitch;
   const size_t used = (size_t)(w - reinterpret_cast<uint8_t *>(workspace));
-  return run_gemm(p, q, b, nullptr, offsets_zero, tensor_cores ? 0 : 1, w, workspace_bytes - used, s);
+  const bool kn = weights_transposed == nullptr || ((flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0 && weights != nullptr);
+  return run_gemm(p, q, kn ? weights : weights_transposed, nullptr, offsets_zero, (flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0, w,
+                  workspace_bytes - used, s, kn);
 }
 
 }  // namespace
@@ -245,9 +269,9 @@ using namespace glowb200;
 
 extern "C" size_t glowb200_dynamic_fc_workspace_bytes(int64_t M, int64_t K, int64_t N) {
   if (M < 0 || N < 0 || K < 0) return 0;
-  // quantized input, row scales, row sums, a transposed copy of the weights, the contraction's own
-  return align_up((size_t)M * K, 256) + 2 * align_up((size_t)M * 4, 256) + align_up((size_t)N * K, 256) +
-         i8_gemm_core_workspace_bytes(M, N);
+  // quantized input, row scales, row sums, the contraction's own and its copy of the weights
+  return align_up((size_t)M * align_up((size_t)K, 16), 256) + 2 * align_up((size_t)M * 4, 256) +
+         i8_gemm_core_workspace_bytes(M, N) + i8_gemm_copies_bytes(M, K, N, false, true);
 }
 
 extern "C" int glowb200_dynamic_rowwise_quantized_fc(void *out, const void *in, const int8_t *weights, const float *bias,

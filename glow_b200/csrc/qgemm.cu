@@ -352,8 +352,9 @@ struct GemmSmem {
 // (column-tile-major, so CTAs running together share weight tiles in L2).  The accumulators are
 // double-buffered in tensor memory: while the epilogue warps drain tile i, the MMA warp is
 // already accumulating tile i+1 into the other buffer.
-// MODE 0: no input row sums take part (every weight offset is 0) and the activation is none or
-// Relu -- the common case, whose drain has neither the row-sum term nor the activation switch;
+// MODE 0: no input row sums take part (every weight offset is 0), the activation is none or Relu and
+// the rows of the result are whole 16-byte pieces -- the common case, whose drain has neither the
+// row-sum term, nor the activation switch, nor the stores of ragged rows;
 // MODE 1: everything else with an int8 result; MODE 2: the floating-point result of the
 // dynamically quantized layers (GemmParams::float_out).  One drain body per kernel keeps the
 // register allocation inside the 96 registers a 576-thread CTA leaves.
@@ -549,7 +550,9 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             if (p.bias)
               term = scale32(load_bias(p, j) - (p.bias_offsets ? p.bias_offsets[j] : p.bias_offset), q.bias_pre, q.bias_post,
                              q.bias_scale, 0);
-            const uint32_t corr = (uint32_t)term - (uint32_t)p.a_offset * (uint32_t)p.b_row_sums[j] +
+            uint32_t b_sum = (uint32_t)p.b_row_sums[j];
+            for (int part = 1; part < p.b_sum_parts; part++) b_sum += (uint32_t)p.b_row_sums[(size_t)part * p.N + j];
+            const uint32_t corr = (uint32_t)term - (uint32_t)p.a_offset * b_sum +
                                   (uint32_t)p.k_corr * (uint32_t)p.a_offset * (uint32_t)q.b_off;
             cp.c = (int32_t)corr;
             cp.scale = q.out_scale;
@@ -625,6 +628,17 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
               for (int v4 = 0; v4 < kChunk / 8; v4++)
                 *reinterpret_cast<uint4 *>(orow + 8 * v4) = make_uint4(h2[4 * v4], h2[4 * v4 + 1], h2[4 * v4 + 2], h2[4 * v4 + 3]);
+            } else if (n0 + c0 + kChunk <= p.N) {  // pairs where the row's words lie
+              uint16_t *o16 = reinterpret_cast<uint16_t *>(orow);
+              if ((reinterpret_cast<uintptr_t>(orow) & 2) == 0) {
+#pragma unroll
+                for (int i = 0; i < kChunk / 2; i++) *reinterpret_cast<uint32_t *>(o16 + 2 * i) = h2[i];
+              } else {
+                o16[0] = (uint16_t)h2[0];
+#pragma unroll
+                for (int i = 0; i + 1 < kChunk / 2; i++) *reinterpret_cast<uint32_t *>(o16 + 2 * i + 1) = __byte_perm(h2[i], h2[i + 1], 0x5432);
+                o16[kChunk - 1] = (uint16_t)(h2[kChunk / 2 - 1] >> 16);
+              }
             } else {
               for (int i = 0; i < kChunk; i++)
                 if (n0 + c0 + i < p.N) orow[i] = __ushort_as_half((unsigned short)((h2[i >> 1] >> (16 * (i & 1))) & 0xffffu));
@@ -709,21 +723,44 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         constexpr int kRowPieces = S::kOutPitch / 16;
         if (col_group == 0) out_rows[quarter * 32 + lane] = row_ok ? out_index : -1;
         asm volatile("bar.sync %0, 128;" ::"r"(2 + quarter) : "memory");  // the quarter's 32 rows are complete
-        const bool whole = vec_ok && n0 + BLOCK_N <= p.N;
+        if (MODE == 0 || vec_ok) {
 #pragma unroll
-        for (int piece = col_group * 32 + lane; piece < 32 * kRowPieces; piece += 128) {
-          const int r = piece / kRowPieces, q16 = piece % kRowPieces;
-          const int dst = out_rows[quarter * 32 + r];
-          if (q16 * 16 >= BLOCK_N || dst < 0) continue;
-          const uint4 v = *reinterpret_cast<const uint4 *>(stage_q + stage_offset<S::kOutPitch>(r, q16));
-          int8_t *o = p.out + (size_t)dst * p.N + n0 + q16 * 16;
-          if (whole) {
-            *reinterpret_cast<uint4 *>(o) = v;
-          } else {
-            const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+          for (int piece = col_group * 32 + lane; piece < 32 * kRowPieces; piece += 128) {
+            const int r = piece / kRowPieces, q16 = piece % kRowPieces;
+            const int dst = out_rows[quarter * 32 + r];
+            if (q16 * 16 >= BLOCK_N || n0 + q16 * 16 >= p.N || dst < 0) continue;
+            *reinterpret_cast<uint4 *>(p.out + (size_t)dst * p.N + n0 + q16 * 16) =
+                *reinterpret_cast<const uint4 *>(stage_q + stage_offset<S::kOutPitch>(r, q16));
+          }
+        } else {
+          // Rows that start anywhere (N not a multiple of 16): the lanes of a warp
+          // write consecutive aligned words of a row, each put together from two staged words; the
+          // bytes at a row's two ends go one by one.  (Byte stores for the whole tile took
+          // 2000 x 30 x 1000 to 21.5 us.)
+          constexpr int kRowWords = BLOCK_N / 4 + 1;
+          const int len = p.N - n0 < BLOCK_N ? p.N - n0 : BLOCK_N;
+          auto staged = [&](int r, int word) -> uint32_t {
+            return *reinterpret_cast<const uint32_t *>(stage_q + stage_offset<S::kOutPitch>(r, word >> 2) + 4 * (word & 3));
+          };
+#pragma unroll 1
+          for (int item = col_group * 32 + lane; item < 32 * kRowWords; item += 128) {
+            const int r = item / kRowWords;
+            const int dst = out_rows[quarter * 32 + r];
+            if (dst < 0) continue;
+            int8_t *o = p.out + (size_t)dst * p.N + n0;
+            const int sh = (int)(reinterpret_cast<uintptr_t>(o) & 3);
+            const int col = 4 * (item % kRowWords) - sh;  // of the word's first byte
+            if (col >= len) continue;
+            const int below = col < 0 ? -1 : col >> 2;    // the staged word that holds it
+            const uint32_t lo = below >= 0 ? staged(r, below) : 0u, hi = below + 1 < BLOCK_N / 4 ? staged(r, below + 1) : 0u;
+            const uint32_t v = __funnelshift_r(lo, hi, 8 * (col & 3));
+            if (col >= 0 && col + 4 <= len) {
+              *reinterpret_cast<uint32_t *>(o + col) = v;
+            } else {
 #pragma unroll
-            for (int b = 0; b < 16; b++)
-              if (n0 + q16 * 16 + b < p.N) o[b] = (int8_t)((w4[b >> 2] >> (8 * (b & 3))) & 0xff);
+              for (int b = 0; b < 4; b++)
+                if (col + b >= 0 && col + b < len) o[col + b] = (int8_t)((v >> (8 * b)) & 0xff);
+            }
           }
         }
       }
@@ -777,17 +814,21 @@ __global__ void __launch_bounds__(256) i8_row_sums_kernel(const int8_t *__restri
 }
 
 // ---------------------------------------------------------------------------------------
-// Any-shape contraction (K not a multiple of 16, unaligned pointers): one thread per output,
-// the reference's loop as written.  Also the cross-check of the tensor-core kernel in tests.
+// Any-shape contraction: one thread per output, the reference's loop as written.  The cross-check of
+// the tensor-core kernels in tests, and what a caller gets whose workspace has no room for the padded
+// copies that a K off the 16-byte grid needs.  b element (j, k) sits at b[j * b_stride_j + k * b_stride_k]
+// ([N, K] or [K, N]).
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) i8_gemm_requant_any_kernel(const int8_t *__restrict__ a, const int8_t *__restrict__ b,
+                                                                   int64_t b_stride_j, int64_t b_stride_k,
                                                                    const __grid_constant__ GemmParams p) {
   const int j = blockIdx.x * 16 + (threadIdx.x & 15), i = blockIdx.y * 16 + (threadIdx.x >> 4);
   if (i >= p.M || j >= p.N) return;
+  const int lda = p.a_pitch ? p.a_pitch : p.K;
   const ColQuant q = col_quant(p, j);
   uint32_t sum = 0;
   for (int k = 0; k < p.k_corr; k++)
-    sum += (uint32_t)(((int32_t)b[(size_t)j * p.K + k] - q.b_off) * ((int32_t)a[(size_t)i * p.K + k] - p.a_offset));
+    sum += (uint32_t)(((int32_t)b[j * b_stride_j + k * b_stride_k] - q.b_off) * ((int32_t)a[(size_t)i * lda + k] - p.a_offset));
   if (p.bias)
     sum += (uint32_t)scale32(load_bias(p, j) - (p.bias_offsets ? p.bias_offsets[j] : p.bias_offset), q.bias_pre, q.bias_post,
                              q.bias_scale, 0);
@@ -795,34 +836,19 @@ __global__ void __launch_bounds__(256) i8_gemm_requant_any_kernel(const int8_t *
       (int8_t)clip_i8(activation_i32(scale32((int32_t)sum, q.out_pre, q.out_post, q.out_scale, p.out_offset), p));
 }
 
-// The floating-point result (GemmParams::float_out) for any shape: b element (j, k) sits at
-// b[j * b_stride_j + k * b_stride_k], so both the [N, K] and the [K, N] form of the weights serve.
+// The same for the floating-point result (GemmParams::float_out).
 __global__ void __launch_bounds__(256) i8_gemm_float_any_kernel(const int8_t *__restrict__ a, const int8_t *__restrict__ b,
                                                                  int64_t b_stride_j, int64_t b_stride_k,
                                                                  const __grid_constant__ GemmParams p) {
   const int j = blockIdx.x * 16 + (threadIdx.x & 15), i = blockIdx.y * 16 + (threadIdx.x >> 4);
   if (i >= p.M || j >= p.N) return;
+  const int lda = p.a_pitch ? p.a_pitch : p.K;
   const int32_t b_off = p.b_offsets ? p.b_offsets[j] : p.u_b_offset;
   uint32_t sum = 0;
   for (int k = 0; k < p.k_corr; k++)
-    sum += (uint32_t)(((int32_t)b[j * b_stride_j + k * b_stride_k] - b_off) * (int32_t)a[(size_t)i * p.K + k]);
+    sum += (uint32_t)(((int32_t)b[j * b_stride_j + k * b_stride_k] - b_off) * (int32_t)a[(size_t)i * lda + k]);
   const float mm = __fmul_rn(p.row_scales[i], p.col_scales ? p.col_scales[j] : p.u_col_scale);
   p.out_f16[(size_t)i * p.N + j] = __float2half_rn(__fadd_rn(__fmul_rn((float)(int32_t)sum, mm), p.bias_f32[j]));
-}
-
-// [R, C] int8 -> [C, R] int8 (32x32 tiles through shared memory)
-__global__ void __launch_bounds__(256) i8_transpose_kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int R, int C) {
-  __shared__ int8_t tile[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int y = threadIdx.y; y < 32; y += 8) {
-    const int r = r0 + y, c = c0 + threadIdx.x;
-    tile[y][threadIdx.x] = (r < R && c < C) ? in[(size_t)r * C + c] : (int8_t)0;
-  }
-  __syncthreads();
-  for (int y = threadIdx.y; y < 32; y += 8) {
-    const int c = c0 + y, r = r0 + threadIdx.x;
-    if (c < C && r < R) out[(size_t)c * R + r] = tile[threadIdx.x][y];
-  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -864,6 +890,13 @@ int make_map(CUtensorMap *map, const void *base, int rows, int K, int box_rows, 
   return GLOWB200_OK;
 }
 
+bool ptr16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// MODE 0 of the tile kernel
+bool plain_drain(const GemmParams &p) {
+  return p.a_row_sums == nullptr && p.act_type <= 1 && (p.N & 15) == 0 && ptr16(p.out);
+}
+
 template <int BLOCK_N, int STAGES, int MODE>
 int launch_tile_mode(const CUtensorMap &ma, const CUtensorMap &mb, const GemmParams &p, cudaStream_t s) {
   using S = GemmSmem<BLOCK_N, STAGES>;
@@ -897,7 +930,7 @@ int &resident_pairs() {
 template <int BLOCK_N, int STAGES>
 int launch_pair_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmParams &p, cudaStream_t s) {
   using S = GemmSmem<BLOCK_N, STAGES, 1>;
-  const bool plain = p.a_row_sums == nullptr && p.act_type <= 1;
+  const bool plain = plain_drain(p);
   auto kernel = plain ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 0, 1> : i8_gemm_requant_kernel<BLOCK_N, STAGES, 1, 1>;
   GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
   const int tiles = ((p.N + BLOCK_N - 1) / BLOCK_N) * ((p.M + 2 * kBlockM - 1) / (2 * kBlockM));
@@ -930,11 +963,9 @@ int launch_pair_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmP
 template <int BLOCK_N, int STAGES>
 int launch_tile_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmParams &p, cudaStream_t s) {
   if (p.float_out) return launch_tile_mode<BLOCK_N, STAGES, 2>(ma, mb, p, s);
-  if (p.a_row_sums == nullptr && p.act_type <= 1) return launch_tile_mode<BLOCK_N, STAGES, 0>(ma, mb, p, s);
+  if (plain_drain(p)) return launch_tile_mode<BLOCK_N, STAGES, 0>(ma, mb, p, s);
   return launch_tile_mode<BLOCK_N, STAGES, 1>(ma, mb, p, s);
 }
-
-bool ptr16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 #ifndef GLOWB200_GEMM_TILE_240
 #define GLOWB200_GEMM_TILE_240 1
@@ -1052,55 +1083,61 @@ int run_gemm_row_windows(GemmParams p, const int8_t *planes, int64_t rows, int o
 }
 
 int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_row_sums_in, bool b_offsets_zero,
-             int force_any, void *ws, size_t ws_bytes, cudaStream_t s) {
+             int force_any, void *ws, size_t ws_bytes, cudaStream_t s, bool b_is_kn) {
   if (p.M == 0 || p.N == 0) return GLOWB200_OK;
   if (p.k_corr == 0) p.k_corr = p.K;
-  const bool tc = !force_any && p.K > 0 && (p.K % 16) == 0 && ptr16(a) && ptr16(b);
+  const int K = p.K, pitch = (int)align_up((size_t)K, 16);
+  const bool copy_a = (pitch != K && p.a_pitch != pitch) || !ptr16(a), copy_b = b_is_kn || pitch != K || !ptr16(b);
+  const size_t core = i8_gemm_core_workspace_bytes(p.M, p.N);
+  if (!force_any && K > 0 && i8_skinny_wins(p.M, p.N, K, b_is_kn)) return run_gemm_skinny(p, a, b, b_is_kn, b_offsets_zero, s);
+  const bool tc = !force_any && K > 0 &&
+                  ((!copy_a && !copy_b) ||
+                   (ws != nullptr && ptr16(ws) && ws_bytes >= core + i8_gemm_copies_bytes(p.M, K, p.N, copy_a, copy_b)));
   if (!tc) {
     dim3 grid((p.N + 15) / 16, (p.M + 15) / 16);
-    if (p.float_out) i8_gemm_float_any_kernel<<<grid, 256, 0, s>>>(a, b, p.K, 1, p);
-    else i8_gemm_requant_any_kernel<<<grid, 256, 0, s>>>(a, b, p);
+    const int64_t stride_j = b_is_kn ? 1 : K, stride_k = b_is_kn ? p.N : 1;
+    if (p.float_out) i8_gemm_float_any_kernel<<<grid, 256, 0, s>>>(a, b, stride_j, stride_k, p);
+    else i8_gemm_requant_any_kernel<<<grid, 256, 0, s>>>(a, b, stride_j, stride_k, p);
     GLOWB200_CUDA_OK(cudaGetLastError());
     return GLOWB200_OK;
   }
-  const size_t need = align_up((size_t)p.N * 4, 256) + align_up((size_t)p.M * 4, 256);
-  if (ws == nullptr || ws_bytes < need)
-    return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", ws_bytes, need);
-  int32_t *bs = reinterpret_cast<int32_t *>(ws);
-  int32_t *as = reinterpret_cast<int32_t *>(reinterpret_cast<uint8_t *>(ws) + align_up((size_t)p.N * 4, 256));
-  if (b_row_sums_in || p.float_out) {  // (the float result has no input offset: the sums are never read)
-    p.b_row_sums = b_row_sums_in;
-  } else {
-    i8_row_sums_kernel<<<(p.N + 7) / 8, 256, 0, s>>>(b, p.N, p.K, bs);
-    GLOWB200_CUDA_OK(cudaGetLastError());
-    p.b_row_sums = bs;
+  if (ws == nullptr || ws_bytes < core)
+    return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", ws_bytes, core);
+  uint8_t *w = reinterpret_cast<uint8_t *>(ws);
+  int32_t *bs = reinterpret_cast<int32_t *>(w), *as = reinterpret_cast<int32_t *>(w + align_up((size_t)p.N * 4, 256));
+  w += core;
+  // (the float result has no input offset: the sums of the right-hand side are never read; those of
+  // the left one are the caller's, written while it quantized the rows)
+  const bool b_sums = b_row_sums_in == nullptr && !p.float_out, a_sums = !b_offsets_zero && !p.float_out;
+  PrepParams prep{};
+  if (copy_a) {
+    prep_side_rows(prep.a, a, reinterpret_cast<int8_t *>(w), a_sums ? as : nullptr, p.M, K, pitch);
+    a = prep.a.dst;
+    w += align_up((size_t)p.M * pitch, 256);
+  } else if (a_sums) {
+    prep_side_rows(prep.a, a, nullptr, as, p.M, K, pitch);
   }
-  if (p.float_out) {
-    if (b_offsets_zero) p.a_row_sums = nullptr;  // else the caller's, written while it quantized the rows
-  } else if (!b_offsets_zero) {
-    i8_row_sums_kernel<<<(p.M + 7) / 8, 256, 0, s>>>(a, p.M, p.K, as);
-    GLOWB200_CUDA_OK(cudaGetLastError());
-    p.a_row_sums = as;
-  } else {
-    p.a_row_sums = nullptr;
+  p.b_row_sums = b_sums ? bs : b_row_sums_in;
+  p.b_sum_parts = 1;
+  if (copy_b && b_is_kn) {
+    int32_t *parts = reinterpret_cast<int32_t *>(w + align_up((size_t)p.N * pitch, 256));
+    prep_side_transposed(prep.b, b, reinterpret_cast<int8_t *>(w), b_sums ? parts : nullptr, p.N, K, pitch);
+    if (b_sums) {
+      p.b_row_sums = parts;
+      p.b_sum_parts = prep_transposed_parts(p.N, pitch);
+    }
+    b = prep.b.dst;
+  } else if (copy_b) {
+    prep_side_rows(prep.b, b, reinterpret_cast<int8_t *>(w), b_sums ? bs : nullptr, p.N, K, pitch);
+    b = prep.b.dst;
+  } else if (b_sums) {
+    prep_side_rows(prep.b, b, nullptr, bs, p.N, K, pitch);
   }
+  if (int rc = run_prepare_operands(prep, s)) return rc;
+  if (b_offsets_zero) p.a_row_sums = nullptr;
+  else if (!p.float_out) p.a_row_sums = as;
+  p.K = pitch;
   return launch_for_block_n(pick_tile(p.M, p.N, !p.float_out), a, p.M, p.K, p.K, b, p, s);
-}
-
-int run_gemm_float_any(const GemmParams &p, const int8_t *a, const int8_t *b_kn, cudaStream_t s) {
-  if (p.M == 0 || p.N == 0) return GLOWB200_OK;
-  dim3 grid((p.N + 15) / 16, (p.M + 15) / 16);
-  i8_gemm_float_any_kernel<<<grid, 256, 0, s>>>(a, b_kn, 1, p.N, p);
-  GLOWB200_CUDA_OK(cudaGetLastError());
-  return GLOWB200_OK;
-}
-
-int transpose_i8(const int8_t *in_rc, int8_t *out_cr, int R, int C, cudaStream_t s) {
-  if (R == 0 || C == 0) return GLOWB200_OK;
-  dim3 grid((C + 31) / 32, (R + 31) / 32), block(32, 8);
-  i8_transpose_kernel<<<grid, block, 0, s>>>(in_rc, out_cr, R, C);
-  GLOWB200_CUDA_OK(cudaGetLastError());
-  return GLOWB200_OK;
 }
 
 namespace {
@@ -1123,8 +1160,9 @@ extern "C" int glowb200_debug_gemm_trace(unsigned long long *host512) {
 
 extern "C" size_t glowb200_i8_gemm_workspace_bytes(int64_t M, int64_t K, int64_t N) {
   if (M < 0 || N < 0 || K < 0) return 0;
-  // row sums of both operands + room for a transposed copy of a [K, N] right-hand side
-  return align_up((size_t)N * 4, 256) + align_up((size_t)M * 4, 256) + align_up((size_t)N * (size_t)K, 256);
+  // row sums of both operands + room for a padded (transposed) copy of the right-hand side and, when
+  // rows are not whole 16-byte pieces, of the left one
+  return i8_gemm_core_workspace_bytes(M, N) + i8_gemm_copies_bytes(M, K, N, (K % 16) != 0, true);
 }
 
 extern "C" int glowb200_i8_mma_issue_probe(int64_t mmas_per_sm, int64_t *ops_per_launch, int32_t *status,
@@ -1184,31 +1222,6 @@ extern "C" int glowb200_rowwise_quantized_fc_i8_i32(
                   reinterpret_cast<cudaStream_t>(stream));
 }
 
-namespace {
-// Shared tail of the two per-tensor entry points, whose right-hand side is [K, N]: transposes it
-// into the workspace (unless the caller already holds the [N, K] form) and runs the contraction
-// with every per-column array read at stride 0.
-int run_per_tensor(GemmParams p, const int8_t *lhs, const int8_t *rhs_kn, const int8_t *rhs_nk, int flags, void *workspace,
-                   size_t workspace_bytes, cudaStream_t s) {
-  const size_t sums = align_up((size_t)p.N * 4, 256) + align_up((size_t)p.M * 4, 256);
-  const int8_t *b = rhs_nk;
-  if (b == nullptr) {
-    const size_t need = sums + align_up((size_t)p.N * (size_t)p.K, 256);
-    if (workspace == nullptr || workspace_bytes < need)
-      return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", workspace_bytes, need);
-    int8_t *t = reinterpret_cast<int8_t *>(workspace) + sums;
-    if (p.K > 0) {
-      dim3 grid((p.N + 31) / 32, (p.K + 31) / 32), block(32, 8);
-      i8_transpose_kernel<<<grid, block, 0, s>>>(rhs_kn, t, p.K, p.N);
-      GLOWB200_CUDA_OK(cudaGetLastError());
-    }
-    b = t;
-  }
-  return run_gemm(p, lhs, b, nullptr, (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) != 0,
-                  (flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0, workspace, workspace_bytes, s);
-}
-}  // namespace
-
 extern "C" int glowb200_fc_i8_i32(int8_t *out, const int8_t *in, const int8_t *weights, const int32_t *bias, int64_t M,
                                   int64_t K, int64_t N, int32_t out_offset, int32_t in_offset, int32_t weights_offset,
                                   int32_t bias_offset, int32_t bias_pre, int32_t bias_post, int32_t bias_scale,
@@ -1230,8 +1243,9 @@ extern "C" int glowb200_fc_i8_i32(int8_t *out, const int8_t *in, const int8_t *w
   p.u_out_pre = out_pre; p.u_out_post = out_post; p.u_out_scale = out_scale;
   p.bias_is_i8 = (flags & GLOWB200_FC_BIAS_INT8) ? 1 : 0;
   if (weights_offset == 0) flags |= GLOWB200_FC_WEIGHT_OFFSETS_ZERO;
-  return run_per_tensor(p, in, weights, weights_transposed, flags, workspace, workspace_bytes,
-                        reinterpret_cast<cudaStream_t>(stream));
+  return run_gemm(p, in, weights_transposed ? weights_transposed : weights, nullptr,
+                  (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) != 0, (flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0, workspace,
+                  workspace_bytes, reinterpret_cast<cudaStream_t>(stream), weights_transposed == nullptr);
 }
 
 extern "C" int glowb200_matmul_i8(int8_t *out, const int8_t *lhs, const int8_t *rhs, int64_t M, int64_t K, int64_t N,
@@ -1251,5 +1265,7 @@ extern "C" int glowb200_matmul_i8(int8_t *out, const int8_t *lhs, const int8_t *
   p.u_b_offset = rhs_offset;
   p.u_out_pre = out_pre; p.u_out_post = out_post; p.u_out_scale = out_scale;
   if (rhs_offset == 0) flags |= GLOWB200_FC_WEIGHT_OFFSETS_ZERO;
-  return run_per_tensor(p, lhs, rhs, nullptr, flags, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+  return run_gemm(p, lhs, rhs, nullptr, (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) != 0,
+                  (flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0, workspace, workspace_bytes,
+                  reinterpret_cast<cudaStream_t>(stream), true);
 }

@@ -11,11 +11,13 @@ struct GemmParams {
   const int32_t *b_offsets;   // weight offsets; index j * stride_b_off
   const int32_t *bias_pre, *bias_post, *bias_scale;  // index j * stride_q
   const int32_t *out_pre, *out_post, *out_scale;      // index j * stride_q
-  const int32_t *b_row_sums;  // [N] sum_k B[j,k]
+  const int32_t *b_row_sums;  // [N] sum_k B[j,k]; b_sum_parts > 1: as many arrays, whose sum it is
+  int b_sum_parts;
   const int32_t *a_row_sums;  // [M] sum_k A[i,k], or nullptr when every b offset is 0
   int32_t *status;
   const int32_t *bias_offsets;  // per-column bias offsets (channelwise conv), or nullptr: bias_offset
   int M, N, K;                  // K: row pitch of both operands in bytes (a multiple of 16 on the TMA path)
+  int a_pitch;                  // row pitch of A when it differs from K (its rows then are zero padded to it); 0 = K
   int k_corr;                   // number of real K entries (<= K; the rest is zero padding); 0 = K
   int32_t a_offset, bias_offset, out_offset;
   // fused activation on the requantised value (glow::FusedActivation: 0 none, 1 relu, 2 clip, 5 leaky relu)
@@ -75,11 +77,38 @@ __device__ __forceinline__ int32_t activation_i32(int32_t x, const GemmParams &p
   return x >= p.out_offset ? x : scale32(x - p.out_offset, p.act_args[0], p.act_args[1], p.act_args[2], p.out_offset);
 }
 
-// out = requant(A[M,K] x B[N,K]^T) with the tensor-core kernel when the shapes allow it (K a
-// multiple of 16, 16-byte aligned operands), else the any-shape kernel.  `ws` must hold
-// i8_gemm_core_workspace_bytes(M, N) bytes.  b_row_sums_in may be nullptr (computed here).
+// out = requant(A[M,K] x B[N,K]^T); b_is_kn: the right-hand side is given as [K, N].  Products with
+// few rows take the one-launch kernel of qgemm_small.cu, the others the tcgen05 kernel -- on the
+// operands as they are when K is a multiple of 16 and both are 16-byte aligned [rows, K] matrices, else
+// on zero-padded (transposed) copies in `ws` -- and the any-shape kernel when asked for (force_any) or
+// when `ws` has no room for the copies.  `ws` must hold i8_gemm_core_workspace_bytes(M, N) bytes, with
+// i8_gemm_copies_bytes(M, K, N, ...) more for the copies.  b_row_sums_in may be nullptr (computed here).
 int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_row_sums_in, bool b_offsets_zero,
-             int force_any, void *ws, size_t ws_bytes, cudaStream_t s);
+             int force_any, void *ws, size_t ws_bytes, cudaStream_t s, bool b_is_kn = false);
+
+// ---- qgemm_small.cu ----
+constexpr int kSkinnyRows = 64;
+bool i8_skinny_wins(int64_t M, int64_t N, int64_t K, bool b_is_kn);
+int run_gemm_skinny(GemmParams p, const int8_t *a, const int8_t *b, bool b_is_kn, bool b_offsets_zero, cudaStream_t s);
+
+// One operand to prepare: src [rows, K] -> dst [rows, pitch] (pitch a multiple of 16, the rest zero;
+// dst may be nullptr: sums only), or with `transpose` src [K, rows] -> dst [rows, pitch].  sums (may be
+// nullptr): per row; a transposed operand's come in prep_transposed_parts() arrays to be added up.
+struct PrepSide {
+  const int8_t *src;
+  int8_t *dst;
+  int32_t *sums;
+  int rows, K, pitch, transpose, k_span;
+};
+struct PrepParams {
+  PrepSide a, b;  // src nullptr: nothing to do on that side
+  int a_blocks;
+};
+constexpr int kMaxSumParts = 16;
+int prep_transposed_parts(int64_t rows, int64_t pitch);
+void prep_side_rows(PrepSide &o, const int8_t *src, int8_t *dst, int32_t *sums, int rows, int K, int pitch);
+void prep_side_transposed(PrepSide &o, const int8_t *src, int8_t *dst, int32_t *sums, int rows, int K, int pitch);
+int run_prepare_operands(PrepParams p, cudaStream_t s);
 
 // The shifted-rows convolution on the same kernel: `padded` holds `rows` padded pixels of `C` bytes
 // (plus 128 readable bytes behind them), p.conv_* describe the taps, p.M = rows, p.K = bytes of a
@@ -88,11 +117,6 @@ int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_ro
 int run_gemm_shifted_rows(GemmParams p, const int8_t *padded, int64_t rows, int C, const int8_t *b,
                           const int32_t *b_row_sums, cudaStream_t s, int64_t buffer_rows = 0);
 
-// The float-result contraction for any shape with the weights in their [K, N] form.
-int run_gemm_float_any(const GemmParams &p, const int8_t *a, const int8_t *b_kn, cudaStream_t s);
-// [R, C] int8 -> [C, R] int8
-int transpose_i8(const int8_t *in_rc, int8_t *out_cr, int R, int C, cudaStream_t s);
-
 // The row-window convolution: `planes` holds two planes of `rows` 32-byte windows each, back to back,
 // with 3 * ow + 1 readable windows behind the second; b is [N, 256] (plane, a, 32 bytes).
 int run_gemm_row_windows(GemmParams p, const int8_t *planes, int64_t rows, int ow, const int8_t *b, const int32_t *b_row_sums,
@@ -100,6 +124,12 @@ int run_gemm_row_windows(GemmParams p, const int8_t *planes, int64_t rows, int o
 
 inline size_t i8_gemm_core_workspace_bytes(int64_t M, int64_t N) {
   return align_up((size_t)N * 4, 256) + align_up((size_t)M * 4, 256);
+}
+// Room for a padded copy of either operand and the partial sums of a transposed one.
+inline size_t i8_gemm_copies_bytes(int64_t M, int64_t K, int64_t N, bool copy_a, bool copy_b) {
+  const size_t pitch = align_up((size_t)K, 16);
+  return (copy_a ? align_up((size_t)M * pitch, 256) : 0) +
+         (copy_b ? align_up((size_t)N * pitch, 256) + align_up((size_t)N * 4 * kMaxSumParts, 256) : 0);
 }
 
 }  // namespace glowb200
