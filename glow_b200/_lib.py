@@ -3,6 +3,7 @@
 There is no fallback: if the CUDA library has not been built, importing an operator raises.
 """
 import ctypes as C
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -153,6 +154,25 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = l
     return _lib
+
+
+_binding = None
+
+
+def binding(explain):
+    """The CPython module of the per-request calls (csrc/binding.cpp), working on this process's library."""
+    global _binding
+    if _binding is None:
+        path = os.path.join(_HERE, "lib", "_binding.so")
+        if not os.path.exists(path):
+            raise ImportError("%s is missing: build it with `python -m glow_b200.build`" % path)
+        l = lib()
+        spec = importlib.util.spec_from_file_location("glow_b200._binding", path)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        m.setup({name: C.cast(getattr(l, name), C.c_void_p).value for name in SIGNATURES}, GlowB200Error, explain)
+        _binding = m
+    return _binding
 
 
 def check(rc):

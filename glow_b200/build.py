@@ -2,7 +2,8 @@
 
 Every .cu file under glow_b200/csrc is compiled for sm_100a only
 (-gencode arch=compute_100a,code=sm_100a) and linked into one shared library that exports
-the C ABI declared in include/glow_b200.h.  Run as `python -m glow_b200.build`.
+the C ABI declared in include/glow_b200.h; csrc/binding.cpp becomes the CPython module
+(glow_b200/lib/_binding.so) through which ops.py calls it.  Run as `python -m glow_b200.build`.
 """
 import os
 import subprocess
@@ -15,6 +16,7 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libglow_b200.so")
+BINDING = os.path.join(LIBDIR, "_binding.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -29,6 +31,20 @@ def _headers():
     hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     hs.append(os.path.join(ROOT, "include", "glow_b200.h"))
     return hs
+
+
+def _binding_command(src):
+    import sysconfig
+
+    import torch
+    t = os.path.dirname(torch.__file__)
+    # (torch's own libraries are in the process before the module is: no path to them is recorded)
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+            "-I", os.path.join(t, "include"), "-I", os.path.join(t, "include", "torch", "csrc", "api", "include"),
+            "-I", os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), "-I", sysconfig.get_paths()["include"],
+            "-I", os.path.join(ROOT, "include"), src, "-o", BINDING, "-L", os.path.join(t, "lib"),
+            "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
 
 def _stale(target, deps):
@@ -55,13 +71,17 @@ def build(verbose=False, extra_flags=()):
             print(" ".join(cmd), flush=True)
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed:\n%s\n%s" % (" ".join(cmd), r.stderr))
+            raise RuntimeError("compilation failed:\n%s\n%s" % (" ".join(cmd), r.stderr))
         if verbose and r.stderr.strip():
             print(r.stderr, flush=True)
         return r.stderr
 
-    with ThreadPoolExecutor(max(1, min(8, len(jobs)))) as ex:
-        list(ex.map(run, jobs))
+    binding_src = os.path.join(CSRC, "binding.cpp")
+    compiles = list(jobs)
+    if _stale(BINDING, [binding_src, os.path.join(ROOT, "include", "glow_b200.h")]):
+        compiles.append(_binding_command(binding_src))
+    with ThreadPoolExecutor(max(1, min(8, len(compiles)))) as ex:
+        list(ex.map(run, compiles))
     if jobs or _stale(LIB, objs):
         run([NVCC, "-shared", "-o", LIB] + objs)
     return LIB

@@ -21,6 +21,18 @@ STATUS_WAIT_TIMEOUT = 16
 STATUS_UNSUPPORTED_TABLE = 32
 
 
+def _explain(name, obj, dtypes):
+    """Raises what is wrong with an argument the native binding turned down."""
+    names = (torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64, torch.float16, torch.float32)
+    _cuda(obj, name, tuple(t for i, t in enumerate(names) if dtypes >> i & 1) or None)
+    raise TypeError("%s is not a suitable tensor" % name)
+
+
+def _native():
+    """The per-request calls as native functions: checks, allocation and the C ABI call in one."""
+    return _lib._binding or _lib.binding(_explain)
+
+
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -73,31 +85,9 @@ def fused_rowwise_quantized_sparse_lengths_weighted_sum(data, weights, indices, 
     weights: result dtype [n]; indices: int32/int64 [n]; lengths: int32 [segments].
     out_line: columns of the result when the rows are padded (see pad_fused_rows); default: the
     whole row is payload + scale/offset."""
-    _cuda(data, "data", (torch.uint8,))
-    _cuda(indices, "indices", (torch.int32, torch.int64))
-    _cuda(lengths, "lengths", (torch.int32,))
-    rows, in_line = data.shape
-    out_line = out_columns(in_line, kind) if out_line is None else int(out_line)
-    odt = result_dtype(kind) if out is None else out.dtype
-    _cuda(weights, "weights", (odt,))
-    segments = lengths.shape[0]
-    if out is None:
-        out = torch.empty((segments, out_line), dtype=odt, device=data.device)
-    n = indices.shape[0] if num_indices is None else int(num_indices)
-    need = slws_workspace_bytes(segments, 1)
-    ws = _workspace(workspace, need, data.device)
-    if low_latency:   # a warp per bag: for small requests; another summation order (see the header)
-        if use_fp16_accumulation:
-            raise ValueError("the low-latency form accumulates in fp32")
-        check(_lib.lib().glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_low_latency(
-            _p(out), _p(data), kind, rows, _p(weights), _p(indices), int(indices.dtype == torch.int64), _p(lengths),
-            segments, n, in_line, out_line, int(odt == torch.float16), _p(ws), ws.numel(), _p(status), _stream()))
-        return out
-    check(_lib.lib().glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum(
-        _p(out), _p(data), kind, rows, _p(weights), _p(indices), int(indices.dtype == torch.int64), _p(lengths),
-        segments, n, in_line, out_line, int(odt == torch.float16), int(use_fp16_accumulation), _p(ws), ws.numel(),
-        _p(status), _stream()))
-    return out
+    # (low latency: a warp per bag: for small requests; another summation order, see the header)
+    return _native().slws(data, weights, indices, lengths, kind, use_fp16_accumulation, out, status, workspace, num_indices,
+                          out_line, low_latency)
 
 
 def fused_rowwise_quantized_sparse_lengths_weighted_sum_static_scratch(data, weights, indices, lengths,
@@ -132,25 +122,8 @@ def embedding_bag_byte_rowwise_offsets(data, weights, indices, offsets, kind=UIN
                                        use_fp16_accumulation=False, out=None, status=None, workspace=None,
                                        num_indices=None):
     """EmbeddingBagByteRowwiseOffsets: bags given by offsets (same integer type as indices)."""
-    _cuda(data, "data", (torch.uint8,))
-    _cuda(indices, "indices", (torch.int32, torch.int64))
-    _cuda(offsets, "offsets", (indices.dtype,))
-    rows, in_line = data.shape
-    out_line = out_columns(in_line, kind)
-    odt = result_dtype(kind) if out is None else out.dtype
-    _cuda(weights, "weights", (odt,))
-    num_offsets = offsets.shape[0]
-    segments = num_offsets - 1 if has_end_offset else num_offsets
-    if out is None:
-        out = torch.empty((max(segments, 0), out_line), dtype=odt, device=data.device)
-    n = indices.shape[0] if num_indices is None else int(num_indices)
-    need = slws_workspace_bytes(max(segments, 0), 1)
-    ws = _workspace(workspace, need, data.device)
-    check(_lib.lib().glowb200_embedding_bag_byte_rowwise_offsets(
-        _p(out), _p(data), kind, rows, _p(weights), _p(indices), _p(offsets), int(indices.dtype == torch.int64),
-        num_offsets, n, in_line, out_line, int(has_end_offset), int(odt == torch.float16),
-        int(use_fp16_accumulation), _p(ws), ws.numel(), _p(status), _stream()))
-    return out
+    return _native().embedding_bag(data, weights, indices, offsets, kind, has_end_offset, use_fp16_accumulation, out, status,
+                                   workspace, num_indices)
 
 
 EST_FLOAT, EST_FLOAT16, EST_INT8, EST_INT4 = 0, 1, 2, 3   # SplitEmbeddingSparseType
@@ -172,32 +145,9 @@ def int_nbit_split_embedding_bags(dev_weights, uvm_weights, weights_placements, 
                                   row_alignment=16, out=None, status=None):
     """IntNBitSplitEmbeddingBags (indice_weights None) / IntNBitSplitEmbeddingWeightedBags:
     T tables in one byte buffer, T*B bags per request, result [B, total_dims]."""
-    _cuda(dev_weights, "dev_weights", (torch.uint8,))
-    _cuda(uvm_weights, "uvm_weights", (torch.uint8,))
-    _cuda(weights_placements, "weights_placements", (torch.int32,))
-    _cuda(weights_offsets, "weights_offsets", (torch.int32, torch.int64))
-    _cuda(weights_tys, "weights_tys", (torch.uint8,))
-    _cuda(dim_offsets, "dim_offsets", (torch.int32,))
-    _cuda(indices, "indices", (torch.int32, torch.int64))
-    _cuda(offsets, "offsets", (indices.dtype,))
-    if indice_weights is not None:
-        _cuda(indice_weights, "indice_weights", (torch.float32, torch.float16))
-    T = dim_offsets.shape[0] - 1
-    if T < 0 or weights_tys.shape[0] != T or weights_placements.shape[0] != T or weights_offsets.shape[0] != T:
-        raise ValueError("table description arrays disagree on the number of tables")
-    if T == 0 or (offsets.shape[0] - 1) % T != 0:
-        raise ValueError("offsets must hold num_tables * bags_per_table + 1 entries")
-    B = (offsets.shape[0] - 1) // T
-    if out is None:
-        out = torch.empty((B, total_dims), dtype=out_dtype, device=indices.device)
-    _cuda(out, "out", (torch.float32, torch.float16))
-    check(_lib.lib().glowb200_int_nbit_split_embedding_bags(
-        _p(out), _p(dev_weights), dev_weights.numel(), _p(uvm_weights), uvm_weights.numel(), _p(weights_placements),
-        _p(weights_offsets), int(weights_offsets.dtype == torch.int64), _p(weights_tys), _p(dim_offsets), T,
-        total_dims, _p(indices), _p(offsets), int(indices.dtype == torch.int64), indices.shape[0], B, pooling_mode,
-        _p(indice_weights), int(indice_weights is not None and indice_weights.dtype == torch.float16),
-        int(out.dtype == torch.float16), int(scale_offset_is_fp32), row_alignment, _p(status), _stream()))
-    return out
+    return _native().split_bags(dev_weights, uvm_weights, weights_placements, weights_offsets, weights_tys, dim_offsets,
+                                total_dims, indices, offsets, pooling_mode, indice_weights, out_dtype == torch.float16,
+                                scale_offset_is_fp32, row_alignment, out, status)
 
 
 # ------------------------------------------------------------------------------------------
@@ -418,55 +368,21 @@ def rowwise_quantized_fc(inp, weights, bias, weights_offsets, bias_triples, out_
                          bias_offset, *, weights_row_sums=None, flags=0, out=None, workspace=None, status=None):
     """RowwiseQuantizedFullyConnected: inp int8 [M,K], weights int8 [N,K], bias int32 [N],
     weights_offsets int32 [N], bias_triples/out_triples = three int32 [N] tensors each."""
-    _cuda(inp, "inp", (torch.int8,))
-    _cuda(weights, "weights", (torch.int8,))
-    M, K = inp.shape
-    N = weights.shape[0]
-    _cuda(bias, "bias", (torch.int32, torch.int8))
-    if bias.dtype == torch.int8:   # the reference's _i8_i8 form
-        flags |= FC_BIAS_INT8
-    for t in (weights_offsets, *bias_triples, *out_triples):
-        _cuda(t, "per-row parameter", (torch.int32,))
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.int8, device=inp.device)
-    ws = _workspace(workspace, i8_gemm_workspace_bytes(M, K, N), inp.device)
-    check(_lib.lib().glowb200_rowwise_quantized_fc_i8_i32(
-        _p(out), _p(inp), _p(weights), _p(bias), _p(weights_offsets), _p(bias_triples[0]), _p(bias_triples[1]),
-        _p(bias_triples[2]), _p(out_triples[0]), _p(out_triples[1]), _p(out_triples[2]), M, K, N, int(out_offset),
-        int(in_offset), int(bias_offset), _p(weights_row_sums), int(flags), _p(ws), ws.numel(), _p(status),
-        _stream()))
-    return out
+    return _native().rowwise_fc(inp, weights, bias, weights_offsets, bias_triples, out_triples, out_offset, in_offset,
+                                bias_offset, weights_row_sums, flags, out, workspace, status)
 
 
 def fully_connected_i8(inp, weights, bias, out_offset, in_offset, weights_offset, bias_offset, bias_triple,
                        out_triple, *, weights_transposed=None, flags=0, out=None, workspace=None, status=None):
     """FullyConnected (int8, per-tensor): inp [M,K], weights [K,N], bias int32 (or int8) [N]."""
-    if bias.dtype == torch.int8:   # the reference's _i8_i8 form
-        flags |= FC_BIAS_INT8
-    M, K = inp.shape
-    N = weights.shape[1] if weights is not None else weights_transposed.shape[0]
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.int8, device=inp.device)
-    ws = _workspace(workspace, i8_gemm_workspace_bytes(M, K, N), inp.device)
-    check(_lib.lib().glowb200_fc_i8_i32(
-        _p(out), _p(inp), _p(weights), _p(bias), M, K, N, int(out_offset), int(in_offset), int(weights_offset),
-        int(bias_offset), *[int(v) for v in bias_triple], *[int(v) for v in out_triple], _p(weights_transposed),
-        int(flags), _p(ws), ws.numel(), _p(status), _stream()))
-    return out
+    return _native().fc_i8(inp, weights, bias, out_offset, in_offset, weights_offset, bias_offset, bias_triple, out_triple,
+                           weights_transposed, flags, out, workspace, status)
 
 
 def matmul_i8(lhs, rhs, out_offset, lhs_offset, rhs_offset, out_triple, *, flags=0, out=None, workspace=None,
               status=None):
     """MatMul (int8): lhs [M,K], rhs [K,N]."""
-    M, K = lhs.shape
-    N = rhs.shape[1]
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.int8, device=lhs.device)
-    ws = _workspace(workspace, i8_gemm_workspace_bytes(M, K, N), lhs.device)
-    check(_lib.lib().glowb200_matmul_i8(
-        _p(out), _p(lhs), _p(rhs), M, K, N, int(out_offset), int(lhs_offset), int(rhs_offset),
-        *[int(v) for v in out_triple], int(flags), _p(ws), ws.numel(), _p(status), _stream()))
-    return out
+    return _native().matmul(lhs, rhs, out_offset, lhs_offset, rhs_offset, out_triple, flags, out, workspace, status)
 
 
 def tensor_rowwise_quantize_i8_device(w, schema=ASYMMETRIC):
@@ -511,31 +427,14 @@ def dynamic_rowwise_quantized_fc(inp, weights, bias, scales, offsets, *, weights
                                  workspace=None, status=None):
     """DynamicRowwiseQuantizedFullyConnected: inp [M,K] fp16, weights [K,N] int8 (or weights_transposed
     [N,K]), bias / scales fp32 [N], offsets int32 [N]; result [M,N] fp16."""
-    _cuda(inp, "inp", (torch.float16,))
-    M, K = inp.shape
-    N = bias.shape[0]
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.float16, device=inp.device)
-    ws = _workspace(workspace, dynamic_fc_workspace_bytes(M, K, N), inp.device)
-    check(_lib.lib().glowb200_dynamic_rowwise_quantized_fc(
-        _p(out), _p(inp), _p(weights), _p(bias), _p(scales), _p(offsets), M, K, N, _p(weights_transposed), int(flags),
-        _p(ws), ws.numel(), _p(status), _stream()))
-    return out
+    return _native().dynamic_rowwise_fc(inp, weights, bias, scales, offsets, weights_transposed, flags, out, workspace, status)
 
 
 def dynamic_quantized_fc(inp, weights, bias, weights_scale, weights_offset, *, weights_transposed=None, flags=0,
                          out=None, workspace=None, status=None):
     """DynamicQuantizedFullyConnected: as above with one scale / offset for the whole weights tensor."""
-    _cuda(inp, "inp", (torch.float16,))
-    M, K = inp.shape
-    N = bias.shape[0]
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.float16, device=inp.device)
-    ws = _workspace(workspace, dynamic_fc_workspace_bytes(M, K, N), inp.device)
-    check(_lib.lib().glowb200_dynamic_quantized_fc(
-        _p(out), _p(inp), _p(weights), _p(bias), float(weights_scale), int(weights_offset), M, K, N,
-        _p(weights_transposed), int(flags), _p(ws), ws.numel(), _p(status), _stream()))
-    return out
+    return _native().dynamic_fc(inp, weights, bias, weights_scale, weights_offset, weights_transposed, flags, out, workspace,
+                                status)
 
 
 # ------------------------------------------------------------------------------------------
@@ -564,20 +463,9 @@ def channelwise_quantized_conv2d(inp, filt, bias, kernels, strides, pads, group,
                                  filter_offsets, bias_offsets, bias_triples, out_triples, act_type=0, act_args=None,
                                  *, filter_row_sums=None, flags=0, out=None, workspace=None, status=None):
     """ChannelwiseQuantizedConvolution: inp int8 NHWC, filt int8 [outC,kH,kW,inC/group], bias int32."""
-    _cuda(inp, "inp", (torch.int8,))
-    _cuda(filt, "filt", (torch.int8,))
-    sh, odims = _conv_shapes(inp, filt, kernels, strides, pads, group, dilation)
-    if out is None:
-        out = torch.empty(odims, dtype=torch.int8, device=inp.device)
-    need = int(_lib.lib().glowb200_conv2d_workspace_bytes(sh[0], sh[1], sh[2], sh[3], sh[4], sh[5], sh[6], sh[7]))
-    ws = _workspace(workspace, need, inp.device)
-    aa = (C.c_int32 * 3)(*([int(v) for v in act_args] + [0, 0, 0])[:3]) if act_args is not None else None
-    check(_lib.lib().glowb200_channelwise_quantized_conv2d_i8_i32(
-        _p(out), _p(inp), _p(filt), _p(bias), sh[0], sh[1], sh[2], sh[3], sh[4], sh[5], sh[6], sh[7], int(out_offset),
-        int(in_offset), _p(filter_offsets), _p(bias_offsets), _p(bias_triples[0]), _p(bias_triples[1]),
-        _p(bias_triples[2]), _p(out_triples[0]), _p(out_triples[1]), _p(out_triples[2]), int(act_type), aa,
-        _p(filter_row_sums), int(flags), _p(ws), ws.numel(), _p(status), _stream()))
-    return out
+    return _native().channelwise_conv(inp, filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset,
+                                      filter_offsets, bias_offsets, bias_triples, out_triples, act_type, act_args,
+                                      filter_row_sums, flags, out, workspace, status)
 
 
 def conv2d_i8(inp, filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset, filter_offset,
@@ -638,12 +526,7 @@ def batched_add_i8(batch, slice_, dest_offset, batch_offset, slice_offset, batch
 
 def element_add_maxsplat_i8(lhs, rhs, dest_offset, lhs_offset, rhs_offset, lhs_triple, rhs_triple, splat, out=None):
     """element_add_i8 followed by element_maxsplat_i8(splat), fused."""
-    if out is None:
-        out = torch.empty_like(lhs)
-    check(_lib.lib().glowb200_element_add_maxsplat_i8(
-        _p(out), _p(lhs), _p(rhs), lhs.numel(), int(dest_offset), int(lhs_offset), int(rhs_offset),
-        *[int(v) for v in lhs_triple], *[int(v) for v in rhs_triple], int(splat), _stream()))
-    return out
+    return _native().add_maxsplat(lhs, rhs, dest_offset, lhs_offset, rhs_offset, lhs_triple, rhs_triple, splat, out)
 
 
 def element_relu_i8(src, src_offset, dest_offset, triple, out=None):
@@ -667,36 +550,19 @@ def element_rescale_i8(src, out_offset, in_offset, triple, out=None):
 
 
 def element_quantize_i8(src, scale, offset, out=None):
-    out = torch.empty(src.shape, dtype=torch.int8, device=src.device) if out is None else out
-    check(_lib.lib().glowb200_element_quantize_i8(_p(out), _p(src), src.numel(), C.c_float(float(scale)), int(offset),
-                                                  _stream()))
-    return out
+    return _native().quantize(src, scale, offset, out)
 
 
 def element_dequantize_i8(src, scale, offset, out=None):
-    out = torch.empty(src.shape, dtype=torch.float32, device=src.device) if out is None else out
-    check(_lib.lib().glowb200_element_dequantize_i8(_p(out), _p(src), src.numel(), C.c_float(float(scale)),
-                                                    int(offset), _stream()))
-    return out
+    return _native().dequantize(src, scale, offset, out)
 
 
 def max_pool_i8(inp, kernels, strides, pads, out_offset, out=None):
-    n, h, w, c = inp.shape
-    oh, ow = conv_out_hw((h, w), kernels, strides, pads)
-    out = torch.empty((n, oh, ow, c), dtype=torch.int8, device=inp.device) if out is None else out
-    check(_lib.lib().glowb200_max_pool_i8(_p(inp), _p(out), _i64arr(inp.shape), _i64arr(out.shape), _i64arr(kernels),
-                                          _i64arr(strides), _i64arr(pads), int(out_offset), _stream()))
-    return out
+    return _native().max_pool(inp, kernels, strides, pads, out_offset, out)
 
 
 def avg_pool_i8(inp, kernels, strides, pads, count_include_pads, out_offset, in_offset, triple, out=None):
-    n, h, w, c = inp.shape
-    oh, ow = conv_out_hw((h, w), kernels, strides, pads)
-    out = torch.empty((n, oh, ow, c), dtype=torch.int8, device=inp.device) if out is None else out
-    check(_lib.lib().glowb200_avg_pool_i8(_p(inp), _p(out), _i64arr(inp.shape), _i64arr(out.shape), _i64arr(kernels),
-                                          _i64arr(strides), _i64arr(pads), int(bool(count_include_pads)),
-                                          int(out_offset), int(in_offset), *[int(v) for v in triple], _stream()))
-    return out
+    return _native().avg_pool(inp, kernels, strides, pads, out_offset, out, count_include_pads, in_offset, triple)
 
 
 def transpose(src, shuffle):
@@ -727,29 +593,14 @@ class programmatic_launch:
 
 def quantize_transpose_i8(src, shuffle, scale, offset):
     """transpose(quantize(src)) in one pass: fp32 in, int8 out with dims[i] = src dims[shuffle[i]]."""
-    _cuda(src, "src", (torch.float32,))
-    out = torch.empty([src.shape[i] for i in shuffle], dtype=torch.int8, device=src.device)
-    check(_lib.lib().glowb200_quantize_transpose_i8(_p(out), _p(src), _i64arr(src.shape), (C.c_int32 * len(shuffle))(*shuffle),
-                                                    len(shuffle), C.c_float(float(scale)), int(offset), _stream()))
-    return out
+    return _native().quantize_transpose(src, shuffle, scale, offset)
 
 
 def pairwise_dot_interaction(dense, pooled, *, quant=None, out=None):
     """dense fp32 [B, D]; pooled fp32 [B, T, D] (or [B, T*D]).  Returns fp32 [B, D + n(n-1)/2]
     (n = T + 1), or int8 when quant=(scale, offset) (the following Quantize node fused)."""
-    _cuda(dense, "dense", (torch.float32,))
-    _cuda(pooled, "pooled", (torch.float32,))
-    B, D = dense.shape
-    T = pooled.numel() // (B * D) if B else 0
-    n = T + 1
-    width = D + n * (n - 1) // 2
-    if out is None:
-        out = torch.empty((B, width), dtype=torch.int8 if quant else torch.float32, device=dense.device)
     q = quant or (1.0, 0)
-    check(_lib.lib().glowb200_pairwise_dot_interaction(
-        _p(dense), D, _p(pooled), T * D, B, T, D, None if quant else _p(out), _p(out) if quant else None, width,
-        C.c_float(float(q[0])), int(q[1]), _stream()))
-    return out
+    return _native().pairwise_dot(dense, pooled, bool(quant), q[0], q[1], out)
 
 
 def device_tensor(ptr, shape, dtype, device="cuda"):
@@ -892,7 +743,5 @@ class SlwsBatch:
                 int(self.index_dtype == torch.int64), self.in_line, self.out_line,
                 _p(self.workspace), self.workspace.numel(), _p(status), _stream()))
             return
-        check(_lib.lib().glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched(
-            _p(self.jobs_dev), self.num_jobs, self.max_segments, self.kind,
-            int(self.index_dtype == torch.int64), self.in_line, self.out_line, self.out_fp16, int(self.fp16_acc),
-            _p(self.workspace), self.workspace.numel(), _p(status), _stream()))
+        _native().slws_batched(self.jobs_dev, self.num_jobs, self.max_segments, self.kind, self.index_dtype == torch.int64,
+                               self.in_line, self.out_line, self.out_fp16, self.fp16_acc, self.workspace, status)
