@@ -197,7 +197,7 @@ PyObject *slws(PyObject *const *a) {
     invoke(fn.glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum, out.data_ptr(), data.data_ptr(), kind, rows,
         weights.data_ptr(), indices.data_ptr(), idx64,
         (const int32_t *)lengths.data_ptr(), segments, n, in_line, out_line, out16, acc16, ws.data(), ws.bytes(), status,
-            stream());
+        stream());
   return given ? same(a[6]) : give(out);
 }
 
@@ -517,8 +517,9 @@ PyObject *setup(PyObject *, PyObject *args) {
   Py_RETURN_NONE;
 }
 
-#define FAST(name, body, n) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<body, n>)),
-    METH_FASTCALL, nullptr}
+#define FAST(name, body, n) \
+  {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<body, n>)), \
+   METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"setup", setup, METH_VARARGS, nullptr},
     FAST("slws", slws, 12),
