@@ -85,7 +85,6 @@ def fused_rowwise_quantized_sparse_lengths_weighted_sum(data, weights, indices, 
     weights: result dtype [n]; indices: int32/int64 [n]; lengths: int32 [segments].
     out_line: columns of the result when the rows are padded (see pad_fused_rows); default: the
     whole row is payload + scale/offset."""
-    # (low latency: a warp per bag: for small requests; another summation order, see the header)
     return _native().slws(data, weights, indices, lengths, kind, use_fp16_accumulation, out, status, workspace, num_indices,
                           out_line, low_latency)
 

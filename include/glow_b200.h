@@ -138,14 +138,11 @@ int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum(
     int64_t in_line_size, int64_t out_line_size, int out_is_fp16, int use_fp16_accumulation,
     void *workspace, size_t workspace_bytes, int32_t *status, glowb200_stream_t stream);
 
-/* The same operator for small requests where latency counts: every bag gets a whole warp (the
- * thread mapping the entry point above gives tables with very uneven bags), so a bag's rows are
- * fetched together instead of four at a time -- the launch of benchmark configuration 1 (1024
- * bags of about 32 rows) takes a quarter of the time; up to 2048 bags the warps also add up the
- * lengths before their bag themselves, so the request is a single launch.  fp32 accumulation only.  The rows of a bag
- * are summed in another order than above: results agree within the operator's tolerance (1e-5
- * relative) but are not bit-identical to the other entry points', which is why the choice is the
- * caller's and not made from the size of the launch. */
+/* The same operator under the name callers use for small requests where latency counts.  It runs the
+ * kernels of the entry point above and gives the same bits: a launch too small to fill the GPU fetches
+ * sixteen rows of a bag at a time, and up to 2048 bags its warps also add up the lengths before their
+ * bags themselves, so that the request is a single launch, whichever of the two is called.  fp32
+ * accumulation only. */
 int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_low_latency(
     void *dest, const void *data, int kind, int64_t rows, const void *weights, const void *indices,
     int indices_are_int64, const int32_t *lengths, int64_t segments, int64_t num_indices,

@@ -1,0 +1,137 @@
+"""The gather-pool's runs of bags at their edges: bags of every length round the 4, 8 and 16 rows of a
+step, among short and empty ones; every width and row alignment the kernel is built for; launches on
+both sides of the sizes where it changes its step, its runs and where bag boundaries come from; weights
+of very different sizes; rows that are not finite.  Against a float64 restatement of the operator."""
+import numpy as np
+import pytest
+import torch
+
+from glow_b200 import ops, workloads
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+EDGES = [0, 1, 2, 31, 32, 33, 5, 0, 0, 7, 9, 3, 1, 1, 63, 64, 65, 255, 256, 257, 0, 288, 600, 15, 16, 17, 30, 2, 1, 4, 8, 0]
+
+
+def make_table(kind, rows, dim, seed):
+    f = workloads.fused_table_u4 if kind >= 2 else workloads.fused_table_u8
+    return f(rows, dim, seed, 0, fp16_scale_offset=bool(kind & 1))
+
+
+def want_and_size(table, kind, dim, w, idx, lengths):
+    tail = 4 if kind & 1 else 8
+    so = table[:, -tail:].copy().view(np.float16 if kind & 1 else np.float32).astype(np.float64)
+    q = table[:, :dim if kind < 2 else dim // 2]
+    if kind >= 2:
+        q = np.stack([q & 15, q >> 4], 2).reshape(len(table), dim)
+    q, sc, of = q.astype(np.float64), so[:, :1], so[:, 1:]
+    w = np.asarray(w, np.float64)[:, None]
+    # (the kernel's association: where a weight is infinite, w * scale * q and w * offset may cancel)
+    terms, size = (w * sc[idx]) * q[idx] + w * of[idx], np.abs(w) * (np.abs(sc[idx] * q[idx]) + np.abs(of[idx]))
+    ends = np.cumsum(lengths)
+    return (np.stack([terms[e - l:e].sum(0) for l, e in zip(lengths, ends)]),
+            np.stack([size[e - l:e].sum(0) for l, e in zip(lengths, ends)]))
+
+
+def dev(a, shift=0):
+    """The array on the device, `shift` bytes behind a 16-byte boundary."""
+    a = np.ascontiguousarray(a)
+    buf = torch.zeros(a.nbytes + 32, dtype=torch.uint8, device=DEV)
+    at = -buf.data_ptr() % 16 + shift
+    view = buf[at:at + a.nbytes].view(torch.from_numpy(a).dtype).view(a.shape)
+    view.copy_(torch.from_numpy(a))
+    return view
+
+
+def check(got, want, size, rel):
+    bound = rel * np.maximum(size, np.abs(want)) + 1e-30
+    err = np.abs(got.astype(np.float64) - want)
+    assert (err <= bound).all(), "largest error / bound %g" % np.max(err / bound)
+
+
+def pool(table, w, idx, lengths, kind, **kw):
+    return ops.fused_rowwise_quantized_sparse_lengths_weighted_sum(table, dev(w), dev(idx), dev(lengths), kind, **kw)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("dim", [8, 16, 24, 32, 40, 64, 96, 128, 136, 256, 1000])
+def test_lengths_widths_and_alignments(kind, dim):
+    rng = np.random.default_rng(dim + kind)
+    rows = 700
+    table = make_table(kind, rows, dim, dim)
+    lengths = np.concatenate([EDGES, rng.integers(0, 9, 40), rng.permutation(EDGES)]).astype(np.int32)
+    n = int(lengths.sum())
+    idx = rng.integers(0, rows, n)
+    w = rng.normal(0, 1, n).astype(np.float16 if kind & 1 else np.float32)
+    want, size = want_and_size(table, kind, dim, w, idx, lengths)
+    status = ops.new_status(DEV)
+    first = None
+    for shift in (0, 4, 1, 2, 8):
+        for idt in (np.int64, np.int32):
+            got = pool(dev(table, shift), w, idx.astype(idt), lengths, kind, status=status)
+            first = got if first is None else first
+            assert torch.equal(got, first)   # neither the alignment nor the index type shows
+    check(first.cpu().numpy(), want, size, 2e-3 if kind & 1 else 1e-5)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    got = ops.embedding_bag_byte_rowwise_offsets(dev(table), dev(w), dev(idx.astype(np.int64)), dev(offsets), kind, status=status)
+    assert torch.equal(got, first)
+    assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("bags", [1, 3, 2048, 2049, 9000, 120_000])
+@pytest.mark.parametrize("kind,dim", [(0, 64), (3, 128)])
+def test_launch_size_does_not_show(bags, kind, dim):
+    """A bag pooled beside any number of others gives the same bits as pooled alone."""
+    rng = np.random.default_rng(bags)
+    table = dev(make_table(kind, 5000, dim, 3))
+    lengths = rng.choice(EDGES if bags < 10_000 else [0, 1, 2, 5, 9, 33], bags).astype(np.int32)
+    lengths[-1] = 300
+    n = int(lengths.sum())
+    idx, w = rng.integers(0, 5000, n), rng.normal(0, 1, n).astype(np.float16 if kind & 1 else np.float32)
+    whole = pool(table, w, idx, lengths, kind)
+    ends = np.cumsum(lengths)
+    for b in [0, bags - 1] + list(rng.integers(0, bags, 12)):
+        e, l = int(ends[b]), int(lengths[b])
+        assert torch.equal(pool(table, w[e - l:e], idx[e - l:e], lengths[b:b + 1], kind)[0], whole[b])
+
+
+@pytest.mark.parametrize("kind", [0, 2])
+def test_weights_of_changing_size(kind):
+    rng = np.random.default_rng(5)
+    table = make_table(kind, 300, 64, 9)
+    lengths = np.array([200, 33, 500, 64, 32, 8], np.int32)
+    n = int(lengths.sum())
+    idx = rng.integers(0, 300, n)
+    w = rng.normal(0, 1, n) * 10.0 ** rng.integers(-8, 8, n)
+    w[200:233] = 0
+    w[232] = 1.5
+    w[233:300] = 1e-30
+    w = w.astype(np.float32)
+    want, size = want_and_size(table, kind, 64, w, idx, lengths)
+    check(pool(dev(table), w, idx, lengths, kind).cpu().numpy(), want, size, 1e-5)
+
+
+@pytest.mark.parametrize("dim", [64, 136])
+def test_rows_that_are_not_finite(dim):
+    """Infinite and undefined scales, offsets and weights reach exactly the bags they belong to."""
+    rng = np.random.default_rng(7)
+    table = make_table(0, 400, dim, 11)
+    sc = table[:, -8:].copy().view(np.float32)
+    sc[3, 0], sc[4, 1], sc[5, 0], sc[6, 1] = np.inf, -np.inf, np.nan, np.nan
+    table[:, -8:] = sc.view(np.uint8)
+    lengths = np.array([5, 3, 40, 2, 100, 1, 7, 33, 6, 300], np.int32)
+    n = int(lengths.sum())
+    idx = rng.integers(10, 400, n)
+    w = rng.normal(0, 1, n).astype(np.float32)
+    ends = np.cumsum(lengths)
+    for b, r in ((1, 3), (2, 4), (4, 5), (7, 6), (9, 3)):
+        idx[ends[b] - 1] = r
+    w[ends[3] - 1] = np.inf
+    table[3, :8] = 0                        # an infinite scale times a zero byte is undefined
+    with np.errstate(all="ignore"):
+        want, size = want_and_size(table, 0, dim, w, idx, lengths)
+    got = pool(dev(table), w, idx, lengths, 0).cpu().numpy()
+    fine = np.isfinite(want)
+    assert (np.isnan(got) == np.isnan(want)).all() and (got[np.isinf(want)] == want[np.isinf(want)]).all()
+    assert fine.any(1).sum() == 4
+    check(got[fine], want[fine], size[fine], 1e-5)
