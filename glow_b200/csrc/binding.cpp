@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "glow_b200.h"
 
@@ -27,13 +28,14 @@ namespace {
   X(glowb200_fc_i8_i32) X(glowb200_matmul_i8) X(glowb200_dynamic_rowwise_quantized_fc) X(glowb200_dynamic_quantized_fc) \
   X(glowb200_conv2d_workspace_bytes) X(glowb200_channelwise_quantized_conv2d_i8_i32) X(glowb200_element_add_maxsplat_i8) \
   X(glowb200_element_quantize_i8) X(glowb200_element_dequantize_i8) X(glowb200_max_pool_i8) X(glowb200_avg_pool_i8)    \
-  X(glowb200_quantize_transpose_i8) X(glowb200_pairwise_dot_interaction)
+  X(glowb200_quantize_transpose_i8) X(glowb200_pairwise_dot_interaction) X(glowb200_device_manager_run_function_io)
 struct Entry {
 #define X(name) decltype(&::name) name = nullptr;
   GLOWB200_ENTRY_POINTS(X)
 #undef X
 } fn;
 PyObject *error_class = nullptr;   // GlowB200Error(code, message)
+PyObject *ndarray = nullptr;       // numpy.ndarray
 PyObject *explain = nullptr;       // ops._explain(name, object, dtypes): raises what is wrong with an argument
 
 struct Raised {};  // a Python exception is set
@@ -497,6 +499,54 @@ PyObject *pairwise_dot(PyObject *const *a) {
   return given ? same(a[5]) : give(out);
 }
 
+// ---- device manager ----
+// handle, network name, {placeholder name: array}, names of the outputs (None: every array goes in and comes back)
+PyObject *run_function(PyObject *const *a) {
+  void *dm = PyLong_AsVoidPtr(a[0]);
+  const char *name = PyUnicode_AsUTF8(a[1]);
+  if (name == nullptr || PyErr_Occurred()) throw Raised{};
+  if (!PyDict_Check(a[2])) {
+    PyErr_SetString(PyExc_TypeError, "bindings must be a dict of placeholder names and arrays");
+    throw Raised{};
+  }
+  const size_t n = (size_t)PyDict_GET_SIZE(a[2]);
+  std::vector<const char *> names;
+  std::vector<void *> buffers;
+  std::vector<size_t> sizes;
+  std::vector<int> directions;
+  struct Views {
+    std::vector<Py_buffer> v;
+    ~Views() { for (Py_buffer &b : v) PyBuffer_Release(&b); }
+  } views;
+  names.reserve(n), buffers.reserve(n), sizes.reserve(n), directions.reserve(n), views.v.reserve(n);
+  PyObject *key, *value;
+  Py_ssize_t pos = 0;
+  while (PyDict_Next(a[2], &pos, &key, &value)) {
+    const char *k = PyUnicode_AsUTF8(key);
+    if (k == nullptr) throw Raised{};
+    Py_buffer b;
+    if (!PyObject_TypeCheck(value, reinterpret_cast<PyTypeObject *>(ndarray)) ||
+        PyObject_GetBuffer(value, &b, PyBUF_WRITABLE | PyBUF_C_CONTIGUOUS) != 0) {
+      PyErr_SetString(PyExc_TypeError, "bindings must be writable C-contiguous numpy arrays");
+      throw Raised{};
+    }
+    views.v.push_back(b);
+    names.push_back(k);
+    buffers.push_back(b.buf);
+    sizes.push_back((size_t)b.len);
+    int direction = GLOWB200_BINDING_INPUT | GLOWB200_BINDING_OUTPUT;
+    if (a[3] != Py_None) {
+      const int is_output = PySequence_Contains(a[3], key);
+      if (is_output < 0) throw Raised{};
+      direction = is_output ? GLOWB200_BINDING_OUTPUT : GLOWB200_BINDING_INPUT;
+    }
+    directions.push_back(direction);
+  }
+  invoke(fn.glowb200_device_manager_run_function_io, static_cast<glowb200_device_manager *>(dm), name, names.data(),
+         buffers.data(), sizes.data(), directions.data(), (int)n);
+  Py_RETURN_NONE;
+}
+
 // setup(addresses by name, error class, explain)
 PyObject *setup(PyObject *, PyObject *args) {
   PyObject *table, *error, *why;
@@ -510,6 +560,11 @@ PyObject *setup(PyObject *, PyObject *args) {
   }
   GLOWB200_ENTRY_POINTS(X)
 #undef X
+  PyObject *numpy = PyImport_ImportModule("numpy");
+  PyObject *array = numpy ? PyObject_GetAttrString(numpy, "ndarray") : nullptr;
+  Py_XDECREF(numpy);
+  if (array == nullptr) return nullptr;
+  Py_XSETREF(ndarray, array);
   Py_INCREF(error);
   Py_INCREF(why);
   Py_XSETREF(error_class, error);
@@ -539,6 +594,7 @@ PyMethodDef methods[] = {
     FAST("avg_pool", pool<true>, 9),
     FAST("quantize_transpose", quantize_transpose, 4),
     FAST("pairwise_dot", pairwise_dot, 6),
+    FAST("run_function", run_function, 4),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -55,7 +55,10 @@ struct Instruction {
   std::vector<int64_t> off;   // byte offset of each operand inside its symbol (a view of a larger tensor)
   int group = -1;             // FRWQ_SLWS: index of the batched launch this instruction is part of
   bool group_leader = false;  // ... and whether it is the one that launches it
-  bool absorbed = false;      // QUANTIZE: done by the TRANSPOSE behind it (nothing to launch)
+  bool absorbed = false;      // QUANTIZE done by the TRANSPOSE behind it, INSERT_TENSOR done by its source (nothing to launch)
+  bool once = false;          // SPLAT whose result nothing else writes: done when the network is loaded
+  bool zero_offsets = false;  // RWQ_FC, CWQ_CONV: every weight offset is a constant 0
+  int64_t dest_stride = 0;    // FRWQ_SLWS: elements between result rows when an INSERT_TENSOR was folded in (else out_line)
   bool quantizes = false;     // TRANSPOSE: reads floats (operand 2) and quantizes them on the way (fa[0], ia[10])
   std::vector<int64_t> ia;    // integer attributes
   std::vector<float> fa;      // float attributes
@@ -105,6 +108,12 @@ struct Context {
   int32_t *status_host = nullptr;      // pinned
   std::vector<glowb200_slws_job *> jobs;  // device descriptor arrays, one per batched pooling launch
   cudaEvent_t in_done = nullptr, run_done = nullptr, out_done = nullptr;
+  // The instruction list as one graph: every address and size of a context is fixed, so the list is
+  // captured at the context's second request (the first runs it launch by launch, which also loads the
+  // kernels' code) and replayed from then on.
+  cudaGraphExec_t graph = nullptr;
+  int runs = 0;
+  bool no_graph = false;               // capture was tried and is not possible
   int64_t ticket = 0;                  // the request in flight on this context (0: none)
 };
 
@@ -190,9 +199,9 @@ namespace {
 // What an instruction addresses, checked against the sizes of the symbols it names: a
 // malformed or mistranslated instruction must fail here, not overwrite a neighbour in the slab.
 // Layouts as in the table above glowb200_function_compile.
-int validate_instruction(const glowb200_function *f, const Instruction &in, size_t ii) {
+struct Need { int op; int64_t bytes; bool optional; };
+int validate_instruction(const glowb200_function *f, const Instruction &in, size_t ii, std::vector<Need> *sizes = nullptr) {
   const auto &a = in.ia;
-  struct Need { int op; int64_t bytes; bool optional; };
   std::vector<Need> needs;
   auto need = [&](int op, int64_t bytes, bool optional = false) { needs.push_back({op, bytes, optional}); };
   auto bad = [&](const char *what) { return set_error(GLOWB200_RUNTIME_ERROR, "instruction %zu: %s", ii, what); };
@@ -205,7 +214,7 @@ int validate_instruction(const glowb200_function *f, const Instruction &in, size
     case GLOWB200_INSTR_FRWQ_SLWS: {
       if (!nonneg({1, 2, 3, 4, 5})) return bad("negative size");
       const int64_t es = a[7] ? 2 : 4;
-      need(0, a[4] * a[3] * es); need(1, a[1] * a[2]); need(2, a[5] * es); need(3, a[5] * (a[6] ? 8 : 4)); need(4, a[4] * 4);
+      need(0, in.dest_stride ? (a[4] > 0 ? (a[4] - 1) * in.dest_stride + a[3] : 0) * es : a[4] * a[3] * es); need(1, a[1] * a[2]); need(2, a[5] * es); need(3, a[5] * (a[6] ? 8 : 4)); need(4, a[4] * 4);
       break;
     }
     case GLOWB200_INSTR_RWQ_FC:
@@ -313,6 +322,7 @@ int validate_instruction(const glowb200_function *f, const Instruction &in, size
     default: break;
   }
   if (needs.size() != in.ops.size()) return bad("operand table out of step with the instruction");
+  if (sizes) *sizes = needs;
   for (const Need &n : needs) {
     const int id = in.ops[n.op];
     if (id < 0) {
@@ -326,6 +336,104 @@ int validate_instruction(const glowb200_function *f, const Instruction &in, size
     if (n.op == 0 && s.kind == kConstant) return set_error(GLOWB200_RUNTIME_ERROR, "instruction %zu: the destination '%s' is a constant", ii, s.name.c_str());
   }
   return GLOWB200_OK;
+}
+
+// Whether `bytes` of a symbol are a constant and all zero.
+bool constant_zeros(const glowb200_function *f, int id, int64_t off, int64_t bytes) {
+  if (id < 0 || f->symbols[id].kind != kConstant) return false;
+  const auto &h = f->symbols[id].host;
+  for (int64_t i = 0; i < bytes; i++)
+    if (h[off + i] != 0) return false;
+  return true;
+}
+
+// Rows of `width` bytes, `pitch` apart, inside a symbol.
+struct Region { int symbol; int64_t at, rows, width, pitch; };
+bool overlap(const Region &x, const Region &y) {
+  if (x.symbol != y.symbol || x.rows <= 0 || y.rows <= 0 || x.width <= 0 || y.width <= 0) return false;
+  const int64_t x1 = x.at + (x.rows - 1) * x.pitch + x.width, y1 = y.at + (y.rows - 1) * y.pitch + y.width;
+  if (x1 <= y.at || y1 <= x.at) return false;
+  if (x.pitch == y.pitch && x.pitch > 0) {  // different columns of the same rows (the parts of a Concat)
+    const int64_t d = ((y.at - x.at) % x.pitch + x.pitch) % x.pitch;
+    if (d >= x.width && d + y.width <= x.pitch) return false;
+  }
+  return true;
+}
+// What operand `op` of an instruction addresses (the rows that lie between are not touched).
+Region region_of(const glowb200_function *f, const Instruction &in, size_t ii, int op) {
+  std::vector<Need> sizes;
+  if (in.ops[op] < 0 || validate_instruction(f, in, ii, &sizes) != GLOWB200_OK) return {in.ops[op], 0, 0, 0, 0};
+  const auto &a = in.ia;
+  if (op == 0 && in.kind == GLOWB200_INSTR_INSERT_TENSOR) return {in.ops[0], in.off[0] + a[3], a[0], a[1], a[2]};
+  if (op == 0 && in.kind == GLOWB200_INSTR_FRWQ_SLWS && in.dest_stride) {
+    const int64_t es = a[7] ? 2 : 4;
+    return {in.ops[0], in.off[0], a[4], a[3] * es, in.dest_stride * es};
+  }
+  for (const Need &n : sizes)
+    if (n.op == op) return {in.ops[op], in.off[op], 1, n.bytes, n.bytes};
+  return {in.ops[op], in.off[op], 1, (int64_t)f->symbols[in.ops[op]].bytes, 0};
+}
+
+// Batched pooling wants 16-byte aligned operands and a result on the boundary of its element type.
+bool batchable(const Instruction &in) {
+  if (in.kind != GLOWB200_INSTR_FRWQ_SLWS || in.off[0] % (in.ia[7] ? 2 : 4)) return false;
+  for (size_t o = 1; o < in.off.size(); o++)
+    if (in.off[o] % 16) return false;
+  return true;
+}
+
+// A pooling result that nothing reads but the InsertTensor which puts it into its columns of a wider tensor
+// (a Concat of pooled vectors, as it is lowered) is pooled there: one copy per table less.
+void fold_inserts(glowb200_function *f) {
+  for (size_t j = 0; j < f->instrs.size(); j++) {
+    Instruction &ins = f->instrs[j];
+    if (ins.kind != GLOWB200_INSTR_INSERT_TENSOR || f->symbols[ins.ops[1]].kind != kActivation) continue;
+    const Region from = region_of(f, ins, j, 1), to = region_of(f, ins, j, 0);
+    int source = -1;
+    bool alone = true;
+    for (size_t i = 0; i < f->instrs.size() && alone; i++) {
+      const Instruction &other = f->instrs[i];
+      if (i == j || other.absorbed) continue;
+      for (size_t o = 0; o < other.ops.size() && alone; o++) {
+        if (other.ops[o] != from.symbol || !overlap(region_of(f, other, i, (int)o), from)) continue;
+        if (o == 0 && i < j && source < 0 && other.kind == GLOWB200_INSTR_FRWQ_SLWS && other.dest_stride == 0 &&
+            other.off[0] == ins.off[1]) source = (int)i;
+        else alone = false;
+      }
+    }
+    if (!alone || source < 0) continue;
+    Instruction &pool = f->instrs[source];
+    const int64_t es = pool.ia[7] ? 2 : 4;
+    if (pool.ia[4] != ins.ia[0] || pool.ia[3] * es != ins.ia[1] || ins.ia[2] % es || (ins.off[0] + ins.ia[3]) % es) continue;
+    if (!batchable(pool)) continue;  // (only a batched launch takes a row stride)
+    // the columns must not be in use between the two instructions, nor be what the pooling reads
+    bool busy = false;
+    for (size_t i = source; i < j && !busy; i++) {
+      const Instruction &other = f->instrs[i];
+      if (other.absorbed) continue;
+      for (size_t o = (int)i == source ? 1 : 0; o < other.ops.size(); o++)
+        busy = busy || (other.ops[o] == to.symbol && overlap(region_of(f, other, i, (int)o), to));
+    }
+    if (busy) continue;
+    pool.ops[0] = ins.ops[0];
+    pool.off[0] = ins.off[0] + ins.ia[3];
+    pool.dest_stride = ins.ia[2] / es;
+    ins.absorbed = true;
+  }
+}
+
+// A Splat whose destination no other instruction writes holds its value for good (the weights of one of a
+// lowered SparseLengthsSum): it is done when the network is loaded.
+void hoist_splats(glowb200_function *f) {
+  for (size_t i = 0; i < f->instrs.size(); i++) {
+    Instruction &sp = f->instrs[i];
+    if (sp.kind != GLOWB200_INSTR_SPLAT || f->symbols[sp.ops[0]].kind != kActivation) continue;
+    const Region r = region_of(f, sp, i, 0);
+    bool written = false;
+    for (size_t k = 0; k < f->instrs.size(); k++)
+      if (k != i && !f->instrs[k].absorbed && f->instrs[k].ops[0] == r.symbol) written = written || overlap(region_of(f, f->instrs[k], k, 0), r);
+    sp.once = !written;
+  }
 }
 
 }  // namespace
@@ -404,6 +512,7 @@ extern "C" int glowb200_function_compile(glowb200_function *f) {
           rs[j] = s;
         }
         in.derived.push_back(f->add_i32_constant(tag + ".row_sums", rs));
+        in.zero_offsets = constant_zeros(f, in.ops[4], in.off[4], N * 4);
         ws = std::max(ws, glowb200_i8_gemm_workspace_bytes(in.ia[0], in.ia[1], N));
         break;
       }
@@ -417,6 +526,15 @@ extern "C" int glowb200_function_compile(glowb200_function *f) {
         const int64_t fd[4] = {in.ia[6], in.ia[7], in.ia[8], in.ia[3] / in.ia[15]}, k[2] = {in.ia[7], in.ia[8]}, s[2] = {in.ia[9], in.ia[10]};
         const int64_t p[4] = {in.ia[11], in.ia[12], in.ia[13], in.ia[14]}, d[2] = {in.ia[16], in.ia[17]};
         ws = std::max(ws, glowb200_conv2d_workspace_bytes(od, id, fd, k, s, p, in.ia[15], d));
+        in.zero_offsets = constant_zeros(f, in.ops[5], in.off[5], OC * 4);
+        const Symbol &flt = f->symbols[in.ops[2]];
+        const int64_t K = fd[1] * fd[2] * fd[3];
+        if (flt.kind == kConstant) {  // row sums of a constant filter, computed once
+          std::vector<int32_t> rs(OC);
+          for (int64_t j = 0; j < OC; j++)
+            for (int64_t q = 0; q < K; q++) rs[j] += (int8_t)flt.host[in.off[2] + j * K + q];
+          in.derived.push_back(f->add_i32_constant(tag + ".row_sums", rs));
+        }
         break;
       }
       case GLOWB200_INSTR_ADD: {
@@ -533,50 +651,37 @@ extern "C" int glowb200_function_compile(glowb200_function *f) {
       default: return set_error(GLOWB200_RUNTIME_ERROR, "instruction %zu: unsupported kind %d (isOpSupported would refuse the node)", ii, in.kind);
     }
   }
+  fold_inserts(f);
+  hoist_splats(f);
   // Pooling instructions that follow one another, read the same kind of table with the same row
   // width and do not feed each other become ONE batched launch (a recommendation model's tables
   // are so many independent SparseLengthsSum nodes): the descriptors are built when the network
-  // is loaded.  The batched kernels want 16-byte aligned operands; views at other offsets stay
-  // single launches.
+  // is loaded.  Views that batchable() turns down stay single launches.
   {
-    auto groupable = [&](const Instruction &in) {
-      if (in.kind != GLOWB200_INSTR_FRWQ_SLWS) return false;
-      for (int64_t o : in.off)
-        if (o % 16) return false;
-      return true;
-    };
     auto same_shape = [](const Instruction &a, const Instruction &b) {
       return a.ia[0] == b.ia[0] && a.ia[2] == b.ia[2] && a.ia[3] == b.ia[3] && a.ia[6] == b.ia[6] && a.ia[7] == b.ia[7] &&
              a.ia[8] == b.ia[8];
     };
     size_t i = 0;
     while (i < f->instrs.size()) {
-      if (!groupable(f->instrs[i])) { i++; continue; }
+      if (!batchable(f->instrs[i])) { i++; continue; }
       std::vector<int> members{(int)i};
       size_t j = i + 1;
-      for (; j < f->instrs.size() && groupable(f->instrs[j]) && same_shape(f->instrs[i], f->instrs[j]); j++) {
+      for (; j < f->instrs.size() && batchable(f->instrs[j]) && same_shape(f->instrs[i], f->instrs[j]); j++) {
         // an earlier member must not write what this one reads, nor the bytes it writes
-        auto dest_range = [](const Instruction &in, int64_t &lo, int64_t &hi) {
-          lo = in.off[0];
-          hi = lo + in.ia[4] * in.ia[3] * (in.ia[7] ? 2 : 4);
-        };
         bool feeds = false;
         const Instruction &cand = f->instrs[j];
+        const Region to = region_of(f, cand, j, 0);
         for (int m : members) {
           const Instruction &prev = f->instrs[m];
           for (size_t o = 1; o < cand.ops.size(); o++) feeds = feeds || cand.ops[o] == prev.ops[0];
           for (size_t o = 1; o < prev.ops.size(); o++) feeds = feeds || prev.ops[o] == cand.ops[0];
-          if (cand.ops[0] == prev.ops[0]) {
-            int64_t a0, a1, b0, b1;
-            dest_range(cand, a0, a1);
-            dest_range(prev, b0, b1);
-            feeds = feeds || (a0 < b1 && b0 < a1);
-          }
+          feeds = feeds || overlap(to, region_of(f, prev, m, 0));
         }
         if (feeds) break;
         members.push_back((int)j);
       }
-      if (members.size() > 1 && members.size() <= 65535) {
+      if ((members.size() > 1 || f->instrs[i].dest_stride) && members.size() <= 65535) {
         int64_t max_segments = 0;
         for (int m : members) {
           f->instrs[m].group = (int)f->slws_groups.size();
@@ -648,6 +753,15 @@ struct glowb200_device_manager {
   std::map<int64_t, int> finished;    // results of requests that were completed on behalf of a later one
   std::map<std::string, LoadedNetwork> networks;
   std::mutex lock;
+  std::map<const uint8_t *, size_t> io;  // pinned buffers handed out (allocate_io_buffer)
+  std::mutex io_lock;
+  bool is_io(const void *p, size_t bytes) {
+    std::lock_guard<std::mutex> g(io_lock);
+    auto it = io.upper_bound(static_cast<const uint8_t *>(p));
+    if (it == io.begin()) return false;
+    --it;
+    return static_cast<const uint8_t *>(p) + bytes <= it->first + it->second;
+  }
 };
 
 extern "C" glowb200_device_manager *glowb200_device_manager_create(int device_id, uint64_t max_memory_bytes) {
@@ -694,6 +808,7 @@ static void free_network(LoadedNetwork &n) {
     if (c.status_dev) cudaFree(c.status_dev);
     if (c.status_host) cudaFreeHost(c.status_host);
     for (auto *j : c.jobs) if (j) cudaFree(j);
+    if (c.graph) cudaGraphExecDestroy(c.graph);
     if (c.in_done) cudaEventDestroy(c.in_done);
     if (c.run_done) cudaEventDestroy(c.run_done);
     if (c.out_done) cudaEventDestroy(c.out_done);
@@ -753,7 +868,7 @@ extern "C" int glowb200_device_manager_add_network(glowb200_device_manager *dm, 
         memset(&j, 0, sizeof(j));
         j.dest = at(0); j.data = at(1); j.weights = at(2); j.indices = at(3);
         j.lengths = reinterpret_cast<const int32_t *>(at(4));
-        j.rows = in.ia[1]; j.num_indices = in.ia[5]; j.dest_stride = in.ia[3]; j.segments = in.ia[4];
+        j.rows = in.ia[1]; j.num_indices = in.ia[5]; j.dest_stride = in.dest_stride ? in.dest_stride : in.ia[3]; j.segments = in.ia[4];
       }
       glowb200_slws_job *dj = nullptr;
       ok = cudaMalloc(&dj, jobs.size() * sizeof(glowb200_slws_job)) == cudaSuccess &&
@@ -765,6 +880,12 @@ extern "C" int glowb200_device_manager_add_network(glowb200_device_manager *dm, 
     for (const Symbol &s : f->symbols)
       if (s.kind == kConstant && s.bytes)
         ok = ok && cudaMemcpyAsync(n.shared[0] + s.offset, s.host.data(), s.bytes, cudaMemcpyHostToDevice, dm->stream) == cudaSuccess;
+  for (Context &c : n.ctx)
+    for (const Instruction &in : f->instrs)
+      if (ok && in.once) {
+        const Symbol &sy = f->symbols[in.ops[0]];
+        ok = glowb200_splat_f(c.slab[sy.kind] + sy.offset + in.off[0], in.ia[0], in.fa[0], (int)in.ia[1], dm->stream) == GLOWB200_OK;
+      }
   if (ok) ok = cudaStreamSynchronize(dm->stream) == cudaSuccess;
   if (!ok) {
     free_network(n);
@@ -838,6 +959,7 @@ int execute(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
       return c.slab[s.kind] + s.offset + in.off[o];
     };
     int rc = GLOWB200_OK;
+    if (in.absorbed || in.once) continue;
     switch (in.kind) {
       case GLOWB200_INSTR_FRWQ_SLWS:
         if (in.group >= 0) {  // part of a batched launch: the first member launches it for all
@@ -861,7 +983,7 @@ int execute(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
         rc = glowb200_rowwise_quantized_fc_i8_i32(
             (int8_t *)P(0), (const int8_t *)P(1), (const int8_t *)P(2), (const int32_t *)P(5),
             (const int32_t *)P(4), d(0), d(1), d(2), d(3), d(4), d(5), a[0], a[1], a[2], (int32_t)a[5], (int32_t)a[3],
-            (int32_t)a[4], d(6), a[6] ? GLOWB200_FC_FUSE_RELU : 0, c.workspace, f->workspace_bytes, c.status_dev, st);
+            (int32_t)a[4], d(6), (a[6] ? GLOWB200_FC_FUSE_RELU : 0) | (in.zero_offsets ? GLOWB200_FC_WEIGHT_OFFSETS_ZERO : 0), c.workspace, f->workspace_bytes, c.status_dev, st);
         break;
       }
       case GLOWB200_INSTR_CWQ_CONV: {
@@ -871,7 +993,8 @@ int execute(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
         rc = glowb200_channelwise_quantized_conv2d_i8_i32(
             (int8_t *)P(0), (const int8_t *)P(1), (const int8_t *)P(2), (const int32_t *)P(3),
             od, id, fd, k, s, p, a[15], dl, (int32_t)a[19], (int32_t)a[18], (const int32_t *)P(5),
-            (const int32_t *)P(7), d(0), d(1), d(2), d(3), d(4), d(5), (int32_t)a[20], nullptr, nullptr, 0, c.workspace,
+            (const int32_t *)P(7), d(0), d(1), d(2), d(3), d(4), d(5), (int32_t)a[20], nullptr, in.derived.size() > 6 ? d(6) : nullptr,
+            in.zero_offsets ? GLOWB200_FC_WEIGHT_OFFSETS_ZERO : 0, c.workspace,
             f->workspace_bytes, c.status_dev, st);
         break;
       }
@@ -884,7 +1007,6 @@ int execute(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
         rc = glowb200_element_maxsplat_i8((int8_t *)P(0), (const int8_t *)P(1), a[0], (int32_t)a[1], st);
         break;
       case GLOWB200_INSTR_QUANTIZE:
-        if (in.absorbed) break;  // the Transpose behind it does both
         rc = glowb200_element_quantize_i8((int8_t *)P(0), (const float *)P(1), a[0], in.fa[0], (int32_t)a[1], st);
         break;
       case GLOWB200_INSTR_DEQUANTIZE:
@@ -1012,6 +1134,75 @@ int execute(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
   return GLOWB200_OK;
 }
 
+// The instruction list on the kernel stream: launch by launch the first time, as a graph from the second.
+int execute_request(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
+  c.runs++;
+  if (c.graph == nullptr && c.runs == 2 && !c.no_graph) {
+    cudaGraph_t g = nullptr;
+    c.no_graph = true;
+    if (cudaStreamBeginCapture(dm->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      const int rc = execute(dm, n, c);
+      const bool captured = cudaStreamEndCapture(dm->stream, &g) == cudaSuccess && g != nullptr;
+      if (captured && rc == GLOWB200_OK && cudaGraphInstantiate(&c.graph, g, 0) == cudaSuccess) c.no_graph = false;
+      else c.graph = nullptr;
+      if (g) cudaGraphDestroy(g);
+    }
+    if (c.no_graph) cudaGetLastError();
+  }
+  if (c.graph != nullptr) {
+    if (cudaGraphLaunch(c.graph, dm->stream) != cudaSuccess)
+      return set_error(GLOWB200_RUNTIME_DEVICE_NONRECOVERABLE, "cannot launch the graph of %s", n.fn->name.c_str());
+    return GLOWB200_OK;
+  }
+  return execute(dm, n, c);
+}
+
+// ---- inputs and outputs of a synchronous request ----
+// A request of a few small tensors spends more time starting copies than copying.  Where every buffer is
+// pinned memory this device manager handed out (the GPU reads and writes it in place), one kernel brings all
+// inputs in and one takes all outputs and the status word out.
+constexpr int kMaxMoves = 16;
+constexpr size_t kMoveBytes = 4 << 20;  // larger requests are the copy engines'
+struct Move { const uint8_t *from; uint8_t *to; uint32_t bytes, zeros; };  // zeros: bytes of `to` to clear behind them
+struct Moves {
+  Move m[kMaxMoves];
+  int n;
+  int32_t *status, *status_host;  // outputs only: the status word goes along and is cleared
+};
+constexpr int kMovePiece = 8192;  // bytes per block and step: 256 threads, two 16-byte pieces each in flight
+__global__ void __launch_bounds__(256) move_kernel(const __grid_constant__ Moves p) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && p.status != nullptr) {
+    *p.status_host = *p.status;
+    *p.status = 0;
+  }
+  int64_t piece = blockIdx.x;
+  for (int i = 0; i < p.n; i++) {
+    const Move &m = p.m[i];
+    const int64_t total = (int64_t)m.bytes + m.zeros, pieces = (total + kMovePiece - 1) / kMovePiece;
+    if (piece >= pieces) { piece -= pieces; continue; }
+    const int64_t begin = piece * kMovePiece, end = begin + kMovePiece < total ? begin + kMovePiece : total;
+    const bool wide = ((reinterpret_cast<uintptr_t>(m.from) | reinterpret_cast<uintptr_t>(m.to)) & 15) == 0;
+    if (wide && end <= m.bytes) {
+#pragma unroll 2
+      for (int64_t at = begin + 16 * threadIdx.x; at + 16 <= end; at += 16 * 256)
+        *reinterpret_cast<uint4 *>(m.to + at) = *reinterpret_cast<const uint4 *>(m.from + at);
+      for (int64_t at = (end & ~15ll) + threadIdx.x; at < end; at += 256)
+        if (at >= begin) m.to[at] = m.from[at];
+    } else {
+#pragma unroll 4
+      for (int64_t at = begin + threadIdx.x; at < end; at += 256) m.to[at] = at < m.bytes ? m.from[at] : 0;
+    }
+    return;
+  }
+}
+int launch_moves(const Moves &p, cudaStream_t s) {
+  int64_t blocks = 0;
+  for (int i = 0; i < p.n; i++) blocks += ((int64_t)p.m[i].bytes + p.m[i].zeros + kMovePiece - 1) / kMovePiece;
+  if (blocks == 0 && p.status == nullptr) return GLOWB200_OK;
+  move_kernel<<<(unsigned)(blocks ? blocks : 1), 256, 0, s>>>(p);
+  return cudaGetLastError() == cudaSuccess ? GLOWB200_OK : set_error(GLOWB200_RUNTIME_ERROR, "cannot move the request's tensors");
+}
+
 }  // namespace
 
 // runFunction: `bindings` pairs placeholder names with HOST buffers (the PlaceholderBindings of
@@ -1032,14 +1223,16 @@ int status_to_error(int32_t status, const char *name) {
   return GLOWB200_OK;
 }
 
-// Finishes a synchronous request: the status word, the stream, the mapping of what went wrong.
-int finish_request(glowb200_device_manager *dm, Context &c, const char *name) {
-  int32_t status = 0;
-  cudaMemcpyAsync(&status, c.status_dev, 4, cudaMemcpyDeviceToHost, dm->stream);
-  cudaMemsetAsync(c.status_dev, 0, 4, dm->stream);
+// Finishes a synchronous request: the status word (unless it is on its way already), the stream, the
+// mapping of what went wrong.
+int finish_request(glowb200_device_manager *dm, Context &c, const char *name, bool status_sent = false) {
+  if (!status_sent) {
+    cudaMemcpyAsync(c.status_host, c.status_dev, 4, cudaMemcpyDeviceToHost, dm->stream);
+    cudaMemsetAsync(c.status_dev, 0, 4, dm->stream);
+  }
   const cudaError_t e = cudaStreamSynchronize(dm->stream);
   if (e != cudaSuccess) return set_error(GLOWB200_RUNTIME_DEVICE_NONRECOVERABLE, "device error while running %s: %s", name, cudaGetErrorString(e));
-  return status_to_error(status, name);
+  return status_to_error(*static_cast<volatile int32_t *>(c.status_host), name);
 }
 
 // A request that failed on the host part-way through: kernels and copies already queued are
@@ -1140,7 +1333,7 @@ extern "C" int glowb200_device_manager_run_function_resident(glowb200_device_man
     const int64_t t = c.ticket;
     dm->finished[t] = complete_context(dm, c, name);
   }
-  if (int rc = execute(dm, it->second, c)) return abort_request(dm, c, rc);
+  if (int rc = execute_request(dm, it->second, c)) return abort_request(dm, c, rc);
   return finish_request(dm, c, name);
 }
 
@@ -1162,6 +1355,26 @@ extern "C" int glowb200_device_manager_run_function_io(glowb200_device_manager *
     const int64_t t = c.ticket;
     dm->finished[t] = complete_context(dm, c, name);
   }
+  Moves in{}, out{};
+  bool in_place = num_bindings <= kMaxMoves;
+  size_t moved = 0;
+  for (int b = 0; b < num_bindings && in_place; b++) {
+    const Symbol &sym = f->symbols[ids[b]];
+    uint8_t *d = c.slab[kPlaceholder] + sym.offset, *h = static_cast<uint8_t *>(host_buffers[b]);
+    const int dir = directions ? directions[b] : GLOWB200_BINDING_INPUT | GLOWB200_BINDING_OUTPUT;
+    in_place = dm->is_io(h, buffer_bytes[b]) && (moved += sym.bytes) <= kMoveBytes;
+    if (dir & GLOWB200_BINDING_INPUT) in.m[in.n++] = {h, d, (uint32_t)buffer_bytes[b], (uint32_t)(sym.bytes - buffer_bytes[b])};
+    if (dir & GLOWB200_BINDING_OUTPUT) out.m[out.n++] = {d, h, (uint32_t)buffer_bytes[b], 0};
+  }
+  if (in_place) {
+    out.status = c.status_dev;
+    out.status_host = c.status_host;
+    int rc = launch_moves(in, dm->stream);
+    if (rc == GLOWB200_OK) rc = execute_request(dm, n, c);
+    if (rc == GLOWB200_OK) rc = launch_moves(out, dm->stream);
+    if (rc != GLOWB200_OK) return abort_request(dm, c, rc);
+    return finish_request(dm, c, name, true);
+  }
   for (int b = 0; b < num_bindings; b++) {
     const Symbol &sym = f->symbols[ids[b]];
     uint8_t *d = c.slab[kPlaceholder] + sym.offset;
@@ -1170,7 +1383,7 @@ extern "C" int glowb200_device_manager_run_function_io(glowb200_device_manager *
     if (ok && buffer_bytes[b] < sym.bytes) ok = cudaMemsetAsync(d + buffer_bytes[b], 0, sym.bytes - buffer_bytes[b], dm->stream) == cudaSuccess;
     if (!ok) return abort_request(dm, c, set_error(GLOWB200_RUNTIME_ERROR, "host-to-device copy of %s failed", sym.name.c_str()));
   }
-  if (int rc = execute(dm, n, c)) return abort_request(dm, c, rc);
+  if (int rc = execute_request(dm, n, c)) return abort_request(dm, c, rc);
   for (int b = 0; b < num_bindings; b++) {
     const Symbol &sym = f->symbols[ids[b]];
     if (directions && !(directions[b] & GLOWB200_BINDING_OUTPUT)) continue;  // an input: nothing to copy back
@@ -1220,7 +1433,7 @@ extern "C" int glowb200_device_manager_run_function_async(glowb200_device_manage
   }
   bool ok = cudaEventRecord(c.in_done, dm->in_stream) == cudaSuccess && cudaStreamWaitEvent(dm->stream, c.in_done, 0) == cudaSuccess;
   if (!ok) return abort_request(dm, c, set_error(GLOWB200_RUNTIME_ERROR, "cannot order the streams of %s", name));
-  if (int rc = execute(dm, n, c)) return abort_request(dm, c, rc);
+  if (int rc = execute_request(dm, n, c)) return abort_request(dm, c, rc);
   ok = cudaEventRecord(c.run_done, dm->stream) == cudaSuccess && cudaStreamWaitEvent(dm->out_stream, c.run_done, 0) == cudaSuccess;
   for (int b = 0; b < num_bindings && ok; b++) {
     const Symbol &sym = f->symbols[ids[b]];
@@ -1265,9 +1478,16 @@ extern "C" void *glowb200_device_manager_allocate_io_buffer(glowb200_device_mana
     set_error(GLOWB200_RUNTIME_ERROR, "cannot allocate %zu bytes of pinned host memory", bytes);
     return nullptr;
   }
+  std::lock_guard<std::mutex> g(dm->io_lock);
+  dm->io[static_cast<const uint8_t *>(p)] = bytes;
   return p;
 }
 
 extern "C" void glowb200_device_manager_free_io_buffer(glowb200_device_manager *dm, void *buffer) {
-  if (dm && buffer) cudaFreeHost(buffer);
+  if (!dm || !buffer) return;
+  {
+    std::lock_guard<std::mutex> g(dm->io_lock);
+    dm->io.erase(static_cast<const uint8_t *>(buffer));
+  }
+  cudaFreeHost(buffer);
 }

@@ -9,7 +9,7 @@ import ctypes as C
 
 import numpy as np
 
-from . import _lib
+from . import _lib, ops
 from ._lib import GlowB200Error
 
 CONSTANT, PLACEHOLDER, ACTIVATION, STATIC = 0, 1, 2, 3
@@ -240,19 +240,7 @@ class DeviceManager:
     def run_function(self, name, bindings, outputs=None):
         """bindings: dict placeholder name -> numpy array.  outputs=None: every array is copied in
         and written back; else the names in `outputs` are copied out only, the others in only."""
-        names = list(bindings)
-        arrs = [bindings[k] for k in names]
-        for a in arrs:
-            if not (isinstance(a, np.ndarray) and a.flags["C_CONTIGUOUS"] and a.flags["WRITEABLE"]):
-                raise TypeError("bindings must be writable C-contiguous numpy arrays")
-        cn = (C.c_char_p * len(names))(*[k.encode() for k in names])
-        cb = (C.c_void_p * len(names))(*[a.ctypes.data for a in arrs])
-        cs = (C.c_size_t * len(names))(*[a.nbytes for a in arrs])
-        if outputs is None:
-            _check(_lib.lib().glowb200_device_manager_run_function(self.h, name.encode(), cn, cb, cs, len(names)))
-        else:
-            cd = (C.c_int * len(names))(*[2 if k in outputs else 1 for k in names])
-            _check(_lib.lib().glowb200_device_manager_run_function_io(self.h, name.encode(), cn, cb, cs, cd, len(names)))
+        ops._native().run_function(self.h, name, bindings, outputs)
 
     def set_context_count(self, contexts):
         """Execution contexts (own placeholders and activations each) of networks added from now on."""
