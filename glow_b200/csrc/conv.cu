@@ -22,10 +22,6 @@
 namespace glowb200 {
 namespace {
 
-struct ConvGeom {
-  int N, H, W, C, OH, OW, OC, KH, KW, SH, SW, PT, PL, DH, DW, G;
-};
-
 // one thread per 16-byte chunk of the im2col matrix (C a multiple of 16: a chunk never
 // straddles two taps)
 __global__ void __launch_bounds__(256) im2col_i8_vec_kernel(const int8_t *__restrict__ x, int8_t *__restrict__ a,
@@ -158,68 +154,86 @@ __global__ void __launch_bounds__(256) im2col_i8_rows_kernel(const int8_t *__res
 // of output pixel (n, oh, ow) is byte kw * C + c of window (n, oh + a, ow) of plane e, so the
 // convolution is a contraction whose left-hand rows are four windows of one plane, Y = OH + 3 rows
 // per image: 2 * 32 bytes per (y, ow) instead of KH * KW * C per output pixel, and no im2col matrix.
-// One thread per window.
+// One thread per window; behind them `tail` zero windows (the four windows of the last rows reach that far)
+// and the filter re-laid to match: [OC, KH, KW, C] -> [OC, 2 planes, 4 rows a, 32 bytes], tap
+// (kh = 2a + e, kw, c) at byte kw * C + c of (e, a), everything else zero.
 __global__ void __launch_bounds__(256) row_windows_i8_kernel(const int8_t *__restrict__ x, int8_t *__restrict__ planes,
                                                               const __grid_constant__ ConvGeom g, int Y, int64_t plane_bytes,
-                                                              int8_t pad) {
+                                                              int8_t pad, int tail, const int8_t *__restrict__ f,
+                                                              int8_t *__restrict__ fb) {
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t per_plane = (int64_t)g.N * Y * g.OW, total = 2 * per_plane;
+  const int64_t per_plane = (int64_t)g.N * Y * g.OW, windows = 2 * per_plane, total = windows + tail + (int64_t)g.OC * 8;
   const int run = g.KW * g.C;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int e = (int)(i / per_plane);
-    int64_t r = i - e * per_plane;
-    const int ow = (int)(r % g.OW);
-    r /= g.OW;
-    const int y = (int)(r % Y), n = (int)(r / Y);
-    const int ih = 2 * y - g.PT + e, b0 = (2 * ow - g.PL) * g.C;  // first byte of the window in its image row
-    const bool row_in = ih >= 0 && ih < g.H;
-    const int8_t *src = x + ((int64_t)n * g.H + (row_in ? ih : 0)) * g.W * g.C;
     uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-    for (int b = 0; b < run; b++) {
-      const int o = b0 + b;
-      const int8_t v = (row_in && o >= 0 && o < g.W * g.C) ? src[o] : pad;
-      w[b >> 2] |= (uint32_t)(uint8_t)v << (8 * (b & 3));
+    int4 *dst;
+    if (i < windows) {
+      const int e = (int)(i / per_plane);
+      int64_t r = i - e * per_plane;
+      const int ow = (int)(r % g.OW);
+      r /= g.OW;
+      const int y = (int)(r % Y), n = (int)(r / Y);
+      const int ih = 2 * y - g.PT + e, b0 = (2 * ow - g.PL) * g.C;  // first byte of the window in its image row
+      const bool row_in = ih >= 0 && ih < g.H;
+      const int8_t *src = x + ((int64_t)n * g.H + (row_in ? ih : 0)) * g.W * g.C;
+      for (int b = 0; b < run; b++) {
+        const int o = b0 + b;
+        const int8_t v = (row_in && o >= 0 && o < g.W * g.C) ? src[o] : pad;
+        w[b >> 2] |= (uint32_t)(uint8_t)v << (8 * (b & 3));
+      }
+      dst = reinterpret_cast<int4 *>(planes + e * plane_bytes + (i - e * per_plane) * 32);
+    } else if (i < windows + tail) {
+      dst = reinterpret_cast<int4 *>(planes + 2 * plane_bytes + (i - windows) * 32);
+    } else {
+      const int64_t r = i - windows - tail;  // 32 bytes (e, a) of a filter
+      const int oc = (int)(r >> 3), e = (int)(r >> 2) & 1, kh = 2 * ((int)r & 3) + e;
+      if (kh < g.KH) {
+        const int8_t *src = f + ((int64_t)oc * g.KH + kh) * run;
+        for (int b = 0; b < run; b++) w[b >> 2] |= (uint32_t)(uint8_t)src[b] << (8 * (b & 3));
+      }
+      dst = reinterpret_cast<int4 *>(fb + r * 32);
     }
-    int4 *dst = reinterpret_cast<int4 *>(planes + e * plane_bytes + (i - e * per_plane) * 32);
     dst[0] = make_int4((int)w[0], (int)w[1], (int)w[2], (int)w[3]);
     dst[1] = make_int4((int)w[4], (int)w[5], (int)w[6], (int)w[7]);
   }
 }
 
-// Filter [OC, KH, KW, C] -> [OC, 2 planes, 4 rows a, 32 bytes]: tap (kh = 2a + e, kw, c) at byte
-// kw * C + c of (e, a); everything else zero.
-__global__ void __launch_bounds__(256) window_filter_i8_kernel(const int8_t *__restrict__ f, int8_t *__restrict__ out, int OC,
-                                                               int KH, int KW, int C) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int64_t total = (int64_t)OC * 256;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int oc = (int)(i >> 8), k = (int)(i & 255);
-    const int e = k >> 7, a = (k >> 5) & 3, b = k & 31;
-    const int kh = 2 * a + e, kw = b / C, c = b - kw * C;
-    out[i] = (kh < KH && kw < KW) ? f[(((int64_t)oc * KH + kh) * KW + kw) * C + c] : (int8_t)0;
-  }
-}
-
 // NHWC input with its padding made real: [N, Hp, Wp, C], the cells outside the image filled with
-// `pad_word` (the input offset, which is how the reference's skipped taps read).  16 bytes per thread.
+// `pad_word` (the input offset, which is how the reference's skipped taps read), and 256 zero bytes
+// behind it (the window of the last rows reads past them).  16 bytes per thread.
+// fb != nullptr (C = 64): the same launch re-lays the filter [OC, KH, KW, 64] -> [OC, KH * ceil(KW / 2), 128],
+// taps (kh, 2j) and (kh, 2j + 1) side by side, the partner of a last odd tap zero -- the right-hand side
+// that matches left-hand rows made of two neighbouring 64-channel pixels.
 __global__ void __launch_bounds__(256) pad_nhwc_i8_kernel(const int8_t *__restrict__ x, int8_t *__restrict__ xp,
-                                                           const __grid_constant__ ConvGeom g, int Hp, int Wp, int pad_word) {
+                                                           const __grid_constant__ ConvGeom g, int Hp, int Wp, int pad_word,
+                                                           const int8_t *__restrict__ f, int8_t *__restrict__ fb) {
   pdl_wait();
   pdl_launch_dependents();
-  const int cc = g.C >> 4;
-  const int64_t total = (int64_t)g.N * Hp * Wp * cc;
+  const int cc = g.C >> 4, pairs = (g.KW + 1) >> 1;
+  const int64_t cells = (int64_t)g.N * Hp * Wp * cc, total = cells + 16 + (fb ? (int64_t)g.OC * g.KH * pairs * 8 : 0);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % cc);
-    int64_t r = i / cc;
-    const int xw = (int)(r % Wp);
-    r /= Wp;
-    const int yh = (int)(r % Hp), n = (int)(r / Hp);
-    const int ih = yh - g.PT, iw = xw - g.PL;
-    int4 v = make_int4(pad_word, pad_word, pad_word, pad_word);
-    if (ih >= 0 && iw >= 0 && ih < g.H && iw < g.W)
-      v = __ldg(reinterpret_cast<const int4 *>(x + (((int64_t)n * g.H + ih) * g.W + iw) * g.C) + c);
+    int4 v = make_int4(0, 0, 0, 0);
+    if (i < cells) {
+      const int c = (int)(i % cc);
+      int64_t r = i / cc;
+      const int xw = (int)(r % Wp);
+      r /= Wp;
+      const int yh = (int)(r % Hp), n = (int)(r / Hp);
+      const int ih = yh - g.PT, iw = xw - g.PL;
+      v = make_int4(pad_word, pad_word, pad_word, pad_word);
+      if (ih >= 0 && iw >= 0 && ih < g.H && iw < g.W)
+        v = __ldg(reinterpret_cast<const int4 *>(x + (((int64_t)n * g.H + ih) * g.W + iw) * g.C) + c);
+    } else if (i >= cells + 16) {
+      const int64_t j = i - cells - 16;
+      const int piece = (int)(j & 7);
+      int64_t r = j >> 3;
+      const int kw = 2 * (int)(r % pairs) + (piece >> 2);
+      r /= pairs;  // oc * KH + kh
+      if (kw < g.KW) v = __ldg(reinterpret_cast<const int4 *>(f + (r * g.KW + kw) * 64) + (piece & 3));
+      reinterpret_cast<int4 *>(fb)[j] = v;
+      continue;
+    }
     reinterpret_cast<int4 *>(xp)[i] = v;
   }
 }
@@ -246,26 +260,6 @@ __global__ void __launch_bounds__(256) pad_parity_nhwc_i8_kernel(const int8_t *_
     if (ih >= 0 && iw >= 0 && ih < g.H && iw < g.W)
       v = __ldg(reinterpret_cast<const int4 *>(x + (((int64_t)n * g.H + ih) * g.W + iw) * g.C) + c);
     reinterpret_cast<int4 *>(xp)[i] = v;
-  }
-}
-
-// Filter [OC, KH, KW, 64] -> [OC, KH * ceil(KW / 2), 128]: taps (kh, 2j) and (kh, 2j + 1) side by
-// side, the partner of a last odd tap zero -- the right-hand side that matches left-hand rows made of
-// two neighbouring 64-channel pixels.
-__global__ void __launch_bounds__(256) pair_taps_c64_kernel(const int8_t *__restrict__ f, int8_t *__restrict__ out, int OC,
-                                                             int KH, int KW) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int pairs = (KW + 1) >> 1;
-  const int64_t total = (int64_t)OC * KH * pairs * 128;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(i & 127);
-    int64_t r = i >> 7;
-    const int pr = (int)(r % pairs);
-    r /= pairs;
-    const int kh = (int)(r % KH), oc = (int)(r / KH);
-    const int kw = 2 * pr + (j >> 6);
-    out[i] = kw < KW ? f[(((int64_t)oc * KH + kh) * KW + kw) * 64 + (j & 63)] : (int8_t)0;
   }
 }
 
@@ -364,6 +358,9 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
     GLOWB200_CUDA_OK(cudaGetLastError());
     return GLOWB200_OK;
   }
+  const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(filter)) & 15) == 0;
+  if (pl.need_im2col && aligned && i8_skinny_conv_wins(g))
+    return run_conv_skinny(p, in, filter, g, (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) != 0, s);
   const size_t need = pl.a_bytes + pl.f_bytes + pl.core_bytes;
   if (workspace == nullptr || workspace_bytes < need)
     return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", workspace_bytes, need);
@@ -392,22 +389,12 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
         xp_bytes + fb_bytes <= pl.a_bytes + pl.f_bytes) {
       int8_t *xp = reinterpret_cast<int8_t *>(ws);
       const uint32_t b = (uint8_t)p.a_offset;
-      const int64_t chunks = rows * (g.C >> 4), blocks = (chunks + 255) / 256;
+      int8_t *fb = g.C == 64 ? reinterpret_cast<int8_t *>(ws + xp_bytes) : nullptr;
+      const int64_t chunks = rows * (g.C >> 4) + 16 + (fb ? (int64_t)g.OC * entries * 8 : 0), blocks = (chunks + 255) / 256;
       GLOWB200_CUDA_OK(launch_pdl(pad_nhwc_i8_kernel, (unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s, in, xp, g, Hp, Wp,
-                                  (int)(b | (b << 8) | (b << 16) | (b << 24))));
-      GLOWB200_CUDA_OK(cudaGetLastError());
-      GLOWB200_CUDA_OK(cudaMemsetAsync(xp + rows * g.C, 0, 256, s));  // the window of the last rows reads past them
-      const int8_t *bmat = filter;
-      p.K = g.KH * g.KW * g.C;
-      if (g.C == 64) {
-        int8_t *fb = reinterpret_cast<int8_t *>(ws + xp_bytes);
-        const int64_t fblocks = ((int64_t)g.OC * entries * 128 + 255) / 256;
-        GLOWB200_CUDA_OK(launch_pdl(pair_taps_c64_kernel, (unsigned)(fblocks < 148 * 16 ? fblocks : 148 * 16), 256, 0, s, filter, fb, g.OC,
-                                    g.KH, g.KW));
-        GLOWB200_CUDA_OK(cudaGetLastError());
-        bmat = fb;
-        p.K = entries * 128;
-      }
+                                  (int)(b | (b << 8) | (b << 16) | (b << 24)), filter, fb));
+      const int8_t *bmat = fb ? fb : filter;
+      p.K = fb ? entries * 128 : g.KH * g.KW * g.C;
       p.k_corr = pl.K;
       p.N = g.OC;
       p.conv_entries = entries;
@@ -477,17 +464,16 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
     if (rows < (1ll << 31) && wp_bytes + fb_bytes <= pl.a_bytes + pl.f_bytes) {
       int8_t *planes = reinterpret_cast<int8_t *>(ws);
       int8_t *fb = reinterpret_cast<int8_t *>(ws + wp_bytes);
-      const int64_t blocks = (2 * rows + 255) / 256;
+      const int tail = (int)((wp_bytes - 2 * plane_bytes) / 32);  // the four windows of the last rows reach past the second plane
+      const int64_t items = 2 * rows + tail + (int64_t)g.OC * 8, blocks = (items + 255) / 256;
       GLOWB200_CUDA_OK(launch_pdl(row_windows_i8_kernel, (unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s, in, planes, g, Y,
-                                  plane_bytes, (int8_t)p.a_offset));
-      GLOWB200_CUDA_OK(cudaGetLastError());
-      // the four windows of the last rows reach past the second plane
-      GLOWB200_CUDA_OK(cudaMemsetAsync(planes + 2 * plane_bytes, 0, wp_bytes - 2 * plane_bytes, s));
-      GLOWB200_CUDA_OK(launch_pdl(window_filter_i8_kernel, (unsigned)((g.OC * 256 + 255) / 256), 256, 0, s, filter, fb, g.OC, g.KH, g.KW,
-                                  g.C));
-      GLOWB200_CUDA_OK(cudaGetLastError());
-      int32_t *bs = reinterpret_cast<int32_t *>(ws + pl.a_bytes + pl.f_bytes);  // zeros do not change the sums, but one path
-      if (int rc = glowb200_i8_row_sums(fb, g.OC, 256, bs, reinterpret_cast<glowb200_stream_t>(s))) return rc;
+                                  plane_bytes, (int8_t)p.a_offset, tail, filter, fb));
+      const int32_t *bs = filter_row_sums;  // (the zeros of the new layout do not change them)
+      if (bs == nullptr) {
+        int32_t *sums = reinterpret_cast<int32_t *>(ws + pl.a_bytes + pl.f_bytes);
+        if (int rc = glowb200_i8_row_sums(fb, g.OC, 256, sums, reinterpret_cast<glowb200_stream_t>(s))) return rc;
+        bs = sums;
+      }
       p.K = 256;
       p.k_corr = pl.K;
       p.N = g.OC;

@@ -86,7 +86,16 @@ __device__ __forceinline__ int32_t activation_i32(int32_t x, const GemmParams &p
 int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_row_sums_in, bool b_offsets_zero,
              int force_any, void *ws, size_t ws_bytes, cudaStream_t s, bool b_is_kn = false);
 
+// An NHWC convolution: input [N, H, W, C], filter [OC, KH, KW, C / G], output [N, OH, OW, OC].
+struct ConvGeom {
+  int N, H, W, C, OH, OW, OC, KH, KW, SH, SW, PT, PL, DH, DW, G;
+};
+
 // ---- qgemm_small.cu ----
+// A convolution of little work as one such product, its left-hand rows read from the input itself (C a
+// multiple of 16, one group, 16-byte aligned operands).
+bool i8_skinny_conv_wins(const ConvGeom &g);
+int run_conv_skinny(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeom &g, bool b_offsets_zero, cudaStream_t s);
 constexpr int kSkinnyRows = 64;
 bool i8_skinny_wins(int64_t M, int64_t N, int64_t K, bool b_is_kn);
 int run_gemm_skinny(GemmParams p, const int8_t *a, const int8_t *b, bool b_is_kn, bool b_offsets_zero, cudaStream_t s);

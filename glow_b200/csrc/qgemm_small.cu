@@ -189,9 +189,12 @@ __device__ __forceinline__ uint4 row16(const int8_t *p, int valid) {
 // MT row tiles of 16, NT column tiles of 8 per block (KN: always 4).  KN: the right-hand side is
 // [K, N], its 4 x 4-byte blocks transposed in registers.  VEC: rows of the operands that are read 16
 // bytes at a time start on 16-byte boundaries and hold a multiple of 16 bytes.
-template <int MT, int NT, bool KN, bool VEC>
-__global__ void __launch_bounds__(512) i8_skinny_kernel(const int8_t *a, const int8_t *b,
-                                                         const __grid_constant__ GemmParams p, int need_a_sums) {
+// CONV: the left-hand row of output pixel (n, oh, ow) is its window of the NHWC input, read where it lies:
+// a lane's 16 bytes never straddle two taps (C a multiple of 16), and a tap outside the image reads as
+// the input offset, which is how the reference's skipped taps count (libjit_conv.cpp:209-212).
+template <int MT, int NT, bool KN, bool VEC, bool CONV>
+__global__ void __launch_bounds__(512) i8_skinny_kernel(const int8_t *a, const int8_t *b, const __grid_constant__ GemmParams p,
+                                                         int need_a_sums, const __grid_constant__ ConvGeom cg) {
   constexpr int kCols = NT * 8;
   // row pitch of the shared sums: the lanes of one atomic (rows g, columns 2t or 8t) meet in no bank, or in pairs
   constexpr int kPitch = KN ? kCols + 1 : (kCols == 8 ? 8 : kCols + 8);
@@ -209,6 +212,22 @@ __global__ void __launch_bounds__(512) i8_skinny_kernel(const int8_t *a, const i
   __syncthreads();
   pdl_wait();
   pdl_launch_dependents();
+
+  // CONV: first pixel and corner of the windows of this lane's rows g and g + 8 of every row tile
+  int pixel[CONV ? MT : 1][2], corner_h[CONV ? MT : 1][2], corner_w[CONV ? MT : 1][2];
+  const uint32_t pad_word = (uint32_t)(uint8_t)p.a_offset * 0x01010101u;
+  if constexpr (CONV) {
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int row = m0 + 16 * mt + 8 * i + g, r = row < p.M ? row : 0;
+        const int ow = r % cg.OW, q = r / cg.OW, oh = q % cg.OH, n = q / cg.OH;
+        corner_h[mt][i] = row < p.M ? oh * cg.SH - cg.PT : -(1 << 20);  // (rows that are not there: never inside the image)
+        corner_w[mt][i] = ow * cg.SW - cg.PL;
+        pixel[mt][i] = (n * cg.H + oh * cg.SH - cg.PT) * cg.W + corner_w[mt][i];
+      }
+  }
 
   int32_t acc[MT][NT][4] = {};
   int32_t a_sums[MT][2] = {}, b_sums[NT] = {};
@@ -251,11 +270,35 @@ __global__ void __launch_bounds__(512) i8_skinny_kernel(const int8_t *a, const i
         const int n = n0 + 8 * nt + g;
         bv[nt] = row16<VEC>(b + (size_t)n * p.K + k, n < p.N ? K - k : 0);
       }
+      int tap_h = 0, tap_w = 0, channel = 0;
+      if constexpr (CONV) {
+        const int tap = k / cg.C, kh = tap / cg.KW;
+        channel = k - tap * cg.C;
+        tap_h = kh * cg.DH;
+        tap_w = (tap - kh * cg.KW) * cg.DW;
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; mt++) {
-        const int row = m0 + 16 * mt + g;
-        const uint4 lo = row16<VEC>(a + (size_t)row * lda + k, row < p.M ? K - k : 0);
-        const uint4 hi = row16<VEC>(a + (size_t)(row + 8) * lda + k, row + 8 < p.M ? K - k : 0);
+        uint4 lo, hi;
+        if constexpr (CONV) {
+          uint4 v[2];
+          bool in[2];
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            in[i] = (unsigned)(corner_h[mt][i] + tap_h) < (unsigned)cg.H && (unsigned)(corner_w[mt][i] + tap_w) < (unsigned)cg.W;
+            v[i] = load_if(reinterpret_cast<const uint4 *>(a + (int64_t)(pixel[mt][i] + tap_h * cg.W + tap_w) * cg.C + channel), in[i] && k < K);
+          }
+          const uint32_t fill = k < K ? pad_word : 0u;
+#pragma unroll
+          for (int i = 0; i < 2; i++)
+            if (!in[i]) v[i] = make_uint4(fill, fill, fill, fill);
+          lo = v[0];
+          hi = v[1];
+        } else {
+          const int row = m0 + 16 * mt + g;
+          lo = row16<VEC>(a + (size_t)row * lda + k, row < p.M ? K - k : 0);
+          hi = row16<VEC>(a + (size_t)(row + 8) * lda + k, row + 8 < p.M ? K - k : 0);
+        }
         if (need_a_sums) {
           a_sums[mt][0] = byte_sum(lo, a_sums[mt][0]);
           a_sums[mt][1] = byte_sum(hi, a_sums[mt][1]);
@@ -327,16 +370,18 @@ __global__ void __launch_bounds__(512) i8_skinny_kernel(const int8_t *a, const i
 }
 
 template <int MT, int NT, bool KN>
-cudaError_t launch_skinny(const GemmParams &p, const int8_t *a, const int8_t *b, bool vec, int need_a_sums, cudaStream_t s) {
+cudaError_t launch_skinny(const GemmParams &p, const int8_t *a, const int8_t *b, bool vec, int need_a_sums, cudaStream_t s,
+                          const ConvGeom *conv = nullptr) {
   const dim3 grid((unsigned)((p.N + 8 * NT - 1) / (8 * NT)), (unsigned)((p.M + 16 * MT - 1) / (16 * MT)));
   // warps share the depth: one step of it each, up to 16.  (CTAs of a cluster sharing it as well, adding
   // up through distributed shared memory, cost more than they brought: 8 x 1024 x 1024 2.5 -> 3.4 us.)
   const int steps = (p.k_corr + (KN ? 31 : 63)) / (KN ? 32 : 64);
   const unsigned threads = steps > 8 ? 512 : steps > 4 ? 256 : 128;
   if constexpr (!KN) {
-    if (vec) return launch_pdl(i8_skinny_kernel<MT, NT, KN, true>, grid, threads, 0, s, a, b, p, need_a_sums);
+    if (conv) return launch_pdl(i8_skinny_kernel<MT, NT, KN, true, true>, grid, threads, 0, s, a, b, p, need_a_sums, *conv);
+    if (vec) return launch_pdl(i8_skinny_kernel<MT, NT, KN, true, false>, grid, threads, 0, s, a, b, p, need_a_sums, ConvGeom{});
   }
-  return launch_pdl(i8_skinny_kernel<MT, NT, KN, false>, grid, threads, 0, s, a, b, p, need_a_sums);
+  return launch_pdl(i8_skinny_kernel<MT, NT, KN, false, false>, grid, threads, 0, s, a, b, p, need_a_sums, ConvGeom{});
 }
 
 }  // namespace
@@ -369,6 +414,29 @@ int run_gemm_skinny(GemmParams p, const int8_t *a, const int8_t *b, bool b_is_kn
 #undef GLOWB200_SKINNY
   }
   if (e != cudaSuccess) return set_error(GLOWB200_ERR_CUDA, "few-row contraction launch failed: %s", cudaGetErrorString(e));
+  return GLOWB200_OK;
+}
+
+bool i8_skinny_conv_wins(const ConvGeom &g) {
+  // (against a padded copy or im2col matrix and the tile kernel, two launches of 2 and 7 us for the 3 x 3
+  // layers of a ResNet-50 on one image)
+  const int64_t M = (int64_t)g.N * g.OH * g.OW, K = (int64_t)g.KH * g.KW * g.C;
+  return g.G == 1 && g.C % 16 == 0 && M * g.OC <= (1 << 19) && M * g.OC * K <= (1ll << 28);
+}
+
+int run_conv_skinny(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeom &g, bool b_offsets_zero, cudaStream_t s) {
+  p.M = g.N * g.OH * g.OW;
+  p.N = g.OC;
+  p.K = p.k_corr = g.KH * g.KW * g.C;
+  const int need = b_offsets_zero ? 0 : 1;
+  // row tiles of 64, smaller ones where those would leave SMs idle
+  const int cols = (p.N + 7) / 8;
+  int mt = 4;
+  while (mt > 1 && (int64_t)((p.M + 16 * mt - 1) / (16 * mt)) * cols < sm_count()) mt /= 2;
+  const cudaError_t e = mt == 4 ? launch_skinny<4, 1, false>(p, in, filter, true, need, s, &g)
+                        : mt == 2 ? launch_skinny<2, 1, false>(p, in, filter, true, need, s, &g)
+                                  : launch_skinny<1, 1, false>(p, in, filter, true, need, s, &g);
+  if (e != cudaSuccess) return set_error(GLOWB200_ERR_CUDA, "small convolution launch failed: %s", cudaGetErrorString(e));
   return GLOWB200_OK;
 }
 
