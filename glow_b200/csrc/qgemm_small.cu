@@ -172,7 +172,6 @@ __global__ void __launch_bounds__(kPrepThreads) i8_prepare_operands_kernel(const
 // the warp-level int8 MMA, and the block adds its warps' partial products in shared memory (integers:
 // exact in any order).  8 x 1024 x 1024: 2.4 us where the tile kernel needs 5.0 and, with weight offsets,
 // its row-sum pass 2.6 more; 8 x 4096 x 4096 (16 MB of weights) 12.4 -> 4.8 us.
-constexpr int kSkinnyMaxCols = 32;
 
 __device__ __forceinline__ void mma_i8(int32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -373,15 +372,49 @@ template <int MT, int NT, bool KN>
 cudaError_t launch_skinny(const GemmParams &p, const int8_t *a, const int8_t *b, bool vec, int need_a_sums, cudaStream_t s,
                           const ConvGeom *conv = nullptr) {
   const dim3 grid((unsigned)((p.N + 8 * NT - 1) / (8 * NT)), (unsigned)((p.M + 16 * MT - 1) / (16 * MT)));
-  // warps share the depth: one step of it each, up to 16.  (CTAs of a cluster sharing it as well, adding
-  // up through distributed shared memory, cost more than they brought: 8 x 1024 x 1024 2.5 -> 3.4 us.)
-  const int steps = (p.k_corr + (KN ? 31 : 63)) / (KN ? 32 : 64);
-  const unsigned threads = steps > 8 ? 512 : steps > 4 ? 256 : 128;
+  // Warps share the depth in equal parts: up to 16 of them, 8 once the blocks alone fill the SMs.  (CTAs of a
+  // cluster sharing it as well, adding up through distributed shared memory, cost more than they brought:
+  // 8 x 1024 x 1024 2.5 -> 3.4 us.)
+  const int steps = (p.k_corr + (KN ? 31 : 63)) / (KN ? 32 : 64), most = (int64_t)grid.x * grid.y >= 220 ? 8 : 16;
+  const int rounds = (steps + most - 1) / most, warps = (steps + rounds - 1) / rounds;
+  const unsigned threads = 32 * (warps < 4 ? 4 : warps);
   if constexpr (!KN) {
     if (conv) return launch_pdl(i8_skinny_kernel<MT, NT, KN, true, true>, grid, threads, 0, s, a, b, p, need_a_sums, *conv);
     if (vec) return launch_pdl(i8_skinny_kernel<MT, NT, KN, true, false>, grid, threads, 0, s, a, b, p, need_a_sums, ConvGeom{});
   }
   return launch_pdl(i8_skinny_kernel<MT, NT, KN, false, false>, grid, threads, 0, s, a, b, p, need_a_sums, ConvGeom{});
+}
+
+// Rows and columns of a block's tile, in MMA tiles of 16 and 8.  Small weights: 16 x 32 (the four column
+// tiles share a row's loads), fewer columns while the tiles leave SMs idle, more rows once they are four
+// to an SM -- 3 x 3 layers of one image, device time: 64 channels at 56 x 56 9.5 (as 64 x 8) -> 3.9 us, 256 at
+// 14 x 14 5.5 -> 4.6, 512 at 7 x 7 9.1 -> 5.0.  Weights of 4 MB and more: all rows in a block as far as they fit,
+// so that the weights are read once.
+struct SkinnyTile { int mt, nt; };
+SkinnyTile skinny_tile(int64_t M, int64_t N, int64_t K, bool kn) {
+  auto blocks = [&](int mt, int nt) { return ((M + 16 * mt - 1) / (16 * mt)) * ((N + 8 * nt - 1) / (8 * nt)); };
+  SkinnyTile t{M <= 16 ? 1 : M <= 32 ? 2 : 4, 4};
+  if (N * K >= (1 << 22)) {
+    if (!kn) t.nt = N >= 8 * 4 * (t.mt == 4 ? 110 : 148 * 2) ? 4 : N >= 8 * 2 * 148 ? 2 : 1;
+    return t;
+  }
+  if (kn) {
+    while (t.mt > 1 && blocks(t.mt, 4) < 100) t.mt /= 2;
+    return t;
+  }
+  t.mt = 1;
+  while (t.nt > 1 && blocks(1, t.nt) < 100) t.nt /= 2;
+  if (K > 64 && blocks(1, 4) >= 148 * 4) t.mt = blocks(2, 4) >= 148 * 6 ? 4 : 2;
+  return t;
+}
+
+cudaError_t launch_skinny_tile(SkinnyTile t, const GemmParams &p, const int8_t *a, const int8_t *b, bool vec, int need, cudaStream_t s,
+                               const ConvGeom *conv) {
+#define GLOWB200_SKINNY(MT)                                                                            \
+  (t.nt == 1 ? launch_skinny<MT, 1, false>(p, a, b, vec, need, s, conv)                                \
+             : t.nt == 2 ? launch_skinny<MT, 2, false>(p, a, b, vec, need, s, conv) : launch_skinny<MT, 4, false>(p, a, b, vec, need, s, conv))
+  return t.mt == 1 ? GLOWB200_SKINNY(1) : t.mt == 2 ? GLOWB200_SKINNY(2) : GLOWB200_SKINNY(4);
+#undef GLOWB200_SKINNY
 }
 
 }  // namespace
@@ -400,18 +433,13 @@ int run_gemm_skinny(GemmParams p, const int8_t *a, const int8_t *b, bool b_is_kn
   if (p.k_corr == 0) p.k_corr = p.K;
   const int need = b_offsets_zero ? 0 : 1;
   const bool vec = (p.K % 16) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
-  const int mt = p.M <= 16 ? 1 : p.M <= 32 ? 2 : 4;
+  const SkinnyTile t = skinny_tile(p.M, p.N, p.k_corr, b_is_kn);
   cudaError_t e;
   if (b_is_kn) {
-    e = mt == 1 ? launch_skinny<1, 4, true>(p, a, b, false, need, s) : mt == 2 ? launch_skinny<2, 4, true>(p, a, b, false, need, s)
-                                                                               : launch_skinny<4, 4, true>(p, a, b, false, need, s);
+    e = t.mt == 1 ? launch_skinny<1, 4, true>(p, a, b, false, need, s) : t.mt == 2 ? launch_skinny<2, 4, true>(p, a, b, false, need, s)
+                                                                                 : launch_skinny<4, 4, true>(p, a, b, false, need, s);
   } else {
-    // wider tiles once narrow ones fill the SMs: the rows of the left operand are read once per block
-    const int nt = p.N >= 8 * 4 * (mt == 4 ? 110 : 148 * 2) ? 4 : p.N >= 8 * 2 * 148 ? 2 : 1;
-#define GLOWB200_SKINNY(MT) (nt == 1 ? launch_skinny<MT, 1, false>(p, a, b, vec, need, s) \
-                           : nt == 2 ? launch_skinny<MT, 2, false>(p, a, b, vec, need, s) : launch_skinny<MT, 4, false>(p, a, b, vec, need, s))
-    e = mt == 1 ? GLOWB200_SKINNY(1) : mt == 2 ? GLOWB200_SKINNY(2) : GLOWB200_SKINNY(4);
-#undef GLOWB200_SKINNY
+    e = launch_skinny_tile(t, p, a, b, vec, need, s, nullptr);
   }
   if (e != cudaSuccess) return set_error(GLOWB200_ERR_CUDA, "few-row contraction launch failed: %s", cudaGetErrorString(e));
   return GLOWB200_OK;
@@ -429,13 +457,7 @@ int run_conv_skinny(GemmParams p, const int8_t *in, const int8_t *filter, const 
   p.N = g.OC;
   p.K = p.k_corr = g.KH * g.KW * g.C;
   const int need = b_offsets_zero ? 0 : 1;
-  // row tiles of 64, smaller ones where those would leave SMs idle
-  const int cols = (p.N + 7) / 8;
-  int mt = 4;
-  while (mt > 1 && (int64_t)((p.M + 16 * mt - 1) / (16 * mt)) * cols < sm_count()) mt /= 2;
-  const cudaError_t e = mt == 4 ? launch_skinny<4, 1, false>(p, in, filter, true, need, s, &g)
-                        : mt == 2 ? launch_skinny<2, 1, false>(p, in, filter, true, need, s, &g)
-                                  : launch_skinny<1, 1, false>(p, in, filter, true, need, s, &g);
+  const cudaError_t e = launch_skinny_tile(skinny_tile(p.M, p.N, p.K, false), p, in, filter, true, need, s, &g);
   if (e != cudaSuccess) return set_error(GLOWB200_ERR_CUDA, "small convolution launch failed: %s", cudaGetErrorString(e));
   return GLOWB200_OK;
 }
