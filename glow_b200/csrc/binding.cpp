@@ -459,7 +459,7 @@ PyObject *pool(PyObject *const *a) {
   return given ? same(a[5]) : give(out);
 }
 
-// src, shuffle, scale, offset
+// src, shuffle, scale, offset, out
 PyObject *quantize_transpose(PyObject *const *a) {
   const Tensor &x = cuda_tensor(a[0], "src", F32);
   PyObject *seq = PySequence_Fast(a[1], "shuffle");
@@ -480,10 +480,11 @@ PyObject *quantize_transpose(PyObject *const *a) {
     PyErr_SetString(PyExc_IndexError, "shuffle does not fit the tensor's dimensions");
     throw Raised{};
   }
-  const Tensor out = empty(c10::IntArrayRef(od, (size_t)n), at::kChar, x);
+  const bool given = a[4] != Py_None;
+  const Tensor out = given ? cuda_tensor(a[4], "out", bit(at::kChar)) : empty(c10::IntArrayRef(od, (size_t)n), at::kChar, x);
   invoke(fn.glowb200_quantize_transpose_i8, (int8_t *)out.data_ptr(), (const float *)x.data_ptr(), dims, sh, n, real(a[2]),
       (int32_t)integer(a[3]), stream());
-  return give(out);
+  return given ? same(a[4]) : give(out);
 }
 
 // dense, pooled, quantize?, scale, offset, out
@@ -592,7 +593,7 @@ PyMethodDef methods[] = {
     FAST("dequantize", element_convert<false>, 4),
     FAST("max_pool", pool<false>, 6),
     FAST("avg_pool", pool<true>, 9),
-    FAST("quantize_transpose", quantize_transpose, 4),
+    FAST("quantize_transpose", quantize_transpose, 5),
     FAST("pairwise_dot", pairwise_dot, 6),
     FAST("run_function", run_function, 4),
     {nullptr, nullptr, 0, nullptr}};

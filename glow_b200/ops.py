@@ -590,9 +590,9 @@ class programmatic_launch:
         return False
 
 
-def quantize_transpose_i8(src, shuffle, scale, offset):
+def quantize_transpose_i8(src, shuffle, scale, offset, out=None):
     """transpose(quantize(src)) in one pass: fp32 in, int8 out with dims[i] = src dims[shuffle[i]]."""
-    return _native().quantize_transpose(src, shuffle, scale, offset)
+    return _native().quantize_transpose(src, shuffle, scale, offset, out)
 
 
 def pairwise_dot_interaction(dense, pooled, *, quant=None, out=None):

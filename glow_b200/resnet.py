@@ -17,6 +17,7 @@ Harness code: builds the network description and drives glow_b200.ops (the tests
 description through the CPU checker).
 """
 import math
+import threading
 
 import numpy as np
 import torch
@@ -187,6 +188,8 @@ class ResNet50Int8:
         self.status = ops.new_status(self.dev)
         self.ws = None
         self.launches = 0
+        self._lock = threading.Lock()
+        self._seen, self._replay = None, None
 
     def _workspace(self, nbytes):
         if self.ws is None or self.ws.numel() < nbytes:
@@ -208,14 +211,62 @@ class ResNet50Int8:
                                                 flags=ops.FC_WEIGHT_OFFSETS_ZERO, workspace=self._workspace(need),
                                                 status=self.status)
 
+    # Images up to which the layers between Quantize and the FC are replayed from a CUDA graph (from the second
+    # call of a shape on): their 73 launches cost the host 4 us each, which is more than the device needs for
+    # them below about 20 images of 224 x 224 (one image: 480 us from the host, 300 replayed).
+    REPLAY_PIXELS = 20 * 224 * 224
+
     def forward(self, x_nchw):
         """x_nchw: fp32 [N,3,H,W] on the device -> fp32 logits [N, classes]."""
-        tqp = self.q["tqp"]
-        self.launches = 0
+        n, _, h, w = shape = tuple(x_nchw.shape)
+        with self._lock:
+            self.launches = 0
+            if n * h * w > self.REPLAY_PIXELS or torch.cuda.is_current_stream_capturing():
+                return self._head(self._features(self._quantize(x_nchw)))
+            r = self._replay
+            if r is None or r["shape"] != shape:
+                if self._seen != shape:
+                    self._seen = shape
+                    return self._head(self._features(self._quantize(x_nchw)))
+                r = self._replay = self._capture(shape)   # the one graph kept: that of the last shape called twice
+            stream = torch.cuda.current_stream()
+            if stream != r["stream"]:   # its buffers are read by the last replay, on another stream
+                stream.wait_event(r["event"])
+                r["stream"] = stream
+            self._quantize(x_nchw, r["input"])
+            r["graph"].replay()
+            self.launches += r["launches"]
+            out = self._head(r["features"])
+            r["event"].record(stream)
+            return out
+
+    def _capture(self, shape):
+        n, c, h, w = shape
+        stream, side = torch.cuda.current_stream(), torch.cuda.Stream()
+        r = {"shape": shape, "graph": torch.cuda.CUDAGraph(), "stream": stream, "event": torch.cuda.Event(), "ws": self.ws,  # the workspace of the first call
+             "input": torch.empty((n, h, w, c), dtype=torch.int8, device=self.dev)}
+        before = self._replay
+        if before is not None:
+            before["event"].synchronize()   # its memory goes with it
+        side.wait_stream(stream)
+        with torch.cuda.stream(side):
+            r["graph"].capture_begin(capture_error_mode="thread_local")
+            try:
+                r["features"] = self._features(r["input"])
+            finally:
+                r["graph"].capture_end()
+        r["launches"], self.launches = self.launches, 0
+        return r
+
+    def _quantize(self, x_nchw, out=None):
         # Quantize, then Transpose: the order Glow's optimizer leaves (it sinks a Transpose below the
         # Quantize that consumes it, GraphOptimizer.cpp:1076-1086) -- the layout change moves bytes, not floats
-        x = ops.quantize_transpose_i8(x_nchw, (0, 2, 3, 1), *tqp["input"])   # one kernel for the pair
         self.launches += 1
+        return ops.quantize_transpose_i8(x_nchw, (0, 2, 3, 1), *self.q["tqp"]["input"], out=out)   # one kernel for the pair
+
+    def _features(self, x):
+        """int8 NHWC images -> the pooled int8 features."""
+        tqp = self.q["tqp"]
         for l in self.layers:
             if l[0] == "conv":
                 x = self._conv(l[1]["name"], x)
@@ -238,17 +289,18 @@ class ResNet50Int8:
                 tr = ops.quantize_scale_offset_32to8(np.float32(tqp[src][0]) / np.float32(tqp["avgpool"][0]) / np.float32(hw * hw))
                 x = ops.avg_pool_i8(x, (hw, hw), (1, 1), (0, 0, 0, 0), True, tqp["avgpool"][1], tqp[src][1], tr)
                 self.launches += 1
-            elif l[0] == "fc":
-                f = self.fc
-                x2 = x.reshape(x.shape[0], -1)
-                y = ops.rowwise_quantized_fc(x2, f["w"], f["bias"], f["w_off"], f["params"][:3], f["params"][3:], tqp["fc"][1],
-                                             tqp[self.q["fc"]["in_name"]][1], 0, weights_row_sums=f["row_sums"],
-                                             workspace=self._workspace(ops.i8_gemm_workspace_bytes(x2.shape[0], x2.shape[1], f["w"].shape[0])),
-                                             status=self.status)
-                self.logits_q = y
-                x = ops.element_dequantize_i8(y, *tqp["fc"])
-                self.launches += 3
         return x
+
+    def _head(self, x):
+        """Pooled features -> fp32 logits: the FC and the Dequantize."""
+        tqp, f = self.q["tqp"], self.fc
+        x2 = x.reshape(x.shape[0], -1)
+        self.logits_q = ops.rowwise_quantized_fc(
+            x2, f["w"], f["bias"], f["w_off"], f["params"][:3], f["params"][3:], tqp["fc"][1], tqp[self.q["fc"]["in_name"]][1], 0,
+            weights_row_sums=f["row_sums"], workspace=self._workspace(ops.i8_gemm_workspace_bytes(x2.shape[0], x2.shape[1], f["w"].shape[0])),
+            status=self.status)
+        self.launches += 3
+        return ops.element_dequantize_i8(self.logits_q, *tqp["fc"])
 
 
 def conv_ops_per_image(layers, hw=224):

@@ -128,3 +128,27 @@ def test_programmatic_launches_do_not_change_results(net):
         torch.cuda.synchronize()
         assert torch.equal(captured, plain)
     assert int(model.status.item()) == 0
+
+
+@pytest.mark.parametrize("shapes", [((1, 3, 64, 64),) * 4, ((2, 3, 64, 64), (3, 3, 96, 96), (3, 3, 96, 96), (2, 3, 64, 64), (2, 3, 64, 64))])
+def test_replayed_forward_equals_the_launches(net, shapes):
+    """From the second call of a shape on the layers are replayed from a graph: other images, other
+    streams and other shapes in between give what the launches give, and results stay the caller's."""
+    layers, w, q = net
+    model, plain = resnet.ResNet50Int8(layers, q, DEV), resnet.ResNet50Int8(layers, q, DEV)
+    plain.REPLAY_PIXELS = 0
+    g = torch.Generator(device=DEV).manual_seed(9)
+    xs = [torch.randn(s, device=DEV, generator=g) for s in shapes]
+    want = [plain.forward(x) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got, quantized = [], []
+    for x, s in zip(xs, streams):
+        with torch.cuda.stream(s):
+            got.append(model.forward(x))
+            quantized.append(model.logits_q)
+    torch.cuda.synchronize()
+    assert model.launches == plain.launches and int(model.status.item()) == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert len({t.data_ptr() for t in quantized}) == len(xs)
