@@ -310,6 +310,12 @@ __device__ __forceinline__ int stage_offset(int r, int q16) {
   return r * PITCH + 16 * (q16 ^ x);
 }
 
+// x / d for 0 <= x < 2^31 with reciprocal = floor((2^32 - 1) / d): the estimate is the quotient or one less.
+__device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
+  const int q = (int)__umulhi((uint32_t)x, reciprocal);
+  return q + (x - q * d >= d ? 1 : 0);
+}
+
 // Optional tracing for tuning builds (python -m glow_b200.build -DGLOWB200_GEMM_TRACE): every CTA
 // stamps %globaltimer (ns) at entry and exit -- entries 2b and 2b + 1 of a device buffer -- and
 // CTA 0 its clock64 at the same two points (entries 510, 511), from which the SM clock a launch really
@@ -340,10 +346,13 @@ struct GemmSmem {
   static constexpr int kBBytes = (PAIR ? BLOCK_N / 2 : BLOCK_N) * kBlockK;  // a pair's CTAs hold half of the rows each
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kTileBytes = STAGES * kStageBytes;
-  static constexpr int kColBytes = BLOCK_N * (int)sizeof(ColParams);
-  // The int8 result of a tile on its way out: 128 rows of kOutPitch bytes, then the output row of each.
-  static constexpr int kOutPitch = BLOCK_N <= 32 ? 32 : BLOCK_N <= 64 ? 64 : BLOCK_N <= 128 ? 128 : 256;
-  static constexpr int kOutBytes = kBlockM * kOutPitch + kBlockM * 4;
+  static constexpr int kColBytes = BLOCK_N * (int)(sizeof(ColParams) + 4);  // the records, then the rounding terms
+  // The int8 result of a tile on its way out.  Each epilogue warp has a piece of 32 rows x kWarpCols bytes
+  // of its own (ragged rows: 128 rows of kOutPitch bytes instead, then the output row of each).
+  static constexpr int kOutPitch = BLOCK_N <= 64 ? 64 : BLOCK_N <= 128 ? 128 : 256;
+  static constexpr int kWarpCols = BLOCK_N <= 128 ? 32 : 64;
+  static constexpr int kOutBytes = kEpilogueWarps * 32 * kWarpCols + kBlockM * 4;
+  static_assert(kOutBytes >= kBlockM * kOutPitch + kBlockM * 4, "the ragged rows' staging area fits as well");
   static constexpr int kTotal = kTileBytes + kColBytes + kOutBytes + 256 /*barriers*/ + 1024 /*alignment slack*/;
   static_assert(kTotal <= 232448, "more shared memory than a CTA can have");
 };
@@ -355,9 +364,9 @@ struct GemmSmem {
 // MODE 0: no input row sums take part (every weight offset is 0), the activation is none or Relu and
 // the rows of the result are whole 16-byte pieces -- the common case, whose drain has neither the
 // row-sum term, nor the activation switch, nor the stores of ragged rows;
-// MODE 1: everything else with an int8 result; MODE 2: the floating-point result of the
-// dynamically quantized layers (GemmParams::float_out).  One drain body per kernel keeps the
-// register allocation inside the 96 registers a 576-thread CTA leaves.
+// MODE 1: every other int8 result in whole 16-byte pieces; MODE 3: int8 results in ragged rows;
+// MODE 2: the floating-point result of the dynamically quantized layers (GemmParams::float_out).
+// One drain body per kernel keeps the register allocation inside the 96 registers a 576-thread CTA leaves.
 // PAIR: the grid is clusters of two CTAs and a tile is 256 rows -- 128 per CTA, whose tensor core
 // reads its own rows of the left operand and HALF of the right operand's rows from its own shared
 // memory and the other half from its partner's (tcgen05.mma.cta_group::2, issued by the even CTA
@@ -379,7 +388,13 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   ColParams *cols = reinterpret_cast<ColParams *>(smem + S::kTileBytes);
   uint8_t *out_stage = smem + S::kTileBytes + S::kColBytes;
-  int32_t *out_rows = reinterpret_cast<int32_t *>(out_stage + kBlockM * S::kOutPitch);
+  [[maybe_unused]] int32_t *out_rows = reinterpret_cast<int32_t *>(out_stage + kBlockM * S::kOutPitch);
+  int32_t *col_rounding = reinterpret_cast<int32_t *>(smem + S::kTileBytes + BLOCK_N * sizeof(ColParams));
+  // MODE 0, 1: every epilogue warp carries its own rows and columns from tensor memory to the result with no
+  // barrier on the way.  Tiles of 64 columns alternate between two halves of the warps (32 columns each: whole
+  // 32-byte sectors), the others are split between all of them.
+  constexpr bool kOwnRows = MODE == 0 || MODE == 1;
+  constexpr bool kAlternate = kOwnRows && BLOCK_N <= 64;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::kTileBytes + S::kColBytes + S::kOutBytes);
   uint64_t *empty = full + STAGES;
   uint64_t *acc_full = empty + STAGES;   // [2]
@@ -403,7 +418,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], (PAIR ? 2 : 1) * kEpilogueWarps);  // one arrival per epilogue warp (of both CTAs)
+      mbar_init(&acc_empty[b], (PAIR ? 2 : 1) * kEpilogueWarps / (kAlternate ? 2 : 1));  // one per warp that drains it (of both CTAs)
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -522,8 +537,10 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     // columns drained from tensor memory per step: 16 keeps the drain loop inside the 96 registers
     // a 576-thread CTA leaves
     constexpr int kChunk = 16;
-    const bool vec_ok = ((p.N & 15) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+    const uint32_t image_div = p.conv_hpwp > 0 ? 0xffffffffu / (uint32_t)p.conv_hpwp : 0u;
+    const uint32_t line_div = p.conv_wp > 0 ? 0xffffffffu / (uint32_t)p.conv_wp : 0u;
     int lt = 0;
+    bool dead = false;
     int cols_n0 = -1;  // column block the records in shared memory belong to
     const uint32_t leader_acc_empty[2] = {PAIR ? map_to_cta(&acc_empty[0], 0) : 0u, PAIR ? map_to_cta(&acc_empty[1], 0) : 0u};
     for (int t = walker; t < tiles; t += walkers, lt++) {
@@ -539,6 +556,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         static_assert(BLOCK_N <= kEpilogueThreads, "one column record per epilogue thread");
         const int j = n0 + et;
         ColParams cp = {0, 0, 0, 0};
+        [[maybe_unused]] int32_t rounding = 0;
         if (et < BLOCK_N && j < p.N) {
           if constexpr (MODE == 2) {  // {unused, column scale, float bias, weight offset}
             cp.scale = __float_as_int(p.col_scales ? p.col_scales[j] : p.u_col_scale);
@@ -556,36 +574,55 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                                   (uint32_t)p.k_corr * (uint32_t)p.a_offset * (uint32_t)q.b_off;
             cp.c = (int32_t)corr;
             cp.scale = q.out_scale;
-            cp.shifts = q.out_pre | (q.out_post << 8);
-            cp.b_off = q.b_off;
+            if constexpr (MODE == 0) {  // nothing to unpack: {c, scale, pre, post}
+              cp.shifts = q.out_pre;
+              cp.b_off = q.out_post;
+            } else {
+              cp.shifts = q.out_pre | (q.out_post << 8);
+              cp.b_off = q.b_off;
+            }
+            rounding = (int32_t)((1u << q.out_post) >> 1);
           }
         }
-        if (et < BLOCK_N) cols[et] = cp;
+        if (et < BLOCK_N) {
+          cols[et] = cp;
+          if constexpr (kOwnRows) col_rounding[et] = rounding;
+        }
         asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");  // epilogue warps only
       }
       // (2) drain the accumulators of this tile
+      if constexpr (kAlternate) {
+        if ((col_group >> 1) != buf) continue;
+      }
       const int row = m0 + quarter * 32 + lane;
-      // All epilogue threads agree on the outcome of the (bounded) wait through a reducing
-      // barrier, so either all of them drain the tile or all of them leave the loop.
-      const uint32_t mine = mbar_wait(&acc_full[buf], (lt >> 1) & 1, abort_flag) ? 1u : 0u;
-      uint32_t ok;
-      asm volatile(
-          "{\n\t.reg .pred p, q;\n\t"
-          "setp.ne.u32 q, %1, 0;\n\t"
-          "barrier.cta.red.and.pred p, 1, %2, q;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(ok)
-          : "r"(mine), "n"(kEpilogueThreads)
-          : "memory");
+      const uint32_t mine = !dead && mbar_wait(&acc_full[buf], (lt >> 1) & 1, abort_flag) ? 1u : 0u;
+      if constexpr (kOwnRows) {
+        // A warp whose (bounded) wait gave up drains nothing any more, but walks on: the barriers around the
+        // column records count every epilogue warp.
+        dead = !__all_sync(0xffffffffu, mine);
+        if (dead) continue;
+      } else {
+        // All epilogue threads agree on the outcome of the (bounded) wait through a reducing
+        // barrier, so either all of them drain the tile or all of them leave the loop.
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.u32 q, %1, 0;\n\t"
+            "barrier.cta.red.and.pred p, 1, %2, q;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(mine), "n"(kEpilogueThreads)
+            : "memory");
+        if (!ok) break;
+      }
       tc_fence_after();
-      if (!ok) break;
       GEMM_TRACE(4, lt == 0 && et == 0);
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * kAccCols;
       int out_index = row;  // row of the result this accumulator row becomes
       bool row_ok = row < p.M;
       if (p.conv_entries > 0 || p.conv_windows) {  // padded pixel -> (image, oh, ow); the halo rows are dropped
-        const int img = row / p.conv_hpwp, rem = row - img * p.conv_hpwp;
-        const int oh = rem / p.conv_wp, ow = rem - oh * p.conv_wp;
+        const int img = fast_div(row, p.conv_hpwp, image_div), rem = row - img * p.conv_hpwp;
+        const int oh = fast_div(rem, p.conv_wp, line_div), ow = rem - oh * p.conv_wp;
         row_ok = row_ok && oh < p.conv_oh && ow < p.conv_ow;
         out_index = (img * p.conv_oh + oh) * p.conv_ow + ow;
       }
@@ -645,28 +682,107 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
           }
         }
-      } else {
-        // The int8 result.  A column's record is 16 bytes, and shared memory delivers 128 bytes
-        // per clock per SM whether the lanes of a load read one address or 32: with one accumulator
-        // row per lane (the 32x32b shape) every element costs a 16-byte broadcast load, 4096 clocks
-        // for a 128 x 256 tile and, measured, the whole duration of its drain.  The 16x256b shape
-        // hands each lane two neighbouring columns of four rows per eight columns instead -- register
-        // i of the load of rows 16h..16h+15 holds row 16h + lane/4 + 8*((i>>1)&1), column
-        // 8*(i>>2) + 2*(lane%4) + (i&1) -- so a record is loaded once per four elements.
-        // A lane then owns two bytes of a row, and a warp's stores would be scattered over 32
-        // lines either way (16-byte stores by row took 6500 clocks per 128 x 256 tile): the tile
-        // passes through shared memory, swizzled in 16-byte pieces so that neither the writes nor
-        // the reads along rows meet in a bank, and leaves as whole rows.
-        const int jq = lane & 3, r0 = lane >> 2;
-        uint8_t *stage_q = out_stage + quarter * 32 * S::kOutPitch;
-        int32_t a_sums[4] = {0, 0, 0, 0};
+      } else if constexpr (kOwnRows) {
+        // The int8 result.  The 16x256b shape hands a lane two neighbouring columns of four rows per eight
+        // columns -- register i of the load of rows 16h..16h+15 holds row 16h + lane/4 + 8*((i>>1)&1), column
+        // 8*(i>>2) + 2*(lane%4) + (i&1) -- so a column's 16-byte record is loaded once per four elements.  (With
+        // a row per lane, the 32x32b shape, each element costs a 16-byte broadcast: 4096 clocks for a
+        // 128 x 256 tile.)  The two bytes a lane has of each of two column groups make one 32-bit word, and four
+        // of these, one per eight rows, are what stmatrix spreads over 32 rows of 16 bytes; a row's 16 bytes then
+        // hold its column pairs in the order 0 4 1 5 2 6 3 7, which four byte permutes undo when they leave.
+        // What bounds it is the ALU: two shifts, an add-and-maximum and half a pack per element, little else
+        // being left.  Byte-pair stores into a tile that four warps shared, with their addresses and two barriers
+        // per tile, took 14 instructions per element: 200,704 x 64 x 256 ran 38.6 us, now 31.2; the stem's
+        // 64-column tiles 65, now 49.6.
+        constexpr int kCols = S::kWarpCols, kPieces = kCols / 16;
+        const int first = (kAlternate ? col_group & 1 : col_group) * kCols;
+        const int last = first + kCols < BLOCK_N ? first + kCols : BLOCK_N;
+        const int jq = lane & 3;
+        uint8_t *stage = out_stage + (warp - 2) * 32 * kCols;
+        const int dst_row = row_ok ? out_index : -1;
+        [[maybe_unused]] int32_t a_sums[4] = {0, 0, 0, 0};
         if constexpr (MODE == 1) {
           if (p.a_row_sums) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-              const int rr = m0 + quarter * 32 + 8 * i + r0;
+              const int rr = m0 + quarter * 32 + 8 * i + (lane >> 2);
               a_sums[i] = rr < p.M ? p.a_row_sums[rr] : 0;
             }
+          }
+        }
+        const int32_t relu_floor = p.act_type == 1 ? p.out_offset : INT32_MIN;
+#pragma unroll 1
+        for (int c0 = first; c0 < last; c0 += 16) {
+          uint32_t acc[16];  // [row half h][column group g][row rr][column cc] -> 8h + 4g + 2rr + cc
+          tmem_ld_16x256b_x2(lane_addr + (uint32_t)c0, &acc[0]);
+          tmem_ld_16x256b_x2(lane_addr + (16u << 16) + (uint32_t)c0, &acc[8]);
+          tmem_ld_wait();
+          if (c0 + 16 >= last) {
+            // everything this warp needs from the buffer is in registers: hand it back
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if constexpr (PAIR) mbar_arrive_cluster(leader_acc_empty[buf]);
+              else mbar_arrive(&acc_empty[buf]);
+            }
+          }
+          // the requantisation: libjit_scale, ((v >> pre) * scale + rtn) >> post, then + offset, with
+          // rtn = 1 << (post - 1) (0 for post 0); Relu is max(x, out_offset), no activation max(x, INT_MIN)
+          uint32_t word[4] = {0u, 0u, 0u, 0u};  // of row 8i + lane/4: {group 0, group 1} x two columns
+#pragma unroll
+          for (int g = 1; g >= 0; g--) {
+            int32_t res[2][4];  // [cc][i]
+            const int2 rtn = *reinterpret_cast<const int2 *>(&col_rounding[c0 + 8 * g + 2 * jq]);
+#pragma unroll
+            for (int cc = 0; cc < 2; cc++) {
+              const int4 cp = *reinterpret_cast<const int4 *>(&cols[c0 + 8 * g + 2 * jq + cc]);
+              const int32_t pre = MODE == 0 ? cp.z : cp.z & 0xff, post = MODE == 0 ? cp.w : cp.z >> 8;
+#pragma unroll
+              for (int i = 0; i < 4; i++) {  // i = 2h + rr
+                uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)cp.x;
+                if constexpr (MODE == 1) v -= (uint32_t)cp.w * (uint32_t)a_sums[i];  // 0 when no row sums take part
+                const int32_t m = (int32_t)((uint32_t)((int32_t)v >> pre) * (uint32_t)cp.y + (uint32_t)(cc ? rtn.y : rtn.x));
+                // max((m >> post) + offset, floor) in one instruction (a wrapping add, like the two it replaces)
+                int32_t x = __viaddmax_s32(m >> post, p.out_offset, relu_floor);
+                if constexpr (MODE == 1) {
+                  if (p.act_type > 1) x = activation_i32(x, p);
+                }
+                res[cc][i] = x;
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)  // sat8 of both columns (libjit_clip_i8) below the other group's two
+              asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(word[i]) : "r"(res[1][i]), "r"(res[0][i]), "r"(word[i]));
+          }
+          asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(
+                           smem_u32(stage + stage_offset<kCols>(lane, (c0 - first) >> 4))),
+                       "r"(word[0]), "r"(word[1]), "r"(word[2]), "r"(word[3])
+                       : "memory");
+        }
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < kPieces; it++) {
+          const int r = it * (32 / kPieces) + lane / kPieces, q16 = lane % kPieces;
+          const int dst = __shfl_sync(0xffffffffu, dst_row, r);
+          const uint4 w = *reinterpret_cast<const uint4 *>(stage + stage_offset<kCols>(r, q16));
+          const uint4 o = make_uint4(__byte_perm(w.x, w.y, 0x5410), __byte_perm(w.z, w.w, 0x5410),
+                                     __byte_perm(w.x, w.y, 0x7632), __byte_perm(w.z, w.w, 0x7632));
+          const int col = first + 16 * q16;
+          if (dst >= 0 && col < last && n0 + col < p.N) *reinterpret_cast<uint4 *>(p.out + (size_t)dst * p.N + n0 + col) = o;
+        }
+        __syncwarp();  // read back before the next tile's pieces arrive
+      } else {
+        // The int8 result in ragged rows (N not a multiple of 16, or an unaligned result): the same loads, but
+        // the whole tile passes through shared memory, swizzled in 16-byte pieces so that neither the writes
+        // nor the reads along rows meet in a bank, and leaves in words across the warps' columns.
+        const int jq = lane & 3, r0 = lane >> 2;
+        uint8_t *stage_q = out_stage + quarter * 32 * S::kOutPitch;
+        int32_t a_sums[4] = {0, 0, 0, 0};
+        if (p.a_row_sums) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const int rr = m0 + quarter * 32 + 8 * i + r0;
+            a_sums[i] = rr < p.M ? p.a_row_sums[rr] : 0;
           }
         }
         const int32_t relu_floor = p.act_type == 1 ? p.out_offset : INT32_MIN;
@@ -700,13 +816,11 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
               for (int i = 0; i < 4; i++) {  // i = 2h + rr
                 uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)cp.x;
-                if constexpr (MODE == 1) v -= (uint32_t)cp.w * (uint32_t)a_sums[i];  // 0 when no row sums take part
+                v -= (uint32_t)cp.w * (uint32_t)a_sums[i];  // 0 when no row sums take part
                 const int32_t m = (int32_t)((uint32_t)((int32_t)v >> pre) * (uint32_t)cp.y + rtn);
                 // max((m >> post) + offset, floor) in one instruction (a wrapping add, like the two it replaces)
                 int32_t x = __viaddmax_s32(m >> post, p.out_offset, relu_floor);
-                if constexpr (MODE == 1) {
-                  if (p.act_type > 1) x = activation_i32(x, p);
-                }
+                if (p.act_type > 1) x = activation_i32(x, p);
                 res[cc][i] = x;
               }
             }
@@ -720,47 +834,35 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           }
           GEMM_TRACE(9, lt == 0 && et == 0 && c0 == 0);
         }
-        constexpr int kRowPieces = S::kOutPitch / 16;
         if (col_group == 0) out_rows[quarter * 32 + lane] = row_ok ? out_index : -1;
         asm volatile("bar.sync %0, 128;" ::"r"(2 + quarter) : "memory");  // the quarter's 32 rows are complete
-        if (MODE == 0 || vec_ok) {
-#pragma unroll
-          for (int piece = col_group * 32 + lane; piece < 32 * kRowPieces; piece += 128) {
-            const int r = piece / kRowPieces, q16 = piece % kRowPieces;
-            const int dst = out_rows[quarter * 32 + r];
-            if (q16 * 16 >= BLOCK_N || n0 + q16 * 16 >= p.N || dst < 0) continue;
-            *reinterpret_cast<uint4 *>(p.out + (size_t)dst * p.N + n0 + q16 * 16) =
-                *reinterpret_cast<const uint4 *>(stage_q + stage_offset<S::kOutPitch>(r, q16));
-          }
-        } else {
-          // Rows that start anywhere (N not a multiple of 16): the lanes of a warp
-          // write consecutive aligned words of a row, each put together from two staged words; the
-          // bytes at a row's two ends go one by one.  (Byte stores for the whole tile took
-          // 2000 x 30 x 1000 to 21.5 us.)
-          constexpr int kRowWords = BLOCK_N / 4 + 1;
-          const int len = p.N - n0 < BLOCK_N ? p.N - n0 : BLOCK_N;
-          auto staged = [&](int r, int word) -> uint32_t {
-            return *reinterpret_cast<const uint32_t *>(stage_q + stage_offset<S::kOutPitch>(r, word >> 2) + 4 * (word & 3));
-          };
+        // Rows that start anywhere (N not a multiple of 16): the lanes of a warp
+        // write consecutive aligned words of a row, each put together from two staged words; the
+        // bytes at a row's two ends go one by one.  (Byte stores for the whole tile took
+        // 2000 x 30 x 1000 to 21.5 us.)
+        constexpr int kRowWords = BLOCK_N / 4 + 1;
+        const int len = p.N - n0 < BLOCK_N ? p.N - n0 : BLOCK_N;
+        auto staged = [&](int r, int word) -> uint32_t {
+          return *reinterpret_cast<const uint32_t *>(stage_q + stage_offset<S::kOutPitch>(r, word >> 2) + 4 * (word & 3));
+        };
 #pragma unroll 1
-          for (int item = col_group * 32 + lane; item < 32 * kRowWords; item += 128) {
-            const int r = item / kRowWords;
-            const int dst = out_rows[quarter * 32 + r];
-            if (dst < 0) continue;
-            int8_t *o = p.out + (size_t)dst * p.N + n0;
-            const int sh = (int)(reinterpret_cast<uintptr_t>(o) & 3);
-            const int col = 4 * (item % kRowWords) - sh;  // of the word's first byte
-            if (col >= len) continue;
-            const int below = col < 0 ? -1 : col >> 2;    // the staged word that holds it
-            const uint32_t lo = below >= 0 ? staged(r, below) : 0u, hi = below + 1 < BLOCK_N / 4 ? staged(r, below + 1) : 0u;
-            const uint32_t v = __funnelshift_r(lo, hi, 8 * (col & 3));
-            if (col >= 0 && col + 4 <= len) {
-              *reinterpret_cast<uint32_t *>(o + col) = v;
-            } else {
+        for (int item = col_group * 32 + lane; item < 32 * kRowWords; item += 128) {
+          const int r = item / kRowWords;
+          const int dst = out_rows[quarter * 32 + r];
+          if (dst < 0) continue;
+          int8_t *o = p.out + (size_t)dst * p.N + n0;
+          const int sh = (int)(reinterpret_cast<uintptr_t>(o) & 3);
+          const int col = 4 * (item % kRowWords) - sh;  // of the word's first byte
+          if (col >= len) continue;
+          const int below = col < 0 ? -1 : col >> 2;    // the staged word that holds it
+          const uint32_t lo = below >= 0 ? staged(r, below) : 0u, hi = below + 1 < BLOCK_N / 4 ? staged(r, below + 1) : 0u;
+          const uint32_t v = __funnelshift_r(lo, hi, 8 * (col & 3));
+          if (col >= 0 && col + 4 <= len) {
+            *reinterpret_cast<uint32_t *>(o + col) = v;
+          } else {
 #pragma unroll
-              for (int b = 0; b < 4; b++)
-                if (col + b >= 0 && col + b < len) o[col + b] = (int8_t)((v >> (8 * b)) & 0xff);
-            }
+            for (int b = 0; b < 4; b++)
+              if (col + b >= 0 && col + b < len) o[col + b] = (int8_t)((v >> (8 * b)) & 0xff);
           }
         }
       }
@@ -892,9 +994,10 @@ int make_map(CUtensorMap *map, const void *base, int rows, int K, int box_rows, 
 
 bool ptr16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// MODE 0 of the tile kernel
-bool plain_drain(const GemmParams &p) {
-  return p.a_row_sums == nullptr && p.act_type <= 1 && (p.N & 15) == 0 && ptr16(p.out);
+// the tile kernel's MODE for an int8 result
+int int8_mode(const GemmParams &p) {
+  if ((p.N & 15) != 0 || !ptr16(p.out)) return 3;
+  return p.a_row_sums == nullptr && p.act_type <= 1 ? 0 : 1;
 }
 
 template <int BLOCK_N, int STAGES, int MODE>
@@ -930,8 +1033,10 @@ int &resident_pairs() {
 template <int BLOCK_N, int STAGES>
 int launch_pair_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmParams &p, cudaStream_t s) {
   using S = GemmSmem<BLOCK_N, STAGES, 1>;
-  const bool plain = plain_drain(p);
-  auto kernel = plain ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 0, 1> : i8_gemm_requant_kernel<BLOCK_N, STAGES, 1, 1>;
+  const int mode = int8_mode(p);
+  auto kernel = mode == 0   ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 0, 1>
+                : mode == 1 ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 1, 1>
+                            : i8_gemm_requant_kernel<BLOCK_N, STAGES, 3, 1>;
   GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
   const int tiles = ((p.N + BLOCK_N - 1) / BLOCK_N) * ((p.M + 2 * kBlockM - 1) / (2 * kBlockM));
   cudaLaunchConfig_t cfg = {};
@@ -963,8 +1068,11 @@ int launch_pair_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmP
 template <int BLOCK_N, int STAGES>
 int launch_tile_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmParams &p, cudaStream_t s) {
   if (p.float_out) return launch_tile_mode<BLOCK_N, STAGES, 2>(ma, mb, p, s);
-  if (plain_drain(p)) return launch_tile_mode<BLOCK_N, STAGES, 0>(ma, mb, p, s);
-  return launch_tile_mode<BLOCK_N, STAGES, 1>(ma, mb, p, s);
+  switch (int8_mode(p)) {
+    case 0: return launch_tile_mode<BLOCK_N, STAGES, 0>(ma, mb, p, s);
+    case 1: return launch_tile_mode<BLOCK_N, STAGES, 1>(ma, mb, p, s);
+    default: return launch_tile_mode<BLOCK_N, STAGES, 3>(ma, mb, p, s);
+  }
 }
 
 #ifndef GLOWB200_GEMM_TILE_240
