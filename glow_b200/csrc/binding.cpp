@@ -26,7 +26,8 @@ namespace {
   X(glowb200_embedding_bag_byte_rowwise_offsets) X(glowb200_int_nbit_split_embedding_bags)                            \
   X(glowb200_i8_gemm_workspace_bytes) X(glowb200_dynamic_fc_workspace_bytes) X(glowb200_rowwise_quantized_fc_i8_i32)  \
   X(glowb200_fc_i8_i32) X(glowb200_matmul_i8) X(glowb200_dynamic_rowwise_quantized_fc) X(glowb200_dynamic_quantized_fc) \
-  X(glowb200_conv2d_workspace_bytes) X(glowb200_channelwise_quantized_conv2d_i8_i32) X(glowb200_element_add_maxsplat_i8) \
+  X(glowb200_conv2d_workspace_bytes) X(glowb200_channelwise_quantized_conv2d_i8_i32) \
+  X(glowb200_channelwise_quantized_conv2d_add_i8) X(glowb200_element_add_maxsplat_i8) \
   X(glowb200_element_quantize_i8) X(glowb200_element_dequantize_i8) X(glowb200_max_pool_i8) X(glowb200_avg_pool_i8)    \
   X(glowb200_quantize_transpose_i8) X(glowb200_pairwise_dot_interaction) X(glowb200_device_manager_run_function_io)
 struct Entry {
@@ -368,6 +369,8 @@ int64_t conv_out(int64_t in, int64_t k, int64_t s, int64_t pads, int64_t d) {
 
 // inp, filt, bias, kernels, strides, pads, group, dilation, out offset, in offset, filter offsets, bias
 // offsets, bias triples, out triples, activation, its arguments, filter row sums, flags, out, workspace, status
+// [, residual, dest offset, lhs offset, residual offset, lhs triple, residual triple, splat]
+template <bool ADD>
 PyObject *channelwise_conv(PyObject *const *a) {
   const Tensor &x = cuda_tensor(a[0], "inp", I8), &f = cuda_tensor(a[1], "filt", I8);
   const Ints<2> k(a[3], "kernels"), s(a[4], "strides"), d(a[7], "dilation");
@@ -392,14 +395,22 @@ PyObject *channelwise_conv(PyObject *const *a) {
     Py_DECREF(seq);
     if (PyErr_Occurred()) throw Raised{};
   }
-  invoke(fn.glowb200_channelwise_quantized_conv2d_i8_i32, (int8_t *)out.data_ptr(), (const int8_t *)x.data_ptr(),
-      (const int8_t *)f.data_ptr(), (const int32_t *)address(a[2], "bias"), od, in,
-      fd, k.v, s.v, p.v, group, d.v, (int32_t)integer(a[8]), (int32_t)integer(a[9]), (const int32_t *)address(a[10],
-          "filter_offsets"),
-      (const int32_t *)address(a[11], "bias_offsets"), bt.p[0], bt.p[1], bt.p[2], ot.p[0], ot.p[1], ot.p[2],
-          (int32_t)integer(a[14]),
-      has_args ? act : nullptr, (const int32_t *)address(a[16], "filter_row_sums"), (int)integer(a[17]), ws.data(), ws.bytes(),
-      (int32_t *)address(a[20], "status"), stream());
+  auto with = [&](auto function, auto... add) {
+    invoke(function, (int8_t *)out.data_ptr(), (const int8_t *)x.data_ptr(), (const int8_t *)f.data_ptr(),
+           (const int32_t *)address(a[2], "bias"), od, in, fd, k.v, s.v, p.v, group, d.v, (int32_t)integer(a[8]),
+           (int32_t)integer(a[9]), (const int32_t *)address(a[10], "filter_offsets"), (const int32_t *)address(a[11], "bias_offsets"),
+           bt.p[0], bt.p[1], bt.p[2], ot.p[0], ot.p[1], ot.p[2], (int32_t)integer(a[14]), has_args ? act : nullptr,
+           (const int32_t *)address(a[16], "filter_row_sums"), (int)integer(a[17]), ws.data(), ws.bytes(),
+           (int32_t *)address(a[20], "status"), add..., stream());
+  };
+  if constexpr (ADD) {
+    const Ints<3> lt(a[25], "lhs_triple"), rt(a[26], "residual_triple");
+    with(fn.glowb200_channelwise_quantized_conv2d_add_i8, (const int8_t *)cuda_tensor(a[21], "residual", I8).data_ptr(),
+         (int32_t)integer(a[22]), (int32_t)integer(a[23]), (int32_t)integer(a[24]), (int32_t)lt.v[0], (int32_t)lt.v[1],
+         (int32_t)lt.v[2], (int32_t)rt.v[0], (int32_t)rt.v[1], (int32_t)rt.v[2], (int32_t)integer(a[27]));
+  } else {
+    with(fn.glowb200_channelwise_quantized_conv2d_i8_i32);
+  }
   return given ? same(a[18]) : give(out);
 }
 
@@ -587,7 +598,8 @@ PyMethodDef methods[] = {
     FAST("matmul", matmul, 10),
     FAST("dynamic_rowwise_fc", dynamic_fc<true>, 10),
     FAST("dynamic_fc", dynamic_fc<false>, 10),
-    FAST("channelwise_conv", channelwise_conv, 21),
+    FAST("channelwise_conv", channelwise_conv<false>, 21),
+    FAST("channelwise_conv_add", channelwise_conv<true>, 28),
     FAST("add_maxsplat", add_maxsplat, 9),
     FAST("quantize", element_convert<true>, 4),
     FAST("dequantize", element_convert<false>, 4),

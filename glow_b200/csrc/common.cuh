@@ -52,6 +52,43 @@ __host__ __device__ __forceinline__ int32_t scale32(int32_t input, int32_t pre, 
   return (int32_t)((uint32_t)(c >> post) + (uint32_t)offset);
 }
 
+// The quantized Add of two int8 values (scale32 of either side, the result's offset, clip, optionally max with
+// a constant) for parameters of the ordinary kind: no shift before the multiplication, a scale of 16 bits, and
+// nothing in 32-bit overflow.  A side then is one dot-product instruction -- byte * scale + constant, the byte
+// picked from its word -- and a shift, and the result's offset rides on the left constant: 3.5 ALU and 2
+// multiplier instructions per element where the formula as written took 10.8 and 4.9.
+struct AddQuant {
+  int32_t l_scale, l_const, l_post, r_scale, r_const, r_post, floor;
+};
+inline bool make_add_quant(AddQuant &q, int32_t dest_off, int32_t l_off, int32_t r_off, int32_t l_pre, int32_t l_post,
+                           int32_t l_scale, int32_t r_pre, int32_t r_post, int32_t r_scale, int32_t splat) {
+  auto off_ok = [](int32_t o) { return o >= -512 && o <= 512; };
+  auto side_ok = [](int32_t pre, int32_t post, int32_t scale) {
+    return pre == 0 && post >= 0 && post <= 20 && scale >= 0 && scale < (1 << 15);
+  };
+  if (!off_ok(dest_off) || !off_ok(l_off) || !off_ok(r_off) || !side_ok(l_pre, l_post, l_scale) || !side_ok(r_pre, r_post, r_scale))
+    return false;
+  // |byte * scale + constant| < 2^22 + 2^19 + 2^24 + 2^29
+  q = {l_scale, ((1 << l_post) >> 1) - l_off * l_scale + dest_off * (1 << l_post), l_post,
+       r_scale, ((1 << r_post) >> 1) - r_off * r_scale, r_post, splat};
+  return true;
+}
+#ifdef __CUDACC__
+// four elements: the bytes of two words
+__device__ __forceinline__ uint32_t add_quant_word(uint32_t l, uint32_t r, const AddQuant &q) {
+  auto one = [&](int32_t a, int32_t b) { return __viaddmax_s32(a >> q.l_post, b >> q.r_post, q.floor); };
+  const int lh = q.l_scale << 16, rh = q.r_scale << 16;
+  const int32_t e0 = one(__dp2a_lo(q.l_scale, (int)l, q.l_const), __dp2a_lo(q.r_scale, (int)r, q.r_const));
+  const int32_t e1 = one(__dp2a_lo(lh, (int)l, q.l_const), __dp2a_lo(rh, (int)r, q.r_const));
+  const int32_t e2 = one(__dp2a_hi(q.l_scale, (int)l, q.l_const), __dp2a_hi(q.r_scale, (int)r, q.r_const));
+  const int32_t e3 = one(__dp2a_hi(lh, (int)l, q.l_const), __dp2a_hi(rh, (int)r, q.r_const));
+  uint32_t w;
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(e3), "r"(e2), "r"(0));
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(e1), "r"(e0), "r"(w));
+  return w;
+}
+#endif
+
 // libjit_clip_i8 (libjit_defs.h:146-148).
 __host__ __device__ __forceinline__ int32_t clip_i8(int32_t v) {
   return v < -128 ? -128 : (v > 127 ? 127 : v);

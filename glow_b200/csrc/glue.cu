@@ -38,6 +38,15 @@ struct AddF {
   }
 };
 
+// The same by make_add_quant's constants, four elements at a time.  51 M elements: 35.1 us by the formula
+// (ALU-bound), 27.5 us so.
+struct AddQuantF {
+  AddQuant q;
+  __device__ __forceinline__ int32_t operator()(int32_t a, int32_t b) const {
+    return (int32_t)(int8_t)add_quant_word((uint32_t)a & 0xffu, (uint32_t)b & 0xffu, q);
+  }
+};
+
 // The other arithmetic mini-kernels of DEFINE_DATA_PARALLEL_KERNEL_QUANTIZED (libjit.cpp:1593-1603,
 // 1675-1682): both sides rescaled to the result's scale, then sub / max / min, offset, clip.
 // OP 1 sub, 2 max, 3 min.
@@ -104,6 +113,8 @@ __device__ __forceinline__ uint32_t map_word(uint32_t a, uint32_t b, const F &f)
   return o;
 }
 
+__device__ __forceinline__ uint32_t map_word(uint32_t a, uint32_t b, const AddQuantF &f) { return add_quant_word(a, b, f.q); }
+
 // dst[i] = f(lhs[i], rhs[i]) (rhs may be NULL: f ignores its second argument).  vec: all three
 // pointers are 16-byte aligned.
 template <typename F>
@@ -131,6 +142,14 @@ cudaError_t launch_map(int8_t *dst, const int8_t *lhs, const int8_t *rhs, int64_
   const int vec = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) & 15u) == 0;
   if (cudaError_t e = launch_pdl(map_i8_kernel<F>, grid_for(vec ? (n + 15) / 16 : n), kThreads, 0, s, dst, lhs, rhs, n, vec, f)) return e;
   return cudaGetLastError();
+}
+
+cudaError_t launch_add(int8_t *dst, const int8_t *lhs, const int8_t *rhs, int64_t n, int32_t dest_off, int32_t lhs_off,
+                       int32_t rhs_off, const Triple &lt, const Triple &rt, int32_t splat, cudaStream_t s) {
+  AddQuant q;
+  if (make_add_quant(q, dest_off, lhs_off, rhs_off, lt.pre, lt.post, lt.scale, rt.pre, rt.post, rt.scale, splat))
+    return launch_map(dst, lhs, rhs, n, AddQuantF{q}, s);
+  return launch_map(dst, lhs, rhs, n, AddF{dest_off, lhs_off, rhs_off, lt, rt, splat}, s);
 }
 
 // libjit_batchedadd_quantized (libjit.cpp:997-1015; entry points libjit_batchedadd_i8 and
@@ -391,10 +410,8 @@ extern "C" int glowb200_element_add_i8(int8_t *dest, const int8_t *lhs, const in
                                        int32_t lhs_scale, int32_t rhs_pre, int32_t rhs_post, int32_t rhs_scale,
                                        glowb200_stream_t stream) {
   GLOWB200_ELEMENTWISE_PROLOGUE(n, dest && lhs && rhs)
-  GLOWB200_CUDA_OK(launch_map(dest, lhs, rhs, n,
-                              AddF{dest_offset, lhs_offset, rhs_offset, Triple{lhs_pre, lhs_post, lhs_scale},
-                                   Triple{rhs_pre, rhs_post, rhs_scale}, -128},
-                              GLOWB200_STREAM));
+  GLOWB200_CUDA_OK(launch_add(dest, lhs, rhs, n, dest_offset, lhs_offset, rhs_offset, Triple{lhs_pre, lhs_post, lhs_scale},
+                              Triple{rhs_pre, rhs_post, rhs_scale}, -128, GLOWB200_STREAM));
   return GLOWB200_OK;
 }
 
@@ -408,7 +425,7 @@ extern "C" int glowb200_element_binary_i8(int op, int8_t *dest, const int8_t *lh
   cudaError_t e;
   switch (op) {
     case GLOWB200_BINARY_ADD:
-      e = launch_map(dest, lhs, rhs, n, AddF{dest_offset, lhs_offset, rhs_offset, lt, rt, -128}, GLOWB200_STREAM);
+      e = launch_add(dest, lhs, rhs, n, dest_offset, lhs_offset, rhs_offset, lt, rt, -128, GLOWB200_STREAM);
       break;
     case GLOWB200_BINARY_SUB:
       e = launch_map(dest, lhs, rhs, n, BinaryF<1>{dest_offset, lhs_offset, rhs_offset, lt, rt}, GLOWB200_STREAM);
@@ -462,10 +479,8 @@ extern "C" int glowb200_element_add_maxsplat_i8(int8_t *dest, const int8_t *lhs,
                                                 int32_t rhs_scale, int32_t splat, glowb200_stream_t stream) {
   GLOWB200_ELEMENTWISE_PROLOGUE(n, dest && lhs && rhs)
   GLOWB200_REQUIRE(splat >= -128 && splat <= 127, "splat value outside int8");
-  GLOWB200_CUDA_OK(launch_map(dest, lhs, rhs, n,
-                              AddF{dest_offset, lhs_offset, rhs_offset, Triple{lhs_pre, lhs_post, lhs_scale},
-                                   Triple{rhs_pre, rhs_post, rhs_scale}, splat},
-                              GLOWB200_STREAM));
+  GLOWB200_CUDA_OK(launch_add(dest, lhs, rhs, n, dest_offset, lhs_offset, rhs_offset, Triple{lhs_pre, lhs_post, lhs_scale},
+                              Triple{rhs_pre, rhs_post, rhs_scale}, splat, GLOWB200_STREAM));
   return GLOWB200_OK;
 }
 

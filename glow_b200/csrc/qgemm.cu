@@ -364,6 +364,7 @@ struct GemmSmem {
 // MODE 0: no input row sums take part (every weight offset is 0), the activation is none or Relu and
 // the rows of the result are whole 16-byte pieces -- the common case, whose drain has neither the
 // row-sum term, nor the activation switch, nor the stores of ragged rows;
+// MODE 4: that with the Add of a residual block behind it (GemmParams::residual);
 // MODE 1: every other int8 result in whole 16-byte pieces; MODE 3: int8 results in ragged rows;
 // MODE 2: the floating-point result of the dynamically quantized layers (GemmParams::float_out).
 // One drain body per kernel keeps the register allocation inside the 96 registers a 576-thread CTA leaves.
@@ -390,10 +391,10 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   uint8_t *out_stage = smem + S::kTileBytes + S::kColBytes;
   [[maybe_unused]] int32_t *out_rows = reinterpret_cast<int32_t *>(out_stage + kBlockM * S::kOutPitch);
   int32_t *col_rounding = reinterpret_cast<int32_t *>(smem + S::kTileBytes + BLOCK_N * sizeof(ColParams));
-  // MODE 0, 1: every epilogue warp carries its own rows and columns from tensor memory to the result with no
+  // MODE 0, 1, 4: every epilogue warp carries its own rows and columns from tensor memory to the result with no
   // barrier on the way.  Tiles of 64 columns alternate between two halves of the warps (32 columns each: whole
   // 32-byte sectors), the others are split between all of them.
-  constexpr bool kOwnRows = MODE == 0 || MODE == 1;
+  constexpr bool kOwnRows = MODE == 0 || MODE == 1 || MODE == 4;
   constexpr bool kAlternate = kOwnRows && BLOCK_N <= 64;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::kTileBytes + S::kColBytes + S::kOutBytes);
   uint64_t *empty = full + STAGES;
@@ -574,7 +575,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                                   (uint32_t)p.k_corr * (uint32_t)p.a_offset * (uint32_t)q.b_off;
             cp.c = (int32_t)corr;
             cp.scale = q.out_scale;
-            if constexpr (MODE == 0) {  // nothing to unpack: {c, scale, pre, post}
+            if constexpr (MODE == 0 || MODE == 4) {  // nothing to unpack: {c, scale, pre, post}
               cp.shifts = q.out_pre;
               cp.b_off = q.out_post;
             } else {
@@ -710,6 +711,18 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
           }
         }
+        // the residual's pieces this lane will add, on their way while the accumulators are drained
+        [[maybe_unused]] uint4 other[kPieces];
+        if constexpr (MODE == 4) {
+#pragma unroll
+          for (int it = 0; it < kPieces; it++) {
+            const int dst = __shfl_sync(0xffffffffu, dst_row, it * (32 / kPieces) + lane / kPieces);
+            const int col = first + 16 * (lane % kPieces);
+            other[it] = make_uint4(0u, 0u, 0u, 0u);
+            if (dst >= 0 && col < last && n0 + col < p.N)
+              other[it] = __ldg(reinterpret_cast<const uint4 *>(p.residual + (size_t)dst * p.N + n0 + col));
+          }
+        }
         const int32_t relu_floor = p.act_type == 1 ? p.out_offset : INT32_MIN;
 #pragma unroll 1
         for (int c0 = first; c0 < last; c0 += 16) {
@@ -736,7 +749,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
             for (int cc = 0; cc < 2; cc++) {
               const int4 cp = *reinterpret_cast<const int4 *>(&cols[c0 + 8 * g + 2 * jq + cc]);
-              const int32_t pre = MODE == 0 ? cp.z : cp.z & 0xff, post = MODE == 0 ? cp.w : cp.z >> 8;
+              const int32_t pre = MODE != 1 ? cp.z : cp.z & 0xff, post = MODE != 1 ? cp.w : cp.z >> 8;
 #pragma unroll
               for (int i = 0; i < 4; i++) {  // i = 2h + rr
                 uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)cp.x;
@@ -765,8 +778,11 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           const int r = it * (32 / kPieces) + lane / kPieces, q16 = lane % kPieces;
           const int dst = __shfl_sync(0xffffffffu, dst_row, r);
           const uint4 w = *reinterpret_cast<const uint4 *>(stage + stage_offset<kCols>(r, q16));
-          const uint4 o = make_uint4(__byte_perm(w.x, w.y, 0x5410), __byte_perm(w.z, w.w, 0x5410),
-                                     __byte_perm(w.x, w.y, 0x7632), __byte_perm(w.z, w.w, 0x7632));
+          uint4 o = make_uint4(__byte_perm(w.x, w.y, 0x5410), __byte_perm(w.z, w.w, 0x5410),
+                               __byte_perm(w.x, w.y, 0x7632), __byte_perm(w.z, w.w, 0x7632));
+          if constexpr (MODE == 4)
+            o = make_uint4(add_quant_word(o.x, other[it].x, p.add), add_quant_word(o.y, other[it].y, p.add),
+                           add_quant_word(o.z, other[it].z, p.add), add_quant_word(o.w, other[it].w, p.add));
           const int col = first + 16 * q16;
           if (dst >= 0 && col < last && n0 + col < p.N) *reinterpret_cast<uint4 *>(p.out + (size_t)dst * p.N + n0 + col) = o;
         }
@@ -997,6 +1013,7 @@ bool ptr16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 // the tile kernel's MODE for an int8 result
 int int8_mode(const GemmParams &p) {
   if ((p.N & 15) != 0 || !ptr16(p.out)) return 3;
+  if (p.residual) return 4;
   return p.a_row_sums == nullptr && p.act_type <= 1 ? 0 : 1;
 }
 
@@ -1071,6 +1088,7 @@ int launch_tile_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmP
   switch (int8_mode(p)) {
     case 0: return launch_tile_mode<BLOCK_N, STAGES, 0>(ma, mb, p, s);
     case 1: return launch_tile_mode<BLOCK_N, STAGES, 1>(ma, mb, p, s);
+    case 4: return launch_tile_mode<BLOCK_N, STAGES, 4>(ma, mb, p, s);
     default: return launch_tile_mode<BLOCK_N, STAGES, 3>(ma, mb, p, s);
   }
 }
@@ -1245,7 +1263,7 @@ int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_ro
   if (b_offsets_zero) p.a_row_sums = nullptr;
   else if (!p.float_out) p.a_row_sums = as;
   p.K = pitch;
-  return launch_for_block_n(pick_tile(p.M, p.N, !p.float_out), a, p.M, p.K, p.K, b, p, s);
+  return launch_for_block_n(pick_tile(p.M, p.N, !p.float_out && !p.residual), a, p.M, p.K, p.K, b, p, s);
 }
 
 namespace {

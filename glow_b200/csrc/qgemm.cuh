@@ -14,6 +14,10 @@ struct GemmParams {
   const int32_t *b_row_sums;  // [N] sum_k B[j,k]; b_sum_parts > 1: as many arrays, whose sum it is
   int b_sum_parts;
   const int32_t *a_row_sums;  // [M] sum_k A[i,k], or nullptr when every b offset is 0
+  // The Add of a residual block behind the layer (residual != nullptr): out = add(layer's int8 result,
+  // residual[M, N]), rows of whole 16-byte pieces, no weight offsets, activation none or Relu.
+  const int8_t *residual;
+  AddQuant add;
   int32_t *status;
   const int32_t *bias_offsets;  // per-column bias offsets (channelwise conv), or nullptr: bias_offset
   int M, N, K;                  // K: row pitch of both operands in bytes (a multiple of 16 on the TMA path)

@@ -363,8 +363,10 @@ __global__ void __launch_bounds__(512) i8_skinny_kernel(const int8_t *a, const i
                               q.bias_scale, 0);
   for (int i = tid / kCols; i < MT * 16 && m0 + i < p.M; i += blockDim.x / kCols) {
     const uint32_t v = (uint32_t)acc_s[i * kPitch + c] + base - (uint32_t)q.b_off * (uint32_t)a_sum_s[i];
-    p.out[(size_t)(m0 + i) * p.N + j] =
-        (int8_t)clip_i8(activation_i32(scale32((int32_t)v, q.out_pre, q.out_post, q.out_scale, p.out_offset), p));
+    int32_t x = clip_i8(activation_i32(scale32((int32_t)v, q.out_pre, q.out_post, q.out_scale, p.out_offset), p));
+    if (p.residual)
+      x = (int32_t)add_quant_word((uint32_t)x & 0xffu, (uint8_t)p.residual[(size_t)(m0 + i) * p.N + j], p.add);
+    p.out[(size_t)(m0 + i) * p.N + j] = (int8_t)x;
   }
 }
 

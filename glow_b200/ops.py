@@ -467,6 +467,18 @@ def channelwise_quantized_conv2d(inp, filt, bias, kernels, strides, pads, group,
                                       filter_row_sums, flags, out, workspace, status)
 
 
+def channelwise_quantized_conv2d_add(inp, filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset,
+                                     filter_offsets, bias_offsets, bias_triples, out_triples, act_type, act_args, residual,
+                                     dest_offset, lhs_offset, residual_offset, lhs_triple, residual_triple, splat,
+                                     *, filter_row_sums=None, flags=0, out=None, workspace=None, status=None):
+    """channelwise_quantized_conv2d, then element_add_maxsplat_i8(its result, residual, dest_offset, ...):
+    the end of a residual block.  Of a pointwise convolution the Add costs no launch and no pass of its own."""
+    return _native().channelwise_conv_add(inp, filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset,
+                                          filter_offsets, bias_offsets, bias_triples, out_triples, act_type, act_args,
+                                          filter_row_sums, flags, out, workspace, status, residual, dest_offset, lhs_offset,
+                                          residual_offset, lhs_triple, residual_triple, splat)
+
+
 def conv2d_i8(inp, filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset, filter_offset,
               bias_offset, bias_triple, out_triple, act_type=0, act_args=None, *, flags=0, out=None, workspace=None,
               status=None):

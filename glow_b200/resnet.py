@@ -196,7 +196,8 @@ class ResNet50Int8:
             self.ws = torch.empty(int(nbytes * 1.1) + 256, dtype=torch.uint8, device=self.dev)
         return self.ws
 
-    def _conv(self, name, x):
+    def _conv(self, name, x, residual=None, add=()):
+        """The convolution; with `residual`, the end of a block: Add and Relu behind it."""
         d = self.conv[name]
         c, spec = d["c"], d["c"]["spec"]
         k, s, p = (spec["k"],) * 2, (spec["stride"],) * 2, (spec["pad"],) * 4
@@ -205,11 +206,12 @@ class ResNet50Int8:
         need = n * oh * ow * ((spec["k"] ** 2 * cin + 15) // 16 * 16) + spec["cout"] * ((spec["k"] ** 2 * cin + 15) // 16 * 16) + \
             ops.i8_gemm_workspace_bytes(n * oh * ow, 16, spec["cout"]) + 4096
         self.launches += 2
-        return ops.channelwise_quantized_conv2d(x, d["filter"], d["bias"], k, s, p, 1, (1, 1), c["out_offset"], c["in_offset"],
-                                                d["fo"], d["bo"], d["params"][:3], d["params"][3:],
-                                                1 if spec["relu"] else 0, None, filter_row_sums=d["row_sums"],
-                                                flags=ops.FC_WEIGHT_OFFSETS_ZERO, workspace=self._workspace(need),
-                                                status=self.status)
+        args = (x, d["filter"], d["bias"], k, s, p, 1, (1, 1), c["out_offset"], c["in_offset"], d["fo"], d["bo"],
+                d["params"][:3], d["params"][3:], 1 if spec["relu"] else 0, None)
+        kw = dict(filter_row_sums=d["row_sums"], flags=ops.FC_WEIGHT_OFFSETS_ZERO, workspace=self._workspace(need), status=self.status)
+        if residual is None:
+            return ops.channelwise_quantized_conv2d(*args, **kw)
+        return ops.channelwise_quantized_conv2d_add(*args, residual, *add, **kw)
 
     # Images up to which the layers between Quantize and the FC are replayed from a CUDA graph (from the second
     # call of a shape on): their 73 launches cost the host 4 us each, which is more than the device needs for
@@ -275,14 +277,13 @@ class ResNet50Int8:
                 self.launches += 1
             elif l[0] == "block":
                 y = x
-                for c in l[2]:
+                for c in l[2][:-1]:
                     y = self._conv(c["name"], y)
                 sc = self._conv(l[3]["name"], x) if l[3] else x
                 a = self.q["add"][l[1]]
                 out_off = tqp[a["out"]][1]
-                x = ops.element_add_maxsplat_i8(y, sc, out_off, tqp[a["lhs"]][1], tqp[a["rhs"]][1], a["lhs_triple"],
-                                                a["rhs_triple"], out_off)
-                self.launches += 1
+                x = self._conv(l[2][-1]["name"], y, sc, (out_off, tqp[a["lhs"]][1], tqp[a["rhs"]][1], a["lhs_triple"],
+                                                         a["rhs_triple"], out_off))
             elif l[0] == "avgpool":
                 src = self.q["avgpool_in"]
                 hw = x.shape[1]

@@ -482,6 +482,23 @@ int glowb200_channelwise_quantized_conv2d_i8_i32(
     const int32_t *filter_row_sums, int flags, void *workspace, size_t workspace_bytes,
     int32_t *status, glowb200_stream_t stream);
 
+/* That convolution followed by glowb200_element_add_maxsplat_i8(out, its result, residual, ...) -- the end of a
+ * residual block -- bit-identical to the two calls.  residual: int8, the result's shape.  Of a pointwise
+ * convolution the Add takes no pass over memory of its own. */
+int glowb200_channelwise_quantized_conv2d_add_i8(
+    int8_t *out, const int8_t *in, const int8_t *filter, const int32_t *bias,
+    const int64_t *out_dims, const int64_t *in_dims, const int64_t *filter_dims,
+    const int64_t *kernels, const int64_t *strides, const int64_t *pads, int64_t group,
+    const int64_t *dilation, int32_t out_offset, int32_t in_offset,
+    const int32_t *filter_offsets, const int32_t *bias_offsets, const int32_t *bias_pre,
+    const int32_t *bias_post, const int32_t *bias_scale, const int32_t *out_pre,
+    const int32_t *out_post, const int32_t *out_scale, int32_t act_type, const int32_t *act_args,
+    const int32_t *filter_row_sums, int flags, void *workspace, size_t workspace_bytes,
+    int32_t *status, const int8_t *residual, int32_t dest_offset,
+    int32_t lhs_offset, int32_t residual_offset, int32_t lhs_pre, int32_t lhs_post, int32_t lhs_scale,
+    int32_t residual_pre, int32_t residual_post, int32_t residual_scale, int32_t splat,
+    glowb200_stream_t stream);
+
 /* Convolution (2-D), int8 with int32 bias, one quantisation per tensor.
  * Replaces libjit_conv2d_i8_i32 (libjit_conv.cpp:496-510, body :49-147; scalars derived at
  * LLVMIRGen.cpp:2501-2599).  The reference's depthUnroll argument only blocks its loops and
