@@ -10,14 +10,14 @@
 // One launch pools every bag of every table.  blockIdx.y is the table; inside a table a group of
 // lanes (as many as a row has 16-byte chunks, 8-byte ones for tables off 16-byte boundaries) owns a bag and walks its
 // rows in index order, each lane keeping the sums of the columns of its own chunk: every result
-// element is accumulated in the reference's order and in the result's type (an fp16 result is
-// rounded after every row, as the reference's float16 sum is), with the multiply and the add
+// element is accumulated in the reference's order and in the result's type, with the multiply and the add
 // kept apart, so results are bit-identical to the Interpreter's.  Four rows are requested before
-// the first is consumed; the loop is bound by random row fetches from HBM.
+// the first is consumed.
 //
-// A lane's chunk is cut from the row start, not from the first column: for int8 / int4 rows the
-// first lane's chunk begins with the scale/offset header, so all loads stay aligned to the chunk
-// size although the columns start 4 (or 8) bytes into the row.
+// A chunk of an fp32 or fp16 row, or of a quantized row off 16-byte boundaries, is cut from the row start, not
+// from the first column: the first lane's chunk of a quantized row begins with the scale/offset header, so all
+// loads stay aligned to the chunk size although the columns start 4 (or 8) bytes into the row.  Quantized rows
+// at 16-byte boundaries go by columns (pool_bag_columns).
 #include "common.cuh"
 
 namespace glowb200 {
@@ -35,20 +35,20 @@ struct SplitLaunch {
   const void *indice_weights;
   int32_t *status;
   int64_t num_indices, bags_per_table, total_dims;
-  int32_t wo64, iw16, so_fp32, row_alignment, pooling_mode;
+  int32_t num_tables, wo64, iw16, so_fp32, row_alignment, pooling_mode;
 };
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;  // (a bag of a warp ends late: small blocks hand their registers on sooner)
 #ifndef GLOWB200_TBE_MIN_BLOCKS
-#define GLOWB200_TBE_MIN_BLOCKS 4
-#endif
-#ifndef GLOWB200_TBE_I4_WIDE
-#define GLOWB200_TBE_I4_WIDE 1
+#define GLOWB200_TBE_MIN_BLOCKS 8
 #endif
 #ifndef GLOWB200_TBE_ROWS
-#define GLOWB200_TBE_ROWS 4
+#define GLOWB200_TBE_ROWS 3
 #endif
-constexpr int kRows = GLOWB200_TBE_ROWS;  // rows in flight per lane
+// Rows in flight per lane.  Four spill under 64 registers (128-column int4 bags of 64 rows: 207 against 190 us),
+// two leave more of the latency bare (210); so do 80 registers and fewer warps (211), and one group of rows being
+// added up while the next is on its way measured no better (190).
+constexpr int kRows = GLOWB200_TBE_ROWS;
 
 enum : int { TY_F32 = 0, TY_F16 = 1, TY_I8 = 2, TY_I4 = 3 };
 
@@ -79,6 +79,24 @@ __device__ __forceinline__ void load_chunk(const uint8_t *base, int64_t at, int6
   }
 }
 
+// N words at p (aligned to their size) if `on`, else 0: a predicate, not a branch, so that the loads of several
+// rows go out together.
+template <int N>
+__device__ __forceinline__ void load_if(bool on, const uint8_t *p, uint32_t (&q)[N]) {
+  if constexpr (N == 4) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+                 "@p ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%5];\n\t}"
+                 : "=&r"(q[0]), "=&r"(q[1]), "=&r"(q[2]), "=&r"(q[3]) : "r"((int)on), "l"(p));
+  } else if constexpr (N == 2) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t"
+                 "@p ld.global.nc.v2.b32 {%0, %1}, [%3];\n\t}"
+                 : "=&r"(q[0]), "=&r"(q[1]) : "r"((int)on), "l"(p));
+  } else {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.b32 %0, [%2];\n\t}"
+                 : "=&r"(q[0]) : "r"((int)on), "l"(p));
+  }
+}
+
 // float(h) for the fp16 number in the low half of `h`, through the mixed-precision add of sm_100
 // (adding -0 keeps every value, the sign of a zero included) instead of a conversion
 // instruction: conversions issue at an eighth of the rate of adds, and this kernel would be
@@ -89,9 +107,6 @@ __device__ __forceinline__ float add_f32_f16(uint16_t h, float c) {
   return d;
 }
 __device__ __forceinline__ float half_bits_to_float(uint32_t h) { return add_f32_f16((uint16_t)(h & 0xFFFFu), -0.0f); }
-#ifndef GLOWB200_TBE_X2
-#define GLOWB200_TBE_X2 1
-#endif
 __device__ __forceinline__ uint64_t pack2f(float lo, float hi) {
   uint64_t v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
@@ -107,19 +122,118 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   return d;
 }
 
+// The sums of a lane's columns: fp32, or -- for an fp16 result -- fp16 pairs, rounded after every row as the
+// reference's float16 sum is (float16::operator+, include/glow/Support/Float16.h:47-49): widened, added to in
+// fp32 and rounded back.
+// Slots (the elements of a lane's words) are handled in pairs: neighbours, except for nibbles, where one
+// mask takes nibbles k and k + 4 of a word.
+template <int TY>
+__device__ __forceinline__ constexpr int slot_of(int pair, int second) {
+  return TY == TY_I4 ? 8 * (pair >> 2) + (pair & 3) + 4 * second : 2 * pair + second;
+}
+
+// Adds one row's words to the sums.  Quantized elements become floats without a conversion instruction: byte
+// or nibble q is merged into the mantissa of the fp16 number 1024 (0x6400 | q = 1024 + q) and 1024 is
+// subtracted in the mixed-precision add.  With fp16 headers q * scale is exact in fp32 (8 + 11 significant
+// bits), so one fused multiply-add gives the reference's separately rounded q * scale + offset.
+// Pairs of fp32 values go through the two-lane fp32 instructions of sm_100 (each lane rounds like the scalar
+// instruction, subnormals included) for the dequantising FMA and for the sums of unweighted quantized rows.
+// The weight multiply and the add behind it stay scalar: issued as a two-lane multiply followed by a two-lane
+// add they did not reproduce the reference's two roundings on its own unit vectors, whereas scalar
+// mul.rn / add.rn are never contracted.
+template <int TY, int CW, bool OUT16, bool WEIGHTED, bool SO32, int NA, int NH>
+__device__ __forceinline__ void add_row(const uint32_t (&q)[CW], uint32_t header0, uint32_t header1, float w, float (&acc)[NA],
+                                        uint32_t (&acch)[NH]) {
+  constexpr int SLOTS = TY == TY_F32 ? CW : TY == TY_F16 ? 2 * CW : TY == TY_I8 ? 4 * CW : 8 * CW;
+  constexpr int PAIRS = SLOTS / 2;
+  float scale = 0.0f, offset = 0.0f;
+  if constexpr (TY == TY_I8 || TY == TY_I4) {
+    if constexpr (SO32) {
+      scale = __uint_as_float(header0);
+      offset = __uint_as_float(header1);
+    } else {
+      scale = half_bits_to_float(header0);
+      offset = half_bits_to_float(header0 >> 16);
+    }
+  }
+  auto dequant2 = [&](uint32_t h2, float &ta, float &tb) {  // h2 = two fp16 numbers 1024 + q
+    const float fa = add_f32_f16((uint16_t)(h2 & 0xFFFFu), -1024.0f), fb = add_f32_f16((uint16_t)(h2 >> 16), -1024.0f);
+    if constexpr (SO32) {
+      ta = __fadd_rn(__fmul_rn(fa, scale), offset);
+      tb = __fadd_rn(__fmul_rn(fb, scale), offset);
+    } else {
+      uint64_t v2;
+      asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v2) : "l"(pack2f(fa, fb)), "l"(pack2f(scale, scale)), "l"(pack2f(offset, offset)));
+      unpack2f(v2, ta, tb);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < PAIRS; i++) {
+    float ta, tb;  // the values of the pair's slots in this row
+    if constexpr (TY == TY_F32) {
+      ta = __uint_as_float(q[2 * i]);
+      tb = __uint_as_float(q[2 * i + 1]);
+    } else if constexpr (TY == TY_F16) {
+      ta = half_bits_to_float(q[i]);
+      tb = half_bits_to_float(q[i] >> 16);
+    } else if constexpr (TY == TY_I8) {
+      dequant2(__byte_perm(q[i >> 1], 0x64646464u, (i & 1) ? 0x4342u : 0x4140u), ta, tb);
+    } else {  // even column = low nibble, odd column = high nibble (InterpreterNodes.cpp:104-109)
+      dequant2(((q[i >> 2] >> (4 * (i & 3))) & 0x000F000Fu) | 0x64006400u, ta, tb);
+    }
+    if constexpr (WEIGHTED) {  // (an unweighted bag multiplies by 1.0)
+      ta = __fmul_rn(w, ta);
+      tb = __fmul_rn(w, tb);
+    }
+    if constexpr (OUT16) {
+      // (keeping fp32 copies of the sums and converting both ways every row was tried: half the speed)
+      const float lo = add_f32_f16((uint16_t)(acch[i] & 0xFFFFu), ta);
+      const float hi = add_f32_f16((uint16_t)(acch[i] >> 16), tb);
+      acch[i] = pack_f16x2(lo, hi);
+    } else if constexpr (!WEIGHTED && !SO32 && (TY == TY_I8 || TY == TY_I4)) {
+      uint64_t s2;
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(s2) : "l"(pack2f(acc[slot_of<TY>(i, 0)], acc[slot_of<TY>(i, 1)])), "l"(pack2f(ta, tb)));
+      unpack2f(s2, acc[slot_of<TY>(i, 0)], acc[slot_of<TY>(i, 1)]);
+    } else {
+      acc[slot_of<TY>(i, 0)] = __fadd_rn(acc[slot_of<TY>(i, 0)], ta);
+      acc[slot_of<TY>(i, 1)] = __fadd_rn(acc[slot_of<TY>(i, 1)], tb);
+    }
+  }
+}
+
+// The sums of columns col0 .. (those below 0 or beyond the table's are nobody's), divided by the row count
+// for mean pooling.
+template <int TY, int SLOTS, bool OUT16, int NA, int NH>
+__device__ __forceinline__ void store_sums(const float (&acc)[NA], const uint32_t (&acch)[NH], int32_t col0, int32_t num_dims,
+                                           bool mean, int64_t rows, void *out_row) {
+  float n = 1.0f;
+  if (mean) {
+    n = (float)rows;
+    if (OUT16) n = __half2float(__float2half_rn(n));
+  }
+#pragma unroll
+  for (int i = 0; i < SLOTS / 2; i++) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int slot = slot_of<TY>(i, e);
+      const int32_t c = col0 + slot;
+      if (c < 0 || c >= num_dims) continue;
+      if constexpr (OUT16) {
+        const __half h = __ushort_as_half((unsigned short)((acch[i] >> (16 * e)) & 0xFFFFu));
+        reinterpret_cast<__half *>(out_row)[c] = mean ? __float2half_rn(__fdiv_rn(__half2float(h), n)) : h;
+      } else {
+        reinterpret_cast<float *>(out_row)[c] = mean ? __fdiv_rn(acc[slot], n) : acc[slot];
+      }
+    }
+  }
+}
+
 // Pools the bag [begin, end) of one table for the lanes of one group.
 //   TY   element type of the table; CW words per lane chunk (2 or 4); SO32: fp32 row headers
 //   gl / lpr  lane within the group / lanes of the group
-// Slots (the elements of a lane's chunk) are handled in pairs.  An fp16 result keeps its running
-// sums as fp16 pairs: per row the sum is widened, added to in fp32 and rounded back
-// (float16::operator+ of the reference, include/glow/Support/Float16.h:47-49).
-// Quantized elements become floats without a conversion instruction: byte or nibble q is merged
-// into the mantissa of the fp16 number 1024 (0x6400 | q = 1024 + q) and 1024 is subtracted in the
-// mixed-precision add.  With fp16 headers q * scale is exact in fp32 (8 + 11 significant bits), so
-// one fused multiply-add gives the reference's separately rounded q * scale + offset.
 template <int TY, int CW, bool OUT16, bool WEIGHTED, bool SO32, typename IdxT>
 __device__ __forceinline__ int32_t pool_bag(const SplitLaunch &p, const uint8_t *base, int64_t limit, int64_t table_at,
-                                            int32_t row_bytes, int32_t touched, int32_t num_dims, bool vec,
+                                            int32_t row_bytes, int32_t touched, int32_t num_dims, int32_t max_row, bool vec,
                                             int64_t begin, int64_t end, int gl, int lpr, void *out_row) {
   constexpr int CB = 4 * CW;                                           // chunk bytes
   constexpr int SLOTS = TY == TY_F32 ? CW : TY == TY_F16 ? 2 * CW : TY == TY_I8 ? 4 * CW : 8 * CW;
@@ -127,14 +241,6 @@ __device__ __forceinline__ int32_t pool_bag(const SplitLaunch &p, const uint8_t 
   constexpr int H = (TY == TY_I8 || TY == TY_I4) ? (SO32 ? 8 : 4) : 0;  // header bytes of a row
   const IdxT *indices = reinterpret_cast<const IdxT *>(p.indices);
   int32_t flags = 0;
-  // the two slots of pair i: neighbours, except for nibbles, where one mask takes nibbles k and k + 4 of a word
-  auto slot_a = [](int i) { return TY == TY_I4 ? 8 * (i >> 2) + (i & 3) : 2 * i; };
-  auto slot_b = [](int i) { return TY == TY_I4 ? 8 * (i >> 2) + (i & 3) + 4 : 2 * i + 1; };
-  // rows whose touched bytes all lie inside the buffer (InterpreterNodes.cpp:6720): 0 .. max_row
-  int64_t max_row = -1;
-  if (table_at >= 0 && table_at + touched <= limit) max_row = (limit - touched - table_at) / row_bytes;
-  if (max_row > 0x7FFFFFFEll) max_row = 0x7FFFFFFEll;
-
   for (int32_t cbase = 0; cbase < touched; cbase += lpr * CB) {
     const int32_t at = cbase + gl * CB;          // byte of the row this lane's chunk starts at
     const bool has = at < touched;
@@ -171,7 +277,7 @@ __device__ __forceinline__ int32_t pool_bag(const SplitLaunch &p, const uint8_t 
       bool live[kRows];
       float w[kRows];
       uint32_t q[kRows][CW];
-      uint32_t hdr[kRows][2];
+      uint32_t hdr[kRows][2] = {};
 #pragma unroll
       for (int u = 0; u < kRows; u++) {
         w[u] = next_w[u];
@@ -197,169 +303,239 @@ __device__ __forceinline__ int32_t pool_bag(const SplitLaunch &p, const uint8_t 
 #pragma unroll
       for (int u = 0; u < kRows; u++) {
         if (!live[u]) continue;
-        float scale = 0.0f, offset = 0.0f;
-        if constexpr (TY == TY_I8 || TY == TY_I4) {
-          if constexpr (SO32) {
-            scale = __uint_as_float(hdr[u][0]);
-            offset = __uint_as_float(hdr[u][1]);
-          } else {
-            scale = half_bits_to_float(hdr[u][0]);
-            offset = half_bits_to_float(hdr[u][0] >> 16);
-          }
-        }
-        // Pairs of fp32 values go through the two-lane fp32 instructions of sm_100 (each lane
-        // rounds like the scalar instruction, subnormals included) for the dequantising FMA and
-        // for the sums of unweighted quantized rows.  The weight multiply and the add behind it
-        // stay scalar: issued as a two-lane multiply followed by a two-lane add they did not
-        // reproduce the reference's two roundings on its own unit vectors, whereas scalar
-        // mul.rn / add.rn are never contracted.
-        auto dequant2 = [&](uint32_t h2, float &ta, float &tb) {  // h2 = two fp16 numbers 1024 + q
-          const float fa = add_f32_f16((uint16_t)(h2 & 0xFFFFu), -1024.0f), fb = add_f32_f16((uint16_t)(h2 >> 16), -1024.0f);
-          if constexpr (SO32) {
-            ta = __fadd_rn(__fmul_rn(fa, scale), offset);
-            tb = __fadd_rn(__fmul_rn(fb, scale), offset);
-          } else if constexpr (GLOWB200_TBE_X2) {
-            uint64_t v2;
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v2) : "l"(pack2f(fa, fb)), "l"(pack2f(scale, scale)), "l"(pack2f(offset, offset)));
-            unpack2f(v2, ta, tb);
-          } else {
-            ta = __fmaf_rn(fa, scale, offset);
-            tb = __fmaf_rn(fb, scale, offset);
-          }
-        };
-#pragma unroll
-        for (int i = 0; i < PAIRS; i++) {
-          float ta, tb;  // the values of the pair's slots in this row
-          if constexpr (TY == TY_F32) {
-            ta = __uint_as_float(q[u][2 * i]);
-            tb = __uint_as_float(q[u][2 * i + 1]);
-          } else if constexpr (TY == TY_F16) {
-            ta = half_bits_to_float(q[u][i]);
-            tb = half_bits_to_float(q[u][i] >> 16);
-          } else if constexpr (TY == TY_I8) {
-            dequant2(__byte_perm(q[u][i >> 1], 0x64646464u, (i & 1) ? 0x4342u : 0x4140u), ta, tb);
-          } else {  // even column = low nibble, odd column = high nibble (InterpreterNodes.cpp:104-109)
-            dequant2(((q[u][i >> 2] >> (4 * (i & 3))) & 0x000F000Fu) | 0x64006400u, ta, tb);
-          }
-          if constexpr (WEIGHTED) {  // (an unweighted bag multiplies by 1.0)
-            ta = __fmul_rn(w[u], ta);
-            tb = __fmul_rn(w[u], tb);
-          }
-          if constexpr (OUT16) {
-            // (keeping fp32 copies of the sums and converting both ways every row was tried: half the speed)
-            const float lo = add_f32_f16((uint16_t)(acch[i] & 0xFFFFu), ta);
-            const float hi = add_f32_f16((uint16_t)(acch[i] >> 16), tb);
-            acch[i] = pack_f16x2(lo, hi);
-          } else if constexpr (GLOWB200_TBE_X2 && !WEIGHTED && !SO32 && (TY == TY_I8 || TY == TY_I4)) {
-            uint64_t s2;
-            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(s2) : "l"(pack2f(acc[slot_a(i)], acc[slot_b(i)])), "l"(pack2f(ta, tb)));
-            unpack2f(s2, acc[slot_a(i)], acc[slot_b(i)]);
-          } else {
-            acc[slot_a(i)] = __fadd_rn(acc[slot_a(i)], ta);
-            acc[slot_b(i)] = __fadd_rn(acc[slot_b(i)], tb);
-          }
-        }
+        add_row<TY, CW, OUT16, WEIGHTED, SO32>(q[u], hdr[u][0], hdr[u][1], w[u], acc, acch);
       }
     }
 
     if (!has) continue;
-    const bool mean = p.pooling_mode == 1 && end > begin;
-    float n = 1.0f;
-    if (mean) {
-      n = (float)(end - begin);
-      if (OUT16) n = __half2float(__float2half_rn(n));
-    }
-#pragma unroll
-    for (int i = 0; i < PAIRS; i++) {
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int slot = e ? slot_b(i) : slot_a(i);
-        const int32_t c = col0 + slot;
-        if (c < 0 || c >= num_dims) continue;
-        if constexpr (OUT16) {
-          const __half h = __ushort_as_half((unsigned short)((acch[i] >> (16 * e)) & 0xFFFFu));
-          reinterpret_cast<__half *>(out_row)[c] = mean ? __float2half_rn(__fdiv_rn(__half2float(h), n)) : h;
-        } else {
-          reinterpret_cast<float *>(out_row)[c] = mean ? __fdiv_rn(acc[slot], n) : acc[slot];
-        }
-      }
-    }
+    store_sums<TY, SLOTS, OUT16>(acc, acch, col0, num_dims, p.pooling_mode == 1 && end > begin, end - begin, out_row);
   }
   return flags;
 }
 
+// The same for quantized rows at 16-byte boundaries whose chunks are cut from the first column instead: a lane's
+// LW words are all columns, where chunks from the row start give the first lane a header and the last one
+// little more than that (five 16-byte chunks for the 68 bytes of a 128-column int4 row: 160 slots for 128
+// columns).  Behind a 4-byte header a lane's four words are three of its aligned 16 bytes and one more load.
+// What bounds it is the arithmetic -- four instructions per element is its least (widen and add for the sum, half
+// a pack, subtract, half an FMA, extract) -- and the rows' latency, which 27 warps of three rows do not hide.
+// 65,536 bags of Poisson(64) int4 rows of 128 columns, fp16 result: 282 us by row chunks and loads in branches, 190 so.
+template <int TY, int LW, bool OUT16, bool WEIGHTED, bool SO32, typename IdxT>
+__device__ __forceinline__ int32_t pool_bag_columns(const SplitLaunch &p, const uint8_t *table,
+                                                    int32_t row_bytes, int32_t touched, int32_t num_dims, int32_t max_row,
+                                                    int64_t begin, int64_t end, int gl, int lpr, void *out_row) {
+  constexpr int H = SO32 ? 8 : 4, SLOTS = (TY == TY_I8 ? 4 : 8) * LW;
+  const IdxT *indices = reinterpret_cast<const IdxT *>(p.indices) + begin;
+  const int32_t count = (int32_t)(end - begin < 0x7FFFFFF0ll ? end - begin : 0x7FFFFFF0ll);
+  int32_t flags = 0;
+  for (int32_t word0 = gl * LW; H + 4 * (word0 - gl * LW) < touched; word0 += lpr * LW) {
+    const int32_t at = H + 4 * word0;   // byte of the row the lane's words start at
+    const bool has = at < touched;
+    const bool more = at + 4 * (LW == 4 && SO32 ? 2 : LW - 1) < touched;  // the second load has something to bring
+    float acc[OUT16 ? 1 : SLOTS];
+    uint32_t acch[OUT16 ? SLOTS / 2 : 1];
+#pragma unroll
+    for (int s = 0; s < (OUT16 ? 1 : SLOTS); s++) acc[s] = 0.0f;
+#pragma unroll
+    for (int s = 0; s < (OUT16 ? SLOTS / 2 : 1); s++) acch[s] = 0u;
+    int32_t next_r[kRows];  // -2 none, -1 refused
+    float next_w[kRows];
+    auto request = [&](int32_t j) {
+#pragma unroll
+      for (int u = 0; u < kRows; u++) {
+        next_r[u] = -2;
+        next_w[u] = 1.0f;
+        if (j + u < count) {
+          const IdxT r = indices[j + u];
+          next_r[u] = (r < 0 || r > (IdxT)max_row) ? -1 : (int32_t)r;
+          if constexpr (WEIGHTED)
+            next_w[u] = p.iw16 ? __half2float(reinterpret_cast<const __half *>(p.indice_weights)[begin + j + u])
+                               : reinterpret_cast<const float *>(p.indice_weights)[begin + j + u];
+        }
+      }
+    };
+    request(0);
+    for (int32_t j = 0; j < count; j += kRows) {
+      bool live[kRows];
+      float w[kRows];
+      uint32_t q[kRows][LW], hdr[kRows][2] = {};
+#pragma unroll
+      for (int u = 0; u < kRows; u++) {
+        w[u] = next_w[u];
+        live[u] = next_r[u] >= 0 && has;
+        if (next_r[u] == -1) flags |= GLOWB200_STATUS_INDEX_OUT_OF_RANGE;
+        const uint8_t *row = table + (int64_t)next_r[u] * row_bytes;
+        if constexpr (SO32) {
+          load_if<2>(live[u], row, hdr[u]);
+#pragma unroll
+          for (int k = 0; k < LW; k += 2)
+            load_if<2>(live[u] && (k == 0 || more), row + at + 4 * k, *reinterpret_cast<uint32_t (*)[2]>(&q[u][k]));
+        } else {
+          load_if<1>(live[u], row, *reinterpret_cast<uint32_t (*)[1]>(&hdr[u][0]));
+          if constexpr (LW == 4) {
+            uint32_t v[4];
+            load_if<4>(live[u], row + at - 4, v);
+            q[u][0] = v[1]; q[u][1] = v[2]; q[u][2] = v[3];
+          } else {
+            load_if<1>(live[u], row + at, *reinterpret_cast<uint32_t (*)[1]>(&q[u][0]));
+          }
+          load_if<1>(live[u] && more, row + at + 4 * (LW - 1), *reinterpret_cast<uint32_t (*)[1]>(&q[u][LW - 1]));
+        }
+      }
+      request(j + kRows);
+#pragma unroll
+      for (int u = 0; u < kRows; u++)
+        if (live[u]) add_row<TY, LW, OUT16, WEIGHTED, SO32>(q[u], hdr[u][0], hdr[u][1], w[u], acc, acch);
+    }
+    if (has)
+      store_sums<TY, SLOTS, OUT16>(acc, acch, (TY == TY_I8 ? 4 : 8) * word0, num_dims, p.pooling_mode == 1 && end > begin, end - begin,
+                                   out_row);
+  }
+  return flags;
+}
+
+// A table as the lanes of one group see it.
+struct TableRows {
+  const uint8_t *base;
+  int64_t limit, table_at;
+  int32_t row_bytes, touched, num_dims, dim_start, table, max_row, gl, lpr;
+  bool vec;
+};
+
+template <bool COLUMNS, int TY, int CW, bool OUT16, bool WEIGHTED, bool SO32, typename IdxT>
+__device__ __forceinline__ int32_t pool_bags(const SplitLaunch &p, const TableRows &r, int64_t first, int64_t step) {
+  const IdxT *offsets = reinterpret_cast<const IdxT *>(p.offsets) + (int64_t)r.table * p.bags_per_table;
+  int32_t flags = 0;
+  for (int64_t b = first; b < p.bags_per_table; b += step) {
+    int64_t begin = (int64_t)offsets[b];
+    int64_t end = (int64_t)offsets[b + 1];
+    if (begin < 0 || end < begin || end > p.num_indices) {
+      if (end >= begin) flags |= GLOWB200_STATUS_BAD_OFFSETS;  // a start above its end is an empty bag
+      begin = end = 0;
+    }
+    void *out_row = reinterpret_cast<char *>(p.dest) + ((size_t)(b * p.total_dims + r.dim_start)) * (OUT16 ? 2 : 4);
+    if constexpr (COLUMNS)
+      flags |= pool_bag_columns<TY, CW, OUT16, WEIGHTED, SO32, IdxT>(p, r.base + r.table_at, r.row_bytes, r.touched, r.num_dims,
+                                                                     r.max_row, begin, end, r.gl, r.lpr, out_row);
+    else
+      flags |= pool_bag<TY, CW, OUT16, WEIGHTED, SO32, IdxT>(p, r.base, r.limit, r.table_at, r.row_bytes, r.touched, r.num_dims, r.max_row, r.vec,
+                                                             begin, end, r.gl, r.lpr, out_row);
+  }
+  return flags;
+}
+
+struct SplitTable {
+  int32_t dim_start, num_dims, ty, placement;
+  bool supported;
+};
+// (int2 rows and tables placed in device-only memory are not supported by the reference
+// either, InterpreterNodes.cpp:6696, 6704: the table's columns stay 0)
+__device__ __forceinline__ SplitTable split_table(const SplitLaunch &p, int t) {
+  SplitTable d;
+  d.dim_start = p.dim_offsets[t];
+  d.num_dims = p.dim_offsets[t + 1] - d.dim_start;
+  d.ty = p.weights_tys[t];
+  d.placement = p.placements[t];
+  d.supported = d.ty <= TY_I4 && d.placement != 0 && d.dim_start >= 0 && (int64_t)d.dim_start + d.num_dims <= p.total_dims &&
+                d.num_dims <= (1 << 27);
+  return d;
+}
+
+// The columns no table writes are 0 (the reference clears the result first, InterpreterNodes.cpp:6672).  The
+// blocks behind the last table look for them -- a fill of the whole result was a launch of its own, 4 us of 16 MB.
+template <bool OUT16>
+__device__ __forceinline__ void clear_uncovered(const SplitLaunch &p) {
+  for (int64_t c = (int64_t)blockIdx.x * kThreads + threadIdx.x; c < p.total_dims; c += (int64_t)gridDim.x * kThreads) {
+    bool covered = false;
+    for (int t = 0; t < p.num_tables && !covered; t++) {
+      const SplitTable d = split_table(p, t);
+      covered = d.supported && c >= d.dim_start && c < (int64_t)d.dim_start + d.num_dims;
+    }
+    if (covered) continue;
+    for (int64_t b = 0; b < p.bags_per_table; b++) {
+      if constexpr (OUT16) reinterpret_cast<uint16_t *>(p.dest)[b * p.total_dims + c] = 0;
+      else reinterpret_cast<float *>(p.dest)[b * p.total_dims + c] = 0.0f;
+    }
+  }
+}
+
 template <bool OUT16, typename IdxT>
 __global__ void __launch_bounds__(kThreads, GLOWB200_TBE_MIN_BLOCKS) split_embedding_bags_kernel(const __grid_constant__ SplitLaunch p) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.y;
-  const int32_t dim_start = p.dim_offsets[t], num_dims = p.dim_offsets[t + 1] - dim_start;
-  const int ty = p.weights_tys[t];
-  const int32_t placement = p.placements[t];
+  if (t == p.num_tables) return clear_uncovered<OUT16>(p);
+  const SplitTable d = split_table(p, t);
+  const int32_t num_dims = d.num_dims;
   if (num_dims <= 0) return;
-  if (ty > TY_I4 || placement == 0 || dim_start < 0 || (int64_t)dim_start + num_dims > p.total_dims || num_dims > (1 << 27)) {
-    // int2 rows and tables placed in device-only memory are not supported by the reference
-    // either (InterpreterNodes.cpp:6696, 6704): the table's columns stay 0
+  if (!d.supported) {
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, GLOWB200_STATUS_UNSUPPORTED_TABLE);
     return;
   }
-  const int so = p.so_fp32 ? 4 : 2;
+  const int ty = d.ty, so = p.so_fp32 ? 4 : 2;
   const int32_t unpadded = ty == TY_F32 ? num_dims * 4 : ty == TY_F16 ? num_dims * 2
                          : ty == TY_I8 ? num_dims + 2 * so : num_dims / 2 + 2 * so;
   const int32_t row_bytes = (unpadded + p.row_alignment - 1) / p.row_alignment * p.row_alignment;
   // bytes of a row the reference touches: the last column of an int4 row with an odd column
   // count sits in the byte after the counted payload (column d reads byte d / 2)
   const int32_t touched = ty == TY_I4 ? (num_dims + 1) / 2 + 2 * so : unpadded;
-  const uint8_t *base = placement == 3 ? p.dev_weights : p.uvm_weights;
-  const int64_t limit = placement == 3 ? p.dev_bytes : p.uvm_bytes;
+  const uint8_t *base = d.placement == 3 ? p.dev_weights : p.uvm_weights;
+  const int64_t limit = d.placement == 3 ? p.dev_bytes : p.uvm_bytes;
   const int64_t table_at = p.wo64 ? reinterpret_cast<const int64_t *>(p.weights_offsets)[t]
                                   : (int64_t)reinterpret_cast<const int32_t *>(p.weights_offsets)[t];
   // 16-byte chunks where the table allows them (rows at 16-byte boundaries), else 8-byte chunks.
   // A bag takes as many lanes as its rows have chunks (32 at most; wider rows take several
-  // passes), not a power of two: a 132-byte int8 row is 9 lanes, three bags to a warp.
+  // passes), not a power of two: a 132-byte row is 9 lanes, three bags to a warp.
   const uint64_t addr = reinterpret_cast<uintptr_t>(base) + (uint64_t)table_at;
   const bool wide = (addr % 16) == 0 && (row_bytes % 16) == 0;
-  // (int4 rows with an fp32 result keep 8-byte chunks: 32 fp32 sums per lane spill, 16.0 against 12.9 G rows/s)
-  const bool wide_i4 = GLOWB200_TBE_I4_WIDE && OUT16;
-  const int cb = (wide && (ty != TY_I4 || wide_i4)) ? 16 : 8;
+  // rows whose touched bytes all lie inside the buffer (InterpreterNodes.cpp:6720): 0 .. max_row
+  int64_t max_row = -1;
+  if (table_at >= 0 && table_at + touched <= limit) max_row = (limit - touched - table_at) / row_bytes;
+  if (max_row > 0x7FFFFFFEll) max_row = 0x7FFFFFFEll;
+  // (a buffer that does not end on a 16-byte boundary may cut the last row's pieces short)
+  const bool columns = wide && ty >= TY_I8 && table_at + max_row * row_bytes + (touched + 15) / 16 * 16 <= limit;
+  // Words of columns per lane: four, but two of int4 rows with an fp32 result (32 fp32 sums per lane spill: 12.9
+  // against 16.0 G rows/s) and of int4 rows that are no longer.
+  const bool pairs = ty == TY_I4 && (!OUT16 || num_dims <= 16);
   const bool vec = wide || ((addr % 8) == 0 && (row_bytes % 8) == 0);
-  const int chunks = (touched + cb - 1) / cb;
+  const int cb = columns ? (pairs ? 8 : 16) : wide ? 16 : 8;
+  const int chunks = ((columns ? touched - 2 * so : touched) + cb - 1) / cb;
   int lpr = chunks > 32 ? 32 : chunks;
-  // Rows of a little more than half a warp (17 chunks: a 260-byte int8 row) would leave the other
+  // Rows of a little more than half a warp (17 chunks: a 260-byte row) would leave the other
   // half idle: half as many lanes then walk the bag twice, one half of the row per pass, when that
   // puts over 2.4 times as many bags into the warp.
   if (chunks <= 32 && 32 / ((chunks + 1) / 2) * 5 > 32 / lpr * 12) lpr = (chunks + 1) / 2;
   const int bags_per_warp = 32 / lpr;
   const int lane = threadIdx.x & 31;
   if (lane >= bags_per_warp * lpr) return;
-  const int64_t b = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * bags_per_warp + lane / lpr;
-  if (b >= p.bags_per_table) return;
   const int gl = lane % lpr;
-
-  const IdxT *offsets = reinterpret_cast<const IdxT *>(p.offsets);
-  int64_t begin = (int64_t)offsets[(int64_t)t * p.bags_per_table + b];
-  int64_t end = (int64_t)offsets[(int64_t)t * p.bags_per_table + b + 1];
+  const int64_t first = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * bags_per_warp + lane / lpr;
+  const int64_t step = (int64_t)gridDim.x * (kThreads / 32) * bags_per_warp;
+  const TableRows rows{base, limit, table_at, row_bytes, touched, num_dims, d.dim_start, t, (int32_t)max_row, gl, lpr, vec};
   int32_t flags = 0;
-  if (begin < 0 || end < begin || end > p.num_indices) {
-    if (end >= begin) flags |= GLOWB200_STATUS_BAD_OFFSETS;  // a start above its end is an empty bag
-    begin = end = 0;
-  }
-  void *out_row = reinterpret_cast<char *>(p.dest) + ((size_t)(b * p.total_dims + dim_start)) * (OUT16 ? 2 : 4);
-
-#define GLOWB200_POOL3(TY, CW, WEIGHTED, SO32)                                                                     \
-  flags |= pool_bag<TY, CW, OUT16, WEIGHTED, SO32, IdxT>(p, base, limit, table_at, row_bytes, touched, num_dims, vec, \
-                                                         begin, end, gl, lpr, out_row)
-#define GLOWB200_POOL2(TY, CW, SO32) \
-  do { if (p.indice_weights != nullptr) GLOWB200_POOL3(TY, CW, true, SO32); else GLOWB200_POOL3(TY, CW, false, SO32); } while (0)
-#define GLOWB200_POOLQ(TY, CW) \
-  do { if (p.so_fp32) GLOWB200_POOL2(TY, CW, true); else GLOWB200_POOL2(TY, CW, false); } while (0)
+#define GLOWB200_POOL2(COLUMNS, TY, CW, SO32)                                                                         \
+  do {                                                                                                               \
+    if (p.indice_weights != nullptr) flags = pool_bags<COLUMNS, TY, CW, OUT16, true, SO32, IdxT>(p, rows, first, step); \
+    else flags = pool_bags<COLUMNS, TY, CW, OUT16, false, SO32, IdxT>(p, rows, first, step);                          \
+  } while (0)
+#define GLOWB200_POOLQ(COLUMNS, TY, CW) \
+  do { if (p.so_fp32) GLOWB200_POOL2(COLUMNS, TY, CW, true); else GLOWB200_POOL2(COLUMNS, TY, CW, false); } while (0)
   switch (ty) {
-    case TY_F32: if (wide) GLOWB200_POOL2(TY_F32, 4, false); else GLOWB200_POOL2(TY_F32, 2, false); break;
-    case TY_F16: if (wide) GLOWB200_POOL2(TY_F16, 4, false); else GLOWB200_POOL2(TY_F16, 2, false); break;
-    case TY_I8: if (wide) GLOWB200_POOLQ(TY_I8, 4); else GLOWB200_POOLQ(TY_I8, 2); break;
-    default: if (wide && wide_i4) GLOWB200_POOLQ(TY_I4, 4); else GLOWB200_POOLQ(TY_I4, 2); break;
+    case TY_F32: if (wide) GLOWB200_POOL2(false, TY_F32, 4, false); else GLOWB200_POOL2(false, TY_F32, 2, false); break;
+    case TY_F16: if (wide) GLOWB200_POOL2(false, TY_F16, 4, false); else GLOWB200_POOL2(false, TY_F16, 2, false); break;
+    case TY_I8: if (columns) GLOWB200_POOLQ(true, TY_I8, 4); else GLOWB200_POOLQ(false, TY_I8, 2); break;
+    default:
+      if (columns && !pairs) {
+        if constexpr (OUT16) GLOWB200_POOLQ(true, TY_I4, 4);
+      } else if (columns) {
+        GLOWB200_POOLQ(true, TY_I4, 2);
+      } else {
+        GLOWB200_POOLQ(false, TY_I4, 2);
+      }
+      break;
   }
 #undef GLOWB200_POOLQ
 #undef GLOWB200_POOL2
-#undef GLOWB200_POOL3
   if (p.status != nullptr && flags != 0) atomicOr(p.status, flags);
 }
 
@@ -384,9 +560,10 @@ extern "C" int glowb200_int_nbit_split_embedding_bags(
   if (bags_per_table == 0 || total_dims == 0) return GLOWB200_OK;
   GLOWB200_REQUIRE(dest != nullptr, "dest is NULL");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // the reference clears the result first (InterpreterNodes.cpp:6672); columns no table covers stay 0
-  GLOWB200_CUDA_OK(cudaMemsetAsync(dest, 0, (size_t)(bags_per_table * total_dims) * (out_is_fp16 ? 2 : 4), s));
-  if (num_tables == 0) return GLOWB200_OK;
+  if (num_tables == 0) {
+    GLOWB200_CUDA_OK(cudaMemsetAsync(dest, 0, (size_t)(bags_per_table * total_dims) * (out_is_fp16 ? 2 : 4), s));
+    return GLOWB200_OK;
+  }
   GLOWB200_REQUIRE(weights_placements != nullptr && weights_offsets != nullptr && weights_tys != nullptr &&
                        dim_offsets != nullptr && offsets != nullptr,
                    "NULL table description or offsets");
@@ -413,16 +590,21 @@ extern "C" int glowb200_int_nbit_split_embedding_bags(
   L.so_fp32 = scale_offset_is_fp32 ? 1 : 0;
   L.row_alignment = row_alignment;
   L.pooling_mode = pooling_mode;
-  // a block holds 8 bags of the widest kind of table (32 lanes a bag); tables with narrower
-  // rows put more bags into a block and their surplus blocks leave at once
-  dim3 grid((unsigned)((bags_per_table + 7) / 8), (unsigned)num_tables);
-  if (out_is_fp16) {
-    if (indices_are_int64) split_embedding_bags_kernel<true, int64_t><<<grid, kThreads, 0, s>>>(L);
-    else split_embedding_bags_kernel<true, int32_t><<<grid, kThreads, 0, s>>>(L);
-  } else {
-    if (indices_are_int64) split_embedding_bags_kernel<false, int64_t><<<grid, kThreads, 0, s>>>(L);
-    else split_embedding_bags_kernel<false, int32_t><<<grid, kThreads, 0, s>>>(L);
-  }
+  L.num_tables = (int32_t)num_tables;
+  // A warp takes 8 bags of rows of 4 lanes; the blocks of tables with wider rows walk on, those of narrower ones
+  // are in part not needed and leave at once.  Few bags: a block for every 8, so that no row is so wide that its
+  // bags would wait for one another while SMs idle (8 tables, 64 bags of 20 int8 rows of 128 columns: 17 -> 12 us).
+  int64_t blocks = (bags_per_table + 7) / 8;
+  if (blocks * num_tables > 2048) blocks = (bags_per_table + 31) / 32;
+  const dim3 grid((unsigned)blocks, (unsigned)num_tables + (num_tables < 65535 ? 1 : 0));
+  if (num_tables == 65535)  // no block row left for the columns without a table
+    GLOWB200_CUDA_OK(cudaMemsetAsync(dest, 0, (size_t)(bags_per_table * total_dims) * (out_is_fp16 ? 2 : 4), s));
+  if (out_is_fp16)
+    GLOWB200_CUDA_OK(indices_are_int64 ? launch_pdl(split_embedding_bags_kernel<true, int64_t>, grid, kThreads, 0, s, L)
+                                       : launch_pdl(split_embedding_bags_kernel<true, int32_t>, grid, kThreads, 0, s, L));
+  else
+    GLOWB200_CUDA_OK(indices_are_int64 ? launch_pdl(split_embedding_bags_kernel<false, int64_t>, grid, kThreads, 0, s, L)
+                                       : launch_pdl(split_embedding_bags_kernel<false, int32_t>, grid, kThreads, 0, s, L));
   GLOWB200_CUDA_OK(cudaGetLastError());
   return GLOWB200_OK;
 }

@@ -131,6 +131,29 @@ def test_row_alignments_and_fp32_headers(oracle, so_fp32, align, first_at):
     assert int(st.item()) == 0
 
 
+@pytest.mark.parametrize("so_fp32", [False, True])
+@pytest.mark.parametrize("out16", [False, True])
+@pytest.mark.parametrize("ty,dims", [(ops.EST_INT4, (1, 16, 17, 33, 127, 1030)), (ops.EST_INT8, (1, 3, 16, 20, 65, 515))])
+def test_quantized_rows_by_columns(oracle, so_fp32, out16, ty, dims):
+    """Rows at 16-byte boundaries whose columns end inside a lane's words, need one lane or several passes;
+    enough bags that a block takes several (few tables, many bags); a buffer that ends inside the last row."""
+    rng = np.random.default_rng(dims[1])
+    specs = [(ty, d, 90 + d, 3) for d in dims]
+    dev, uvm, offs = random_tables(rng, specs, so_fp32, 16)
+    for cut, bags in ((0, 3000), (21 if so_fp32 else 25, 40)):
+        idx, offsets = random_request(rng, specs, bags, 3, np.int32)
+        d = np.array([0] + list(dims), np.int64).cumsum().astype(np.int32)
+        a = dict(dev_weights=dev[:dev.size - cut], uvm_weights=uvm, placements=np.full(len(dims), 3, np.int32),
+                 weights_offsets=offs.astype(np.int64), weights_tys=np.full(len(dims), ty, np.uint8), dim_offsets=d + 5,
+                 total_dims=int(d[-1]) + 7, indices=idx, offsets=offsets, pooling_mode=ops.EP_SUM, out_fp16=out16, indice_weights=None)
+        st = ops.new_status(DEV)
+        got = run_gpu(a, so_fp32=so_fp32, status=st)
+        want = oracle.int_nbit_split_embedding_bags(so_fp32=so_fp32, row_alignment=16, **a)
+        np.testing.assert_array_equal(bits(got), bits(want))
+        assert not got[:, :5].any() and not got[:, -2:].any()
+        assert int(st.item()) == 0
+
+
 def test_bad_rows_and_tables_are_reported():
     rng = np.random.default_rng(5)
     specs = [(ops.EST_INT8, 32, 100, 3), (ops.EST_INT8, 32, 100, 3), (ops.EST_INT8, 32, 100, 0)]
