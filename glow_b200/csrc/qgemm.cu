@@ -544,8 +544,11 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     bool dead = false;
     int cols_n0 = -1;  // column block the records in shared memory belong to
     const uint32_t leader_acc_empty[2] = {PAIR ? map_to_cta(&acc_empty[0], 0) : 0u, PAIR ? map_to_cta(&acc_empty[1], 0) : 0u};
+    int m_tile = walker % m_tiles, n_tile = walker / m_tiles;
     for (int t = walker; t < tiles; t += walkers, lt++) {
-      const int m0 = (t % m_tiles) * kTileM + (int)rank * kBlockM, n0 = (t / m_tiles) * BLOCK_N;
+      for (; m_tile >= m_tiles; m_tile -= m_tiles) n_tile++;
+      const int m0 = m_tile * kTileM + (int)rank * kBlockM, n0 = n_tile * BLOCK_N;
+      m_tile += walkers;
       const int buf = lt & 1;
       // (1) per-column constants of this tile (the main loop of this or the next tile is running).
       // Tiles are numbered row-block fastest, so a CTA's consecutive tiles mostly share their
