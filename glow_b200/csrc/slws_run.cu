@@ -23,7 +23,8 @@
 //   * large launches: U = 4, ten blocks of 64 threads on an SM (96 registers); 4-bit rows with four chunks
 //     per lane U = 8 and six blocks;
 //   * a launch too small to fill the SMs: U = 16, so that a bag of 32 rows is two dependent steps instead of
-//     eight (1024 bags of 64 columns: 18.3 + 3.5 us for the boundaries in a launch of their own -> 8.3 us).
+//     eight (1024 bags of 64 columns: 18.3 + 3.5 us for the boundaries in a launch of their own -> 8.3 us);
+//   * in between: U = 8, eight blocks.
 #include <climits>
 
 #include "slws.cuh"
@@ -67,7 +68,8 @@ __device__ __forceinline__ uint32_t ldg_any(const uint8_t *p, int valid, int row
   return __funnelshift_r(lo, hi, 8 * sh);
 }
 
-// Rows: BITS of a column, SO16 (scale and offset are halves), ALIGN (bytes every row starts on: 8, 4, 1)
+// Rows: BITS of a column, SO16 (scale and offset are halves), ALIGN (bytes every row starts on: 8, 4, 1 -- where
+// scale and offset are floats, 8 makes them one load: 91 bags of 4-bit rows as above 28.2 -> 17.2 us)
 template <int BITS, bool SO16, int ALIGN>
 struct Rows {
   static constexpr int kBytes = BITS;  // bytes of 8 columns
@@ -147,7 +149,7 @@ struct Rows {
 
 // P chunks per lane, U rows per step.
 template <int BITS, bool SO16, int ALIGN, int P, int U>
-__global__ void __launch_bounds__(kThreads, U == 16 ? 4 : P == 4 ? 6 : 10)
+__global__ void __launch_bounds__(kThreads, U == 16 ? 4 : P == 4 ? 6 : U == 8 ? 8 : 10)
 slws_run_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp) {
   pdl_wait();
   pdl_launch_dependents();
@@ -379,8 +381,9 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp) {
 }
 
 template <int BITS, bool SO16, int ALIGN>
-cudaError_t launch_rows(const SlwsLaunch &L, int P, bool small, dim3 grid, int bpw, cudaStream_t s) {
-  if (small) {
+cudaError_t launch_rows(const SlwsLaunch &L, int P, int U, dim3 grid, int bpw, cudaStream_t s) {
+  if (U == 8) return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 1, 8>, grid, kThreads, 0, s, L, bpw);
+  if (U == 16) {
     if (P == 1) return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 1, 16>, grid, kThreads, 0, s, L, bpw);
     if (P == 2) return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 2, 16>, grid, kThreads, 0, s, L, bpw);
     return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 4, 16>, grid, kThreads, 0, s, L, bpw);
@@ -393,27 +396,51 @@ cudaError_t launch_rows(const SlwsLaunch &L, int P, bool small, dim3 grid, int b
 }  // namespace
 
 cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
-  const int chunks = L.out_line / 8, P = chunks_per_lane(chunks, L.kind >= 2);
-  L.lpr_log2 = 2;  // (four lanes at least: they hold a step's indices)
-  while ((P << L.lpr_log2) < chunks) L.lpr_log2++;
-  // A warp's run: one bag per group in small launches; up to 32 bags once that still leaves every SM two
-  // dozen warps (skewed bags even out over a run: 8 bags per warp took 702 us where 32 take 540).
+  const int chunks = L.out_line / 8;
   const int64_t total = max_segments * num_jobs, sms = sm_count();
-  int bpw = 32 >> L.lpr_log2;
-  while (bpw < kMaxRun && total / (2 * bpw) >= sms * 24) bpw *= 2;
-  const int64_t warps = (max_segments + bpw - 1) / bpw;
-  const bool small = warps * num_jobs <= sms * 8;
+  auto lanes_log2 = [&](int per_lane) {
+    int l = 2;  // (four lanes at least: they hold a step's indices)
+    while ((per_lane << l) < chunks) l++;
+    return l;
+  };
+  auto warps_for = [&](int bags) { return (max_segments + bags - 1) / bags; };
+  // Small and medium launches are bound by the chain of steps of the longest bag, and with a warp or two per
+  // scheduler by that warp's own instructions: 16 (8) rows per step, and one chunk per lane, so that a bag is
+  // spread over more lanes and the bags over more warps.  A column's sum is the same either way.  18 tables,
+  // 91 bags of up to 200 rows of 64 columns: 20.8 -> 15.9 us; 16 tables, 256 bags of 192 columns: 55 -> 37;
+  // 1024 bags of 64 columns: 8.2 -> 7.0.  Above 32 warps per SM the fewer rows in flight of more warps win.
+  int P = 1, bpw = 0, U = 4;
+  if (chunks <= 32) {
+    L.lpr_log2 = lanes_log2(1);
+    bpw = 32 >> L.lpr_log2;
+    const int64_t n = warps_for(bpw) * num_jobs;
+    U = n <= sms * 8 ? 16 : n <= sms * 32 ? 8 : 4;
+  }
+  if (U == 4) {
+    P = chunks_per_lane(chunks, L.kind >= 2);
+    L.lpr_log2 = lanes_log2(P);
+    // A warp's run: one bag per group in small launches; up to 32 bags once that still leaves every SM two
+    // dozen warps (skewed bags even out over a run: 8 bags per warp took 702 us where 32 take 540), one dozen
+    // where eight groups of a warp would wait for its longest bag (20 tables, 2000 skewed bags of 64 columns:
+    // 99 -> 72 us; with four chunks per lane half the runs cost 4-bit tables 147 against 119).
+    bpw = 32 >> L.lpr_log2;
+    const int64_t enough = sms * (bpw >= 8 && P <= 2 ? 12 : 24);
+    while (bpw < kMaxRun && total / (2 * bpw) >= enough) bpw *= 2;
+    if (warps_for(bpw) * num_jobs <= sms * 8) U = 16;
+  }
+  const int64_t warps = warps_for(bpw);
   const dim3 grid((unsigned)((warps + kWarps - 1) / kWarps), (unsigned)num_jobs);
   switch (L.kind) {
     case GLOWB200_UINT8_FUSED:
-      if (align == 8) return launch_rows<8, false, 8>(L, P, small, grid, bpw, s);
-      return align == 4 ? launch_rows<8, false, 4>(L, P, small, grid, bpw, s) : launch_rows<8, false, 1>(L, P, small, grid, bpw, s);
+      if (align == 8) return launch_rows<8, false, 8>(L, P, U, grid, bpw, s);
+      return align == 4 ? launch_rows<8, false, 4>(L, P, U, grid, bpw, s) : launch_rows<8, false, 1>(L, P, U, grid, bpw, s);
     case GLOWB200_UINT8_FUSED_FP16:
-      return align >= 4 ? launch_rows<8, true, 4>(L, P, small, grid, bpw, s) : launch_rows<8, true, 1>(L, P, small, grid, bpw, s);
+      return align >= 4 ? launch_rows<8, true, 4>(L, P, U, grid, bpw, s) : launch_rows<8, true, 1>(L, P, U, grid, bpw, s);
     case GLOWB200_UINT4_FUSED:
-      return align >= 4 ? launch_rows<4, false, 4>(L, P, small, grid, bpw, s) : launch_rows<4, false, 1>(L, P, small, grid, bpw, s);
+      if (align == 8) return launch_rows<4, false, 8>(L, P, U, grid, bpw, s);
+      return align >= 4 ? launch_rows<4, false, 4>(L, P, U, grid, bpw, s) : launch_rows<4, false, 1>(L, P, U, grid, bpw, s);
     default:
-      return align >= 4 ? launch_rows<4, true, 4>(L, P, small, grid, bpw, s) : launch_rows<4, true, 1>(L, P, small, grid, bpw, s);
+      return align >= 4 ? launch_rows<4, true, 4>(L, P, U, grid, bpw, s) : launch_rows<4, true, 1>(L, P, U, grid, bpw, s);
   }
 }
 

@@ -135,3 +135,21 @@ def test_rows_that_are_not_finite(dim):
     assert (np.isnan(got) == np.isnan(want)).all() and (got[np.isinf(want)] == want[np.isinf(want)]).all()
     assert fine.any(1).sum() == 4
     check(got[fine], want[fine], size[fine], 1e-5)
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 64), (2, 64), (2, 40), (1, 192), (3, 256)])
+@pytest.mark.parametrize("bags", [600, 5000, 20_000, 70_000])
+def test_launches_of_every_tier_agree(bags, kind, dim):
+    """Sixteen, eight and four rows per step, one chunk per lane and several, runs of one bag per group and of more:
+    the same bits as the bag pooled alone."""
+    rng = np.random.default_rng(bags + dim)
+    table = dev(make_table(kind, 3000, dim, 3))
+    lengths = rng.choice([0, 1, 3, 7, 8, 9, 16, 17, 40], bags).astype(np.int32)
+    lengths[bags // 2] = 200
+    n = int(lengths.sum())
+    idx, w = rng.integers(0, 3000, n), rng.normal(0, 1, n).astype(np.float16 if kind & 1 else np.float32)
+    whole = pool(table, w, idx, lengths, kind)
+    ends = np.cumsum(lengths)
+    for b in [0, bags // 2, bags - 1] + list(rng.integers(0, bags, 5)):
+        e, l = int(ends[b]), int(lengths[b])
+        assert torch.equal(pool(table, w[e - l:e], idx[e - l:e], lengths[b:b + 1], kind)[0], whole[b])
