@@ -382,6 +382,9 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp) {
 
 template <int BITS, bool SO16, int ALIGN>
 cudaError_t launch_rows(const SlwsLaunch &L, int P, int U, dim3 grid, int bpw, cudaStream_t s) {
+  if constexpr (BITS == 4) {
+    if (U == 8 && P == 2) return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 2, 8>, grid, kThreads, 0, s, L, bpw);
+  }
   if (U == 8) return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 1, 8>, grid, kThreads, 0, s, L, bpw);
   if (U == 16) {
     if (P == 1) return launch_pdl(slws_run_kernel<BITS, SO16, ALIGN, 1, 16>, grid, kThreads, 0, s, L, bpw);
@@ -426,7 +429,11 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
     bpw = 32 >> L.lpr_log2;
     const int64_t enough = sms * (bpw >= 8 && P <= 2 ? 12 : 24);
     while (bpw < kMaxRun && total / (2 * bpw) >= enough) bpw *= 2;
-    if (warps_for(bpw) * num_jobs <= sms * 8) U = 16;
+    const int64_t n = warps_for(bpw) * num_jobs;
+    if (n <= sms * 8) U = 16;
+    // (two 4-bit chunks are eight bytes: eight rows of them still fit the registers.  64 tables, 1000 skewed bags
+    // of 64 columns: 131 -> 92 us; two uint8 chunks would make it eight rows for 20 tables 43 -> 51)
+    else if (P == 2 && L.kind >= 2 && n <= sms * 48) U = 8;
   }
   const int64_t warps = warps_for(bpw);
   const dim3 grid((unsigned)((warps + kWarps - 1) / kWarps), (unsigned)num_jobs);
