@@ -52,30 +52,31 @@ __global__ void __launch_bounds__(256) pairwise_dot_kernel(const float *__restri
   }
 }
 
-// (Measured on B200, 512 and 4096 samples of 65 x 128: this kernel 21 / 138 us.  An 8 x 4 tile
-// variant over a transposed copy in shared memory with packed f32x2 FMAs and a staged, coalesced
-// result row executed 15 % fewer instructions but ran at half the warps per SM and came out at
-// 27 / 138 us: both forms issue about one instruction every other cycle per scheduler, so it is
-// latency at low occupancy, not shared-memory bandwidth, that bounds them.)
-// The same result from 4 x 4 register tiles (D a multiple of 4): a thread owns the dots of rows
-// bi + r*nb against rows bj + s*nb (r, s = 0..3, nb = ceil(n / 4), bj <= bi) and walks k four at a time with 16-byte
-// shared-memory loads -- 8 loads feed 64 FMAs instead of 2 loads per FMA, which is what bounded
+// The same result from R x R register tiles (D a multiple of 4): a thread owns the dots of rows
+// bi + r*nb against rows bj + s*nb (r, s < R, nb = ceil(n / R), bj <= bi) and walks k four at a time with 16-byte
+// shared-memory loads -- with R = 4, 8 loads feed 64 FMAs instead of 2 loads per FMA, which is what bounded
 // the kernel above.  Every dot still is the sequential FMA chain over k = 0..D-1, so the bits are
 // the same.  Rows are padded by 4 floats (D + 4, an odd number of 16-byte units for D a multiple of 8) so that
 // the neighbouring rows a warp reads fall into different banks.
-__global__ void __launch_bounds__(256) pairwise_dot_tiled_kernel(const float *__restrict__ dense, int64_t ld_dense,
+// What bounds it is latency: both forms tried for many vectors -- this one, and 8 x 4 tiles over a transposed copy with
+// packed FMAs -- issue about one instruction every other cycle per scheduler (4096 samples of 65 x 128: 138 us;
+// smaller blocks or fewer registers per thread did not help).  Few vectors have few tiles -- 28 of 4 x 4 for 27
+// vectors, the rest of the block idle -- and go in 2 x 2 tiles with no more warps than those fill: 128 samples of
+// 27 x 64 5.4 -> 3.5 us, 4096 samples 35 -> 22, 2048 of 17 x 32 15.0 -> 5.4.
+template <int R>
+__global__ void __launch_bounds__(256, 4) pairwise_dot_tiled_kernel(const float *__restrict__ dense, int64_t ld_dense,
                                                                  const float *__restrict__ pooled, int64_t ld_pooled,
                                                                  int tables, int D, float *__restrict__ out_f,
                                                                  int8_t *__restrict__ out_q, int64_t ld_out, float q_scale,
                                                                  int32_t q_offset, int vec_in) {
   pdl_wait();               // (launched as a programmatic dependent of the pooling kernel)
   pdl_launch_dependents();  // a contraction that follows may set up now (it waits for this kernel before its loads)
-  extern __shared__ __align__(16) float v[];  // [4 * ceil(n / 4)][D + 4]; rows beyond n are zero
-  const int n = tables + 1, pitch = D + 4, nb = (n + 3) >> 2;
+  extern __shared__ __align__(16) float v[];  // [R * ceil(n / R)][D + 4]; rows beyond n are zero
+  const int n = tables + 1, pitch = D + 4, nb = (n + R - 1) / R;
   const int64_t b = blockIdx.x;
   if (vec_in) {
     const int q = D >> 2;
-    for (int i = threadIdx.x; i < nb * 4 * q; i += blockDim.x) {
+    for (int i = threadIdx.x; i < nb * R * q; i += blockDim.x) {
       const int r = i / q, k = (i - r * q) * 4;
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
       if (r < n) x = r == 0 ? __ldg(reinterpret_cast<const float4 *>(dense + b * ld_dense + k))
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256) pairwise_dot_tiled_kernel(const float *__
       *reinterpret_cast<float4 *>(v + r * pitch + k) = x;
     }
   } else {
-    for (int i = threadIdx.x; i < nb * 4 * D; i += blockDim.x) {
+    for (int i = threadIdx.x; i < nb * R * D; i += blockDim.x) {
       const int r = i / D, k = i - r * D;
       v[r * pitch + k] = r >= n ? 0.0f : (r == 0 ? dense[b * ld_dense + k] : pooled[b * ld_pooled + (int64_t)(r - 1) * D + k]);
     }
@@ -110,22 +111,22 @@ __global__ void __launch_bounds__(256) pairwise_dot_tiled_kernel(const float *__
     // threads then read neighbouring rows, which the odd pitch / 4 spreads over all banks
     const float *a = v + bi * pitch, *c = v + bj * pitch;
     const int tile_step = nb * pitch;
-    float acc[4][4];
+    float acc[R][R];
 #pragma unroll
-    for (int r = 0; r < 4; r++)
+    for (int r = 0; r < R; r++)
 #pragma unroll
-      for (int s = 0; s < 4; s++) acc[r][s] = 0.0f;
+      for (int s = 0; s < R; s++) acc[r][s] = 0.0f;
     for (int k = 0; k < D; k += 4) {
-      float4 x[4], y[4];
+      float4 x[R], y[R];
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
+      for (int r = 0; r < R; r++) {
         x[r] = *reinterpret_cast<const float4 *>(a + r * tile_step + k);
         y[r] = *reinterpret_cast<const float4 *>(c + r * tile_step + k);
       }
 #pragma unroll
-      for (int r = 0; r < 4; r++)
+      for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int s = 0; s < 4; s++) {
+        for (int s = 0; s < R; s++) {
           acc[r][s] = fmaf(x[r].x, y[s].x, acc[r][s]);
           acc[r][s] = fmaf(x[r].y, y[s].y, acc[r][s]);
           acc[r][s] = fmaf(x[r].z, y[s].z, acc[r][s]);
@@ -133,9 +134,9 @@ __global__ void __launch_bounds__(256) pairwise_dot_tiled_kernel(const float *__
         }
     }
 #pragma unroll
-    for (int r = 0; r < 4; r++)
+    for (int r = 0; r < R; r++)
 #pragma unroll
-      for (int s = 0; s < 4; s++) {
+      for (int s = 0; s < R; s++) {
         // a dot product is symmetric: the tile of two different residue classes holds every
         // pair between them once; the diagonal tile holds each pair twice and keeps one
         const int i = bi + r * nb, j = bj + s * nb;
@@ -162,18 +163,18 @@ extern "C" int glowb200_pairwise_dot_interaction(const float *dense, int64_t ld_
   const int64_t n = tables + 1, width = dim + n * (n - 1) / 2;
   GLOWB200_REQUIRE(ld_out >= width && ld_dense >= dim && ld_pooled >= tables * dim, "row pitch smaller than the row");
   cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
-  const size_t tiled_smem = (size_t)((n + 3) / 4 * 4) * (dim + 4) * sizeof(float);
+  auto tiles_of = [&](int64_t r) { return ((n + r - 1) / r) * ((n + r - 1) / r + 1) / 2; };
+  const int R = tiles_of(4) >= 80 ? 4 : 2;  // (66 tiles -- 41 vectors -- still gain from the smaller ones)
+  const size_t tiled_smem = (size_t)((n + R - 1) / R * R) * (dim + 4) * sizeof(float);
   if ((dim % 4) == 0 && tiled_smem <= 200 * 1024) {
-    static int raised_for[64];  // largest dynamic shared-memory size enabled so far, per device
-    int dev = 0;
-    GLOWB200_CUDA_OK(cudaGetDevice(&dev));
-    if (tiled_smem > 48 * 1024 && (int)tiled_smem > raised_for[dev & 63]) {
-      GLOWB200_CUDA_OK(cudaFuncSetAttribute(pairwise_dot_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_smem));
-      raised_for[dev & 63] = (int)tiled_smem;
-    }
+    auto kernel = R == 4 ? pairwise_dot_tiled_kernel<4> : pairwise_dot_tiled_kernel<2>;
+    if (tiled_smem > 48 * 1024)
+      GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_smem));
+    const int64_t warps = (tiles_of(R) + 31) / 32;
+    const unsigned threads = R == 4 ? 256 : 32 * (unsigned)(warps < 2 ? 2 : warps > 8 ? 8 : warps);
     const int vec_in = (reinterpret_cast<uintptr_t>(dense) % 16 == 0) && (ld_dense % 4 == 0) &&
                        (tables == 0 || (reinterpret_cast<uintptr_t>(pooled) % 16 == 0 && ld_pooled % 4 == 0));
-    GLOWB200_CUDA_OK(launch_pdl(pairwise_dot_tiled_kernel, (unsigned)batch, 256, tiled_smem, cs, dense, ld_dense, pooled, ld_pooled,
+    GLOWB200_CUDA_OK(launch_pdl(kernel, (unsigned)batch, threads, tiled_smem, cs, dense, ld_dense, pooled, ld_pooled,
                                 (int)tables, (int)dim, out_f32, out_i8, ld_out, quant_scale, quant_offset, vec_in));
     return GLOWB200_OK;
   }

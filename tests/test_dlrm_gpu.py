@@ -92,6 +92,15 @@ def test_interaction_kernel_bit_exact(oracle, B, T, D):
     np.testing.assert_array_equal(gq.cpu().numpy(), oracle.element_quantize_i8(want, sc, off))
 
 
+@pytest.mark.parametrize("T,D", [(1, 4), (2, 16), (26, 64), (43, 12), (44, 12), (47, 64), (48, 64)])
+def test_interaction_tiles_bit_exact(oracle, T, D):
+    """Numbers of vectors round the change of tile size and off both tiles' multiples."""
+    rng = np.random.default_rng(T)
+    dense, pooled = rng.standard_normal((7, D)).astype(np.float32), rng.standard_normal((7, T, D)).astype(np.float32)
+    got = ops.pairwise_dot_interaction(torch.from_numpy(dense).to(DEV), torch.from_numpy(pooled).to(DEV))
+    np.testing.assert_array_equal(got.cpu().numpy().view(np.uint32), oracle.pairwise_dot_interaction(dense, pooled).view(np.uint32))
+
+
 @pytest.mark.parametrize("world", [2, 3])
 def test_partitioned_equals_unpartitioned(model, world):
     cfg, tables, fm, qm = model
