@@ -1099,7 +1099,7 @@ def run_slws4_line(args):
                          # DRAM bytes per launch: 196 B per row in the ncu capture of a smaller case of D=128
                          # (profiles/), scaled by the rows of a launch; not captured for the other widths
                          "traffic": 196.0 * float(np.mean([int(rq[3][-1]) for rq in reqs])) if D == 128 else None,
-                         "kernel": "slws_gather_select_kernel<4,1,1,long,P>",
+                         "kernel": "slws_run_kernel<4,1,4,P,U>",
                          "rows_per_s": sum(int(reqs[i % R][3][-1]) for i in range(args.steps)) / (ms * 1e-3)},
             "gpu_launches": 2 * args.steps, "clocks": clocks}
         if world == 1 and not args.no_cpu_baseline:
@@ -1467,7 +1467,7 @@ def run_slws4_sharded_line(args):
                        "dim": D, "tables": T, "l2_policy": "tables far larger than L2, uniform indices"},
             "roofline": {"bound": "hbm", "achieved": per_gpu, "peak": peak, "unit": "GB/s", "frac": per_gpu / peak,
                          "peak_source": src, "traffic": None,
-                         "kernel": "slws_gather_select_kernel<4,1,0,long,P,U,sharded> + sum_partials_kernel"},
+                         "kernel": "slws_run_kernel<4,1,4,P,U> over shards + sum_partials_kernel"},
             "gpu_launches": 3 * args.steps, "clocks": clocks}))
     if world > 1:
         dist.destroy_process_group()
@@ -1795,7 +1795,7 @@ def main():
                          "nominal_peak": 8000.0, "frac_of_nominal": achieved / 8000.0,
                          # DRAM bytes per launch: bytes per gathered row from the ncu capture x the rows
                          "traffic": (None if args.row_bytes else NCU_DRAM_BYTES_PER_ROW * rows_per_launch),
-                         "kernel": "slws_gather_select_kernel<8,0,0,long,2,4> (+ slws_segments_from_lengths_kernel, timed together)",
+                         "kernel": "slws_run_kernel<8,0,8,2,4> (one launch: the warps add up the lengths themselves)",
                          "launch_us": launch_us, "algorithmic_bytes_per_launch": moved / args.steps},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d // e2e_steps,
                     "d2h_bytes_per_step": d2h // e2e_steps, "steps": e2e_steps,

@@ -214,7 +214,7 @@ class ResNet50Int8:
         return ops.channelwise_quantized_conv2d_add(*args, residual, *add, **kw)
 
     # Images up to which the layers between Quantize and the FC are replayed from a CUDA graph (from the second
-    # call of a shape on): their 73 launches cost the host 4 us each, which is more than the device needs for
+    # call of a shape on): their 56 launches cost the host 4 us each, which is more than the device needs for
     # them below about 20 images of 224 x 224 (one image: 480 us from the host, 300 replayed).
     REPLAY_PIXELS = 20 * 224 * 224
 
