@@ -67,6 +67,9 @@ __global__ void __launch_bounds__(kSegThreads) slws_segments_from_lengths_kernel
   pdl_wait();               // the gather before this one may still read the boundaries this kernel rewrites
   pdl_launch_dependents();  // this launch's gather may take its place on the SMs (it waits before reading them)
   __shared__ int64_t warp_tot[33];
+  __shared__ int longest;
+  if (threadIdx.x == 0) longest = 0;
+  int32_t my_longest = 0;
   const glowb200_slws_job job = p.jobs ? p.jobs[blockIdx.x] : p.single;
   int64_t *out = p.seg_begin + (int64_t)blockIdx.x * p.seg_stride;
   int32_t flags = 0;
@@ -84,6 +87,7 @@ __global__ void __launch_bounds__(kSegThreads) slws_segments_from_lengths_kernel
       if (l < 0) { l = 0; flags |= GLOWB200_STATUS_NEGATIVE_LENGTH; }
       v[i] = l;
       sum += l;
+      my_longest = max(my_longest, (int32_t)l);
     }
     int64_t tile_total;
     int64_t run = carry + block_exclusive_scan(sum, warp_tot, tile_total);
@@ -94,9 +98,14 @@ __global__ void __launch_bounds__(kSegThreads) slws_segments_from_lengths_kernel
     }
     carry += tile_total;
   }
+  my_longest = __reduce_max_sync(0xffffffffu, my_longest);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicMax(&longest, my_longest);
+  __syncthreads();
   if (threadIdx.x == 0) {
     if (carry > N) flags |= GLOWB200_STATUS_LENGTHS_OVERRUN;
     out[S] = carry < N ? carry : N;
+    out[S + 1] = 2 * S * ((int64_t)longest - 16) > 5 * carry;  // skewed: the longest bag a step's rows beyond 2.5 times the mean
   }
   raise_status(p.status, flags);
 }
@@ -111,6 +120,7 @@ __global__ void __launch_bounds__(256) slws_segments_from_offsets_kernel(const _
     if (v < 0) { v = 0; flags |= GLOWB200_STATUS_BAD_OFFSETS; }
     if (v > N) { v = N; flags |= GLOWB200_STATUS_BAD_OFFSETS; }
     p.seg_begin[i] = v;
+    if (i == S) p.seg_begin[S + 1] = 0;
   }
   raise_status(p.status, flags);
 }

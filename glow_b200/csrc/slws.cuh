@@ -8,7 +8,7 @@ namespace glowb200 {
 struct SlwsLaunch {
   const glowb200_slws_job *jobs;  // device array, or nullptr when `single` is the only job
   glowb200_slws_job single;
-  int64_t *seg_begin;  // workspace: per job an int64 [segments + 1] array
+  int64_t *seg_begin;  // workspace: per job an int64 [segments + 1] array, then a word: are its lengths skewed?
   int64_t seg_stride;  // int64 elements between the arrays of consecutive jobs
   int64_t max_segments;  // bags a table's array has room for (a descriptor naming more is cut short)
   int32_t *status;
@@ -19,6 +19,7 @@ struct SlwsLaunch {
   // slws_run.cu: element types that need no kernel of their own, and whether the warps add up the
   // lengths before their bags themselves (no boundary array exists then)
   int32_t kind, idx64, out16, inline_lengths;
+  int32_t skewed_run;  // bags of a warp of a table with skewed lengths (the word behind its boundaries is not 0)
 };
 
 // Bags of a table as the kernels walk them: never more than its boundary array has room for.

@@ -150,7 +150,7 @@ struct Rows {
 // P chunks per lane, U rows per step.
 template <int BITS, bool SO16, int ALIGN, int P, int U>
 __global__ void __launch_bounds__(kThreads, U == 16 ? 4 : P == 4 ? 6 : U == 8 ? 8 : 10)
-slws_run_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp) {
+slws_run_kernel(const __grid_constant__ SlwsLaunch p, int even_run) {
   pdl_wait();
   pdl_launch_dependents();
   using R = Rows<BITS, SO16, ALIGN>;
@@ -158,6 +158,9 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp) {
   const glowb200_slws_job *jp = p.jobs ? p.jobs + blockIdx.y : &p.single;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t segments = bags_of(p, jp);
+  // (a table whose longest bag stands out: longer runs, the surplus blocks leave)
+  const int bags_per_warp =
+      !p.inline_lengths && p.seg_begin[(int64_t)blockIdx.y * p.seg_stride + segments + 1] != 0 ? p.skewed_run : even_run;
   const int64_t first_bag = ((int64_t)blockIdx.x * kWarps + warp) * bags_per_warp;
   if (first_bag >= segments) return;  // whole warps leave together
   const int n_bags = (int)(first_bag + bags_per_warp < segments ? bags_per_warp : segments - first_bag);
@@ -423,18 +426,31 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
     P = chunks_per_lane(chunks, L.kind >= 2);
     L.lpr_log2 = lanes_log2(P);
     // A warp's run: one bag per group in small launches; up to 32 bags once that still leaves every SM two
-    // dozen warps (skewed bags even out over a run: 8 bags per warp took 702 us where 32 take 540), one dozen
-    // where eight groups of a warp would wait for its longest bag (20 tables, 2000 skewed bags of 64 columns:
-    // 99 -> 72 us; with four chunks per lane half the runs cost 4-bit tables 147 against 119).
+    // dozen warps, one dozen where eight groups of a warp would wait for its longest bag.  Skewed tables (the
+    // boundaries' kernel knows) even out over such runs: 702 us with runs of 8, 540 with 32.  The others
+    // take them as long as the warps still fill the rounds in which they become resident, or all fit one:
+    // 12 tables, 8192 bags of 64 rows of 64 columns, 1.04 rounds of runs of 32 295 us, 4.2 rounds of 8 221; 20
+    // tables, 2000 skewed bags, 1.7 rounds of 8 99 us, one of 16 72.
+    const bool wide_steps = L.kind >= 2 && P == 2;
+    const int64_t resident = sms * (P == 4 ? 12 : wide_steps ? 16 : 20);
+    auto filled = [&](int bags) {  // of the slots of those rounds, per cent
+      const int64_t n = warps_for(bags) * num_jobs;
+      return 100 * n / ((n + resident - 1) / resident * resident);
+    };
     bpw = 32 >> L.lpr_log2;
     const int64_t enough = sms * (bpw >= 8 && P <= 2 ? 12 : 24);
-    while (bpw < kMaxRun && total / (2 * bpw) >= enough) bpw *= 2;
-    const int64_t n = warps_for(bpw) * num_jobs;
-    if (n <= sms * 8) U = 16;
+    int64_t best = filled(bpw);
+    for (int run = 2 * bpw; run <= kMaxRun && total / run >= enough; run *= 2) {
+      L.skewed_run = run;
+      if (filled(run) * 100 >= best * 95 || warps_for(run) * num_jobs <= resident) bpw = run;
+      if (filled(run) > best) best = filled(run);
+    }
+    if (warps_for(bpw) * num_jobs <= sms * 8) U = 16;
     // (two 4-bit chunks are eight bytes: eight rows of them still fit the registers.  64 tables, 1000 skewed bags
     // of 64 columns: 131 -> 92 us; two uint8 chunks would make it eight rows for 20 tables 43 -> 51)
-    else if (P == 2 && L.kind >= 2 && n <= sms * 48) U = 8;
+    else if (wide_steps) U = 8;
   }
+  if (L.skewed_run < bpw) L.skewed_run = bpw;
   const int64_t warps = warps_for(bpw);
   const dim3 grid((unsigned)((warps + kWarps - 1) / kWarps), (unsigned)num_jobs);
   switch (L.kind) {
