@@ -430,7 +430,9 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
     // boundaries' kernel knows) even out over such runs: 702 us with runs of 8, 540 with 32.  The others
     // take them as long as the warps still fill the rounds in which they become resident, or all fit one:
     // 12 tables, 8192 bags of 64 rows of 64 columns, 1.04 rounds of runs of 32 295 us, 4.2 rounds of 8 221; 20
-    // tables, 2000 skewed bags, 1.7 rounds of 8 99 us, one of 16 72.
+    // tables, 2000 skewed bags, 1.7 rounds of 8 99 us, one of 16 72.  With eight groups to a warp and the skew
+    // known a bag per group is the better run even in full rounds (40 4-bit tables of 32 columns 524 -> 502 us);
+    // with four the blocks that skewed tables then leave over cost more (64 of them: 569 -> 606).
     const bool wide_steps = L.kind >= 2 && P == 2;
     const int64_t resident = sms * (P == 4 ? 12 : wide_steps ? 16 : 20);
     auto filled = [&](int bags) {  // of the slots of those rounds, per cent
@@ -439,10 +441,11 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
     };
     bpw = 32 >> L.lpr_log2;
     const int64_t enough = sms * (bpw >= 8 && P <= 2 ? 12 : 24);
+    const int lpr = 1 << L.lpr_log2;
     int64_t best = filled(bpw);
     for (int run = 2 * bpw; run <= kMaxRun && total / run >= enough; run *= 2) {
       L.skewed_run = run;
-      if (filled(run) * 100 >= best * 95 || warps_for(run) * num_jobs <= resident) bpw = run;
+      if (((lpr > 4 || L.inline_lengths) && filled(run) * 100 >= best * 95) || warps_for(run) * num_jobs <= resident) bpw = run;
       if (filled(run) > best) best = filled(run);
     }
     if (warps_for(bpw) * num_jobs <= sms * 8) U = 16;
