@@ -274,9 +274,9 @@ __global__ void __launch_bounds__(kGatherThreads, P == 4 ? 8 : 12) slws_gather_k
     for (int i = 0; i < 4; i++) h[i] = __floats2half2_rn(acc[c][2 * i], acc[c][2 * i + 1]);
     if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
       *reinterpret_cast<uint4 *>(d) = *reinterpret_cast<const uint4 *>(h);
-    } else {
+    } else {  // a result may start at any element
 #pragma unroll
-      for (int i = 0; i < 4; i++) *reinterpret_cast<__half2 *>(d + 2 * i) = h[i];
+      for (int i = 0; i < 8; i++) d[i] = i & 1 ? __high2half(h[i / 2]) : __low2half(h[i / 2]);
     }
   }
   raise_status(p.status, flags);

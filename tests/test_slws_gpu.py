@@ -146,6 +146,29 @@ def test_parity_fp16_accumulation_is_bit_exact(oracle, kind, dim):
     np.testing.assert_array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("kind", [1, 3])
+@pytest.mark.parametrize("shift,stride", [(0, 0), (1, 0), (2, 0), (3, 1)])
+def test_fp16_accumulation_into_rows_at_any_element(oracle, kind, shift, stride):
+    """A result may begin at any element, and a batched launch's rows may lie any number of elements apart."""
+    dim, rows, B = 24, 900, 70
+    table = make_table(kind, rows, dim, 3)
+    lengths, idx, w = workloads.bags_poisson(B, 9, 0, 20, rows, 5, 1, np.int64, np.float16)
+    want = oracle.frwq_slws_interp(table, kind, w, idx, lengths, fp16_acc=True)
+    dev = lambda a: torch.from_numpy(a).to(DEV)
+    st, pitch = ops.new_status(DEV), dim + stride
+    flat = torch.full((shift + B * pitch,), 7.0, dtype=torch.float16, device=DEV)
+    args = dev(table), dev(w), dev(idx), dev(lengths)
+    if stride:
+        batch = ops.SlwsBatch(kind, table.shape[1], torch.int64, use_fp16_accumulation=True, device=DEV)
+        batch.bind(*[[a] for a in args], [flat[shift:]], dest_stride=pitch).run(st)
+    else:
+        ops.fused_rowwise_quantized_sparse_lengths_weighted_sum(*args, kind, use_fp16_accumulation=True, status=st,
+                                                                out=flat[shift:].view(B, dim))
+    got = flat[shift:].view(B, pitch).cpu().numpy()
+    assert int(st.item()) == 0 and (got[:, dim:] == 7).all() and (flat[:shift] == 7).all()
+    np.testing.assert_array_equal(got[:, :dim].view(np.uint16), want.view(np.uint16))
+
+
 @pytest.mark.parametrize("kind,dim", [(0, 1), (0, 3), (0, 12), (1, 6), (2, 2), (3, 10), (3, 36), (0, 2000)])
 def test_any_shape_rows_are_bit_exact(oracle, kind, dim):
     """Odd widths take the any-shape kernel, which keeps the reference's operation order."""
