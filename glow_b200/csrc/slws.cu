@@ -4,9 +4,10 @@
 //
 // Launches:
 //   * a "segments" kernel turns lengths (or offsets) into validated bag boundaries in the caller's
-//     workspace, one int64 array per table (tables of up to 2048 bags pooled by slws_run.cu need none:
+//     workspace, one int64 array per table (tables of up to 2048 bags pooled with fp32 accumulation need none:
 //     their warps add up the lengths before their bags themselves);
-//   * fp32 accumulation over rows of a multiple of 8 columns is slws_run.cu's;
+//   * fp32 accumulation over rows of a multiple of 8 columns is slws_run.cu's and, in launches where the longest
+//     bag decides, slws_spread.cu's;
 //   * fp16 accumulation, which the reference rounds at every step, is done exactly that way, step by
 //     step, by slws_gather_kernel below: a group of `lpr` lanes (a power of two, 1..32) per bag, each
 //     lane with P chunks of 8 columns, indices read coalesced and handed round by shuffles, kUnroll rows
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(kSegThreads) slws_segments_from_lengths_kernel
   if (threadIdx.x == 0) {
     if (carry > N) flags |= GLOWB200_STATUS_LENGTHS_OVERRUN;
     out[S] = carry < N ? carry : N;
-    out[S + 1] = 2 * S * ((int64_t)longest - 16) > 5 * carry;  // skewed: the longest bag a step's rows beyond 2.5 times the mean
+    out[S + 1] = lengths_skewed(longest, carry, S);
   }
   raise_status(p.status, flags);
 }
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(256) slws_gather_any_kernel(const __grid_const
 struct GatherConfig {
   int kind, idx64, out16, acc16;
 };
-enum class Form { kAnyShape, kRuns, kFp16Steps };  // the any-shape kernel, slws_run.cu, slws_gather_kernel
+enum class Form { kAnyShape, kRuns, kFp16Steps };  // the any-shape kernel, slws_run.cu / slws_spread.cu, slws_gather_kernel
 
 template <int BITS, typename IdxT>
 cudaError_t launch_fp16_steps(SlwsLaunch L, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
@@ -412,7 +413,7 @@ int run_gather(const SlwsLaunch &L, const GatherConfig &g, Form form, int align,
   if (max_segments == 0 || num_jobs == 0) return GLOWB200_OK;
   cudaError_t e;
   if (form == Form::kRuns) {
-    e = launch_slws_run(L, align, max_segments, num_jobs, s);
+    e = launch_slws(L, align, max_segments, num_jobs, s);
   } else if (form == Form::kFp16Steps) {
     if (g.kind >= 2)
       e = g.idx64 ? launch_fp16_steps<4, int64_t>(L, max_segments, num_jobs, s) : launch_fp16_steps<4, int32_t>(L, max_segments, num_jobs, s);

@@ -6,8 +6,8 @@
 //     acc[k] = fma(w * scale, q[k], acc[k])   and   offsets = fma(w, offset, offsets)
 // (the reference's CPU backend is itself compiled with fast-math, so its float result is defined only
 // up to reassociation; tolerance 1e-5 relative).  Every bag is summed by one group in the same order
-// whatever else the launch holds, so a table gives the same bits pooled alone, beside others, in runs
-// or one bag per group.
+// whatever else the launch holds, so a table gives the same bits pooled alone, beside others, in runs,
+// one bag per group, or by slws_spread.cu.
 //
 // Why this shape.  The kernels before it gave an evenly filled table's bags one group each -- the groups of
 // a warp then wait for its longest bag -- and a skewed table's bags a whole warp each, which spent 42 warp
@@ -25,6 +25,7 @@
 //   * a launch too small to fill the SMs: U = 16, so that a bag of 32 rows is two dependent steps instead of
 //     eight (1024 bags of 64 columns: 18.3 + 3.5 us for the boundaries in a launch of their own -> 8.3 us);
 //   * in between: U = 8, eight blocks.
+// (The launches that slws_spread.cu takes are the smallest of rows of up to 256 columns.)
 #include <climits>
 
 #include "slws.cuh"
@@ -34,118 +35,6 @@ namespace {
 
 constexpr int kThreads = 64;  // a block's SM slots stay taken until its slowest warp is done: small blocks
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxRun = 32;   // bags of a warp: their boundaries live one per lane
-constexpr unsigned kAllLanes = 0xffffffffu;
-
-// Loads taken when `row` is not negative; otherwise the result is whatever the register held (such rows
-// get the weight 0).  Single volatile instructions: neither a branch round one nor a conversion of its
-// value may stand between the loads of a step.
-__device__ __forceinline__ uint32_t ldg_if(const void *p, int row) {
-  uint32_t v;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}" : "=r"(v) : "l"(p), "r"(row));
-  return v;
-}
-__device__ __forceinline__ uint2 ldg2_if(const void *p, int row) {
-  uint2 v;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %3, 0;\n\t@p ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
-      : "=r"(v.x), "=r"(v.y) : "l"(p), "r"(row));
-  return v;
-}
-// an index of either width
-__device__ __forceinline__ uint2 ldg_index(const void *p, int row, bool wide) {
-  uint2 v;
-  asm volatile("{\n\t.reg .pred p, q, a, b;\n\tsetp.ge.s32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tand.pred a, p, q;\n\tnot.pred q, q;\n\t"
-      "and.pred b, p, q;\n\t@a ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t@b ld.global.nc.u32 %0, [%2];\n\t}"
-      : "=r"(v.x), "=r"(v.y) : "l"(p), "r"(row), "r"((uint32_t)wide));
-  return v;
-}
-// four bytes at any address, `valid` of them (none if not positive) inside the row
-__device__ __forceinline__ uint32_t ldg_any(const uint8_t *p, int valid, int row) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-  const int sh = (int)(a & 3);
-  const uint8_t *w = p - sh;
-  const uint32_t lo = ldg_if(w, valid > 0 ? row : -1), hi = ldg_if(w + 4, sh != 0 && valid > 4 - sh ? row : -1);
-  return __funnelshift_r(lo, hi, 8 * sh);
-}
-
-// Rows: BITS of a column, SO16 (scale and offset are halves), ALIGN (bytes every row starts on: 8, 4, 1 -- where
-// scale and offset are floats, 8 makes them one load: 91 bags of 4-bit rows as above 28.2 -> 17.2 us)
-template <int BITS, bool SO16, int ALIGN>
-struct Rows {
-  static constexpr int kBytes = BITS;  // bytes of 8 columns
-
-  __device__ static __forceinline__ uint2 chunk(const uint8_t *at, int valid, int row) {
-    if constexpr (BITS == 4) {
-      if constexpr (ALIGN >= 4) return make_uint2(ldg_if(at, row), 0u);
-      else return make_uint2(ldg_any(at, valid, row), 0u);
-    } else {
-      if constexpr (ALIGN == 8) return ldg2_if(at, row);
-      else if constexpr (ALIGN == 4) return make_uint2(ldg_if(at, row), ldg_if(at + 4, row));
-      else return make_uint2(ldg_any(at, valid, row), ldg_any(at + 4, valid - 4, row));
-    }
-  }
-  // raw scale / offset words from the end of the row
-  __device__ static __forceinline__ uint2 tail(const uint8_t *end, int row) {
-    if constexpr (SO16) {
-      if constexpr (ALIGN >= 4) return make_uint2(ldg_if(end - 4, row), 0u);
-      else return make_uint2(ldg_any(end - 4, 4, row), 0u);
-    } else {
-      if constexpr (ALIGN == 8) return ldg2_if(end - 8, row);
-      else if constexpr (ALIGN == 4) return make_uint2(ldg_if(end - 8, row), ldg_if(end - 4, row));
-      else return make_uint2(ldg_any(end - 8, 8, row), ldg_any(end - 4, 4, row));
-    }
-  }
-  __device__ static __forceinline__ void scale_offset(uint2 t, float &scale, float &offset) {
-    if constexpr (SO16) {
-      const __half2 h = *reinterpret_cast<const __half2 *>(&t.x);
-      scale = __low2float(h);
-      offset = __high2float(h);
-    } else {
-      scale = __uint_as_float(t.x);
-      offset = __uint_as_float(t.y);
-    }
-  }
-  // acc[i] += a * q_i for the 8 columns of a chunk.
-  //  * uint8 rows: the byte dropped into the mantissa of 2^23, minus 2^23, is q exactly; sm_100's packed
-  //    two-lane add and fma (the roundings of the scalar forms, element by element).
-  //  * 4-bit rows: column 2m is the low nibble of byte m, column 2m+1 the high one
-  //    (include/glow/Quantization/Base/Base.h:399-406).  The nibbles are spread into bytes 0x8q (three
-  //    logic ops per 8 columns), a byte permute drops each into bits 16..23 of 0x3F80'0000, which
-  //    reads as m = 1 + q/128, and acc[i] += (128*a) * m.  The surplus sum_j 128*a_j is the same for
-  //    every column and is taken out once per row through the shared offset sum.  m is exact; the
-  //    products are about 8-128 times larger than the wanted a*q, which costs at most 7 of the 24
-  //    mantissa bits -- inside the fp32 tolerance.
-  static constexpr float kUnit = BITS == 4 ? 128.0f : 1.0f;
-  __device__ static __forceinline__ void pool(uint2 c, float a, uint64_t (&acc)[4]) {
-    uint64_t a2;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(a2) : "f"(a));
-    if constexpr (BITS == 8) {
-      uint64_t magic2;
-      asm("mov.b64 %0, {%1, %1};" : "=l"(magic2) : "f"(-8388608.0f));
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const uint32_t w = i < 2 ? c.x : c.y;
-        const uint32_t m0 = __byte_perm(w, 0x4B000000u, 0x7440 + 2 * (i & 1));  // {byte, 0, 0, 0x4B} = 2^23 + q
-        const uint32_t m1 = __byte_perm(w, 0x4B000000u, 0x7441 + 2 * (i & 1));
-        uint64_t q2;
-        asm("mov.b64 %0, {%1, %2};" : "=l"(q2) : "r"(m0), "r"(m1));
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(q2) : "l"(q2), "l"(magic2));
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(acc[i]) : "l"(a2), "l"(q2), "l"(acc[i]));
-      }
-    } else {
-      const uint32_t lo = (c.x & 0x0F0F0F0Fu) | 0x80808080u;         // columns 0,2,4,6 as bytes 0x8q
-      const uint32_t hi = ((c.x >> 4) & 0x0F0F0F0Fu) | 0x80808080u;  // columns 1,3,5,7
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const uint32_t m0 = __byte_perm(lo, 0x3F000000u, 0x7044 + (i << 8));  // {0, 0, byte i, 0x3F}
-        const uint32_t m1 = __byte_perm(hi, 0x3F000000u, 0x7044 + (i << 8));
-        uint64_t m2;
-        asm("mov.b64 %0, {%1, %2};" : "=l"(m2) : "r"(m0), "r"(m1));
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(acc[i]) : "l"(a2), "l"(m2), "l"(acc[i]));
-      }
-    }
-  }
-};
 
 // P chunks per lane, U rows per step.
 template <int BITS, bool SO16, int ALIGN, int P, int U>
@@ -162,7 +51,7 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int even_run) {
   const int bags_per_warp =
       !p.inline_lengths && p.seg_begin[(int64_t)blockIdx.y * p.seg_stride + segments + 1] != 0 ? p.skewed_run : even_run;
   const int64_t first_bag = ((int64_t)blockIdx.x * kWarps + warp) * bags_per_warp;
-  if (first_bag >= segments) return;  // whole warps leave together
+  if (first_bag >= segments || bags_per_warp == 0) return;  // whole warps leave together (0: the skewed tables are another launch's)
   const int n_bags = (int)(first_bag + bags_per_warp < segments ? bags_per_warp : segments - first_bag);
   const int lpr = 1 << p.lpr_log2, gl = lane & (lpr - 1);
   const int64_t N = jp->num_indices;
@@ -171,7 +60,7 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int even_run) {
   int32_t flags = 0;
 
   // ---- bag boundaries: lane l holds where bag l of the run begins, relative to the run, and how many
-  // rows it has ----
+  // rows it has (take_run, written out: behind a call the 256 even tables above took 0.7 % longer) ----
   int64_t begin = 0, len = 0;
   if (p.inline_lengths) {
     const int32_t *lengths = jp->lengths;
@@ -401,7 +290,7 @@ cudaError_t launch_rows(const SlwsLaunch &L, int P, int U, dim3 grid, int bpw, c
 
 }  // namespace
 
-cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
+cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s, bool skip_skewed) {
   const int chunks = L.out_line / 8;
   const int64_t total = max_segments * num_jobs, sms = sm_count();
   auto lanes_log2 = [&](int per_lane) {
@@ -412,9 +301,9 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
   auto warps_for = [&](int bags) { return (max_segments + bags - 1) / bags; };
   // Small and medium launches are bound by the chain of steps of the longest bag, and with a warp or two per
   // scheduler by that warp's own instructions: 16 (8) rows per step, and one chunk per lane, so that a bag is
-  // spread over more lanes and the bags over more warps.  A column's sum is the same either way.  18 tables,
-  // 91 bags of up to 200 rows of 64 columns: 20.8 -> 15.9 us; 16 tables, 256 bags of 192 columns: 55 -> 37;
-  // 1024 bags of 64 columns: 8.2 -> 7.0.  Above 32 warps per SM the fewer rows in flight of more warps win.
+  // spread over more lanes and the bags over more warps.  A column's sum is the same either way.  (Measured
+  // on launches that slws_spread.cu has taken since: 18 tables, 91 bags of up to 200 rows of 64 columns 20.8 -> 15.9 us;
+  // 1024 bags of 64 columns 8.2 -> 7.0.)  Above 32 warps per SM the fewer rows in flight of more warps win.
   int P = 1, bpw = 0, U = 4;
   if (chunks <= 32) {
     L.lpr_log2 = lanes_log2(1);
@@ -453,7 +342,8 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
     // of 64 columns: 131 -> 92 us; two uint8 chunks would make it eight rows for 20 tables 43 -> 51)
     else if (wide_steps) U = 8;
   }
-  if (L.skewed_run < bpw) L.skewed_run = bpw;
+  if (skip_skewed) L.skewed_run = 0;
+  else if (L.skewed_run < bpw) L.skewed_run = bpw;
   const int64_t warps = warps_for(bpw);
   const dim3 grid((unsigned)((warps + kWarps - 1) / kWarps), (unsigned)num_jobs);
   switch (L.kind) {

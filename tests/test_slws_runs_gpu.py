@@ -153,3 +153,71 @@ def test_launches_of_every_tier_agree(bags, kind, dim):
     for b in [0, bags // 2, bags - 1] + list(rng.integers(0, bags, 5)):
         e, l = int(ends[b]), int(lengths[b])
         assert torch.equal(pool(table, w[e - l:e], idx[e - l:e], lengths[b:b + 1], kind)[0], whole[b])
+
+
+def with_4bit_surplus(size, table, kind, w, idx, lengths):
+    """`size`, such that 1e-5 of it also holds what a bag of 4-bit rows may be off by that has q = 0 and hardly an
+    offset: the columns are summed as 128 * w * scale * (1 + q / 128) and the ones taken out again, two roundings of
+    2^-24 of sums of that size."""
+    if kind < 2:
+        return size
+    so = table[:, -(4 if kind & 1 else 8):].copy().view(np.float16 if kind & 1 else np.float32).astype(np.float64)
+    terms = np.concatenate([[0], np.cumsum(128 * np.abs(np.asarray(w, np.float64) * so[idx, 0])[:int(np.sum(lengths))])])
+    ends = np.cumsum(lengths)
+    return size + 1e5 * 2.0 ** -23 * (terms[ends] - terms[ends - lengths])[:, None]
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 48), (1, 64), (2, 40), (3, 64), (2, 96), (3, 128), (2, 136), (3, 256), (1, 128)])
+@pytest.mark.parametrize("bags", [700, 2500, 6000])
+def test_tables_of_every_skew_in_one_launch(kind, dim, bags):
+    """Even tables, skewed ones, an empty one and one of a single long bag, pooled by one launch whose tables may take
+    different kernels: the sums of the operator, and the bits of each table pooled alone."""
+    rng = np.random.default_rng(dim + bags)
+    laws = [rng.integers(18, 23, bags), rng.choice(EDGES[:24] + [200] * 2, bags), np.zeros(bags, int),
+            np.eye(1, bags, bags // 3, dtype=int)[0] * 600, rng.integers(0, 3, bags)]
+    tables, w, idx, lengths, alone = [], [], [], [], []
+    status = ops.new_status(DEV)
+    for law in laws:
+        t, l = make_table(kind, 900, dim, len(tables)), law.astype(np.int32)
+        n = int(l.sum())
+        i, x = rng.integers(0, 900, n + 1), rng.normal(0, 1, n + 1).astype(np.float16 if kind & 1 else np.float32)
+        tables.append(dev(t)), w.append(dev(x)), idx.append(dev(i)), lengths.append(dev(l))
+        alone.append(pool(tables[-1], x, i, l, kind, status=status))
+        want, size = want_and_size(t, kind, dim, x, i, l)
+        size = with_4bit_surplus(size, t, kind, x, i, l)
+        check(alone[-1].cpu().numpy(), want, size, 2e-3 if kind & 1 else 1e-5)
+    out = torch.full((len(laws), bags, dim), 7.0, dtype=alone[0].dtype, device=DEV)
+    batch = ops.SlwsBatch(kind, tables[0].shape[1], torch.int64, device=DEV)
+    batch.bind(tables, w, idx, lengths, list(out)).run(status)
+    for programmatic in (False, True):
+        with ops.programmatic_launch(programmatic):
+            batch.run(status)
+        for got, one in zip(out, alone):
+            assert torch.equal(got, one)
+        out.fill_(7.0)
+    assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 64), (3, 96), (2, 256)])
+@pytest.mark.parametrize("bags", [60, 4000, 15_000])
+def test_offsets_that_go_backwards_and_rows_that_are_not_there(kind, dim, bags):
+    """Bags with a start above their end are empty and reported; others are pooled from where they begin."""
+    rng = np.random.default_rng(bags)
+    table = make_table(kind, 500, dim, 2)
+    lengths = rng.choice([0, 1, 5, 17, 33, 64, 130], bags)
+    offsets = np.concatenate([[0], np.cumsum(lengths)])
+    n = int(offsets[-1])
+    for b in rng.integers(1, bags, 8):
+        offsets[b] = rng.integers(0, n)
+    idx = rng.integers(0, 500, n)
+    idx[::97], idx[::89] = 500, -1
+    w = rng.normal(0, 1, n).astype(np.float16 if kind & 1 else np.float32)
+    w64, good = np.where((idx >= 0) & (idx < 500), w, 0), np.clip(idx, 0, 499)
+    spans = [np.arange(a, b) for a, b in zip(offsets[:-1], offsets[1:])]
+    rows, sizes = np.concatenate(spans), np.array([len(s) for s in spans])
+    want, size = want_and_size(table, kind, dim, w64[rows], good[rows], sizes)
+    size = with_4bit_surplus(size, table, kind, w64[rows], good[rows], sizes)
+    status = ops.new_status(DEV)
+    got = ops.embedding_bag_byte_rowwise_offsets(dev(table), dev(w), dev(idx), dev(offsets), kind, status=status)
+    check(got.cpu().numpy(), want, size, 2e-3 if kind & 1 else 1e-5)
+    assert int(status.item()) & (ops.STATUS_BAD_OFFSETS | ops.STATUS_INDEX_OUT_OF_RANGE) == int(status.item()) != 0
