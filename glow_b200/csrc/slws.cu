@@ -121,9 +121,29 @@ __global__ void __launch_bounds__(256) slws_segments_from_offsets_kernel(const _
     if (v < 0) { v = 0; flags |= GLOWB200_STATUS_BAD_OFFSETS; }
     if (v > N) { v = N; flags |= GLOWB200_STATUS_BAD_OFFSETS; }
     p.seg_begin[i] = v;
-    if (i == S) p.seg_begin[S + 1] = 0;
   }
   raise_status(p.status, flags);
+  if (blockIdx.x != 0) return;
+  // Whether the lengths are skewed, from up to kSampled bags spread over the table: the word decides only which
+  // kernel pools the table, and in runs of how many bags.
+  constexpr int64_t kSampled = 2048;
+  __shared__ int longest;
+  if (threadIdx.x == 0) longest = 0;
+  __syncthreads();
+  auto at = [&](int64_t i) {
+    const int64_t v = (i < S || has_end) ? (int64_t)offsets[i] : N;
+    return v < 0 ? 0 : v > N ? N : v;
+  };
+  const int64_t sampled = S < kSampled ? S : kSampled;
+  int64_t mine = 0;
+  for (int64_t k = threadIdx.x; k < sampled; k += blockDim.x) {
+    const int64_t i = k * S / sampled, len = at(i + 1) - at(i);
+    mine = mine > len ? mine : len;
+  }
+  const int most = __reduce_max_sync(0xffffffffu, (int)(mine < INT32_MAX ? mine : INT32_MAX));
+  if ((threadIdx.x & 31) == 0) atomicMax(&longest, most);
+  __syncthreads();
+  if (threadIdx.x == 0) p.seg_begin[S + 1] = lengths_skewed(longest, at(S) > at(0) ? at(S) - at(0) : 0, S);
 }
 
 // ------------------------------------------------------------------------------------------

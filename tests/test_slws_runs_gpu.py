@@ -221,3 +221,24 @@ def test_offsets_that_go_backwards_and_rows_that_are_not_there(kind, dim, bags):
     got = ops.embedding_bag_byte_rowwise_offsets(dev(table), dev(w), dev(idx), dev(offsets), kind, status=status)
     check(got.cpu().numpy(), want, size, 2e-3 if kind & 1 else 1e-5)
     assert int(status.item()) & (ops.STATUS_BAD_OFFSETS | ops.STATUS_INDEX_OUT_OF_RANGE) == int(status.item()) != 0
+
+
+@pytest.mark.parametrize("bags", [2049, 3000, 40_000])
+@pytest.mark.parametrize("skewed", [False, True])
+def test_both_forms_know_a_skewed_table(bags, skewed):
+    """The word behind the boundaries of a table, by which its kernel is chosen, from lengths and from offsets."""
+    rng = np.random.default_rng(bags)
+    lengths = rng.integers(10, 14, bags).astype(np.int32)
+    if skewed:
+        lengths[rng.choice(bags, bags // 50, replace=False)] = 150
+    n = int(lengths.sum())
+    table, idx, w = make_table(0, 400, 64, 1), rng.integers(0, 400, n), rng.normal(0, 1, n).astype(np.float32)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    got = []
+    for form, bounds in ((ops.fused_rowwise_quantized_sparse_lengths_weighted_sum, lengths), (ops.embedding_bag_byte_rowwise_offsets, offsets)):
+        ws = torch.full((ops.slws_workspace_bytes(bags),), 255, dtype=torch.uint8, device=DEV)
+        got.append(form(dev(table), dev(w), dev(idx), dev(bounds), 0, workspace=ws))
+        words = ws.view(torch.int64)[:bags + 2].cpu().numpy()
+        np.testing.assert_array_equal(words[:-1], offsets)
+        assert words[-1] == int(skewed)
+    assert torch.equal(got[0], got[1])
