@@ -16,6 +16,7 @@ residual add is the max-with-constant the CPU backend lowers it to.
 Harness code: builds the network description and drives glow_b200.ops (the tests run the same
 description through the CPU checker).
 """
+import collections
 import math
 import threading
 
@@ -170,6 +171,41 @@ def quantize_network(layers, w, ranges):
     return q
 
 
+class Replays:
+    """Which input shapes have a graph, and which is to get one next.
+
+    A capture costs as much as some ten replays save, so it has to be earned: a shape gets its graph at its second
+    call while there is room for another, and when KEPT shapes have one only after PATIENCE calls without, in
+    place of the one that was used longest ago.  Callers whose shapes alternate keep their graphs; with more
+    shapes than KEPT, taken in turn, at most one call in PATIENCE captures."""
+    KEPT, PATIENCE, REMEMBERED = 4, 16, 64
+
+    def __init__(self):
+        self.graphs, self.calls = collections.OrderedDict(), collections.OrderedDict()
+
+    def find(self, shape):
+        if shape in self.graphs:
+            self.graphs.move_to_end(shape)
+            return self.graphs[shape]
+        return None
+
+    def earned(self, shape):
+        """Counts a call without a graph; whether the shape is to get one now."""
+        n = self.calls[shape] = self.calls.pop(shape, 0) + 1
+        if len(self.calls) > self.REMEMBERED:
+            self.calls.popitem(last=False)
+        return n >= (2 if len(self.graphs) < self.KEPT else self.PATIENCE)
+
+    def make_room(self):
+        """The graph that has to go before another is captured, or None."""
+        return self.graphs.popitem(last=False)[1] if len(self.graphs) >= self.KEPT else None
+
+    def keep(self, shape, graph):
+        self.calls.pop(shape, None)
+        self.graphs[shape] = graph
+        return graph
+
+
 class ResNet50Int8:
     """The quantized network resident on one GPU."""
 
@@ -187,9 +223,10 @@ class ResNet50Int8:
         self.fc["row_sums"] = ops.i8_row_sums(self.fc["w"])
         self.status = ops.new_status(self.dev)
         self.ws = None
-        self.launches = 0
+        self.launches = 0   # of the last call, at most: a convolution counts as two (windows, contraction)
         self._lock = threading.Lock()
-        self._seen, self._replay = None, None
+        self._replays = Replays()
+        self._stream, self._event = None, torch.cuda.Event()   # of the last call: the calls share a workspace
 
     def _workspace(self, nbytes):
         if self.ws is None or self.ws.numel() < nbytes:
@@ -213,9 +250,9 @@ class ResNet50Int8:
             return ops.channelwise_quantized_conv2d(*args, **kw)
         return ops.channelwise_quantized_conv2d_add(*args, residual, *add, **kw)
 
-    # Images up to which the layers between Quantize and the FC are replayed from a CUDA graph (from the second
-    # call of a shape on): their 56 launches cost the host 4 us each, which is more than the device needs for
-    # them below about 20 images of 224 x 224 (one image: 480 us from the host, 300 replayed).
+    # Images up to which the layers between Quantize and the FC are replayed from a CUDA graph (see Replays for
+    # when): their 56 launches cost the host 4 us each, which is more than the device needs for them below
+    # about 20 images of 224 x 224 (one image: 480 us from the host, 300 replayed).
     REPLAY_PIXELS = 20 * 224 * 224
 
     def forward(self, x_nchw):
@@ -223,34 +260,36 @@ class ResNet50Int8:
         n, _, h, w = shape = tuple(x_nchw.shape)
         with self._lock:
             self.launches = 0
-            if n * h * w > self.REPLAY_PIXELS or torch.cuda.is_current_stream_capturing():
+            if torch.cuda.is_current_stream_capturing():
                 return self._head(self._features(self._quantize(x_nchw)))
-            r = self._replay
-            if r is None or r["shape"] != shape:
-                if self._seen != shape:
-                    self._seen = shape
-                    return self._head(self._features(self._quantize(x_nchw)))
-                r = self._replay = self._capture(shape)   # the one graph kept: that of the last shape called twice
             stream = torch.cuda.current_stream()
-            if stream != r["stream"]:   # its buffers are read by the last replay, on another stream
-                stream.wait_event(r["event"])
-                r["stream"] = stream
-            self._quantize(x_nchw, r["input"])
-            r["graph"].replay()
-            self.launches += r["launches"]
-            out = self._head(r["features"])
-            r["event"].record(stream)
+            if stream != self._stream:   # the last call may still run on the other stream
+                if self._stream is not None:
+                    stream.wait_event(self._event)
+                self._stream = stream
+            r = self._replays.find(shape)
+            if r is None and n * h * w <= self.REPLAY_PIXELS and self._replays.earned(shape):
+                r = self._replays.keep(shape, self._capture(shape))
+            if r is None:
+                out = self._head(self._features(self._quantize(x_nchw)))
+            else:
+                self._quantize(x_nchw, r["input"])
+                r["graph"].replay()
+                self.launches += r["launches"]
+                out = self._head(r["features"])
+            self._event.record(stream)
             return out
 
     def _capture(self, shape):
         n, c, h, w = shape
-        stream, side = torch.cuda.current_stream(), torch.cuda.Stream()
-        r = {"shape": shape, "graph": torch.cuda.CUDAGraph(), "stream": stream, "event": torch.cuda.Event(), "ws": self.ws,  # the workspace of the first call
-             "input": torch.empty((n, h, w, c), dtype=torch.int8, device=self.dev)}
-        before = self._replay
+        before = self._replays.make_room()
         if before is not None:
-            before["event"].synchronize()   # its memory goes with it
-        side.wait_stream(stream)
+            self._event.synchronize()   # its memory goes with it
+            del before
+        side = torch.cuda.Stream()
+        r = {"graph": torch.cuda.CUDAGraph(), "ws": self.ws,   # the workspace of the calls before, large enough for this shape
+             "input": torch.empty((n, h, w, c), dtype=torch.int8, device=self.dev)}
+        side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
             r["graph"].capture_begin(capture_error_mode="thread_local")
             try:

@@ -152,3 +152,27 @@ def test_replayed_forward_equals_the_launches(net, shapes):
     for a, b in zip(got, want):
         assert torch.equal(a, b)
     assert len({t.data_ptr() for t in quantized}) == len(xs)
+
+
+def test_alternating_shapes_are_captured_once(net):
+    """Shapes that take turns are replayed, each from its own graph; more of them than are kept run launch by launch;
+    calls on several streams wait for one another."""
+    layers, w, q = net
+    model, plain = resnet.ResNet50Int8(layers, q, DEV), resnet.ResNet50Int8(layers, q, DEV)
+    plain.REPLAY_PIXELS = 0
+    captures, capture = [], model._capture
+    model._capture = lambda shape: captures.append(shape) or capture(shape)
+    g = torch.Generator(device=DEV).manual_seed(2)
+    xs = [torch.randn((n, 3, 64, 64), device=DEV, generator=g) for n in (1, 2, 3, 4, 5, 6)]
+    want = [plain.forward(x) for x in xs]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    got, call = [], 0
+    for turn in range(12):
+        for i in ((0, 1, 2) if turn < 6 else range(6)):
+            with torch.cuda.stream(streams[call % 3]):
+                got.append((i, model.forward(xs[i])))
+            call += 1
+    torch.cuda.synchronize()
+    assert int(model.status.item()) == 0 and all(torch.equal(out, want[i]) for i, out in got)
+    assert len(captures) == resnet.Replays.KEPT and len(set(captures)) == len(captures)
