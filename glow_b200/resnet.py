@@ -222,7 +222,7 @@ class ResNet50Int8:
         self.fc = dict(w=to(fc["w"]), w_off=to(fc["w_offsets"]), bias=to(fc["bias"]), params=[to(a) for a in fc["params"]])
         self.fc["row_sums"] = ops.i8_row_sums(self.fc["w"])
         self.status = ops.new_status(self.dev)
-        self.ws = None
+        self.ws, self._captured = None, []
         self.launches = 0   # of the last call, at most: a convolution counts as two (windows, contraction)
         self._lock = threading.Lock()
         self._replays = Replays()
@@ -231,6 +231,8 @@ class ResNet50Int8:
     def _workspace(self, nbytes):
         if self.ws is None or self.ws.numel() < nbytes:
             self.ws = torch.empty(int(nbytes * 1.1) + 256, dtype=torch.uint8, device=self.dev)
+        if torch.cuda.is_current_stream_capturing() and (not self._captured or self._captured[-1] is not self.ws):
+            self._captured.append(self.ws)   # a graph addresses it from now on: kept when a larger one takes its place
         return self.ws
 
     def _conv(self, name, x, residual=None, add=()):
@@ -287,7 +289,7 @@ class ResNet50Int8:
             self._event.synchronize()   # its memory goes with it
             del before
         side = torch.cuda.Stream()
-        r = {"graph": torch.cuda.CUDAGraph(), "ws": self.ws,   # the workspace of the calls before, large enough for this shape
+        r = {"graph": torch.cuda.CUDAGraph(),   # (the workspace of the calls before is large enough for this shape)
              "input": torch.empty((n, h, w, c), dtype=torch.int8, device=self.dev)}
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):

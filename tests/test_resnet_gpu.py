@@ -176,3 +176,28 @@ def test_alternating_shapes_are_captured_once(net):
     torch.cuda.synchronize()
     assert int(model.status.item()) == 0 and all(torch.equal(out, want[i]) for i, out in got)
     assert len(captures) == resnet.Replays.KEPT and len(set(captures)) == len(captures)
+
+
+def test_a_captured_forward_outlives_larger_calls(net):
+    """A graph that a caller captured addresses the workspace of that time: it stays when a later call needs more."""
+    layers, w, q = net
+    model = resnet.ResNet50Int8(layers, q, DEV)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    x = torch.randn((1, 3, 64, 64), device=DEV, generator=g)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = model.forward(x).clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = model.forward(x)
+        small = model.ws
+        model.forward(torch.randn((6, 3, 128, 128), device=DEV, generator=g))
+        assert model.ws is not small and any(t is small for t in model._captured)
+        address = small.data_ptr()
+        del small
+        fill = [torch.full((1 << 20,), 85, dtype=torch.uint8, device=DEV) for _ in range(64)]
+        assert all(not f.data_ptr() <= address < f.data_ptr() + f.numel() for f in fill)
+        graph.replay()
+        torch.cuda.synchronize()
+    assert torch.equal(out, want) and int(model.status.item()) == 0
