@@ -247,3 +247,35 @@ def test_properties_on_large_tables():
             idx[lo:hi], t(offsets_h[i * B:(i + 1) * B + 1] - lo), ops.EP_SUM, status=st)
         assert torch.equal(single, base[:, int(dims[i]):int(dims[i + 1])])
     assert int(st.item()) == 0
+
+
+@pytest.mark.parametrize("out_fp16", [False, True])
+@pytest.mark.parametrize("order", ["ascending", "gaps_and_empty", "descending", "reaching_out"])
+def test_columns_of_no_table_are_zero(order, out_fp16):
+    """Every column of the result is a table's or 0, wherever the tables lie: offsets that ascend, with tables
+    without columns and unsupported ones among them, that fall, and tables that reach out of the result."""
+    rng = np.random.default_rng(8)
+    T, B = 300, 5
+    widths = rng.choice([8, 16] if order == "ascending" else [0, 4, 8], T)
+    starts = 3 + np.concatenate([[0], np.cumsum(widths)])
+    if order == "descending":          # table t: columns [starts[t], starts[t + 1]), none where that falls
+        starts[100:200] = starts[100:200][::-1]
+    if order == "reaching_out":
+        starts -= 20
+    total = int(starts.max()) + (5 if order != "reaching_out" else -6)
+    tys = rng.choice([ops.EST_FLOAT, ops.EST_FLOAT16, ops.EST_INT8, 4], T, p=[.4, .25, .25, .1]).astype(np.uint8)
+    placements = rng.choice([ops.PLACEMENT_HOST, ops.PLACEMENT_DEVICE], T, p=[.9, .1]).astype(np.int32)
+    # rows of ones: 1.0f, 1.0h, or scale 0 and offset 1
+    table = {ops.EST_FLOAT: np.full(1024, 1, np.float32).tobytes(), ops.EST_FLOAT16: np.full(2048, 1, np.float16).tobytes()}
+    table[ops.EST_INT8] = table[4] = np.array([0, 1] * 2, np.float16).tobytes() + bytes(4088)
+    data = np.frombuffer(b"".join(table[k] for k in (ops.EST_FLOAT, ops.EST_FLOAT16, ops.EST_INT8)), np.uint8).copy()
+    at = np.array([{ops.EST_FLOAT: 0, ops.EST_FLOAT16: 4096}.get(k, 8192) for k in tys], np.int64)
+    want = np.zeros(total, np.float32)
+    for k in range(T):
+        a, b = int(starts[k]), int(starts[k + 1])
+        if a < b and tys[k] <= ops.EST_INT4 and placements[k] != 0 and a >= 0 and b <= total:
+            want[a:b] = 1
+    out = torch.full((B, total), 7.0, dtype=torch.float16 if out_fp16 else torch.float32, device=DEV)
+    ops.int_nbit_split_embedding_bags(t(data), t(data), t(placements), t(at), t(tys), t(starts.astype(np.int32)), total,
+                                      t(np.zeros(T * B, np.int64)), t(np.arange(T * B + 1, dtype=np.int64)), out=out)
+    np.testing.assert_array_equal(out.float().cpu().numpy(), np.broadcast_to(want, (B, total)))
