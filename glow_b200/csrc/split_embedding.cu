@@ -36,6 +36,7 @@ struct SplitLaunch {
   int32_t *status;
   int64_t num_indices, bags_per_table, total_dims;
   int32_t num_tables, wo64, iw16, so_fp32, row_alignment, pooling_mode;
+  int32_t first_column_ty;  // the types from here on take pool_bag_columns where the rows allow it
 };
 
 constexpr int kThreads = 128;  // (a bag of a warp ends late: small blocks hand their registers on sooner)
@@ -326,6 +327,7 @@ __device__ __forceinline__ int32_t pool_bag_columns(const SplitLaunch &p, const 
                                                     int64_t begin, int64_t end, int gl, int lpr, void *out_row) {
   constexpr int H = SO32 ? 8 : 4, SLOTS = (TY == TY_I8 ? 4 : 8) * LW;
   const IdxT *indices = reinterpret_cast<const IdxT *>(p.indices) + begin;
+  // (longer bags do not come here; without the minimum the compiler spills in this loop)
   const int32_t count = (int32_t)(end - begin < 0x7FFFFFF0ll ? end - begin : 0x7FFFFFF0ll);
   int32_t flags = 0;
   for (int32_t word0 = gl * LW; H + 4 * (word0 - gl * LW) < touched; word0 += lpr * LW) {
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, GLOWB200_TBE_MIN_BLOCKS) split_embed
   if (table_at >= 0 && table_at + touched <= limit) max_row = (limit - touched - table_at) / row_bytes;
   if (max_row > 0x7FFFFFFEll) max_row = 0x7FFFFFFEll;
   // (a buffer that does not end on a 16-byte boundary may cut the last row's pieces short)
-  const bool columns = wide && ty >= TY_I8 && table_at + max_row * row_bytes + (touched + 15) / 16 * 16 <= limit;
+  const bool columns = wide && ty >= p.first_column_ty && table_at + max_row * row_bytes + (touched + 15) / 16 * 16 <= limit;
   // Words of columns per lane: four, but two of int4 rows with an fp32 result (32 fp32 sums per lane spill: 12.9
   // against 16.0 G rows/s) and of int4 rows that are no longer.
   const bool pairs = ty == TY_I4 && (!OUT16 || num_dims <= 16);
@@ -619,6 +621,8 @@ extern "C" int glowb200_int_nbit_split_embedding_bags(
   L.row_alignment = row_alignment;
   L.pooling_mode = pooling_mode;
   L.num_tables = (int32_t)num_tables;
+  // (pool_bag_columns counts the rows of a bag in 32 bits; a long bag in pieces cost its loop 2 to 15 %)
+  L.first_column_ty = num_indices <= 0x7FFFFFF0ll ? TY_I8 : TY_I4 + 1;
   // A warp takes 8 bags of rows of 4 lanes; the blocks of tables with wider rows walk on, those of narrower ones
   // are in part not needed and leave at once.  Few bags: a block for every 8, so that no row is so wide that its
   // bags would wait for one another while SMs idle (8 tables, 64 bags of 20 int8 rows of 128 columns: 17 -> 12 us).

@@ -279,3 +279,31 @@ def test_columns_of_no_table_are_zero(order, out_fp16):
     ops.int_nbit_split_embedding_bags(t(data), t(data), t(placements), t(at), t(tys), t(starts.astype(np.int32)), total,
                                       t(np.zeros(T * B, np.int64)), t(np.arange(T * B + 1, dtype=np.int64)), out=out)
     np.testing.assert_array_equal(out.float().cpu().numpy(), np.broadcast_to(want, (B, total)))
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("ty,dim", [(ops.EST_INT8, 40), (ops.EST_INT4, 72)])
+def test_requests_of_more_indices_than_32_bits_count(ty, dim, weighted):
+    """A request that may hold bags of 2^31 rows takes the loop that counts in 64 bits, with the same bits.  (The bags
+    are short: only the length of the index array, which bounds the offsets and nothing else, is that large.)"""
+    import ctypes as C
+
+    from glow_b200 import _lib
+    rng = np.random.default_rng(dim)
+    T, B, rows = 2, 70, 300
+    dev, uvm, offs = random_tables(rng, [(ty, dim, rows, 3)] * T, False, 16)
+    lengths = rng.integers(0, 30, T * B)
+    n = int(lengths.sum())
+    place, wo, tys = t(np.full(T, 3, np.int32)), t(offs.astype(np.int64)), t(np.full(T, ty, np.uint8))
+    dims, data = t((np.arange(T + 1) * dim).astype(np.int32)), t(dev)
+    idx, bounds = t(rng.integers(0, rows, n)), t(np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64))
+    w = t(rng.normal(0, 1, n).astype(np.float32)) if weighted else None
+    st, p = ops.new_status(DEV), lambda a: C.c_void_p(0 if a is None else a.data_ptr())
+    got = []
+    for claimed in (n, 2 ** 31 + 5):
+        out = torch.empty((B, T * dim), dtype=torch.float16, device=DEV)
+        _lib.check(_lib.lib().glowb200_int_nbit_split_embedding_bags(
+            p(out), p(data), data.numel(), p(data), data.numel(), p(place), p(wo), 1, p(tys), p(dims), T, T * dim, p(idx), p(bounds),
+            1, claimed, B, ops.EP_SUM, p(w), 0, 1, 0, 16, p(st), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        got.append(out)
+    assert torch.equal(got[0], got[1]) and got[0].abs().max() > 0 and int(st.item()) == 0
