@@ -1218,10 +1218,17 @@ int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_ro
   const int K = p.K, pitch = (int)align_up((size_t)K, 16);
   const bool copy_a = (pitch != K && p.a_pitch != pitch) || !ptr16(a), copy_b = b_is_kn || pitch != K || !ptr16(b);
   const size_t core = i8_gemm_core_workspace_bytes(p.M, p.N);
+  // (a right-hand side to be turned round has always asked for room for it, whichever kernel then takes the product)
+  const size_t least = b_is_kn ? core + align_up((size_t)p.N * K, 256) : 0;
+  if (least > 0 && (ws == nullptr || ws_bytes < least))
+    return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", ws_bytes,
+                     core + i8_gemm_copies_bytes(p.M, K, p.N, copy_a, true));
   if (!force_any && K > 0 && i8_skinny_wins(p.M, p.N, K, b_is_kn)) return run_gemm_skinny(p, a, b, b_is_kn, b_offsets_zero, s);
-  const bool tc = !force_any && K > 0 &&
-                  ((!copy_a && !copy_b) ||
-                   (ws != nullptr && ptr16(ws) && ws_bytes >= core + i8_gemm_copies_bytes(p.M, K, p.N, copy_a, copy_b)));
+  // Room for the copies; a transposed one's sums come in parts, or are added up by a launch of their own.
+  const size_t a_copy = copy_a ? align_up((size_t)p.M * pitch, 256) : 0, b_copy = copy_b ? align_up((size_t)p.N * pitch, 256) : 0;
+  const bool room = ws != nullptr && ptr16(ws) && ws_bytes >= core + a_copy + b_copy;
+  const bool sum_parts = room && ws_bytes >= core + i8_gemm_copies_bytes(p.M, K, p.N, copy_a, copy_b);
+  const bool tc = !force_any && K > 0 && ((!copy_a && !copy_b) || room);
   if (!tc) {
     dim3 grid((p.N + 15) / 16, (p.M + 15) / 16);
     const int64_t stride_j = b_is_kn ? 1 : K, stride_k = b_is_kn ? p.N : 1;
@@ -1242,16 +1249,17 @@ int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_ro
   if (copy_a) {
     prep_side_rows(prep.a, a, reinterpret_cast<int8_t *>(w), a_sums ? as : nullptr, p.M, K, pitch);
     a = prep.a.dst;
-    w += align_up((size_t)p.M * pitch, 256);
+    w += a_copy;
   } else if (a_sums) {
     prep_side_rows(prep.a, a, nullptr, as, p.M, K, pitch);
   }
   p.b_row_sums = b_sums ? bs : b_row_sums_in;
   p.b_sum_parts = 1;
+  const bool sums_after = copy_b && b_is_kn && b_sums && !sum_parts;
   if (copy_b && b_is_kn) {
-    int32_t *parts = reinterpret_cast<int32_t *>(w + align_up((size_t)p.N * pitch, 256));
-    prep_side_transposed(prep.b, b, reinterpret_cast<int8_t *>(w), b_sums ? parts : nullptr, p.N, K, pitch);
-    if (b_sums) {
+    int32_t *parts = reinterpret_cast<int32_t *>(w + b_copy);
+    prep_side_transposed(prep.b, b, reinterpret_cast<int8_t *>(w), b_sums && sum_parts ? parts : nullptr, p.N, K, pitch);
+    if (b_sums && sum_parts) {
       p.b_row_sums = parts;
       p.b_sum_parts = prep_transposed_parts(p.N, pitch);
     }
@@ -1263,6 +1271,10 @@ int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_ro
     prep_side_rows(prep.b, b, nullptr, bs, p.N, K, pitch);
   }
   if (int rc = run_prepare_operands(prep, s)) return rc;
+  if (sums_after) {
+    i8_row_sums_kernel<<<(p.N + 7) / 8, 256, 0, s>>>(b, p.N, pitch, bs);
+    GLOWB200_CUDA_OK(cudaGetLastError());
+  }
   if (b_offsets_zero) p.a_row_sums = nullptr;
   else if (!p.float_out) p.a_row_sums = as;
   p.K = pitch;
@@ -1289,9 +1301,9 @@ extern "C" int glowb200_debug_gemm_trace(unsigned long long *host512) {
 
 extern "C" size_t glowb200_i8_gemm_workspace_bytes(int64_t M, int64_t K, int64_t N) {
   if (M < 0 || N < 0 || K < 0) return 0;
-  // row sums of both operands + room for a padded (transposed) copy of the right-hand side and, when
-  // rows are not whole 16-byte pieces, of the left one
-  return i8_gemm_core_workspace_bytes(M, N) + i8_gemm_copies_bytes(M, K, N, (K % 16) != 0, true);
+  // row sums of both operands + room for a padded (transposed) copy of either: where the operands will lie
+  // is not known here, and off a 16-byte boundary both are copied
+  return i8_gemm_core_workspace_bytes(M, N) + i8_gemm_copies_bytes(M, K, N, true, true);
 }
 
 extern "C" int glowb200_i8_mma_issue_probe(int64_t mmas_per_sm, int64_t *ops_per_launch, int32_t *status,

@@ -86,7 +86,8 @@ __device__ __forceinline__ int32_t activation_i32(int32_t x, const GemmParams &p
 // operands as they are when K is a multiple of 16 and both are 16-byte aligned [rows, K] matrices, else
 // on zero-padded (transposed) copies in `ws` -- and the any-shape kernel when asked for (force_any) or
 // when `ws` has no room for the copies.  `ws` must hold i8_gemm_core_workspace_bytes(M, N) bytes, with
-// i8_gemm_copies_bytes(M, K, N, ...) more for the copies.  b_row_sums_in may be nullptr (computed here).
+// i8_gemm_copies_bytes(M, K, N, ...) more for the copies; a [K, N] right-hand side for which it could not hold
+// the N * K bytes is an error.  b_row_sums_in may be nullptr (computed here).
 int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_row_sums_in, bool b_offsets_zero,
              int force_any, void *ws, size_t ws_bytes, cudaStream_t s, bool b_is_kn = false);
 

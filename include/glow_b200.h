@@ -370,7 +370,11 @@ int glowb200_wait_limit_selftest(int64_t limit_cycles, int32_t *status, int32_t 
 int glowb200_i8_mma_issue_probe(int64_t mmas_per_sm, int64_t *ops_per_launch, int32_t *status,
                                 glowb200_stream_t stream);
 
-/* Scratch bytes the three entry points below may need for an [M,K] x [N,K]^T problem. */
+/* Scratch bytes the three entry points below may need for an [M,K] x [N,K]^T problem, wherever its operands
+ * lie: row sums, and a copy of either operand for rows that are not whole 16-byte pieces, operands off 16-byte
+ * boundaries and right-hand sides given as [K,N].  Less is enough for many products; where the copies do not fit, the
+ * product runs in the reference's loop, a thread per output, except that a [K,N] right-hand side whose
+ * workspace has no room for its N * K bytes is GLOWB200_ERR_WORKSPACE_TOO_SMALL. */
 size_t glowb200_i8_gemm_workspace_bytes(int64_t M, int64_t K, int64_t N);
 
 /* sums[r] = sum_k matrix[r,k] (int8 [rows,K] -> int32 [rows]).  Lets a caller compute the row

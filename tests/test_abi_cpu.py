@@ -63,3 +63,19 @@ def test_host_side_argument_errors_need_no_gpu(built):
     assert l.glowb200_set_programmatic_launch(-1) == 1
     assert l.glowb200_set_programmatic_launch(before) in (0, 1)
     l.glowb200_set_programmatic_launch(-1)
+
+
+@pytest.mark.parametrize("M,K,N", [(8, 64, 32), (300, 64, 32), (300, 33, 40), (300, 0, 40)])
+def test_a_right_hand_side_to_turn_round_needs_its_room(built, M, K, N):
+    """[K, N] products refuse a workspace without room for the N * K bytes, on the host; the size that the library names
+    holds a copy of both operands, wherever they lie."""
+    from glow_b200 import _lib
+    l, fake, up = _lib.lib(), ctypes.c_void_p(4096), lambda v, a: (v + a - 1) // a * a
+    least = up(N * 4, 256) + up(M * 4, 256) + up(N * K, 256)
+    named = l.glowb200_i8_gemm_workspace_bytes(M, K, N)
+    assert named >= least + up(M * up(K, 16), 256)
+    for ws, size in ((None, 0), (None, named), (fake, least - 1)):
+        rc = l.glowb200_matmul_i8(fake, fake, fake, M, K, N, 0, 0, 0, 0, 0, 1, 0, ws, size, None, None)
+        assert rc == 3 and b"needed" in l.glowb200_last_error()
+        rc = l.glowb200_fc_i8_i32(fake, fake, fake, fake, M, K, N, 0, 0, 0, 0, 0, 0, 1, 0, 0, 1, None, 0, ws, size, None, None)
+        assert rc == 3

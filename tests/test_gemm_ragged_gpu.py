@@ -71,3 +71,37 @@ def test_dynamic_products(oracle, M, K, N, zero_offsets):
                                                    flags=ops.FC_WEIGHT_OFFSETS_ZERO if zero_offsets else 0, status=status, **kw)
             np.testing.assert_array_equal(got.cpu().numpy().view(np.uint16), want.view(np.uint16))
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(300, 160, 48), (300, 33, 48), (2100, 64, 40), (8, 64, 24)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_workspaces_of_every_size(oracle, M, K, N, shift):
+    """From the least that a [K, N] product asks for to what the library names: the same results, operands off
+    16-byte boundaries included; [N, K] products run with any."""
+    rng = np.random.default_rng(M + K)
+    x, kn = rng.integers(-128, 128, (M, K)).astype(np.int8), rng.integers(-128, 128, (K, N)).astype(np.int8)
+    ot = ops.quantize_scale_offset_32to8(np.float32(0.004 / np.sqrt(K)))
+    want = oracle.matmul_i8(x, kn, 5, -3, 7, ot, threads=4)
+    up = lambda v, a: (v + a - 1) // a * a
+    least = up(N * 4, 256) + up(M * 4, 256) + up(N * K, 256)
+    pitch = up(K, 16)
+    sizes = [least, least + up(M * pitch, 256), least - up(N * K, 256) + up(N * pitch, 256) + (up(M * pitch, 256) if shift else 0),
+             ops.i8_gemm_workspace_bytes(M, K, N)]
+    status = ops.new_status(DEV)
+    for size in sizes:
+        ws = torch.full((size,), 77, dtype=torch.uint8, device=DEV)
+        got = ops.matmul_i8(dev(x, shift), dev(kn, 2 * shift), 5, -3, 7, ot, workspace=ws, status=status)
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
+    with pytest.raises(Exception, match="needed"):
+        ops.matmul_i8(dev(x), dev(kn), 5, -3, 7, ot, workspace=ws[:least - 1])
+    bias = rng.integers(-2 ** 15, 2 ** 15, N).astype(np.int32)
+    offs = rng.integers(-20, 20, N).astype(np.int32)
+    p = ops.rowwise_requant_params(rng.uniform(0.001, 0.02, N).astype(np.float32), 0.05, np.float32(5e-4), np.float32(0.1))
+    want = oracle.rowwise_quantized_fc_i8_i32(x, np.ascontiguousarray(kn.T), bias, offs, p[:3], p[3:], -2, 3, 1, threads=4)
+    dp = [dev(a) for a in p]
+    for size in (up(N * 4, 256) + up(M * 4, 256), ops.i8_gemm_workspace_bytes(M, K, N)):
+        ws = torch.full((size,), 77, dtype=torch.uint8, device=DEV)
+        got = ops.rowwise_quantized_fc(dev(x, shift), dev(kn.T, 3 * shift), dev(bias), dev(offs), dp[:3], dp[3:], -2, 3, 1, workspace=ws,
+                                       status=status)
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
+    assert int(status.item()) == 0
