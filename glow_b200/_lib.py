@@ -5,6 +5,7 @@ There is no fallback: if the CUDA library has not been built, importing an opera
 import ctypes as C
 import importlib.util
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # GLOW_B200_LIBRARY selects another build of the same library (e.g. one compiled with
@@ -161,11 +162,18 @@ def lib():
 _binding = None
 
 
+def binding_path():
+    """The CPython module for this interpreter and this torch: it is compiled against both, and another one's must
+    neither be loaded nor taken for built."""
+    import torch
+    return os.path.join(_HERE, "lib", "_binding.%s.torch-%s.so" % (sys.implementation.cache_tag, torch.__version__))
+
+
 def binding(explain):
     """The CPython module of the per-request calls (csrc/binding.cpp), working on this process's library."""
     global _binding
     if _binding is None:
-        path = os.path.join(_HERE, "lib", "_binding.so")
+        path = binding_path()
         if not os.path.exists(path):
             raise ImportError("%s is missing: build it with `python -m glow_b200.build`" % path)
         l = lib()

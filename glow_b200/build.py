@@ -3,12 +3,14 @@
 Every .cu file under glow_b200/csrc is compiled for sm_100a only
 (-gencode arch=compute_100a,code=sm_100a) and linked into one shared library that exports
 the C ABI declared in include/glow_b200.h; csrc/binding.cpp becomes the CPython module
-(glow_b200/lib/_binding.so) through which ops.py calls it.  Run as `python -m glow_b200.build`.
+(glow_b200/lib/_binding.<interpreter>.torch-<version>.so) through which ops.py calls it.  Run as `python -m glow_b200.build`.
 """
 import os
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
+
+from ._lib import binding_path
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -16,7 +18,6 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libglow_b200.so")
-BINDING = os.path.join(LIBDIR, "_binding.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -33,7 +34,7 @@ def _headers():
     return hs
 
 
-def _binding_command(src):
+def _binding_command(src, target):
     import sysconfig
 
     import torch
@@ -43,7 +44,7 @@ def _binding_command(src):
             "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
             "-I", os.path.join(t, "include"), "-I", os.path.join(t, "include", "torch", "csrc", "api", "include"),
             "-I", os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), "-I", sysconfig.get_paths()["include"],
-            "-I", os.path.join(ROOT, "include"), src, "-o", BINDING, "-L", os.path.join(t, "lib"),
+            "-I", os.path.join(ROOT, "include"), src, "-o", target, "-L", os.path.join(t, "lib"),
             "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
 
@@ -77,11 +78,15 @@ def build(verbose=False, extra_flags=()):
         return r.stderr
 
     binding_src = os.path.join(CSRC, "binding.cpp")
+    binding = binding_path()
     compiles = list(jobs)
-    if _stale(BINDING, [binding_src, os.path.join(ROOT, "include", "glow_b200.h")]):
-        compiles.append(_binding_command(binding_src))
+    if _stale(binding, [binding_src, os.path.join(ROOT, "include", "glow_b200.h")]):
+        compiles.append(_binding_command(binding_src, binding))
     with ThreadPoolExecutor(max(1, min(8, len(compiles)))) as ex:
         list(ex.map(run, compiles))
+    for f in os.listdir(LIBDIR):  # those of another interpreter or torch
+        if f.startswith("_binding") and f != os.path.basename(binding):
+            os.remove(os.path.join(LIBDIR, f))
     if jobs or _stale(LIB, objs):
         run([NVCC, "-shared", "-o", LIB] + objs)
     return LIB

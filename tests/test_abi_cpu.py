@@ -34,6 +34,19 @@ def test_binding_table_matches_header(built):
     assert _lib.lib().glowb200_version().startswith(b"glow_b200")
 
 
+def test_binding_is_of_this_interpreter_and_torch(built, monkeypatch):
+    """The CPython module is compiled against both: another torch in the same tree finds none, and builds its own."""
+    import torch
+    from glow_b200 import _lib
+    path = _lib.binding_path()
+    assert os.path.exists(path) and torch.__version__ in path and os.path.dirname(path) == os.path.dirname(built)
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    monkeypatch.setattr(_lib, "_binding", None)
+    assert _lib.binding_path() != path
+    with pytest.raises(ImportError, match="0.0.1.*build it"):
+        _lib.binding(None)
+
+
 def test_host_side_argument_errors_need_no_gpu(built):
     from glow_b200 import _lib
     l = _lib.lib()
