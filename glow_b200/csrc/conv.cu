@@ -14,13 +14,14 @@
 #include "common.cuh"
 #include "qgemm.cuh"
 
-// 1: stride-1 windows take the shifted-rows path (no im2col matrix) when the shapes allow
-#ifndef GLOWB200_CONV_SHIFTED_ROWS
-#define GLOWB200_CONV_SHIFTED_ROWS 1
-#endif
-
 namespace glowb200 {
 namespace {
+
+// Blocks of a kernel that walks on: `per_sm` to an SM at most.
+unsigned grid_of(int64_t blocks, int per_sm) {
+  const int64_t most = (int64_t)kB200Sms * per_sm;
+  return (unsigned)(blocks < most ? blocks : most);
+}
 
 // one thread per 16-byte chunk of the im2col matrix (C a multiple of 16: a chunk never
 // straddles two taps)
@@ -354,7 +355,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
   const ConvPlan pl = plan_conv(g, (flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0);
   if (pl.direct) {
     const int64_t blocks = (outputs + 255) / 256;
-    conv2d_i8_direct_kernel<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, s>>>(in, filter, g, p);
+    conv2d_i8_direct_kernel<<<grid_of(blocks, 32), 256, 0, s>>>(in, filter, g, p);
     GLOWB200_CUDA_OK(cudaGetLastError());
     return GLOWB200_OK;
   }
@@ -366,7 +367,6 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
     return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", workspace_bytes, need);
   GLOWB200_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
   uint8_t *ws = reinterpret_cast<uint8_t *>(workspace);
-#if GLOWB200_CONV_SHIFTED_ROWS
   // Stride-1 windows over 64 or a multiple of 128 channels, symmetric filters: no im2col matrix.
   // The input is copied once into a padded NHWC buffer; tap (kh, kw) of output row q then is row
   // q + kh * Wp + kw of that buffer, which the contraction's loads address directly (the rows of
@@ -391,7 +391,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       const uint32_t b = (uint8_t)p.a_offset;
       int8_t *fb = g.C == 64 ? reinterpret_cast<int8_t *>(ws + xp_bytes) : nullptr;
       const int64_t chunks = rows * (g.C >> 4) + 16 + (fb ? (int64_t)g.OC * entries * 8 : 0), blocks = (chunks + 255) / 256;
-      GLOWB200_CUDA_OK(launch_pdl(pad_nhwc_i8_kernel, (unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s, in, xp, g, Hp, Wp,
+      GLOWB200_CUDA_OK(launch_pdl(pad_nhwc_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, xp, g, Hp, Wp,
                                   (int)(b | (b << 8) | (b << 16) | (b << 24)), filter, fb));
       const int8_t *bmat = fb ? fb : filter;
       p.K = fb ? entries * 128 : g.KH * g.KW * g.C;
@@ -414,7 +414,6 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       return run_gemm_shifted_rows(p, xp, rows, g.C, bmat, sums, s);
     }
   }
-#endif
   // Stride-2 windows over a multiple of 128 channels, symmetric filters: the shifted-rows form over
   // four parity planes of the padded input (see pad_parity_nhwc_i8_kernel) instead of an im2col matrix.
   if (pl.need_im2col && g.SH == 2 && g.SW == 2 && g.DH == 1 && g.DW == 1 && (g.KH > 1 || g.KW > 1) &&
@@ -427,7 +426,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       int8_t *xp = reinterpret_cast<int8_t *>(ws);
       const uint32_t b = (uint8_t)p.a_offset;
       const int64_t chunks = 4 * rows * (g.C >> 4), blocks = (chunks + 255) / 256;
-      GLOWB200_CUDA_OK(launch_pdl(pad_parity_nhwc_i8_kernel, (unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s, in, xp, g, Hq,
+      GLOWB200_CUDA_OK(launch_pdl(pad_parity_nhwc_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, xp, g, Hq,
                                   Wq, (int)(b | (b << 8) | (b << 16) | (b << 24))));
       GLOWB200_CUDA_OK(cudaGetLastError());
       p.K = g.KH * g.KW * g.C;
@@ -466,7 +465,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       int8_t *fb = reinterpret_cast<int8_t *>(ws + wp_bytes);
       const int tail = (int)((wp_bytes - 2 * plane_bytes) / 32);  // the four windows of the last rows reach past the second plane
       const int64_t items = 2 * rows + tail + (int64_t)g.OC * 8, blocks = (items + 255) / 256;
-      GLOWB200_CUDA_OK(launch_pdl(row_windows_i8_kernel, (unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s, in, planes, g, Y,
+      GLOWB200_CUDA_OK(launch_pdl(row_windows_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, planes, g, Y,
                                   plane_bytes, (int8_t)p.a_offset, tail, filter, fb));
       const int32_t *bs = filter_row_sums;  // (the zeros of the new layout do not change them)
       if (bs == nullptr) {
@@ -492,7 +491,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       const int64_t chunks = pl.M * (pl.Kpad >> 4);
       const int64_t blocks = (chunks + 255) / 256;
       const uint32_t b = (uint8_t)pad;
-      GLOWB200_CUDA_OK(launch_pdl(im2col_i8_vec_kernel, (unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s, in, abuf, g, pl.Kpad,
+      GLOWB200_CUDA_OK(launch_pdl(im2col_i8_vec_kernel, grid_of(blocks, 64), 256, 0, s, in, abuf, g, pl.Kpad,
                                   (int)(b | (b << 8) | (b << 16) | (b << 24))));
     } else if ((int64_t)g.KH * rows_pitch(g) <= 48 * 1024 && (int64_t)g.N * g.OH < (1ll << 31) && (pl.Kpad >> 4) <= 256 &&
                (reinterpret_cast<uintptr_t>(abuf) & 15) == 0) {
@@ -501,7 +500,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       im2col_i8_rows_kernel<<<(unsigned)(g.N * g.OH), 256, (size_t)g.KH * pitch, s>>>(in, abuf, g, pl.K, pl.Kpad, pad, pitch);
     } else {
       const int64_t blocks = (pl.M * pl.Kpad + 255) / 256;
-      im2col_i8_kernel<<<(unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, s>>>(in, abuf, g, pl.K, pl.Kpad, pad);
+      im2col_i8_kernel<<<grid_of(blocks, 64), 256, 0, s>>>(in, abuf, g, pl.K, pl.Kpad, pad);
     }
     GLOWB200_CUDA_OK(cudaGetLastError());
     a = abuf;
@@ -510,7 +509,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
   if (pl.f_bytes) {
     int8_t *fbuf = reinterpret_cast<int8_t *>(ws + pl.a_bytes);
     const int64_t blocks = ((int64_t)g.OC * pl.Kpad + 255) / 256;
-    pad_rows_i8_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(filter, fbuf, g.OC, pl.K, pl.Kpad);
+    pad_rows_i8_kernel<<<grid_of(blocks, 16), 256, 0, s>>>(filter, fbuf, g.OC, pl.K, pl.Kpad);
     GLOWB200_CUDA_OK(cudaGetLastError());
     b = fbuf;
     filter_row_sums = nullptr;  // recomputed over the padded copy (same values; keeps one code path)

@@ -213,7 +213,7 @@ cudaError_t launch_quantize_rows(bool vec, const __half *x, int M, int K, int pi
 cudaError_t quantize_rows(bool vec, const __half *x, int M, int K, int pitch, int8_t *q, float *scales, int32_t *sums,
                           int32_t *status, cudaStream_t s) {
   if (K <= 256 * 2) return launch_quantize_rows<1, 2>(vec, x, M, K, pitch, q, scales, sums, status, s);
-  if (M >= 8 * 2 * 148) return launch_quantize_rows<1, 0>(vec, x, M, K, pitch, q, scales, sums, status, s);
+  if (M >= 8 * 2 * kB200Sms) return launch_quantize_rows<1, 0>(vec, x, M, K, pitch, q, scales, sums, status, s);
   if (K <= 8 * 256 * 2) return launch_quantize_rows<8, 2>(vec, x, M, K, pitch, q, scales, sums, status, s);
   return launch_quantize_rows<8, 0>(vec, x, M, K, pitch, q, scales, sums, status, s);
 }

@@ -20,6 +20,7 @@
 // kernel returns.
 #include <cuda.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <cstdio>
 #include <mutex>
@@ -1044,19 +1045,17 @@ int launch_tile_mode(const CUtensorMap &ma, const CUtensorMap &mb, const GemmPar
 
 // CTA pairs of the int8 kernel that fit the device at once (0: not asked yet).  The kernels' shapes differ
 // only in shared memory, of which every one takes more than half an SM: one number serves them all.
-int &resident_pairs() {
-  static int n = 0;
+std::atomic<int> &resident_pairs() {
+  static std::atomic<int> n{0};
   return n;
 }
 
-// The same for clusters of two CTAs walking 256-row tiles (int8 results only).
+// The same for clusters of two CTAs walking 256-row tiles (int8 results in whole 16-byte pieces only).
 template <int BLOCK_N, int STAGES>
 int launch_pair_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmParams &p, cudaStream_t s) {
   using S = GemmSmem<BLOCK_N, STAGES, 1>;
   const int mode = int8_mode(p);
-  auto kernel = mode == 0   ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 0, 1>
-                : mode == 1 ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 1, 1>
-                            : i8_gemm_requant_kernel<BLOCK_N, STAGES, 3, 1>;
+  auto kernel = mode == 0 ? i8_gemm_requant_kernel<BLOCK_N, STAGES, 0, 1> : i8_gemm_requant_kernel<BLOCK_N, STAGES, 1, 1>;
   GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
   const int tiles = ((p.N + BLOCK_N - 1) / BLOCK_N) * ((p.M + 2 * kBlockM - 1) / (2 * kBlockM));
   cudaLaunchConfig_t cfg = {};
@@ -1096,9 +1095,6 @@ int launch_tile_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const GemmP
   }
 }
 
-#ifndef GLOWB200_GEMM_TILE_240
-#define GLOWB200_GEMM_TILE_240 1
-#endif
 // Columns of an output tile.  64 for narrow results; 128 when 256-column tiles would leave half
 // a tile (or more) of padding; else 256 -- unless 240-column tiles finish in fewer, or as many
 // but narrower, rounds over the SMs: 2048 x 4096 is 256 tiles of 256 columns (two rounds on 148
@@ -1114,10 +1110,8 @@ int pick_block_n(int M, int N) {
   if (((N + 127) / 128) & 1) {
     bn = 128;
   } else {
-#if GLOWB200_GEMM_TILE_240
     auto cost = [&](long b) { return ((tiles(b) + sms - 1) / sms) * (b + 16); };
     if (cost(240) * 100 < cost(256) * 97) bn = 240;
-#endif
   }
   if (bn > 128 && tiles(bn) * 2 <= sms) bn = 128;
   if (bn == 128 && tiles(128) * 2 <= sms) bn = 64;
@@ -1278,7 +1272,7 @@ int run_gemm(GemmParams p, const int8_t *a, const int8_t *b, const int32_t *b_ro
   if (b_offsets_zero) p.a_row_sums = nullptr;
   else if (!p.float_out) p.a_row_sums = as;
   p.K = pitch;
-  return launch_for_block_n(pick_tile(p.M, p.N, !p.float_out && !p.residual), a, p.M, p.K, p.K, b, p, s);
+  return launch_for_block_n(pick_tile(p.M, p.N, !p.float_out && int8_mode(p) <= 1), a, p.M, p.K, p.K, b, p, s);
 }
 
 namespace {

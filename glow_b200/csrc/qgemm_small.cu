@@ -395,9 +395,10 @@ cudaError_t launch_skinny(const GemmParams &p, const int8_t *a, const int8_t *b,
 struct SkinnyTile { int mt, nt; };
 SkinnyTile skinny_tile(int64_t M, int64_t N, int64_t K, bool kn) {
   auto blocks = [&](int mt, int nt) { return ((M + 16 * mt - 1) / (16 * mt)) * ((N + 8 * nt - 1) / (8 * nt)); };
+  constexpr int64_t sms = kB200Sms;
   SkinnyTile t{M <= 16 ? 1 : M <= 32 ? 2 : 4, 4};
   if (N * K >= (1 << 22)) {
-    if (!kn) t.nt = N >= 8 * 4 * (t.mt == 4 ? 110 : 148 * 2) ? 4 : N >= 8 * 2 * 148 ? 2 : 1;
+    if (!kn) t.nt = N >= 8 * 4 * (t.mt == 4 ? 110 : sms * 2) ? 4 : N >= 8 * 2 * sms ? 2 : 1;
     return t;
   }
   if (kn) {
@@ -406,7 +407,7 @@ SkinnyTile skinny_tile(int64_t M, int64_t N, int64_t K, bool kn) {
   }
   t.mt = 1;
   while (t.nt > 1 && blocks(1, t.nt) < 100) t.nt /= 2;
-  if (K > 64 && blocks(1, 4) >= 148 * 4) t.mt = blocks(2, 4) >= 148 * 6 ? 4 : 2;
+  if (K > 64 && blocks(1, 4) >= sms * 4) t.mt = blocks(2, 4) >= sms * 6 ? 4 : 2;
   return t;
 }
 
@@ -470,7 +471,7 @@ void prep_side_rows(PrepSide &o, const int8_t *src, int8_t *dst, int32_t *sums, 
 
 int prep_transposed_parts(int64_t rows, int64_t pitch) {
   const int64_t strips = (rows + kPrepTile - 1) / kPrepTile, steps = (pitch + kPrepTile - 1) / kPrepTile;
-  int64_t parts = (8 * 148 + strips - 1) / strips;
+  int64_t parts = (8 * kB200Sms + strips - 1) / strips;
   if (parts > kMaxSumParts) parts = kMaxSumParts;
   if (parts > steps) parts = steps;
   const int64_t span = (steps + parts - 1) / parts;  // steps per part; no part may be empty

@@ -618,18 +618,9 @@ extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_low_
     int indices_are_int64, const int32_t *lengths, int64_t segments, int64_t num_indices, int64_t in_line_size,
     int64_t out_line_size, int out_is_fp16, void *workspace, size_t workspace_bytes, int32_t *status,
     glowb200_stream_t stream) {
-  SlwsLaunch L;
-  GatherConfig g;
-  Form form;
-  int align;
-  if (int rc = fill_single(L, g, form, align, dest, data, kind, rows, weights, indices, indices_are_int64, lengths, segments,
-                           num_indices, in_line_size, out_line_size, out_is_fp16, 0, workspace, workspace_bytes, status))
-    return rc;
-  if (segments == 0) return GLOWB200_OK;
-  GLOWB200_REQUIRE(lengths != nullptr, "lengths is NULL");
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  GLOWB200_CUDA_OK(segments_from_lengths(L, form, segments, 1, s));
-  return run_gather(L, g, form, align, segments, 1, s);
+  return glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum(dest, data, kind, rows, weights, indices, indices_are_int64,
+                                                                      lengths, segments, num_indices, in_line_size, out_line_size,
+                                                                      out_is_fp16, 0, workspace, workspace_bytes, status, stream);
 }
 
 extern "C" int glowb200_embedding_bag_byte_rowwise_offsets(

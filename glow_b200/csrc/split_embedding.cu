@@ -11,7 +11,7 @@
 // lanes (as many as a row has 16-byte chunks, 8-byte ones for tables off 16-byte boundaries) owns a bag and walks its
 // rows in index order, each lane keeping the sums of the columns of its own chunk: every result
 // element is accumulated in the reference's order and in the result's type, with the multiply and the add
-// kept apart, so results are bit-identical to the Interpreter's.  Four rows are requested before
+// kept apart, so results are bit-identical to the Interpreter's.  Three rows are requested before
 // the first is consumed.
 //
 // A chunk of an fp32 or fp16 row, or of a quantized row off 16-byte boundaries, is cut from the row start, not
@@ -40,16 +40,11 @@ struct SplitLaunch {
 };
 
 constexpr int kThreads = 128;  // (a bag of a warp ends late: small blocks hand their registers on sooner)
-#ifndef GLOWB200_TBE_MIN_BLOCKS
-#define GLOWB200_TBE_MIN_BLOCKS 8
-#endif
-#ifndef GLOWB200_TBE_ROWS
-#define GLOWB200_TBE_ROWS 3
-#endif
+constexpr int kMinBlocks = 8;  // on an SM: 64 registers
 // Rows in flight per lane.  Four spill under 64 registers (128-column int4 bags of 64 rows: 207 against 190 us),
 // two leave more of the latency bare (210); so do 80 registers and fewer warps (211), and one group of rows being
 // added up while the next is on its way measured no better (190).
-constexpr int kRows = GLOWB200_TBE_ROWS;
+constexpr int kRows = 3;
 
 enum : int { TY_F32 = 0, TY_F16 = 1, TY_I8 = 2, TY_I4 = 3 };
 
@@ -490,7 +485,7 @@ __device__ __forceinline__ void clear_uncovered(const SplitLaunch &p) {
 }
 
 template <bool OUT16, typename IdxT>
-__global__ void __launch_bounds__(kThreads, GLOWB200_TBE_MIN_BLOCKS) split_embedding_bags_kernel(const __grid_constant__ SplitLaunch p) {
+__global__ void __launch_bounds__(kThreads, kMinBlocks) split_embedding_bags_kernel(const __grid_constant__ SplitLaunch p) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.y;
