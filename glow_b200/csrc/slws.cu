@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kSegThreads) slws_segments_from_lengths_kernel
   if (threadIdx.x == 0) {
     if (carry > N) flags |= GLOWB200_STATUS_LENGTHS_OVERRUN;
     out[S] = carry < N ? carry : N;
-    out[S + 1] = lengths_skewed(longest, carry, S);
+    out[S + 1] = skew_word(longest, carry, S);
   }
   raise_status(p.status, flags);
 }
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) slws_segments_from_offsets_kernel(const _
   const int most = __reduce_max_sync(0xffffffffu, (int)(mine < INT32_MAX ? mine : INT32_MAX));
   if ((threadIdx.x & 31) == 0) atomicMax(&longest, most);
   __syncthreads();
-  if (threadIdx.x == 0) p.seg_begin[S + 1] = lengths_skewed(longest, at(S) > at(0) ? at(S) - at(0) : 0, S);
+  if (threadIdx.x == 0) p.seg_begin[S + 1] = skew_word(longest, at(S) > at(0) ? at(S) - at(0) : 0, S);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -8,7 +8,7 @@ namespace glowb200 {
 struct SlwsLaunch {
   const glowb200_slws_job *jobs;  // device array, or nullptr when `single` is the only job
   glowb200_slws_job single;
-  int64_t *seg_begin;  // workspace: per job an int64 [segments + 1] array, then a word: are its lengths skewed?
+  int64_t *seg_begin;  // workspace: per job an int64 [segments + 1] array, then a word: the longest length if they are skewed, else 0
   int64_t seg_stride;  // int64 elements between the arrays of consecutive jobs
   int64_t max_segments;  // bags a table's array has room for (a descriptor naming more is cut short)
   int32_t *status;
@@ -19,8 +19,10 @@ struct SlwsLaunch {
   // slws_run.cu, slws_spread.cu: element types that need no kernel of their own, and whether the warps add up the
   // lengths before their bags themselves (no boundary array exists then)
   int32_t kind, idx64, out16, inline_lengths;
-  int32_t skewed_only;  // slws_spread.cu: the launch before this one pools the even tables
-  int32_t skewed_run;  // slws_run.cu: bags of a warp of a table with skewed lengths (the word behind its boundaries is not 0); 0: none
+  int32_t skewed_run;   // slws_run.cu: bags of a warp of a table with skewed lengths (the word behind its boundaries is not 0)
+  // Two launches that share the tables: slws_run.cu leaves those alone whose word is skip_from or more (0: pools all), and
+  // slws_spread.cu, launched behind it, pools those whose word is only_from or more (0: all).
+  int32_t skip_from, only_from;
 };
 
 // Bags of a table as the kernels walk them: never more than its boundary array has room for.
@@ -113,8 +115,11 @@ __device__ __forceinline__ bool take_run(const SlwsLaunch &p, const glowb200_slw
   return true;
 }
 
-// Whether the longest of the lengths is a step's rows beyond 2.5 times their mean.
-__host__ __device__ __forceinline__ bool lengths_skewed(int64_t longest, int64_t sum, int64_t bags) { return 2 * bags * (longest - 16) > 5 * sum; }
+// The word behind a table's boundaries: the longest of its lengths if that is a step's rows beyond 2.5 times their
+// mean, else 0.
+__device__ __forceinline__ int64_t skew_word(int32_t longest, int64_t sum, int64_t bags) {
+  return 2 * bags * ((int64_t)longest - 16) > 5 * sum ? longest : 0;
+}
 
 // The row an index (as ldg_index gives it) names, or -1: out of range, or another shard's.
 __device__ __forceinline__ int32_t row_number(const SlwsLaunch &p, const glowb200_slws_job *jp, int32_t rows, uint2 index, bool idx64,
@@ -287,7 +292,6 @@ constexpr int64_t kInlineLengthsMax = 2048;
 // Gather-pool with fp32 accumulation for rows of a multiple of 8 columns, any alignment (align: what
 // every row of every table starts on -- 8, 4 or 1 bytes): chooses between the two kernels (slws_spread.cu).
 cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s);
-// skip_skewed: tables whose lengths are known to be skewed are left to another launch.
-cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s, bool skip_skewed);
+cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s);
 
 }  // namespace glowb200

@@ -48,10 +48,10 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int even_run) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t segments = bags_of(p, jp);
   // (a table whose longest bag stands out: longer runs, the surplus blocks leave)
-  const int bags_per_warp =
-      !p.inline_lengths && p.seg_begin[(int64_t)blockIdx.y * p.seg_stride + segments + 1] != 0 ? p.skewed_run : even_run;
+  const int64_t word = p.inline_lengths ? 0 : p.seg_begin[(int64_t)blockIdx.y * p.seg_stride + segments + 1];
+  const int bags_per_warp = word != 0 ? p.skewed_run : even_run;
   const int64_t first_bag = ((int64_t)blockIdx.x * kWarps + warp) * bags_per_warp;
-  if (first_bag >= segments || bags_per_warp == 0) return;  // whole warps leave together (0: the skewed tables are another launch's)
+  if (first_bag >= segments || (p.skip_from != 0 && word >= p.skip_from)) return;  // whole warps leave together
   const int n_bags = (int)(first_bag + bags_per_warp < segments ? bags_per_warp : segments - first_bag);
   const int lpr = 1 << p.lpr_log2, gl = lane & (lpr - 1);
   const int64_t N = jp->num_indices;
@@ -290,7 +290,7 @@ cudaError_t launch_rows(const SlwsLaunch &L, int P, int U, dim3 grid, int bpw, c
 
 }  // namespace
 
-cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s, bool skip_skewed) {
+cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
   const int chunks = L.out_line / 8;
   const int64_t total = max_segments * num_jobs, sms = sm_count();
   auto lanes_log2 = [&](int per_lane) {
@@ -342,8 +342,7 @@ cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64
     // of 64 columns: 131 -> 92 us; two uint8 chunks would make it eight rows for 20 tables 43 -> 51)
     else if (wide_steps) U = 8;
   }
-  if (skip_skewed) L.skewed_run = 0;
-  else if (L.skewed_run < bpw) L.skewed_run = bpw;
+  if (L.skewed_run < bpw) L.skewed_run = bpw;
   const int64_t warps = warps_for(bpw);
   const dim3 grid((unsigned)((warps + kWarps - 1) / kWarps), (unsigned)num_jobs);
   switch (L.kind) {

@@ -57,7 +57,7 @@ constexpr int blocks_per_sm(int bits, int v, int lanes, int r) {
 template <int BITS, bool SO16, int ALIGN, int V, int LANES, int R>
 __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) slws_spread_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp) {
   // (beside the launch of the even tables, which has waited already; whoever waits for this one waits for both)
-  if (!p.skewed_only) pdl_wait();
+  if (!p.only_from) pdl_wait();
   pdl_launch_dependents();
   using Row = Rows<BITS, SO16, ALIGN>;
   constexpr int kBytes = V * BITS / 8, kWords = (kBytes + 3) / 4, kPairs = V / 2;
@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
   SlwsRun run;
   int32_t flags = 0;
   const int64_t segments = bags_of(p, jp);
-  auto leave = [&]() { if (p.skewed_only && blockIdx.x == 0 && blockIdx.y == 0) pdl_wait(); };
-  if (p.skewed_only && p.seg_begin[(int64_t)blockIdx.y * p.seg_stride + segments + 1] == 0) return leave();
+  auto leave = [&]() { if (p.only_from && blockIdx.x == 0 && blockIdx.y == 0) pdl_wait(); };
+  if (p.only_from && p.seg_begin[(int64_t)blockIdx.y * p.seg_stride + segments + 1] < p.only_from) return leave();
   if (!take_run(p, jp, segments, ((int64_t)blockIdx.x * kWarps + warp) * bags_per_warp, bags_per_warp, lane, run, flags)) return leave();  // whole warps leave together
   const int32_t rows = (int32_t)jp->rows;
   const int in_line = p.in_line;
@@ -264,7 +264,7 @@ cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t n
     return SpreadShape{v, lanes, rows, (int)std::min<int64_t>(kMaxRun, std::max<int64_t>(32 / lanes, (total + slots - 1) / slots))};
   };
   const int64_t small = sms * (columns <= 32 ? 14 : columns <= 64 ? 24 : 84);
-  if (align < 4 || columns > 256) return launch_slws_run(L, align, max_segments, num_jobs, s, false);
+  if (align < 4 || columns > 256) return launch_slws_run(L, align, max_segments, num_jobs, s);
   if (total <= small) {
     // (two bags to a warp once it has many; half the rows in flight, and more warps, where 4-bit rows fill it)
     const SpreadShape c = columns <= 64    ? shape(2, 32, 32, 1)
@@ -272,12 +272,12 @@ cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t n
                                            : shape(8, 32, four_bit && total <= sms * 12 ? 32 : 16, 1);
     return launch_slws_spread(L, c, align, max_segments, num_jobs, s);
   }
-  const bool two_launches = columns > 32 && (four_bit || columns <= 64) && max_segments > kInlineLengthsMax && total <= sms * 384;
-  if (cudaError_t e = launch_slws_run(L, align, max_segments, num_jobs, s, two_launches)) return e;
-  if (!two_launches) return cudaSuccess;
-  L.skewed_only = 1;
-  return launch_slws_spread(L, columns <= 64 ? shape(4, 16, 16, 1) : columns <= 128 ? shape(8, 16, 16, 3) : shape(8, 32, 16, 3), align,
-                            max_segments, num_jobs, s);
+  if (columns > 32 && max_segments > kInlineLengthsMax && total <= sms * 384) L.skip_from = four_bit || columns <= 64 ? 1 : 128;
+  if (cudaError_t e = launch_slws_run(L, align, max_segments, num_jobs, s)) return e;
+  if (L.skip_from == 0) return cudaSuccess;
+  L.only_from = L.skip_from;
+  const SpreadShape c = columns <= 64 ? shape(4, 16, 16, 1) : columns > 128 ? shape(8, 32, 16, 3) : four_bit ? shape(8, 16, 16, 3) : shape(4, 32, 32, 3);
+  return launch_slws_spread(L, c, align, max_segments, num_jobs, s);
 }
 
 }  // namespace glowb200

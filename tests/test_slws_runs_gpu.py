@@ -240,5 +240,5 @@ def test_both_forms_know_a_skewed_table(bags, skewed):
         got.append(form(dev(table), dev(w), dev(idx), dev(bounds), 0, workspace=ws))
         words = ws.view(torch.int64)[:bags + 2].cpu().numpy()
         np.testing.assert_array_equal(words[:-1], offsets)
-        assert words[-1] == int(skewed)
+        assert words[-1] == (150 if skewed else 0)
     assert torch.equal(got[0], got[1])
