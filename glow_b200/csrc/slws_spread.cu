@@ -10,12 +10,12 @@
 //     acc[k] = fma(w * scale, q[k], acc[k])   and   offsets = fma(w, offset, offsets)
 // row by row, so a bag has the same bits in either kernel.
 //
-// What bounds it is that chain.  Row numbers, and later {w * scale, w, offset}, pass from the lane that has them
+// What bounds it is that chain.  Row numbers, and later {w * scale twice, w, offset}, pass from the lane that has them
 // to the group through shared memory, four rows (one row) per load: a shuffle per row in front of each row's load
 // cost 115 - 190 cycles a row, the whole chain now takes about 60.  What decides beside it is that no load in flight
-// is spilled (blocks_per_sm).  18 tables, 91 skewed bags of up to 200 rows of 64 columns: 16.5 -> 12.4 us, of 4-bit
-// rows 16.8 -> 14.5; even bags of 40 rows 7.2 -> 6.3; 64 x 100 skewed bags of 128 columns 41 -> 35, even ones
-// 24.6 -> 17.8; 1024 even bags of 64 columns, one table 6.8 -> 5.8.
+// is spilled (blocks_per_sm).  18 tables, 91 skewed bags of up to 200 rows of 64 columns: 16.5 -> 12.0 us, of 4-bit
+// rows 16.8 -> 14.3; even bags of 40 rows 7.2 -> 6.2; 64 x 100 skewed bags of 128 columns 41 -> 33, even ones
+// 24.6 -> 18.0; 1024 even bags of 64 columns, one table 6.8 -> 5.6.
 #include <algorithm>
 
 
@@ -27,25 +27,20 @@ namespace {
 constexpr int kThreads = 64;
 constexpr int kWarps = kThreads / 32;
 
-// The V columns of a lane (1, 2, 4 or 8 bytes), as they lie in a row; like ldg_if.
-template <int BYTES, int ALIGN>
-__device__ __forceinline__ void ldg_columns(uint32_t (&v)[(BYTES + 3) / 4], const uint8_t *p, int row) {
+// The V columns of a lane, one word of them, as they lie in a row.
+template <int BYTES>
+__device__ __forceinline__ uint32_t ldg_columns(const uint8_t *p) {
+  uint32_t v;
   if constexpr (BYTES == 1) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p ld.global.nc.u8 %0, [%1];\n\t}" : "=r"(v[0]) : "l"(p), "r"(row));
+    asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(v) : "l"(p));
   } else if constexpr (BYTES == 2) {
     uint16_t h;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p ld.global.nc.u16 %0, [%1];\n\t}" : "=h"(h) : "l"(p), "r"(row));
-    v[0] = h;
-  } else if constexpr (BYTES == 4) {
-    v[0] = ldg_if(p, row);
-  } else if constexpr (ALIGN == 8) {
-    const uint2 q = ldg2_if(p, row);
-    v[0] = q.x;
-    v[1] = q.y;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(h) : "l"(p));
+    v = h;
   } else {
-    v[0] = ldg_if(p, row);
-    v[1] = ldg_if(p + 4, row);
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
   }
+  return v;
 }
 
 // Blocks on an SM: as many as leave every load in flight a register.
@@ -76,7 +71,7 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
   if (!take_run(p, jp, segments, ((int64_t)blockIdx.x * kWarps + warp) * bags_per_warp, bags_per_warp, lane, run, flags)) return leave();  // whole warps leave together
   const int32_t rows = (int32_t)jp->rows;
   const int in_line = p.in_line;
-  float4 *terms = shared_terms[warp] + group * R;  // of the rows being added up: {w * scale, w, offset, -}
+  float4 *terms = shared_terms[warp] + group * R;  // of the rows being added up: {w * scale, the same, w, offset}
   int4 *row_numbers = shared_rows[warp] + group * (R / 4);
   const bool idx64 = p.idx64 != 0, out16 = p.out16 != 0;
   const int idx_bytes = idx64 ? 8 : 4, w_bytes = out16 ? 2 : 4;
@@ -84,7 +79,7 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
   const char *weights = reinterpret_cast<const char *>(jp->weights) + (run.begin + gl) * w_bytes;
   const int column = gl * V;
   const bool active = column < p.out_line;
-  const uint8_t *data = reinterpret_cast<const uint8_t *>(jp->data);
+  const uint8_t *data = reinterpret_cast<const uint8_t *>(jp->data), *columns_at = data + (active ? gl * kBytes : 0);
 
   uint64_t acc[kPairs];
   float bias = 0.0f;  // sum of w * offset (and, 4-bit, minus the surplus)
@@ -139,9 +134,12 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
     __syncwarp();
     b.r = gl < s.n ? row_number(p, jp, rows, q.index, idx64, flags) : -1;
     b.w = out16 ? __half2float(__ushort_as_half((unsigned short)(q.high ? q.word >> 16 : q.word))) : __uint_as_float(q.word);
-    if (gl < R) reinterpret_cast<int32_t *>(row_numbers)[gl] = b.r;
+    // One word of columns: a row that is not there is read as row 0, without a predicate, and adds nothing (13 tables,
+    // 2164 skewed 4-bit bags 94 -> 80 us; where a lane has two words of them 131 -> 144).
+    if (gl < R) reinterpret_cast<int32_t *>(row_numbers)[gl] = kWords == 1 && b.r < 0 ? 0 : b.r;
     __syncwarp();
     b.tail = Row::tail(data + (int64_t)b.r * in_line + in_line, b.r);
+    if (kWords == 1 && rows == 0) return;  // (the whole warp)
     const int n = most(s.n);
     constexpr int kAtOnce = 8;
 #pragma unroll
@@ -153,7 +151,14 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
 #pragma unroll
       for (int k = 0; k < kAtOnce; k++) {
         const int32_t r = k % 4 == 0 ? r4[k / 4].x : k % 4 == 1 ? r4[k / 4].y : k % 4 == 2 ? r4[k / 4].z : r4[k / 4].w;
-        ldg_columns<kBytes, ALIGN>(b.columns[u0 + k], data + (int64_t)r * in_line + gl * kBytes, active ? r : -1);
+        if constexpr (kWords == 1) {
+          b.columns[u0 + k][0] = ldg_columns<kBytes>(columns_at + (int64_t)r * in_line);
+        } else {
+          const uint8_t *at = data + (int64_t)r * in_line + gl * kBytes;
+          const uint2 q = ALIGN == 8 ? ldg2_if(at, active ? r : -1) : make_uint2(ldg_if(at, active ? r : -1), ldg_if(at + 4, active ? r : -1));
+          b.columns[u0 + k][0] = q.x;
+          b.columns[u0 + k][kWords - 1] = q.y;
+        }
       }
     }
   };
@@ -161,8 +166,9 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
     __syncwarp();
     float scale, offset;
     Row::scale_offset(b.tail, scale, offset);
+    const float a = b.w * scale * Row::kUnit;
     // (a row that is not there adds nothing: -0 leaves every sum as it is)
-    if (gl < R) terms[gl] = b.r >= 0 ? make_float4(b.w * scale * Row::kUnit, b.w, offset, 0.0f) : make_float4(0.0f, 0.0f, -0.0f, 0.0f);
+    if (gl < R) terms[gl] = b.r >= 0 ? make_float4(a, a, b.w, offset) : make_float4(0.0f, 0.0f, 0.0f, -0.0f);
     __syncwarp();
     const int n = most(s.n);
 #pragma unroll
@@ -170,10 +176,10 @@ __global__ void __launch_bounds__(kThreads, blocks_per_sm(BITS, V, LANES, R)) sl
       if ((u & 3) == 0 && u >= n) break;
       const float4 c = terms[u];
       uint64_t a2;
-      asm("mov.b64 %0, {%1, %1};" : "=l"(a2) : "f"(c.x));
+      asm("mov.b64 %0, {%1, %2};" : "=l"(a2) : "f"(c.x), "f"(kWords == 1 ? c.y : c.x));
 #pragma unroll
       for (int k = 0; k < kWords; k++) pool_word<BITS, kPairsOfWord>(b.columns[u][k], a2, acc + k * kPairsOfWord);
-      bias = fmaf(c.y, c.z, bias);
+      bias = fmaf(c.z, c.w, bias);
       if (BITS == 4) bias -= c.x;
     }
     if (s.last) {
@@ -246,14 +252,15 @@ cudaError_t launch_slws_spread(const SlwsLaunch &L, SpreadShape c, int align, in
 // Which kernel pools a launch.  Rows of up to 256 columns at 4-byte boundaries; wider ones fill a warp in
 // slws_run.cu as well.
 //   * small launches take this one: up to some 24 bags per SM of narrow rows (64 columns), 84 of wider ones, which
-//     occupy a warp per bag in either kernel (30 tables, 400 skewed 4-bit bags of 96 columns: 67 -> 53 us, even ones
-//     31.3 -> 33.3; 14 x 567, 192 columns 73 -> 52; 5 x 1465 even uint8 bags of 256 columns 45 -> 41).  Above that
+//     occupy a warp per bag in either kernel (30 tables, 400 skewed 4-bit bags of 96 columns: 67 -> 50 us, even ones
+//     31.3 -> 31.3; 14 x 567, 192 columns 73 -> 50; 5 x 1465 even uint8 bags of 256 columns 45 -> 41).  Above that
 //     even bags are slws_run.cu's (86 x 244 of 128 columns 32.7 against 38.6).  Rows of 32 columns and less leave
 //     half of the lanes idle here: only where the warps are fewer than the SMs hold (2 x 211 skewed bags 16.9 -> 11.4).
 //   * in launches of up to 384 bags per SM whose boundaries' kernel knows which tables are skewed, those are a
-//     launch of their own beside that of the even tables: 13 tables, 2164 skewed 4-bit bags of 48 columns 104 -> 80 us,
-//     2 x 6965 of 64 68 -> 54, 8 x 4000 of 256 75 -> 66; where no table is skewed it costs 0.5 us.  uint8 rows of more than
-//     64 columns stay (10 x 4000 of 128: 156 -> 146 with 40 rows on average, 57 -> 62 with 12).
+//     launch of their own beside that of the even tables: 13 tables, 2164 skewed 4-bit bags of 48 columns 108 -> 80 us,
+//     2 x 6965 of 64 68 -> 45, 8 x 4000 of 256 177 -> 136; where no table is skewed it costs 0.3 us.  uint8 rows of more
+//     than 64 columns only with bags of 128 rows and more: 8 x 4096 of 128 144 -> 130 (10 x 4000 with bags of 12 rows
+//     on average, 78 at most, would take 62 instead of 54).
 cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
   const int64_t total = max_segments * num_jobs, sms = sm_count();
   const int columns = L.out_line;
