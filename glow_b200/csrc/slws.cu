@@ -561,9 +561,9 @@ int fill_single(SlwsLaunch &L, GatherConfig &g, Form &form, int &align, void *de
   GLOWB200_REQUIRE(rows >= 0 && rows < (1ll << 31) && num_indices >= 0, "rows must be in [0, 2^31), num_indices >= 0");
   GLOWB200_REQUIRE(segments == 0 || (dest && (num_indices == 0 || (data && weights && indices))),
                    "NULL tensor pointer");
-  // (slws_run.cu counts positions in 32 bits)
+  // (slws_run.cu counts rows in 32 bits)
   const bool fit = aligned_to(dest, out16 ? 2 : 4) && aligned_to(weights, out16 ? 2 : 4) && aligned_to(indices, idx64 ? 8 : 4) &&
-                   num_indices < (1ll << 31);
+                   num_indices <= kMostRows;
   g = GatherConfig{kind, idx64 ? 1 : 0, out16 ? 1 : 0, (acc16 && out16 && (kind & 1)) ? 1 : 0};
   align = (int)(reinterpret_cast<uintptr_t>(data) & 15) | 16;
   if (int rc = plan(g, in_line, out_line, fit, align, form)) return rc;

@@ -1,6 +1,8 @@
 // What the gather-pool sources (slws.cu, slws_run.cu, slws_spread.cu) share: the description of a launch
 // and the small device helpers.
 #pragma once
+#include <climits>
+
 #include "common.cuh"
 
 namespace glowb200 {
@@ -288,6 +290,11 @@ inline int chunks_per_lane(int chunks, bool four_bit) {
 
 // Bags of a table up to which the warps of slws_run.cu add up the lengths before their bags themselves.
 constexpr int64_t kInlineLengthsMax = 2048;
+
+// Rows of a warp's run that slws_run.cu counts: while one group walks a bag, four rows to a step, up to seven others
+// ask for one at every step, and how often they asked is a 32-bit number.  (A minimum on that count instead cost the
+// 256 even tables 12 % and the recommendation model's pooling 30 %: the registers.)
+constexpr int64_t kMostRows = INT32_MAX / 7 * 4ll;
 
 // Gather-pool with fp32 accumulation for rows of a multiple of 8 columns, any alignment (align: what
 // every row of every table starts on -- 8, 4 or 1 bytes): chooses between the two kernels (slws_spread.cu).

@@ -99,11 +99,11 @@ slws_run_kernel(const __grid_constant__ SlwsLaunch p, int even_run) {
     len = sb[1] - begin;
     if (len < 0) { len = 0; flags |= GLOWB200_STATUS_BAD_OFFSETS; }
   }
-  // Positions are 32-bit, relative to where the run begins.  (Index arrays of 2^31 entries and more are the
+  // Positions are 32-bit, relative to where the run begins.  (Index arrays of more than kMostRows entries are the
   // any-shape kernel's where the host can see them; here a run that long is cut short and reported.)
   const int64_t run0 = __shfl_sync(kAllLanes, begin, 0);
   int64_t rel = begin - run0;
-  if (lane < n_bags && (rel + len > INT32_MAX || rel < INT32_MIN)) { rel = 0; len = 0; flags |= GLOWB200_STATUS_LENGTHS_OVERRUN; }
+  if (lane < n_bags && (rel + len > kMostRows || rel < INT32_MIN)) { rel = 0; len = 0; flags |= GLOWB200_STATUS_LENGTHS_OVERRUN; }
   const int32_t from_l = (int32_t)rel, len_l = (int32_t)len;
 
   // ---- what a group is doing: its bag, where its next row is, how many are left ----

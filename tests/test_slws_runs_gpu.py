@@ -242,3 +242,28 @@ def test_both_forms_know_a_skewed_table(bags, skewed):
         np.testing.assert_array_equal(words[:-1], offsets)
         assert words[-1] == (150 if skewed else 0)
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 16), (3, 64)])
+def test_index_arrays_too_long_to_count(kind, dim):
+    """An index array of more entries than the kernels count takes the kernel that counts in 64 bits.  (The bags are
+    short and lie at its beginning: only its length, which bounds them and nothing else, is that large.)"""
+    import ctypes as C
+
+    from glow_b200 import _lib
+    rng = np.random.default_rng(1)
+    table, lengths = make_table(kind, 300, dim, 4), rng.integers(0, 40, 33).astype(np.int32)
+    n, dt = int(lengths.sum()), torch.float16 if kind & 1 else torch.float32
+    idx, w = rng.integers(0, 300, n), rng.normal(0, 1, n).astype(np.float16 if kind & 1 else np.float32)
+    want, size = want_and_size(table, kind, dim, w, idx, lengths)
+    size = with_4bit_surplus(size, table, kind, w, idx, lengths)
+    held, status = (dev(table), dev(w), dev(idx), dev(lengths)), ops.new_status(DEV)
+    ws = torch.empty(ops.slws_workspace_bytes(33), dtype=torch.uint8, device=DEV)
+    p = lambda a: C.c_void_p(a.data_ptr())
+    for claimed in (n, 2 ** 31 // 7 * 4 + 8, 2 ** 31 + 1):
+        out = torch.empty((33, dim), dtype=dt, device=DEV)
+        _lib.check(_lib.lib().glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum(
+            p(out), p(held[0]), kind, 300, p(held[1]), p(held[2]), 1, p(held[3]), 33, claimed, table.shape[1], dim,
+            int(dt == torch.float16), 0, p(ws), ws.numel(), p(status), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        check(out.cpu().numpy(), want, size, 2e-3 if kind & 1 else 1e-5)
+    assert int(status.item()) == 0
