@@ -521,7 +521,13 @@ PyObject *run_function(PyObject *const *a) {
     PyErr_SetString(PyExc_TypeError, "bindings must be a dict of placeholder names and arrays");
     throw Raised{};
   }
-  const size_t n = (size_t)PyDict_GET_SIZE(a[2]);
+  // (a list of its own: the names and arrays stay what they are whatever becomes of the dict during the call)
+  struct Items {
+    PyObject *list;
+    ~Items() { Py_XDECREF(list); }
+  } items{PyDict_Items(a[2])};
+  if (items.list == nullptr) throw Raised{};
+  const size_t n = (size_t)PyList_GET_SIZE(items.list);
   std::vector<const char *> names;
   std::vector<void *> buffers;
   std::vector<size_t> sizes;
@@ -531,9 +537,8 @@ PyObject *run_function(PyObject *const *a) {
     ~Views() { for (Py_buffer &b : v) PyBuffer_Release(&b); }
   } views;
   names.reserve(n), buffers.reserve(n), sizes.reserve(n), directions.reserve(n), views.v.reserve(n);
-  PyObject *key, *value;
-  Py_ssize_t pos = 0;
-  while (PyDict_Next(a[2], &pos, &key, &value)) {
+  for (size_t i = 0; i < n; i++) {
+    PyObject *item = PyList_GET_ITEM(items.list, (Py_ssize_t)i), *key = PyTuple_GET_ITEM(item, 0), *value = PyTuple_GET_ITEM(item, 1);
     const char *k = PyUnicode_AsUTF8(key);
     if (k == nullptr) throw Raised{};
     Py_buffer b;

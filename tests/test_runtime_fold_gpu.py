@@ -76,3 +76,25 @@ def test_folded_networks(oracle, dm, variant, pinned):
         dm.run_function("net", io, outputs={"out"})
     io["idx"][0, 0] = 0
     dm.run_function("net", io, outputs={"out"})
+
+
+def test_bindings_that_change_during_the_call(dm):
+    """The request is of the names and arrays that were bound when it was made, whatever becomes of the dict."""
+    tables = [workloads.fused_table_u8(ROWS, D, 3, t) for t in range(T)]
+    dm.add_network(network("net", tables, "plain"))
+    make = lambda: {"".join(["i", "dx"]): np.zeros((T, CAP), np.int32), "".join(["le", "n"]): np.full((T, B), 2, np.int32),
+                    "".join(["o", "ut"]): np.full((B, T * D + 8), -1, np.float32)}
+    want = make()
+    dm.run_function("net", want, outputs={"out"})
+    assert (want["out"][:, :T * D] != -1).any()
+
+    class Emptying:
+        def __contains__(self, name):
+            io.clear()
+            return name == "out"
+
+    io = make()
+    out = io["out"]
+    dm.run_function("net", io, outputs=Emptying())
+    assert not io
+    np.testing.assert_array_equal(out, want["out"])
