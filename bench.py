@@ -32,11 +32,11 @@ sys.path.insert(0, ROOT)
 ROWS, DIM, BATCH = 1_000_000, 64, 1024
 IN_LINE = DIM + 8
 # DRAM bytes per gathered 72-byte row of the uint8 gather kernel: dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch over 64 tables (4.6 waves of blocks, 2.10 M rows), from the
+# dram__bytes_write.sum of one launch of slws_run_kernel over 64 tables (2.10 M rows), from the
 # ncu capture summarised in profiles/.  ncu cannot run inside the timed region, so `traffic` is
 # this figure x the rows of the timed launch (traffic is proportional to rows: every row is
 # fetched once, L2 hit rate 13 %).
-NCU_DRAM_BYTES_PER_ROW = 205.6
+NCU_DRAM_BYTES_PER_ROW = 209.7
 METRIC = "frwq_slws_hbm_gbps"
 UNIT = "GB/s"
 
@@ -655,6 +655,16 @@ def dlrm_measure(torch, dist, dev, rank, world, steps, warmup, exchanges, as_ran
                                  "interaction; dense layers batch-sharded", "tables": 64, "batch": 4096}
 
 
+def kernel_nodes(graph):
+    """Kernel launches of one replay of a graph captured with keep_graph=True."""
+    from cuda.bindings import driver
+    handle = driver.CUgraph(graph.raw_cuda_graph())
+    _, _, n = driver.cuGraphGetNodes(handle, 0)
+    err, nodes, _ = driver.cuGraphGetNodes(handle, n)
+    assert err == driver.CUresult.CUDA_SUCCESS
+    return sum(driver.cuGraphNodeGetType(node)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL for node in nodes)
+
+
 def resnet_measure(torch, dev, steps, cpu_threads=0):
     """ResNet-50 v1.5, fully int8 channelwise-quantized, batch 64 at 224x224x3 (third benchmark
     configuration): images/s with the batch resident in HBM (CUDA-graph replay of the whole
@@ -671,14 +681,14 @@ def resnet_measure(torch, dev, steps, cpu_threads=0):
     for _ in range(3):
         out = model.forward(x)
     torch.cuda.synchronize()
-    launches = model.launches
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        graph = torch.cuda.CUDAGraph()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
         with torch.cuda.graph(graph, stream=side):
             out = model.forward(x)
+        launches = kernel_nodes(graph)
         graph.replay()
         torch.cuda.synchronize()
         e0.record()
@@ -1096,12 +1106,13 @@ def run_slws4_line(args):
                        "dim": D, "tables_per_gpu": T, "l2_policy": "tables far larger than L2, uniform indices"},
             "roofline": {"bound": "hbm", "achieved": per_gpu, "peak": peak, "unit": "GB/s", "frac": per_gpu / peak,
                          "peak_source": src,
-                         # DRAM bytes per launch: 196 B per row in the ncu capture of a smaller case of D=128
+                         # DRAM bytes per launch: 198 B per row in the ncu capture of a smaller case of D=128
                          # (profiles/), scaled by the rows of a launch; not captured for the other widths
-                         "traffic": 196.0 * float(np.mean([int(rq[3][-1]) for rq in reqs])) if D == 128 else None,
+                         "traffic": 198.0 * float(np.mean([int(rq[3][-1]) for rq in reqs])) if D == 128 else None,
                          "kernel": "slws_run_kernel<4,1,4,P,U>",
                          "rows_per_s": sum(int(reqs[i % R][3][-1]) for i in range(args.steps)) / (ms * 1e-3)},
-            "gpu_launches": 2 * args.steps, "clocks": clocks}
+            # boundaries and pooling; few enough bags add the launch that would take skewed tables
+            "gpu_launches": (3 if D > 32 and T * B <= 384 * 148 else 2) * args.steps, "clocks": clocks}
         if world == 1 and not args.no_cpu_baseline:
             threads = os.cpu_count() or 1
             v, passes, dt = slws4_cpu_rate(D, min(args.cpu_seconds, 10.0), threads)
@@ -1298,7 +1309,7 @@ def run_tbe_line(args):
             "roofline": {"bound": "hbm", "achieved": per_gpu, "peak": peak, "unit": "GB/s", "frac": per_gpu / peak,
                          "peak_source": src,
                          # DRAM bytes per launch from the ncu captures of smaller cases (profiles/), per row x rows
-                         "traffic": ({("int4", 128): 198.0, ("fp16", 128): 264.0}.get((args.tbe_type, D), 0.0) *
+                         "traffic": ({("int4", 128): 203.0, ("fp16", 128): 271.0}.get((args.tbe_type, D), 0.0) *
                                      float(np.mean([int(rq[0].shape[0]) for rq in reqs]))) or None,
                          "kernel": "split_embedding_bags_kernel<%s,long>" % ("true" if out16 else "false"),
                          "rows_per_s": sum(int(reqs[i % R][0].shape[0]) for i in range(args.steps)) / (ms * 1e-3)},
@@ -1716,7 +1727,7 @@ def main():
         q1.record()
         torch.cuda.synchronize()
         us = q0.elapsed_time(q1) * 1e3 / 200
-        # the same 200 launches replayed as one CUDA graph: the device's own latency per launch pair,
+        # the same 200 launches replayed as one CUDA graph: the device's own latency per launch,
         # without the host's call-and-launch pace
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
@@ -1729,7 +1740,7 @@ def main():
         q1.record()
         torch.cuda.synchronize()
         us_graph = q0.elapsed_time(q1) * 1e3 / 200
-        # the low-latency entry point (a warp per bag) on the same request
+        # the low-latency entry point on the same request
         def ll():
             ops.fused_rowwise_quantized_sparse_lengths_weighted_sum(
                 tables[0], weights_d[:starts[1]], indices_d[:starts[1]], lengths_d[0], ops.UINT8_FUSED, out=out[0],

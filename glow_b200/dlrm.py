@@ -420,8 +420,10 @@ class DLRMRank:
 
     @property
     def launches_per_step(self):
-        # segments + gather, quantize, FCs, dequantize x2, interaction
-        return 2 + 1 + len(self.bottom) + 1 + 1 + len(self.top) + 1
+        # pooling (boundaries and sums; up to 384 bags per SM a third that takes skewed tables), quantize,
+        # FCs, dequantize x2, interaction
+        pooling = 3 if self.cfg.batch > 2048 and len(self.my_tables) * self.cfg.batch <= 384 * 148 else 2
+        return pooling + 1 + len(self.bottom) + 1 + 1 + len(self.top) + 1
 
 
 def fixed_ranges(cfg):

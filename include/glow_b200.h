@@ -139,9 +139,9 @@ int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum(
     void *workspace, size_t workspace_bytes, int32_t *status, glowb200_stream_t stream);
 
 /* The same operator under the name callers use for small requests where latency counts.  It runs the
- * kernels of the entry point above and gives the same bits: a launch too small to fill the GPU fetches
- * sixteen rows of a bag at a time, and up to 2048 bags its warps also add up the lengths before their
- * bags themselves, so that the request is a single launch, whichever of the two is called.  fp32
+ * kernels of the entry point above and gives the same bits: a launch too small to fill the GPU spreads
+ * every bag over a warp or half a warp, and up to 2048 bags its warps also add up the lengths before
+ * their bags themselves, so that the request is a single launch, whichever of the two is called.  fp32
  * accumulation only. */
 int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_low_latency(
     void *dest, const void *data, int kind, int64_t rows, const void *weights, const void *indices,
