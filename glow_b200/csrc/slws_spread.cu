@@ -18,7 +18,6 @@
 // 24.6 -> 18.0; 1024 even bags of 64 columns, one table 6.8 -> 5.6.
 #include <algorithm>
 
-
 #include "slws.cuh"
 
 namespace glowb200 {
