@@ -33,6 +33,8 @@ SIGNATURES = {
         _int, [_vp, _vp, _int, _i64, _vp, _vp, _int, _vp, _i64, _i64, _i64, _i64, _int, _vp, _sz, _vp, _vp]),
     "glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched": (
         _int, [_vp, _i64, _i64, _int, _int, _i64, _i64, _int, _int, _vp, _sz, _vp, _vp]),
+    "glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched_sized": (
+        _int, [_vp, _i64, _i64, _int, _int, _i64, _i64, _int, _int, _i64, _vp, _sz, _vp, _vp]),
     "glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_row_sharded": (
         _int, [_vp, _i64, _i64, _int, _int, _i64, _i64, _vp, _sz, _vp, _vp]),
     "glowb200_slws_static_scratch_max_segments": (_i64, []),

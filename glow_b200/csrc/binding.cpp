@@ -22,7 +22,7 @@ namespace {
 #define GLOWB200_ENTRY_POINTS(X)                                                                                     \
   X(glowb200_last_error) X(glowb200_slws_workspace_bytes) X(glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum) \
   X(glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_low_latency)                                         \
-  X(glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched)                                             \
+  X(glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched_sized)                                       \
   X(glowb200_embedding_bag_byte_rowwise_offsets) X(glowb200_int_nbit_split_embedding_bags)                            \
   X(glowb200_i8_gemm_workspace_bytes) X(glowb200_dynamic_fc_workspace_bytes) X(glowb200_rowwise_quantized_fc_i8_i32)  \
   X(glowb200_fc_i8_i32) X(glowb200_matmul_i8) X(glowb200_dynamic_rowwise_quantized_fc) X(glowb200_dynamic_quantized_fc) \
@@ -225,12 +225,13 @@ PyObject *embedding_bag(PyObject *const *a) {
   return given ? same(a[7]) : give(out);
 }
 
-// jobs, count, max_segments, kind, int64 indices, in_line, out_line, fp16 result, fp16 accumulation, workspace, status
+// jobs, count, max_segments, kind, int64 indices, in_line, out_line, fp16 result, fp16 accumulation, workspace, status,
+// indices of all jobs
 PyObject *slws_batched(PyObject *const *a) {
   const Tensor &ws = any_tensor(a[9], "workspace");
-  invoke(fn.glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched, (const glowb200_slws_job *)address(a[0],
+  invoke(fn.glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched_sized, (const glowb200_slws_job *)address(a[0],
       "jobs"), integer(a[1]), integer(a[2]), (int)integer(a[3]), (int)integer(a[4]),
-      integer(a[5]), integer(a[6]), (int)integer(a[7]), (int)integer(a[8]), ws.data_ptr(), (size_t)ws.numel(),
+      integer(a[5]), integer(a[6]), (int)integer(a[7]), (int)integer(a[8]), integer(a[11]), ws.data_ptr(), (size_t)ws.numel(),
       (int32_t *)address(a[10], "status"), stream());
   Py_RETURN_NONE;
 }
@@ -596,7 +597,7 @@ PyMethodDef methods[] = {
     {"setup", setup, METH_VARARGS, nullptr},
     FAST("slws", slws, 12),
     FAST("embedding_bag", embedding_bag, 11),
-    FAST("slws_batched", slws_batched, 11),
+    FAST("slws_batched", slws_batched, 12),
     FAST("split_bags", split_bags, 16),
     FAST("rowwise_fc", rowwise_fc, 14),
     FAST("fc_i8", fc_i8, 14),

@@ -965,11 +965,14 @@ int execute(glowb200_device_manager *dm, LoadedNetwork &n, Context &c) {
         if (in.group >= 0) {  // part of a batched launch: the first member launches it for all
           if (in.group_leader) {
             const auto &grp = f->slws_groups[in.group];
-            int64_t max_segments = 0;
-            for (int m : grp) max_segments = std::max(max_segments, f->instrs[m].ia[4]);
-            rc = glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched(
+            int64_t max_segments = 0, num_indices = 0;
+            for (int m : grp) {
+              max_segments = std::max(max_segments, f->instrs[m].ia[4]);
+              num_indices += f->instrs[m].ia[5];
+            }
+            rc = glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched_sized(
                 c.jobs[in.group], (int64_t)grp.size(), max_segments, (int)a[0], (int)a[6], a[2], a[3], (int)a[7], (int)a[8],
-                c.workspace, f->workspace_bytes, c.status_dev, st);
+                num_indices, c.workspace, f->workspace_bytes, c.status_dev, st);
           }
           break;
         }

@@ -428,12 +428,12 @@ int plan(const GatherConfig &g, int64_t in_line, int64_t out_line, bool operands
   return GLOWB200_OK;
 }
 
-int run_gather(const SlwsLaunch &L, const GatherConfig &g, Form form, int align, int64_t max_segments, int64_t num_jobs,
+int run_gather(const SlwsLaunch &L, const GatherConfig &g, Form form, int align, int64_t max_segments, int64_t num_jobs, int64_t rows,
                cudaStream_t s) {
   if (max_segments == 0 || num_jobs == 0) return GLOWB200_OK;
   cudaError_t e;
   if (form == Form::kRuns) {
-    e = launch_slws(L, align, max_segments, num_jobs, s);
+    e = launch_slws(L, align, max_segments, num_jobs, rows, s);
   } else if (form == Form::kFp16Steps) {
     if (g.kind >= 2)
       e = g.idx64 ? launch_fp16_steps<4, int64_t>(L, max_segments, num_jobs, s) : launch_fp16_steps<4, int32_t>(L, max_segments, num_jobs, s);
@@ -503,7 +503,7 @@ extern "C" size_t glowb200_slws_workspace_bytes(int64_t max_segments, int64_t nu
 namespace {
 int run_batched(const glowb200_slws_job *jobs, int64_t num_jobs, int64_t max_segments, int kind, int indices_are_int64,
                 int64_t in_line_size, int64_t out_line_size, int out_is_fp16, int use_fp16_accumulation,
-                void *workspace, size_t workspace_bytes, int32_t *status, glowb200_stream_t stream, bool sharded) {
+                int64_t num_indices, void *workspace, size_t workspace_bytes, int32_t *status, glowb200_stream_t stream, bool sharded) {
   GLOWB200_REQUIRE(num_jobs >= 0 && num_jobs <= 65535, "num_jobs must be in [0, 65535]");
   GLOWB200_REQUIRE(max_segments >= 0 && max_segments < (1ll << 31), "max_segments out of range");
   if (num_jobs == 0 || max_segments == 0) return GLOWB200_OK;
@@ -532,7 +532,7 @@ int run_batched(const glowb200_slws_job *jobs, int64_t num_jobs, int64_t max_seg
   set_types(L, g);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   GLOWB200_CUDA_OK(segments_from_lengths(L, form, max_segments, num_jobs, s));
-  return run_gather(L, g, form, align, max_segments, num_jobs, s);
+  return run_gather(L, g, form, align, max_segments, num_jobs, num_indices, s);
 }
 }  // namespace
 
@@ -541,7 +541,15 @@ extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batc
     int64_t in_line_size, int64_t out_line_size, int out_is_fp16, int use_fp16_accumulation, void *workspace,
     size_t workspace_bytes, int32_t *status, glowb200_stream_t stream) {
   return run_batched(jobs, num_jobs, max_segments, kind, indices_are_int64, in_line_size, out_line_size, out_is_fp16,
-                     use_fp16_accumulation, workspace, workspace_bytes, status, stream, false);
+                     use_fp16_accumulation, kRowsUnknown, workspace, workspace_bytes, status, stream, false);
+}
+
+extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched_sized(
+    const glowb200_slws_job *jobs, int64_t num_jobs, int64_t max_segments, int kind, int indices_are_int64,
+    int64_t in_line_size, int64_t out_line_size, int out_is_fp16, int use_fp16_accumulation, int64_t num_indices,
+    void *workspace, size_t workspace_bytes, int32_t *status, glowb200_stream_t stream) {
+  return run_batched(jobs, num_jobs, max_segments, kind, indices_are_int64, in_line_size, out_line_size, out_is_fp16,
+                     use_fp16_accumulation, num_indices, workspace, workspace_bytes, status, stream, false);
 }
 
 extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_row_sharded(
@@ -549,7 +557,7 @@ extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_row_
     int64_t in_line_size, int64_t out_line_size, void *workspace, size_t workspace_bytes, int32_t *status,
     glowb200_stream_t stream) {
   return run_batched(jobs, num_jobs, max_segments, kind, indices_are_int64, in_line_size, out_line_size, 0, 0,
-                     workspace, workspace_bytes, status, stream, true);
+                     kRowsUnknown, workspace, workspace_bytes, status, stream, true);
 }
 
 namespace {
@@ -610,7 +618,7 @@ extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum(
   GLOWB200_REQUIRE(lengths != nullptr, "lengths is NULL");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   GLOWB200_CUDA_OK(segments_from_lengths(L, form, segments, 1, s));
-  return run_gather(L, g, form, align, segments, 1, s);
+  return run_gather(L, g, form, align, segments, 1, num_indices, s);
 }
 
 extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_low_latency(
@@ -647,7 +655,7 @@ extern "C" int glowb200_embedding_bag_byte_rowwise_offsets(
   else
     slws_segments_from_offsets_kernel<int32_t><<<blocks, 256, 0, s>>>(L, reinterpret_cast<const int32_t *>(offsets), has_end_offset ? 1 : 0);
   GLOWB200_CUDA_OK(cudaGetLastError());
-  return run_gather(L, g, form, align, segments, 1, s);
+  return run_gather(L, g, form, align, segments, 1, num_indices, s);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -733,5 +741,5 @@ extern "C" int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_stat
   // The segments kernel rewrites everything this call reads (segments + 1 boundaries); nothing in the
   // array has to start at zero, and whatever an earlier call left beyond them is never read.
   GLOWB200_CUDA_OK(segments_from_lengths(L, form, segments, 1, s));
-  return run_gather(L, g, form, align, segments, 1, s);
+  return run_gather(L, g, form, align, segments, 1, num_indices, s);
 }

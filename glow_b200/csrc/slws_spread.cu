@@ -250,17 +250,22 @@ cudaError_t launch_slws_spread(const SlwsLaunch &L, SpreadShape c, int align, in
 
 // Which kernel pools a launch.  Rows of up to 256 columns at 4-byte boundaries; wider ones fill a warp in
 // slws_run.cu as well.
-//   * small launches take this one: up to some 24 bags per SM of narrow rows (64 columns), 84 of wider ones, which
-//     occupy a warp per bag in either kernel (30 tables, 400 skewed 4-bit bags of 96 columns: 67 -> 50 us, even ones
-//     31.3 -> 31.3; 14 x 567, 192 columns 73 -> 50; 5 x 1465 even uint8 bags of 256 columns 45 -> 41).  Above that
-//     even bags are slws_run.cu's (86 x 244 of 128 columns 32.7 against 38.6).  Rows of 32 columns and less leave
-//     half of the lanes idle here: only where the warps are fewer than the SMs hold (2 x 211 skewed bags 16.9 -> 11.4).
+//   * small launches take this one: up to the 12 bags per SM that are resident at once of rows of 32 columns, which leave
+//     half of the lanes idle here (2 x 211 skewed bags 16.9 -> 11.4 us); up to 24 of 64 columns (26 x 128 13.7 -> 11.7); up to 84 of
+//     wider rows, which occupy a warp per bag in either kernel (30 tables, 400 skewed 4-bit bags of 96 columns: 67 -> 50,
+//     even ones 31.3 -> 31.3; 14 x 567, 192 columns 73 -> 50; 5 x 1465 even uint8 bags of 256 columns 45 -> 41). Above that even
+//     bags are slws_run.cu's (86 x 244 of 128 columns 32.7 against 38.6), and so are those just above 12 per SM, where
+//     half of the warps would have two (5 x 400 of 64 columns 5.0 against 5.6, of 128 5.4 against 5.8), and uint8
+//     rows of more than 128 columns as long as slws_run.cu gives them a warp per bag and 8 or 16 rows per step as well
+//     (5 x 400 of 192 columns 29.3 against 32.2).
+//   * bags of fewer than eight rows on average are one step in either kernel, and slws_run.cu has fewer warps to start
+//     (12 x 100 bags of 3 rows of 64 columns 3.8 against 4.3 us, 40 x 64 4.2 against 5.2, one table of 4 bags 3.3 against 3.5).
 //   * in launches of up to 384 bags per SM whose boundaries' kernel knows which tables are skewed, those are a
 //     launch of their own beside that of the even tables: 13 tables, 2164 skewed 4-bit bags of 48 columns 108 -> 80 us,
-//     2 x 6965 of 64 68 -> 45, 8 x 4000 of 256 177 -> 136; where no table is skewed it costs 0.3 us.  uint8 rows of more
-//     than 64 columns only with bags of 128 rows and more: 8 x 4096 of 128 144 -> 130 (10 x 4000 with bags of 12 rows
-//     on average, 78 at most, would take 62 instead of 54).
-cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
+//     2 x 6965 of 64 68 -> 45, 8 x 4000 of 256 177 -> 136; where no table is skewed it costs 0.3 to 0.7 us, so not with less than
+//     2^17 rows (2 x 2100 even bags of 10 rows 8.4 -> 9.1).  uint8 rows of more than 64 columns only with bags of 128 rows and
+//     more: 8 x 4096 of 128 144 -> 130 (10 x 4000 with bags of 12 rows on average, 78 at most, would take 62 instead of 54).
+cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, int64_t rows, cudaStream_t s) {
   const int64_t total = max_segments * num_jobs, sms = sm_count();
   const int columns = L.out_line;
   const bool four_bit = L.kind >= 2;
@@ -269,16 +274,18 @@ cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t n
     const int64_t slots = sms * kWarps * blocks_per_sm(four_bit ? 4 : 8, v, lanes, rows) * times;
     return SpreadShape{v, lanes, rows, (int)std::min<int64_t>(kMaxRun, std::max<int64_t>(32 / lanes, (total + slots - 1) / slots))};
   };
-  const int64_t small = sms * (columns <= 32 ? 14 : columns <= 64 ? 24 : 84);
-  if (align < 4 || columns > 256) return launch_slws_run(L, align, max_segments, num_jobs, s);
-  if (total <= small) {
+  const int64_t small = sms * (columns <= 32 ? 12 : columns <= 64 ? 24 : 84);
+  const bool short_bags = rows >= 0 && rows < total * 8, wide_bytes = !four_bit && columns > 128;
+  if (align < 4 || columns > 256 || (wide_bytes && total <= sms * 32)) return launch_slws_run(L, align, max_segments, num_jobs, s);
+  if (total <= small && !short_bags && !(columns <= 128 && total > sms * 12 && total <= sms * 16)) {
     // (two bags to a warp once it has many; half the rows in flight, and more warps, where 4-bit rows fill it)
     const SpreadShape c = columns <= 64    ? shape(2, 32, 32, 1)
                           : columns <= 128 ? (total <= sms * 54 ? shape(4, 32, 32, 1) : shape(8, 16, 16, 1))
                                            : shape(8, 32, four_bit && total <= sms * 12 ? 32 : 16, 1);
     return launch_slws_spread(L, c, align, max_segments, num_jobs, s);
   }
-  if (columns > 32 && max_segments > kInlineLengthsMax && total <= sms * 384) L.skip_from = four_bit || columns <= 64 ? 1 : 128;
+  if (columns > 32 && max_segments > kInlineLengthsMax && total <= sms * 384 && (rows < 0 || rows >= 1 << 17))
+    L.skip_from = four_bit || columns <= 64 ? 1 : 128;
   if (cudaError_t e = launch_slws_run(L, align, max_segments, num_jobs, s)) return e;
   if (L.skip_from == 0) return cudaSuccess;
   L.only_from = L.skip_from;

@@ -689,6 +689,7 @@ class SlwsBatch:
         self.sharded = False
         self.num_jobs = 0
         self.max_segments = 0
+        self.num_indices = -1
         self.workspace = None
         self._keep = None
 
@@ -739,6 +740,7 @@ class SlwsBatch:
         host = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8) if n else torch.empty(0, dtype=torch.uint8)
         self.jobs_dev = host.to(self.device)
         self.num_jobs = n
+        self.num_indices = sum(j.num_indices for j in arr)
         need = slws_workspace_bytes(self.max_segments, max(n, 1))
         if self.workspace is None or self.workspace.numel() < need:
             self.workspace = torch.empty(max(need, 8), dtype=torch.uint8, device=self.device)
@@ -755,4 +757,4 @@ class SlwsBatch:
                 _p(self.workspace), self.workspace.numel(), _p(status), _stream()))
             return
         _native().slws_batched(self.jobs_dev, self.num_jobs, self.max_segments, self.kind, self.index_dtype == torch.int64,
-                               self.in_line, self.out_line, self.out_fp16, self.fp16_acc, self.workspace, status)
+                               self.in_line, self.out_line, self.out_fp16, self.fp16_acc, self.workspace, status, self.num_indices)

@@ -160,6 +160,13 @@ int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched(
     int indices_are_int64, int64_t in_line_size, int64_t out_line_size, int out_is_fp16,
     int use_fp16_accumulation, void *workspace, size_t workspace_bytes, int32_t *status,
     glowb200_stream_t stream);
+/* The same for a caller who knows the indices of all jobs together (negative: unknown).  The number only helps to
+ * choose a kernel for the length of the bags; results do not depend on it. */
+int glowb200_fused_rowwise_quantized_sparse_lengths_weighted_sum_batched_sized(
+    const glowb200_slws_job *jobs, int64_t num_jobs, int64_t max_segments, int kind,
+    int indices_are_int64, int64_t in_line_size, int64_t out_line_size, int out_is_fp16,
+    int use_fp16_accumulation, int64_t num_indices, void *workspace, size_t workspace_bytes, int32_t *status,
+    glowb200_stream_t stream);
 
 /* The batched operator over row-range SHARDS of tables (row_begin / global_rows of every
  * descriptor are honoured): each launch gives the fp32 partial sums of the rows this GPU holds;

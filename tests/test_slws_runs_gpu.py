@@ -267,3 +267,30 @@ def test_index_arrays_too_long_to_count(kind, dim):
             int(dt == torch.float16), 0, p(ws), ws.numel(), p(status), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
         check(out.cpu().numpy(), want, size, 2e-3 if kind & 1 else 1e-5)
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 64), (0, 96), (2, 128), (0, 192), (3, 256)])
+@pytest.mark.parametrize("tables,bags,mean", [(3, 591, 7), (3, 592, 9), (3, 593, 9), (5, 400, 20), (4, 700, 3), (2, 2100, 12), (3, 2100, 30)])
+def test_kernels_chosen_by_the_rows_of_a_launch_agree(kind, dim, tables, bags, mean):
+    """Bags of a few rows and of more, on both sides of the launch sizes at which the length of bags decides: a caller who
+    says how many rows there are, one who does not, and one table at a time get the same bits."""
+    g = np.random.Generator(np.random.PCG64(tables * bags + mean))
+    dt = ops.result_dtype(kind)
+    data = [dev(make_table(kind, 500, dim, 20 + t)) for t in range(tables)]
+    lengths = [g.poisson(mean, bags).astype(np.int32) for _ in range(tables)]
+    lengths[0][1::9] = 0
+    lengths[1][5] = 150
+    idx = [dev(g.integers(0, 500, int(l.sum()))) for l in lengths]
+    w = [torch.rand(len(i), device=DEV).to(dt) for i in idx]
+    ln = [dev(l) for l in lengths]
+    out = torch.zeros((tables, bags, dim), dtype=dt, device=DEV)
+    status = ops.new_status(DEV)
+    batch = ops.SlwsBatch(kind, data[0].shape[1], torch.int64, device=DEV)
+    batch.bind(data, w, idx, ln, list(out))
+    batch.run(status)
+    known = out.clone()
+    out.zero_()
+    batch.num_indices = -1
+    batch.run(status)
+    one = torch.stack([ops.fused_rowwise_quantized_sparse_lengths_weighted_sum(*a, kind) for a in zip(data, w, idx, ln)])
+    assert torch.equal(out, known) and torch.equal(one, known) and int(status.item()) == 0
