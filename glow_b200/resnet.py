@@ -266,10 +266,10 @@ class ResNet50Int8:
             if self._capturing:
                 return self._head(self._features(self._quantize(x_nchw)))
             stream = torch.cuda.current_stream()
-            if stream != self._stream:   # the last call may still run on the other stream
-                if self._stream is not None:
+            if stream.cuda_stream != self._stream:   # (the handle: a Stream is "not unequal" to None)
+                if self._stream is not None:   # the last call may still run on the other stream
                     stream.wait_event(self._event)
-                self._stream = stream
+                self._stream = stream.cuda_stream
             r = self._replays.find(shape)
             if r is None and n * h * w <= self.REPLAY_PIXELS and self._replays.earned(shape):
                 r = self._replays.keep(shape, self._capture(shape))

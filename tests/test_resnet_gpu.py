@@ -178,6 +178,30 @@ def test_alternating_shapes_are_captured_once(net):
     assert len(captures) == resnet.Replays.KEPT and len(set(captures)) == len(captures)
 
 
+@pytest.mark.parametrize("replayed", [False, True])
+def test_a_call_on_another_stream_waits_for_the_last(net, replayed):
+    """The calls of a model share its workspace and buffers: one on a second stream does not start before the first
+    one, still queued behind other work of its stream, has ended."""
+    layers, w, q = net
+    model = resnet.ResNet50Int8(layers, q, DEV)
+    if not replayed:
+        model.REPLAY_PIXELS = 0
+    g = torch.Generator(device=DEV).manual_seed(8)
+    xs = [torch.randn((n, 3, 64, 64), device=DEV, generator=g) for n in (3, 2, 1)]
+    want = [[model.forward(x) for _ in range(3)][-1] for x in xs]   # (captured by now, each shape a graph)
+    streams, ended, got = [torch.cuda.Stream() for _ in xs], [torch.cuda.Event() for _ in xs], []
+    torch.cuda.synchronize()
+    for x, s, e in zip(xs, streams, ended):
+        with torch.cuda.stream(s):
+            if x is xs[0]:
+                torch.cuda._sleep(100_000_000)   # some 50 ms
+            got.append(model.forward(x))
+            e.record()
+    streams[-1].synchronize()
+    assert all(e.query() for e in ended)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_a_captured_forward_outlives_larger_calls(net):
     """A graph that a caller captured addresses the workspace of that time: it stays when a later call needs more."""
     layers, w, q = net
