@@ -76,9 +76,13 @@ inline bool make_add_quant(AddQuant &q, int32_t dest_off, int32_t l_off, int32_t
   return true;
 }
 #ifdef __CUDACC__
-// four elements: the bytes of two words
+// four elements: the bytes of two words (FLOOR false: saturation alone reaches q.floor)
+template <bool FLOOR = true>
 __device__ __forceinline__ uint32_t add_quant_word(uint32_t l, uint32_t r, const AddQuant &q) {
-  auto one = [&](int32_t a, int32_t b) { return __viaddmax_s32(a >> q.l_post, b >> q.r_post, q.floor); };
+  auto one = [&](int32_t a, int32_t b) {
+    if constexpr (FLOOR) return __viaddmax_s32(a >> q.l_post, b >> q.r_post, q.floor);
+    else return (a >> q.l_post) + (b >> q.r_post);
+  };
   const int lh = q.l_scale << 16, rh = q.r_scale << 16;
   const int32_t e0 = one(__dp2a_lo(q.l_scale, (int)l, q.l_const), __dp2a_lo(q.r_scale, (int)r, q.r_const));
   const int32_t e1 = one(__dp2a_lo(lh, (int)l, q.l_const), __dp2a_lo(rh, (int)r, q.r_const));

@@ -311,6 +311,20 @@ __device__ __forceinline__ int stage_offset(int r, int q16) {
   return r * PITCH + 16 * (q16 ^ x);
 }
 
+// Whether all epilogue threads say yes.
+__device__ __forceinline__ bool barrier_and(bool mine) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.and.pred p, 1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"((uint32_t)mine), "n"(kEpilogueThreads)
+      : "memory");
+  return ok != 0;
+}
+
 // x / d for 0 <= x < 2^31 with reciprocal = floor((2^32 - 1) / d): the estimate is the quotient or one less.
 __device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
   const int q = (int)__umulhi((uint32_t)x, reciprocal);
@@ -396,6 +410,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   // barrier on the way.  Tiles of 64 columns alternate between two halves of the warps (32 columns each: whole
   // 32-byte sectors), the others are split between all of them.
   constexpr bool kOwnRows = MODE == 0 || MODE == 1 || MODE == 4;
+  constexpr bool kFolds = MODE == 0 || MODE == 4;  // columns may be of the kind offset_folds admits
   constexpr bool kAlternate = kOwnRows && BLOCK_N <= 64;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::kTileBytes + S::kColBytes + S::kOutBytes);
   uint64_t *empty = full + STAGES;
@@ -543,6 +558,10 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const uint32_t line_div = p.conv_wp > 0 ? 0xffffffffu / (uint32_t)p.conv_wp : 0u;
     int lt = 0;
     bool dead = false;
+    // The column records in shared memory are {c, scale} and, behind them, pre, of columns that share `tile_post` and
+    // whose result offset rides on the rounding term; else ColParams and the rounding term.
+    [[maybe_unused]] bool folded = false;
+    [[maybe_unused]] int32_t tile_post = 0;
     int cols_n0 = -1;  // column block the records in shared memory belong to
     const uint32_t leader_acc_empty[2] = {PAIR ? map_to_cta(&acc_empty[0], 0) : 0u, PAIR ? map_to_cta(&acc_empty[1], 0) : 0u};
     int m_tile = walker % m_tiles, n_tile = walker / m_tiles;
@@ -556,12 +575,13 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       // column block: the records are rebuilt only when it changes (all epilogue threads see the
       // same n0, so the barriers stay matched).
       if (n0 != cols_n0) {
-        if (cols_n0 >= 0) asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");  // everyone is done with the old records
         cols_n0 = n0;
         static_assert(BLOCK_N <= kEpilogueThreads, "one column record per epilogue thread");
         const int j = n0 + et;
         ColParams cp = {0, 0, 0, 0};
-        [[maybe_unused]] int32_t rounding = 0;
+        [[maybe_unused]] int32_t pre = 0, post = 0;
+        [[maybe_unused]] bool narrow = true;
+        if constexpr (kFolds) tile_post = p.uniform ? p.u_out_post : p.out_post[n0];
         if (et < BLOCK_N && j < p.N) {
           if constexpr (MODE == 2) {  // {unused, column scale, float bias, weight offset}
             cp.scale = __float_as_int(p.col_scales ? p.col_scales[j] : p.u_col_scale);
@@ -579,19 +599,32 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                                   (uint32_t)p.k_corr * (uint32_t)p.a_offset * (uint32_t)q.b_off;
             cp.c = (int32_t)corr;
             cp.scale = q.out_scale;
-            if constexpr (MODE == 0 || MODE == 4) {  // nothing to unpack: {c, scale, pre, post}
-              cp.shifts = q.out_pre;
-              cp.b_off = q.out_post;
-            } else {
-              cp.shifts = q.out_pre | (q.out_post << 8);
-              cp.b_off = q.b_off;
-            }
-            rounding = (int32_t)((1u << q.out_post) >> 1);
+            cp.shifts = q.out_pre | (q.out_post << 8);
+            cp.b_off = q.b_off;
+            pre = q.out_pre;
+            post = q.out_post;
+            if constexpr (kFolds) narrow = post == tile_post && offset_folds(p.k_corr, cp.c, pre, post, cp.scale, p.out_offset);
           }
         }
-        if (et < BLOCK_N) {
-          cols[et] = cp;
-          if constexpr (kOwnRows) col_rounding[et] = rounding;
+        if constexpr (kFolds) {
+          // Whether every column of the tile is of the ordinary kind (offset_folds), agreed on by the epilogue warps, who
+          // are done with the old records then.
+          folded = barrier_and(narrow);
+          if (et < BLOCK_N) {
+            if (folded) {
+              reinterpret_cast<int2 *>(cols)[et] = make_int2(cp.c, cp.scale);
+              reinterpret_cast<int32_t *>(cols)[2 * BLOCK_N + et] = pre;
+            } else {
+              cols[et] = cp;
+              col_rounding[et] = (int32_t)((1u << post) >> 1);
+            }
+          }
+        } else {
+          if (lt > 0) asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");  // everyone is done with the old records
+          if (et < BLOCK_N) {
+            cols[et] = cp;
+            if constexpr (kOwnRows) col_rounding[et] = (int32_t)((1u << post) >> 1);
+          }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");  // epilogue warps only
       }
@@ -609,15 +642,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       } else {
         // All epilogue threads agree on the outcome of the (bounded) wait through a reducing
         // barrier, so either all of them drain the tile or all of them leave the loop.
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p, q;\n\t"
-            "setp.ne.u32 q, %1, 0;\n\t"
-            "barrier.cta.red.and.pred p, 1, %2, q;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(mine), "n"(kEpilogueThreads)
-            : "memory");
+        const bool ok = barrier_and(mine != 0);
         if (!ok) break;
       }
       tc_fence_after();
@@ -695,10 +720,13 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // 128 x 256 tile.)  The two bytes a lane has of each of two column groups make one 32-bit word, and four
         // of these, one per eight rows, are what stmatrix spreads over 32 rows of 16 bytes; a row's 16 bytes then
         // hold its column pairs in the order 0 4 1 5 2 6 3 7, which four byte permutes undo when they leave.
-        // What bounds it is the ALU: two shifts, an add-and-maximum and half a pack per element, little else
-        // being left.  Byte-pair stores into a tile that four warps shared, with their addresses and two barriers
-        // per tile, took 14 instructions per element: 200,704 x 64 x 256 ran 38.6 us, now 31.2; the stem's
-        // 64-column tiles 65, now 49.6.
+        // What bounds it is the ALU, where a shift, a pack or an add-and-maximum takes a scheduler two cycles.  The last of
+        // these falls away where the offset rides on the rounding term and saturation does a Relu's work (offset_folds;
+        // 7.7 -> 5.5 cycles per element in a loop of its own), and records of 12 bytes instead of 20 cost fewer
+        // shared-memory cycles: 200,704 x 64 x 256 26.9 -> 24.8 us, 50,176 x 128 x 512 16.6 -> 15.6, with a residual's Add 23.5 ->
+        // 21.3.  (The same formula as the upper half of a 64-bit multiply-add has no second shift, but takes 10.9 cycles.)
+        // Byte-pair stores into a tile that four warps shared, with their addresses and two barriers
+        // per tile, took 14 instructions per element: 200,704 x 64 x 256 ran 38.6 us.
         constexpr int kCols = S::kWarpCols, kPieces = kCols / 16;
         const int first = (kAlternate ? col_group & 1 : col_group) * kCols;
         const int last = first + kCols < BLOCK_N ? first + kCols : BLOCK_N;
@@ -728,68 +756,97 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           }
         }
         const int32_t relu_floor = p.act_type == 1 ? p.out_offset : INT32_MIN;
+        // FOLDED: see `folded`; FLOOR: a Relu whose floor saturation does not reach by itself
+        auto drain = [&](auto folded_tag, auto floor_tag) {
+          constexpr bool FOLDED = decltype(folded_tag)::value, FLOOR = decltype(floor_tag)::value;
+          [[maybe_unused]] const int32_t rounding = FOLDED ? (int32_t)(((1u << tile_post) >> 1) + ((uint32_t)p.out_offset << tile_post)) : 0;
 #pragma unroll 1
-        for (int c0 = first; c0 < last; c0 += 16) {
-          uint32_t acc[16];  // [row half h][column group g][row rr][column cc] -> 8h + 4g + 2rr + cc
-          tmem_ld_16x256b_x2(lane_addr + (uint32_t)c0, &acc[0]);
-          tmem_ld_16x256b_x2(lane_addr + (16u << 16) + (uint32_t)c0, &acc[8]);
-          tmem_ld_wait();
-          if (c0 + 16 >= last) {
-            // everything this warp needs from the buffer is in registers: hand it back
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              if constexpr (PAIR) mbar_arrive_cluster(leader_acc_empty[buf]);
-              else mbar_arrive(&acc_empty[buf]);
-            }
-          }
-          // the requantisation: libjit_scale, ((v >> pre) * scale + rtn) >> post, then + offset, with
-          // rtn = 1 << (post - 1) (0 for post 0); Relu is max(x, out_offset), no activation max(x, INT_MIN)
-          uint32_t word[4] = {0u, 0u, 0u, 0u};  // of row 8i + lane/4: {group 0, group 1} x two columns
-#pragma unroll
-          for (int g = 1; g >= 0; g--) {
-            int32_t res[2][4];  // [cc][i]
-            const int2 rtn = *reinterpret_cast<const int2 *>(&col_rounding[c0 + 8 * g + 2 * jq]);
-#pragma unroll
-            for (int cc = 0; cc < 2; cc++) {
-              const int4 cp = *reinterpret_cast<const int4 *>(&cols[c0 + 8 * g + 2 * jq + cc]);
-              const int32_t pre = MODE != 1 ? cp.z : cp.z & 0xff, post = MODE != 1 ? cp.w : cp.z >> 8;
-#pragma unroll
-              for (int i = 0; i < 4; i++) {  // i = 2h + rr
-                uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)cp.x;
-                if constexpr (MODE == 1) v -= (uint32_t)cp.w * (uint32_t)a_sums[i];  // 0 when no row sums take part
-                const int32_t m = (int32_t)((uint32_t)((int32_t)v >> pre) * (uint32_t)cp.y + (uint32_t)(cc ? rtn.y : rtn.x));
-                // max((m >> post) + offset, floor) in one instruction (a wrapping add, like the two it replaces)
-                int32_t x = __viaddmax_s32(m >> post, p.out_offset, relu_floor);
-                if constexpr (MODE == 1) {
-                  if (p.act_type > 1) x = activation_i32(x, p);
-                }
-                res[cc][i] = x;
+          for (int c0 = first; c0 < last; c0 += 16) {
+            uint32_t acc[16];  // [row half h][column group g][row rr][column cc] -> 8h + 4g + 2rr + cc
+            tmem_ld_16x256b_x2(lane_addr + (uint32_t)c0, &acc[0]);
+            tmem_ld_16x256b_x2(lane_addr + (16u << 16) + (uint32_t)c0, &acc[8]);
+            tmem_ld_wait();
+            if (c0 + 16 >= last) {
+              // everything this warp needs from the buffer is in registers: hand it back
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) {
+                if constexpr (PAIR) mbar_arrive_cluster(leader_acc_empty[buf]);
+                else mbar_arrive(&acc_empty[buf]);
               }
             }
+            uint32_t word[4] = {0u, 0u, 0u, 0u};  // of row 8i + lane/4: {group 0, group 1} x two columns
 #pragma unroll
-            for (int i = 0; i < 4; i++)  // sat8 of both columns (libjit_clip_i8) below the other group's two
-              asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(word[i]) : "r"(res[1][i]), "r"(res[0][i]), "r"(word[i]));
+            for (int g = 1; g >= 0; g--) {
+              int32_t res[2][4];  // [cc][i]
+              const int j = c0 + 8 * g + 2 * jq;
+              if constexpr (FOLDED) {
+                const int4 rec = *reinterpret_cast<const int4 *>(reinterpret_cast<const int2 *>(cols) + j);  // {c, scale} of both
+                const int2 pre = *reinterpret_cast<const int2 *>(reinterpret_cast<const int32_t *>(cols) + 2 * BLOCK_N + j);
+#pragma unroll
+                for (int cc = 0; cc < 2; cc++)
+#pragma unroll
+                  for (int i = 0; i < 4; i++) {  // i = 2h + rr
+                    uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)(cc ? rec.z : rec.x);
+                    int32_t x = (((int32_t)v >> (cc ? pre.y : pre.x)) * (cc ? rec.w : rec.y) + rounding) >> tile_post;
+                    if constexpr (FLOOR) x = max(x, relu_floor);
+                    res[cc][i] = x;
+                  }
+              } else {
+                // libjit_scale as it is written, ((v >> pre) * scale + rtn) >> post, then + offset, with
+                // rtn = 1 << (post - 1) (0 for post 0); Relu is max(x, out_offset), no activation max(x, INT_MIN)
+                const int2 rtn = *reinterpret_cast<const int2 *>(&col_rounding[j]);
+#pragma unroll
+                for (int cc = 0; cc < 2; cc++) {
+                  const int4 cp = *reinterpret_cast<const int4 *>(&cols[j + cc]);
+                  const int32_t pre = cp.z & 0xff, post = cp.z >> 8;
+#pragma unroll
+                  for (int i = 0; i < 4; i++) {
+                    uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)cp.x;
+                    if constexpr (MODE == 1) v -= (uint32_t)cp.w * (uint32_t)a_sums[i];  // 0 when no row sums take part
+                    const int32_t m = (int32_t)((uint32_t)((int32_t)v >> pre) * (uint32_t)cp.y + (uint32_t)(cc ? rtn.y : rtn.x));
+                    // max((m >> post) + offset, floor) in one instruction (a wrapping add, like the two it replaces)
+                    int32_t x = __viaddmax_s32(m >> post, p.out_offset, relu_floor);
+                    if constexpr (MODE == 1) {
+                      if (p.act_type > 1) x = activation_i32(x, p);
+                    }
+                    res[cc][i] = x;
+                  }
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 4; i++)  // sat8 of both columns (libjit_clip_i8) below the other group's two
+                asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(word[i]) : "r"(res[1][i]), "r"(res[0][i]), "r"(word[i]));
+            }
+            asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(
+                             smem_u32(stage + stage_offset<kCols>(lane, (c0 - first) >> 4))),
+                         "r"(word[0]), "r"(word[1]), "r"(word[2]), "r"(word[3])
+                         : "memory");
           }
-          asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(
-                           smem_u32(stage + stage_offset<kCols>(lane, (c0 - first) >> 4))),
-                       "r"(word[0]), "r"(word[1]), "r"(word[2]), "r"(word[3])
-                       : "memory");
-        }
+        };
+        if (!kFolds || !folded) drain(std::false_type{}, std::false_type{});
+        else if (relu_floor > -128) drain(std::true_type{}, std::true_type{});
+        else drain(std::true_type{}, std::false_type{});
         __syncwarp();
+        // (FLOOR: the Add's floor is one that saturation alone does not reach)
+        auto leave = [&](auto floor_tag) {
+          constexpr bool FLOOR = decltype(floor_tag)::value;
 #pragma unroll
-        for (int it = 0; it < kPieces; it++) {
-          const int r = it * (32 / kPieces) + lane / kPieces, q16 = lane % kPieces;
-          const int dst = __shfl_sync(0xffffffffu, dst_row, r);
-          const uint4 w = *reinterpret_cast<const uint4 *>(stage + stage_offset<kCols>(r, q16));
-          uint4 o = make_uint4(__byte_perm(w.x, w.y, 0x5410), __byte_perm(w.z, w.w, 0x5410),
-                               __byte_perm(w.x, w.y, 0x7632), __byte_perm(w.z, w.w, 0x7632));
-          if constexpr (MODE == 4)
-            o = make_uint4(add_quant_word(o.x, other[it].x, p.add), add_quant_word(o.y, other[it].y, p.add),
-                           add_quant_word(o.z, other[it].z, p.add), add_quant_word(o.w, other[it].w, p.add));
-          const int col = first + 16 * q16;
-          if (dst >= 0 && col < last && n0 + col < p.N) *reinterpret_cast<uint4 *>(p.out + (size_t)dst * p.N + n0 + col) = o;
-        }
+          for (int it = 0; it < kPieces; it++) {
+            const int r = it * (32 / kPieces) + lane / kPieces, q16 = lane % kPieces;
+            const int dst = __shfl_sync(0xffffffffu, dst_row, r);
+            const uint4 w = *reinterpret_cast<const uint4 *>(stage + stage_offset<kCols>(r, q16));
+            uint4 o = make_uint4(__byte_perm(w.x, w.y, 0x5410), __byte_perm(w.z, w.w, 0x5410),
+                                 __byte_perm(w.x, w.y, 0x7632), __byte_perm(w.z, w.w, 0x7632));
+            if constexpr (MODE == 4)
+              o = make_uint4(add_quant_word<FLOOR>(o.x, other[it].x, p.add), add_quant_word<FLOOR>(o.y, other[it].y, p.add),
+                             add_quant_word<FLOOR>(o.z, other[it].z, p.add), add_quant_word<FLOOR>(o.w, other[it].w, p.add));
+            const int col = first + 16 * q16;
+            if (dst >= 0 && col < last && n0 + col < p.N) *reinterpret_cast<uint4 *>(p.out + (size_t)dst * p.N + n0 + col) = o;
+          }
+        };
+        if (MODE == 4 && p.add.floor > -128) leave(std::true_type{});
+        else leave(std::false_type{});
         __syncwarp();  // read back before the next tile's pieces arrive
       } else {
         // The int8 result in ragged rows (N not a multiple of 16, or an unaligned result): the same loads, but

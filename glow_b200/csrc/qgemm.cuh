@@ -66,6 +66,16 @@ __device__ __forceinline__ ColQuant col_quant(const GemmParams &p, int j) {
           p.out_pre[j], p.out_post[j], p.out_scale[j]};
 }
 
+// Whether the result offset of a column may ride on its rounding term, (((v >> pre) * scale + rtn) >> post) + offset ==
+// ((v >> pre) * scale + rtn + (offset << post)) >> post, for every v = dot + c that `k` products of two bytes
+// can give: nothing may pass 32 bits, where both wrap, each in its own place.
+__host__ __device__ inline bool offset_folds(int64_t k, int32_t c, int32_t pre, int32_t post, int32_t scale, int32_t offset) {
+  if (pre < 0 || pre > 30 || post < 1 || post > 30 || scale < 0 || k >= 1ll << 24) return false;
+  const auto size = [](int32_t x) { return x < 0 ? -(int64_t)x : (int64_t)x; };
+  const int64_t most = size(c) + k * (128 * 128);
+  return most < 1ll << 31 && ((most >> pre) + 1) * scale + (1ll << (post - 1)) + (size(offset) << post) < 1ll << 31;
+}
+
 // bias[j] of either element type (libjit_fc_generic / libjit_rowwise_quantized_fc_generic /
 // libjit_*_conv2d_generic are templates over BiasElemTy: int32 for the _i8_i32 entry points, int8 for _i8_i8).
 __device__ __forceinline__ int32_t load_bias(const GemmParams &p, int j) {

@@ -195,3 +195,26 @@ def test_bounded_wait_gives_up_and_leaves_the_context_usable(oracle):
     got, status = run_rwq(c)
     assert status == 0
     np.testing.assert_array_equal(got, oracle_rwq(oracle, c))
+
+
+@pytest.mark.parametrize("k", [64, 1120])
+@pytest.mark.parametrize("pre,post,scale,offset,relu", [
+    ((2, 3), (15, 15), (255, 510), -128, True),        # the ordinary kind: the offset rides on the rounding term
+    ((0, 5), (15, 15), (255, 510), 7, True),           # with a floor of its own
+    ((2, 3), (14, 15), (255, 510), -3, False),         # columns that do not share the last shift
+    ((0, 1), (0, 0), (1, 2), 4, False),                # no last shift, no rounding term
+    ((0, 0), (15, 15), (20000, 32767), 0, False),      # products that wrap in 32 bits
+    ((0, 1), (30, 30), (1, 400), 90, True),
+    ((3, 3), (15, 15), (255, 510), 1 << 18, False),    # an offset that would wrap on the rounding term
+])
+def test_tile_drain_of_any_requantisation(k, pre, post, scale, offset, relu):
+    """Integers bit for bit: the loop as the reference writes it is what the tile kernel has to give."""
+    rng = np.random.default_rng(k + post[1] + scale[0])
+    m, n = 1500, 272
+    x, w = (torch.from_numpy(rng.integers(-128, 128, s, dtype=np.int8)).to(DEV) for s in ((m, k), (n, k)))
+    col = lambda lo, hi: torch.from_numpy(rng.integers(lo, hi + 1, n, dtype=np.int32)).to(DEV)
+    bias, zero = col(-40000, 40000), col(0, 0)
+    args = (x, w, bias, zero, (col(0, 2), col(0, 15), col(1, 400)), (col(*pre), col(*post), col(*scale)), offset, -5, 0)
+    flags = ops.FC_WEIGHT_OFFSETS_ZERO | (ops.FC_FUSE_RELU if relu else 0)
+    want = ops.rowwise_quantized_fc(*args, flags=flags | ops.FC_FORCE_ANY_SHAPE_KERNEL)
+    assert torch.equal(ops.rowwise_quantized_fc(*args, flags=flags), want)
