@@ -69,6 +69,8 @@ SIGNATURES = {
         _int, [_vp] * 10 + [_i64, _vp, _i32, _i32] + [_vp] * 8 + [_i32, _vp, _vp, _int, _vp, _sz, _vp, _vp]),
     "glowb200_channelwise_quantized_conv2d_add_i8": (
         _int, [_vp] * 10 + [_i64, _vp, _i32, _i32] + [_vp] * 8 + [_i32, _vp, _vp, _int, _vp, _sz, _vp, _vp] + [_i32] * 10 + [_vp]),
+    "glowb200_channelwise_quantized_conv2d_pair_workspace_bytes": (_sz, [_vp] * 5),
+    "glowb200_channelwise_quantized_conv2d_pair_i8_i32": (_int, [_vp] * 8 + [_sz, _vp, _vp]),
     "glowb200_conv2d_i8_i32": (
         _int, [_vp] * 10 + [_i64] + [_i32] * 10 + [_vp, _i32, _vp, _int, _vp, _sz, _vp, _vp]),
     "glowb200_element_add_i8": (_int, [_vp, _vp, _vp, _i64] + [_i32] * 9 + [_vp]),

@@ -27,6 +27,7 @@ namespace {
   X(glowb200_i8_gemm_workspace_bytes) X(glowb200_dynamic_fc_workspace_bytes) X(glowb200_rowwise_quantized_fc_i8_i32)  \
   X(glowb200_fc_i8_i32) X(glowb200_matmul_i8) X(glowb200_dynamic_rowwise_quantized_fc) X(glowb200_dynamic_quantized_fc) \
   X(glowb200_conv2d_workspace_bytes) X(glowb200_channelwise_quantized_conv2d_i8_i32) \
+  X(glowb200_channelwise_quantized_conv2d_pair_workspace_bytes) X(glowb200_channelwise_quantized_conv2d_pair_i8_i32) \
   X(glowb200_channelwise_quantized_conv2d_add_i8) X(glowb200_element_add_maxsplat_i8) \
   X(glowb200_element_quantize_i8) X(glowb200_element_dequantize_i8) X(glowb200_max_pool_i8) X(glowb200_avg_pool_i8)    \
   X(glowb200_quantize_transpose_i8) X(glowb200_pairwise_dot_interaction) X(glowb200_device_manager_run_function_io)
@@ -415,6 +416,55 @@ PyObject *channelwise_conv(PyObject *const *a) {
   return given ? same(a[18]) : give(out);
 }
 
+// A layer of a pair: filt, bias, kernels, strides, pads, group, dilation, out offset, in offset, filter offsets, bias
+// offsets, bias triples, out triples, activation, its arguments, filter row sums, flags
+struct ConvLayer {
+  const Items<17> a;
+  const Tensor &f;
+  const Ints<2> k, s, d;
+  const Ints<4> p;
+  const Triples bt, ot;
+  const int64_t fd[4];
+  int32_t act[3] = {0, 0, 0};
+  glowb200_conv_layer layer;
+  ConvLayer(PyObject *o, const char *which)
+      : a(o, which), f(cuda_tensor(a[0], "filt", I8)), k(a[2], "kernels"), s(a[3], "strides"), d(a[6], "dilation"), p(a[4], "pads"),
+        bt(a[11], false), ot(a[12], false), fd{f.size(0), f.size(1), f.size(2), f.size(3)} {
+    if (a[14] != Py_None) {
+      const Ints<3> v(a[14], "act_args");
+      for (int i = 0; i < 3; i++) act[i] = (int32_t)v.v[i];
+    }
+    auto ints = [&](int i, const char *name) { return (const int32_t *)address(a[i], name); };
+    layer = glowb200_conv_layer{(const int8_t *)f.data_ptr(), ints(1, "bias"), ints(9, "filter_offsets"), ints(10, "bias_offsets"),
+                                bt.p[0], bt.p[1], bt.p[2], ot.p[0], ot.p[1], ot.p[2], ints(15, "filter_row_sums"),
+                                fd, k.v, s.v, p.v, d.v, integer(a[5]), (int32_t)integer(a[8]), (int32_t)integer(a[7]),
+                                (int32_t)integer(a[13]), a[14] != Py_None ? act : nullptr, (int)integer(a[16])};
+  }
+  // dims of its result over an input of dims `in`
+  void result(const int64_t (&in)[4], int64_t (&out)[4]) const {
+    out[0] = in[0];
+    for (int i = 0; i < 2; i++) out[1 + i] = conv_out(in[1 + i], k.v[i], s.v[i], p.v[i] + p.v[2 + i], d.v[i]);
+    out[3] = fd[0];
+  }
+};
+
+// inp, first layer, second layer, out, workspace, status
+PyObject *channelwise_conv_pair(PyObject *const *a) {
+  const Tensor &x = cuda_tensor(a[0], "inp", I8);
+  const ConvLayer first(a[1], "first"), second(a[2], "second");
+  const int64_t in[4] = {x.size(0), x.size(1), x.size(2), x.size(3)};
+  int64_t mid[4], od[4];
+  first.result(in, mid);
+  second.result(mid, od);
+  const bool given = a[3] != Py_None;
+  const Tensor out = given ? any_tensor(a[3], "out") : empty({od[0], od[1], od[2], od[3]}, at::kChar, x);
+  const Workspace ws(a[4], a[4] == Py_None ? fn.glowb200_channelwise_quantized_conv2d_pair_workspace_bytes(in, mid, od, &first.layer,
+                                                                                                           &second.layer) : 0, x);
+  invoke(fn.glowb200_channelwise_quantized_conv2d_pair_i8_i32, (int8_t *)out.data_ptr(), (const int8_t *)x.data_ptr(), in, mid, od,
+         &first.layer, &second.layer, ws.data(), ws.bytes(), (int32_t *)address(a[5], "status"), stream());
+  return given ? same(a[3]) : give(out);
+}
+
 // lhs, rhs, dest offset, lhs offset, rhs offset, lhs triple, rhs triple, splat, out
 PyObject *add_maxsplat(PyObject *const *a) {
   const Tensor &l = any_tensor(a[0], "lhs"), &r = any_tensor(a[1], "rhs");
@@ -606,6 +656,7 @@ PyMethodDef methods[] = {
     FAST("dynamic_fc", dynamic_fc<false>, 10),
     FAST("channelwise_conv", channelwise_conv<false>, 21),
     FAST("channelwise_conv_add", channelwise_conv<true>, 28),
+    FAST("channelwise_conv_pair", channelwise_conv_pair, 6),
     FAST("add_maxsplat", add_maxsplat, 9),
     FAST("quantize", element_convert<true>, 4),
     FAST("dequantize", element_convert<false>, 4),

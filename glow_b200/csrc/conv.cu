@@ -348,6 +348,72 @@ ConvPlan plan_conv(const ConvGeom &g, bool force_direct) {
   return pl;
 }
 
+int pad_word(int32_t offset) {
+  const uint32_t b = (uint8_t)offset;
+  return (int)(b | (b << 8) | (b << 16) | (b << 24));
+}
+
+// Windows over 64 or a multiple of 128 channels, symmetric filters: no im2col matrix.
+// Stride 1: the input lies in a padded NHWC buffer [N, h, w, C]; tap (kh, kw) of output row q then is row q + kh * w + kw
+// of that buffer, which the contraction's loads address directly (the rows of the product that fall on the
+// padding are computed and dropped).  Stride 2 (multiples of 128 channels): the same over four planes by the parity of
+// the padded coordinates (see pad_parity_nhwc_i8_kernel).  The scratch sized for the im2col matrix is more than this needs.
+// 64 channels: two neighbouring pixels per 128-byte row against a filter re-laid in tap pairs (the
+// partner of an odd last tap zero).  One tap per 64-byte k-block in the 64-byte swizzle -- no
+// wasted MMAs, a quarter fewer operand bytes, nine k-blocks instead of six for a 3 x 3 window --
+// gave the same results and a slower network (1.590 against 1.562 ms per ResNet-50 batch).
+struct ShiftedRows {
+  int planes, h, w, pairs, entries;  // pairs: of taps in a filter row (64 channels; else 0)
+  int64_t rows;                      // pixels of a plane
+  size_t input_bytes, pair_bytes;    // of the buffer, and of the filter re-laid behind it
+};
+bool shifted_rows(const ConvGeom &g, const ConvPlan &pl, int flags, ShiftedRows &r) {
+  if (!pl.need_im2col || g.SH != g.SW || g.SH > 2 || g.DH != 1 || g.DW != 1 || !(flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO)) return false;
+  r = ShiftedRows{};
+  if (g.SH == 1) {
+    if (g.C != 64 && g.C % 128 != 0) return false;
+    r.planes = 1;
+    r.h = g.OH + g.KH - 1;
+    r.w = g.OW + g.KW - 1;
+    if (r.h < g.H + g.PT || r.w < g.W + g.PL) return false;
+    r.pairs = g.C == 64 ? (g.KW + 1) / 2 : 0;
+  } else {
+    if (g.C % 128 != 0 || (g.KH == 1 && g.KW == 1)) return false;
+    r.planes = 4;
+    r.h = g.OH + (g.KH - 1) / 2;
+    r.w = g.OW + (g.KW - 1) / 2;
+  }
+  r.entries = g.KH * (r.pairs ? r.pairs : g.KW);
+  r.rows = (int64_t)g.N * r.h * r.w;
+  r.input_bytes = align_up((size_t)(r.planes * r.rows) * g.C + 256, 256);
+  r.pair_bytes = r.pairs ? align_up((size_t)g.OC * r.entries * 128, 256) : 0;
+  return r.entries <= 32 && r.planes * r.rows < (1ll << 31) && r.input_bytes + r.pair_bytes <= pl.a_bytes + pl.f_bytes;
+}
+
+// The contraction over such a buffer; b: the filter, in tap pairs where r.pairs.
+int run_shifted_rows(GemmParams p, const ConvGeom &g, const ConvPlan &pl, const ShiftedRows &r, const int8_t *xp, const int8_t *b,
+                     const int32_t *filter_row_sums, uint8_t *sums_ws, cudaStream_t s) {
+  p.K = r.pairs ? r.entries * 128 : g.KH * g.KW * g.C;
+  p.k_corr = pl.K;
+  p.N = g.OC;
+  p.conv_entries = r.entries;
+  p.conv_cpb = r.pairs ? 1 : g.C / 128;
+  for (int e = 0; e < r.entries; e++) {
+    const int kh = e / (r.pairs ? r.pairs : g.KW), kw = r.pairs ? 2 * (e % r.pairs) : e % g.KW;
+    p.conv_row_off[e] = r.planes == 1 ? kh * r.w + kw : (int)(((kh & 1) * 2 + (kw & 1)) * r.rows) + (kh >> 1) * r.w + (kw >> 1);
+  }
+  p.conv_hpwp = r.h * r.w;
+  p.conv_wp = r.w;
+  p.conv_oh = g.OH;
+  p.conv_ow = g.OW;
+  if (filter_row_sums == nullptr) {  // zeros added by the pairing do not change the sums
+    int32_t *sums = reinterpret_cast<int32_t *>(sums_ws);
+    if (int rc = glowb200_i8_row_sums(b, g.OC, p.K, sums, reinterpret_cast<glowb200_stream_t>(s))) return rc;
+    filter_row_sums = sums;
+  }
+  return run_gemm_shifted_rows(p, xp, r.rows, g.C, b, filter_row_sums, s, r.planes * r.rows);
+}
+
 int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeom &g, const int32_t *filter_row_sums,
              int flags, void *workspace, size_t workspace_bytes, cudaStream_t s) {
   const int64_t outputs = (int64_t)g.N * g.OH * g.OW * g.OC;
@@ -367,89 +433,18 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
     return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", workspace_bytes, need);
   GLOWB200_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
   uint8_t *ws = reinterpret_cast<uint8_t *>(workspace);
-  // Stride-1 windows over 64 or a multiple of 128 channels, symmetric filters: no im2col matrix.
-  // The input is copied once into a padded NHWC buffer; tap (kh, kw) of output row q then is row
-  // q + kh * Wp + kw of that buffer, which the contraction's loads address directly (the rows of
-  // the product that fall on the padding are computed and dropped).  The scratch sized for the
-  // im2col matrix is more than this needs.
-  if (pl.need_im2col && g.SH == 1 && g.SW == 1 && g.DH == 1 && g.DW == 1 && (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) &&
-      (g.C == 64 || g.C % 128 == 0) && (reinterpret_cast<uintptr_t>(in) & 15) == 0 &&
-      (reinterpret_cast<uintptr_t>(filter) & 15) == 0) {
-    const int Hp = g.OH + g.KH - 1, Wp = g.OW + g.KW - 1;
-    // 64 channels: two neighbouring pixels per 128-byte row against a filter re-laid in tap pairs (the
-    // partner of an odd last tap zero).  One tap per 64-byte k-block in the 64-byte swizzle -- no
-    // wasted MMAs, a quarter fewer operand bytes, nine k-blocks instead of six for a 3 x 3 window --
-    // gave the same results and a slower network (1.590 against 1.562 ms per ResNet-50 batch).
-    const int pairs = (g.KW + 1) / 2;
-    const int entries = g.C == 64 ? g.KH * pairs : g.KH * g.KW;
-    const int64_t rows = (int64_t)g.N * Hp * Wp;
-    const size_t xp_bytes = align_up((size_t)rows * g.C + 256, 256);
-    const size_t fb_bytes = g.C == 64 ? align_up((size_t)g.OC * entries * 128, 256) : 0;
-    if (entries <= 32 && Hp >= g.H + g.PT && Wp >= g.W + g.PL && rows < (1ll << 31) &&
-        xp_bytes + fb_bytes <= pl.a_bytes + pl.f_bytes) {
-      int8_t *xp = reinterpret_cast<int8_t *>(ws);
-      const uint32_t b = (uint8_t)p.a_offset;
-      int8_t *fb = g.C == 64 ? reinterpret_cast<int8_t *>(ws + xp_bytes) : nullptr;
-      const int64_t chunks = rows * (g.C >> 4) + 16 + (fb ? (int64_t)g.OC * entries * 8 : 0), blocks = (chunks + 255) / 256;
-      GLOWB200_CUDA_OK(launch_pdl(pad_nhwc_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, xp, g, Hp, Wp,
-                                  (int)(b | (b << 8) | (b << 16) | (b << 24)), filter, fb));
-      const int8_t *bmat = fb ? fb : filter;
-      p.K = fb ? entries * 128 : g.KH * g.KW * g.C;
-      p.k_corr = pl.K;
-      p.N = g.OC;
-      p.conv_entries = entries;
-      p.conv_cpb = g.C == 64 ? 1 : g.C / 128;
-      for (int e = 0; e < entries; e++)
-        p.conv_row_off[e] = g.C == 64 ? (e / pairs) * Wp + 2 * (e % pairs) : (e / g.KW) * Wp + (e % g.KW);
-      p.conv_hpwp = Hp * Wp;
-      p.conv_wp = Wp;
-      p.conv_oh = g.OH;
-      p.conv_ow = g.OW;
-      const int32_t *sums = filter_row_sums;
-      if (sums == nullptr) {  // zeros added by the pairing do not change the sums
-        int32_t *bs = reinterpret_cast<int32_t *>(ws + pl.a_bytes + pl.f_bytes);
-        if (int rc = glowb200_i8_row_sums(bmat, g.OC, p.K, bs, reinterpret_cast<glowb200_stream_t>(s))) return rc;
-        sums = bs;
-      }
-      return run_gemm_shifted_rows(p, xp, rows, g.C, bmat, sums, s);
+  ShiftedRows sr;
+  if (aligned && shifted_rows(g, pl, flags, sr)) {
+    int8_t *xp = reinterpret_cast<int8_t *>(ws), *pairs = sr.pair_bytes ? reinterpret_cast<int8_t *>(ws + sr.input_bytes) : nullptr;
+    const int word = pad_word(p.a_offset);
+    if (sr.planes == 1) {
+      const int64_t chunks = sr.rows * (g.C >> 4) + 16 + (pairs ? (int64_t)g.OC * sr.entries * 8 : 0), blocks = (chunks + 255) / 256;
+      GLOWB200_CUDA_OK(launch_pdl(pad_nhwc_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, xp, g, sr.h, sr.w, word, filter, pairs));
+    } else {
+      const int64_t chunks = 4 * sr.rows * (g.C >> 4), blocks = (chunks + 255) / 256;
+      GLOWB200_CUDA_OK(launch_pdl(pad_parity_nhwc_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, xp, g, sr.h, sr.w, word));
     }
-  }
-  // Stride-2 windows over a multiple of 128 channels, symmetric filters: the shifted-rows form over
-  // four parity planes of the padded input (see pad_parity_nhwc_i8_kernel) instead of an im2col matrix.
-  if (pl.need_im2col && g.SH == 2 && g.SW == 2 && g.DH == 1 && g.DW == 1 && (g.KH > 1 || g.KW > 1) &&
-      (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) && g.C % 128 == 0 && g.KH * g.KW <= 32 &&
-      (reinterpret_cast<uintptr_t>(in) & 15) == 0 && (reinterpret_cast<uintptr_t>(filter) & 15) == 0) {
-    const int Hq = g.OH + (g.KH - 1) / 2, Wq = g.OW + (g.KW - 1) / 2;
-    const int64_t rows = (int64_t)g.N * Hq * Wq;  // per plane
-    const size_t xp_bytes = align_up((size_t)(4 * rows) * g.C + 256, 256);
-    if (4 * rows < (1ll << 31) && xp_bytes <= pl.a_bytes + pl.f_bytes) {
-      int8_t *xp = reinterpret_cast<int8_t *>(ws);
-      const uint32_t b = (uint8_t)p.a_offset;
-      const int64_t chunks = 4 * rows * (g.C >> 4), blocks = (chunks + 255) / 256;
-      GLOWB200_CUDA_OK(launch_pdl(pad_parity_nhwc_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, xp, g, Hq,
-                                  Wq, (int)(b | (b << 8) | (b << 16) | (b << 24))));
-      GLOWB200_CUDA_OK(cudaGetLastError());
-      p.K = g.KH * g.KW * g.C;
-      p.k_corr = pl.K;
-      p.N = g.OC;
-      p.conv_entries = g.KH * g.KW;
-      p.conv_cpb = g.C / 128;
-      for (int e = 0; e < p.conv_entries; e++) {
-        const int kh = e / g.KW, kw = e % g.KW;
-        p.conv_row_off[e] = (int)(((kh & 1) * 2 + (kw & 1)) * rows) + (kh >> 1) * Wq + (kw >> 1);
-      }
-      p.conv_hpwp = Hq * Wq;
-      p.conv_wp = Wq;
-      p.conv_oh = g.OH;
-      p.conv_ow = g.OW;
-      const int32_t *sums = filter_row_sums;
-      if (sums == nullptr) {
-        int32_t *bs = reinterpret_cast<int32_t *>(ws + pl.a_bytes + pl.f_bytes);
-        if (int rc = glowb200_i8_row_sums(filter, g.OC, p.K, bs, reinterpret_cast<glowb200_stream_t>(s))) return rc;
-        sums = bs;
-      }
-      return run_gemm_shifted_rows(p, xp, rows, g.C, filter, sums, s, 4 * rows);
-    }
+    return run_shifted_rows(p, g, pl, sr, xp, pairs ? pairs : filter, filter_row_sums, ws + pl.a_bytes + pl.f_bytes, s);
   }
   // Stride-2 windows over few channels with symmetric filters (the 7 x 7 stem over 3 channels): row
   // windows instead of an im2col matrix (see row_windows_i8_kernel).
@@ -583,6 +578,93 @@ extern "C" int glowb200_channelwise_quantized_conv2d_i8_i32(    int8_t *out, con
                                   out_offset, in_offset, filter_offsets, bias_offsets, bias_pre, bias_post, bias_scale, out_pre,
                                   out_post, out_scale, act_type, act_args, flags, status)) return rc;
   return run_conv(p, in, filter, g, filter_row_sums, flags, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+}
+
+namespace {
+int pair_geometry(ConvGeom &a, ConvGeom &b, const int64_t *in_dims, const int64_t *mid_dims, const int64_t *out_dims,
+                  const glowb200_conv_layer *first, const glowb200_conv_layer *second) {
+  GLOWB200_REQUIRE(first && second, "NULL layer");
+  if (int rc = geom_from_dims(a, mid_dims, in_dims, first->filter_dims, first->kernels, first->strides, first->pads, first->group,
+                              first->dilation)) return rc;
+  return geom_from_dims(b, out_dims, mid_dims, second->filter_dims, second->kernels, second->strides, second->pads, second->group,
+                        second->dilation);
+}
+// What a convolution may ask of the workspace, and the bytes of a pair's tensor in between.
+size_t conv_bytes(const ConvGeom &g) {
+  const ConvPlan pl = plan_conv(g, false);
+  return pl.a_bytes + pl.f_bytes + pl.core_bytes;
+}
+size_t mid_bytes(const ConvGeom &a) { return align_up((size_t)a.N * a.OH * a.OW * a.OC, 256); }
+}  // namespace
+
+extern "C" size_t glowb200_channelwise_quantized_conv2d_pair_workspace_bytes(
+    const int64_t *in_dims, const int64_t *mid_dims, const int64_t *out_dims, const glowb200_conv_layer *first,
+    const glowb200_conv_layer *second) {
+  ConvGeom a, b;
+  if (pair_geometry(a, b, in_dims, mid_dims, out_dims, first, second) != GLOWB200_OK) return 0;
+  const size_t x = conv_bytes(a), y = conv_bytes(b);
+  return mid_bytes(a) + (x > y ? x : y);
+}
+
+// A pointwise layer in front of a window over 64 or a multiple of 128 channels writes the padded buffer itself
+// (PaddedOut): as launches of their own the copies into it took 139 + 45 us of 1128 of a ResNet-50 batch of 64.
+extern "C" int glowb200_channelwise_quantized_conv2d_pair_i8_i32(
+    int8_t *out, const int8_t *in, const int64_t *in_dims, const int64_t *mid_dims, const int64_t *out_dims,
+    const glowb200_conv_layer *first, const glowb200_conv_layer *second, void *workspace, size_t workspace_bytes,
+    int32_t *status, glowb200_stream_t stream) {
+  ConvGeom a, b;
+  if (int rc = pair_geometry(a, b, in_dims, mid_dims, out_dims, first, second)) return rc;
+  if ((int64_t)b.N * b.OH * b.OW * b.OC == 0) return GLOWB200_OK;
+  GLOWB200_REQUIRE((int64_t)a.N * a.OH * a.OW * a.OC > 0, "a result of an empty tensor");
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const size_t mid = mid_bytes(a);
+  if (workspace == nullptr || workspace_bytes < mid)
+    return set_error(GLOWB200_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", workspace_bytes,
+                     glowb200_channelwise_quantized_conv2d_pair_workspace_bytes(in_dims, mid_dims, out_dims, first, second));
+  GLOWB200_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
+  uint8_t *ws = reinterpret_cast<uint8_t *>(workspace);
+  GemmParams p, q;
+  auto params = [&](GemmParams &p, ConvGeom &g, const glowb200_conv_layer *l, int8_t *to, const int8_t *from, const int64_t *from_dims,
+                    const int64_t *to_dims) {
+    return channelwise_params(p, g, to, from, l->filter, l->bias, to_dims, from_dims, l->filter_dims, l->kernels, l->strides, l->pads,
+                              l->group, l->dilation, l->out_offset, l->in_offset, l->filter_offsets, l->bias_offsets, l->bias_pre,
+                              l->bias_post, l->bias_scale, l->out_pre, l->out_post, l->out_scale, l->act_type, l->act_args, l->flags, status);
+  };
+  int8_t *between = reinterpret_cast<int8_t *>(ws);
+  if (int rc = params(p, a, first, between, in, in_dims, mid_dims)) return rc;
+  if (int rc = params(q, b, second, out, between, mid_dims, out_dims)) return rc;
+  const ConvPlan pa = plan_conv(a, (first->flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0);
+  const ConvPlan pb = plan_conv(b, (second->flags & GLOWB200_FC_FORCE_ANY_SHAPE_KERNEL) != 0);
+  ShiftedRows r;
+  if (!pa.direct && !pa.need_im2col && !pb.direct && (reinterpret_cast<uintptr_t>(second->filter) & 15) == 0 &&
+      i8_tiles_direct(pa.M, a.OC, pa.K, in, first->filter, between) && !i8_skinny_conv_wins(b) && shifted_rows(b, pb, second->flags, r)) {
+    const int sides = r.planes == 1 ? 1 : 2;  // (a parity plane is half as high and wide as the padded input)
+    const size_t need = r.input_bytes + r.pair_bytes + (pa.core_bytes > pb.core_bytes ? pa.core_bytes : pb.core_bytes);
+    if (sides * r.h >= b.H + b.PT && sides * r.w >= b.W + b.PL && workspace_bytes >= need) {
+      PaddedOut &o = p.padded;
+      o.kind = sides;
+      o.images = b.N; o.h = b.H; o.w = b.W;
+      o.hp = sides * r.h; o.wp = sides * r.w;
+      o.top = b.PT; o.left = b.PL;
+      o.plane = (int)r.rows;
+      o.word = (uint32_t)pad_word(q.a_offset);
+      if (r.pairs) {
+        o.filter = second->filter;
+        o.pairs = reinterpret_cast<int8_t *>(ws + r.input_bytes);
+        o.filter_rows = b.OC * b.KH;
+        o.kw = b.KW;
+      }
+      uint8_t *core = ws + r.input_bytes + r.pair_bytes;
+      p.M = (int)pa.M;
+      p.N = a.OC;
+      p.K = p.k_corr = pa.K;
+      if (int rc = run_gemm(p, in, first->filter, first->filter_row_sums, (first->flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) != 0, 0, core,
+                            pa.core_bytes, s)) return rc;
+      return run_shifted_rows(q, b, pb, r, between, o.pairs ? o.pairs : second->filter, second->filter_row_sums, core, s);
+    }
+  }
+  if (int rc = run_conv(p, in, first->filter, a, first->filter_row_sums, first->flags, ws + mid, workspace_bytes - mid, s)) return rc;
+  return run_conv(q, between, second->filter, b, second->filter_row_sums, second->flags, ws + mid, workspace_bytes - mid, s);
 }
 
 // The Add rides in the contraction's drain when the layer is a plain product with whole 16-byte rows and the

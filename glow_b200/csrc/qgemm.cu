@@ -331,6 +331,44 @@ __device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
   return q + (x - q * d >= d ? 1 : 0);
 }
 
+// The halo of a PaddedOut, and the next layer's filter in tap pairs: 16-byte pieces dealt to `threads` threads.
+__device__ void fill_padded(const PaddedOut &o, int8_t *out, int channels, int64_t thread, int64_t threads) {
+  const int pieces = channels >> 4, side = o.wp - o.w;
+  const int above = o.top * o.wp, below = (o.hp - o.top - o.h) * o.wp, cells = above + below + o.h * side;
+  const uint4 word = make_uint4(o.word, o.word, o.word, o.word);
+  for (int64_t i = thread; i < (int64_t)o.images * cells * pieces; i += threads) {
+    const int64_t cell = i / pieces;
+    const int image = (int)(cell / cells);
+    int c = (int)(cell - (int64_t)image * cells), y, x;
+    if (c < above) {
+      y = c / o.wp;
+      x = c - y * o.wp;
+    } else if (c < above + below) {
+      c -= above;
+      y = c / o.wp;
+      x = c - y * o.wp;
+      y += o.top + o.h;
+    } else {
+      c -= above + below;
+      y = c / side;
+      x = c - y * side;
+      y += o.top;
+      if (x >= o.left) x += o.w;
+    }
+    reinterpret_cast<uint4 *>(out + (size_t)o.pixel(image, y, x) * channels)[(int)(i - cell * pieces)] = word;
+  }
+  if (o.pairs == nullptr) return;
+  const int pairs = (o.kw + 1) >> 1;
+  for (int64_t i = thread; i < (int64_t)o.filter_rows * pairs * 8; i += threads) {
+    const int piece = (int)(i & 7);
+    const int64_t r = (i >> 3) / pairs;  // oc * KH + kh
+    const int kw = 2 * (int)((i >> 3) - r * pairs) + (piece >> 2);
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (kw < o.kw) v = __ldg(reinterpret_cast<const uint4 *>(o.filter + (r * o.kw + kw) * 64) + (piece & 3));
+    reinterpret_cast<uint4 *>(o.pairs)[i] = v;
+  }
+}
+
 // Optional tracing for tuning builds (python -m glow_b200.build -DGLOWB200_GEMM_TRACE): every CTA
 // stamps %globaltimer (ns) at entry and exit -- entries 2b and 2b + 1 of a device buffer -- and
 // CTA 0 its clock64 at the same two points (entries 510, 511), from which the SM clock a launch really
@@ -410,6 +448,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   // barrier on the way.  Tiles of 64 columns alternate between two halves of the warps (32 columns each: whole
   // 32-byte sectors), the others are split between all of them.
   constexpr bool kOwnRows = MODE == 0 || MODE == 1 || MODE == 4;
+  constexpr bool kPads = MODE == 0 || MODE == 1;   // the result may go into the padded input of a convolution
   constexpr bool kFolds = MODE == 0 || MODE == 4;  // columns may be of the kind offset_folds admits
   constexpr bool kAlternate = kOwnRows && BLOCK_N <= 64;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::kTileBytes + S::kColBytes + S::kOutBytes);
@@ -558,6 +597,12 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const uint32_t line_div = p.conv_wp > 0 ? 0xffffffffu / (uint32_t)p.conv_wp : 0u;
     int lt = 0;
     bool dead = false;
+    if constexpr (kPads) {
+      if (p.padded.kind)
+        fill_padded(p.padded, p.out, p.N, (int64_t)blockIdx.x * kEpilogueThreads + et, (int64_t)gridDim.x * kEpilogueThreads);
+    }
+    [[maybe_unused]] const uint32_t out_image_div = kPads && p.padded.kind ? 0xffffffffu / (uint32_t)(p.padded.h * p.padded.w) : 0u;
+    [[maybe_unused]] const uint32_t out_line_div = kPads && p.padded.kind ? 0xffffffffu / (uint32_t)p.padded.w : 0u;
     // The column records in shared memory are {c, scale} and, behind them, pre, of columns that share `tile_post` and
     // whose result offset rides on the rounding term; else ColParams and the rounding term.
     [[maybe_unused]] bool folded = false;
@@ -655,6 +700,13 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const int oh = fast_div(rem, p.conv_wp, line_div), ow = rem - oh * p.conv_wp;
         row_ok = row_ok && oh < p.conv_oh && ow < p.conv_ow;
         out_index = (img * p.conv_oh + oh) * p.conv_ow + ow;
+      }
+      if constexpr (kPads) {
+        if (p.padded.kind) {
+          const int img = fast_div(row, p.padded.h * p.padded.w, out_image_div), rem = row - img * (p.padded.h * p.padded.w);
+          const int y = fast_div(rem, p.padded.w, out_line_div);
+          out_index = p.padded.pixel(img, y + p.padded.top, rem - y * p.padded.w + p.padded.left);
+        }
       }
       const int c_end = (col_group + 1) * kGroupCols < BLOCK_N ? (col_group + 1) * kGroupCols : BLOCK_N;
       if constexpr (MODE == 2) {

@@ -5,6 +5,26 @@
 
 namespace glowb200 {
 
+// Where a layer's result goes when it is the input of a convolution that wants its padding made real (conv.cu): straight
+// into that padded buffer, whose halo the epilogue warps fill beside it.  kind 1: [images, hp, wp, N], pixel (y, x) of an
+// image at (y + top, x + left); kind 2: the same split by the parity of the padded coordinates into four planes
+// [images, hp / 2, wp / 2, N].  Rows of the product are the images' h * w pixels.
+struct PaddedOut {
+  int kind;  // 0: no, the result is a matrix
+  int images, h, w, hp, wp, top, left, plane;  // plane: pixels of one of the four
+  uint32_t word;                               // of the halo
+  // the next layer's filter [filter_rows, kw, 64] -> pairs [filter_rows, ceil(kw / 2), 128] (64 channels; else nullptr)
+  const int8_t *filter;
+  int8_t *pairs;
+  int filter_rows, kw;
+#ifdef __CUDACC__
+  __device__ __forceinline__ int pixel(int image, int y, int x) const {  // padded coordinates
+    if (kind == 1) return (image * hp + y) * wp + x;
+    return ((y & 1) * 2 + (x & 1)) * plane + (image * (hp >> 1) + (y >> 1)) * (wp >> 1) + (x >> 1);
+  }
+#endif
+};
+
 struct GemmParams {
   int8_t *out;                // [M, N]
   const int32_t *bias;        // [N] or nullptr (MatMul); int8 values when bias_is_i8 (the _i8_i8 kernels)
@@ -18,6 +38,7 @@ struct GemmParams {
   // residual[M, N]), rows of whole 16-byte pieces, no weight offsets, activation none or Relu.
   const int8_t *residual;
   AddQuant add;
+  PaddedOut padded;  // (the TMA path, rows of whole 16-byte pieces)
   int32_t *status;
   const int32_t *bias_offsets;  // per-column bias offsets (channelwise conv), or nullptr: bias_offset
   int M, N, K;                  // K: row pitch of both operands in bytes (a multiple of 16 on the TMA path)
@@ -113,6 +134,11 @@ bool i8_skinny_conv_wins(const ConvGeom &g);
 int run_conv_skinny(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeom &g, bool b_offsets_zero, cudaStream_t s);
 constexpr int kSkinnyRows = 64;
 bool i8_skinny_wins(int64_t M, int64_t N, int64_t K, bool b_is_kn);
+// Whether run_gemm takes a [M, K] x [N, K] product with the tile kernel, its operands as they are: what can write a PaddedOut.
+inline bool i8_tiles_direct(int64_t M, int64_t N, int64_t K, const void *a, const void *b, const void *out) {
+  auto whole = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  return K > 0 && K % 16 == 0 && N % 16 == 0 && whole(a) && whole(b) && whole(out) && !i8_skinny_wins(M, N, K, false);
+}
 int run_gemm_skinny(GemmParams p, const int8_t *a, const int8_t *b, bool b_is_kn, bool b_offsets_zero, cudaStream_t s);
 
 // One operand to prepare: src [rows, K] -> dst [rows, pitch] (pitch a multiple of 16, the rest zero;

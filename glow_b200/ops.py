@@ -479,6 +479,13 @@ def channelwise_quantized_conv2d_add(inp, filt, bias, kernels, strides, pads, gr
                                           residual_offset, lhs_triple, residual_triple, splat)
 
 
+def channelwise_quantized_conv2d_pair(inp, first, second, *, out=None, workspace=None, status=None):
+    """channelwise_quantized_conv2d(inp, ...), then another over its result, which nothing else reads.  `first` and
+    `second`: (filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset, filter_offsets, bias_offsets,
+    bias_triples, out_triples, act_type, act_args, filter_row_sums, flags), as of the single call."""
+    return _native().channelwise_conv_pair(inp, first, second, out, workspace, status)
+
+
 def conv2d_i8(inp, filt, bias, kernels, strides, pads, group, dilation, out_offset, in_offset, filter_offset,
               bias_offset, bias_triple, out_triple, act_type=0, act_args=None, *, flags=0, out=None, workspace=None,
               status=None):

@@ -235,22 +235,37 @@ class ResNet50Int8:
             self._captured.append(self.ws)   # a graph addresses it from now on: kept when a larger one takes its place
         return self.ws
 
-    def _conv(self, name, x, residual=None, add=()):
-        """The convolution; with `residual`, the end of a block: Add and Relu behind it."""
+    def _layer(self, name):
         d = self.conv[name]
         c, spec = d["c"], d["c"]["spec"]
-        k, s, p = (spec["k"],) * 2, (spec["stride"],) * 2, (spec["pad"],) * 4
-        n, h, w_, cin = x.shape
-        oh, ow = ops.conv_out_hw((h, w_), k, s, p)
-        need = n * oh * ow * ((spec["k"] ** 2 * cin + 15) // 16 * 16) + spec["cout"] * ((spec["k"] ** 2 * cin + 15) // 16 * 16) + \
-            ops.i8_gemm_workspace_bytes(n * oh * ow, 16, spec["cout"]) + 4096
+        return (d["filter"], d["bias"], (spec["k"],) * 2, (spec["stride"],) * 2, (spec["pad"],) * 4, 1, (1, 1), c["out_offset"],
+                c["in_offset"], d["fo"], d["bo"], d["params"][:3], d["params"][3:], 1 if spec["relu"] else 0, None)
+
+    def _result(self, name, shape):
+        """(shape of the layer's result over an NHWC input of `shape`, bytes of scratch it may ask for)"""
+        spec = self.conv[name]["c"]["spec"]
+        n, h, w_, cin = shape
+        oh, ow = ops.conv_out_hw((h, w_), (spec["k"],) * 2, (spec["stride"],) * 2, (spec["pad"],) * 4)
+        row = (spec["k"] ** 2 * cin + 15) // 16 * 16
+        return (n, oh, ow, spec["cout"]), (n * oh * ow + spec["cout"]) * row + ops.i8_gemm_workspace_bytes(n * oh * ow, 16, spec["cout"]) + 4096
+
+    def _conv(self, name, x, residual=None, add=()):
+        """The convolution; with `residual`, the end of a block: Add and Relu behind it."""
+        need = self._result(name, x.shape)[1]
         self.launches += 2
-        args = (x, d["filter"], d["bias"], k, s, p, 1, (1, 1), c["out_offset"], c["in_offset"], d["fo"], d["bo"],
-                d["params"][:3], d["params"][3:], 1 if spec["relu"] else 0, None)
-        kw = dict(filter_row_sums=d["row_sums"], flags=ops.FC_WEIGHT_OFFSETS_ZERO, workspace=self._workspace(need), status=self.status)
+        kw = dict(filter_row_sums=self.conv[name]["row_sums"], flags=ops.FC_WEIGHT_OFFSETS_ZERO, workspace=self._workspace(need),
+                  status=self.status)
         if residual is None:
-            return ops.channelwise_quantized_conv2d(*args, **kw)
-        return ops.channelwise_quantized_conv2d_add(*args, residual, *add, **kw)
+            return ops.channelwise_quantized_conv2d(x, *self._layer(name), **kw)
+        return ops.channelwise_quantized_conv2d_add(x, *self._layer(name), residual, *add, **kw)
+
+    def _conv_pair(self, first, second, x):
+        """Two convolutions of which only the second reads the first's result."""
+        mid, need = self._result(first, x.shape)
+        need = max(need, self._result(second, mid)[1]) + math.prod(mid) + 256
+        self.launches += 4   # (at most; two where the first writes the padded buffer of the second)
+        layers = [self._layer(name) + (self.conv[name]["row_sums"], ops.FC_WEIGHT_OFFSETS_ZERO) for name in (first, second)]
+        return ops.channelwise_quantized_conv2d_pair(x, *layers, workspace=self._workspace(need), status=self.status)
 
     # Images up to which the layers between Quantize and the FC are replayed from a CUDA graph (see Replays for
     # when): their 56 launches cost the host 4 us each, which is more than the device needs for them below
@@ -320,9 +335,7 @@ class ResNet50Int8:
                 x = ops.max_pool_i8(x, (3, 3), (2, 2), (1, 1, 1, 1), tqp["conv1"][1])
                 self.launches += 1
             elif l[0] == "block":
-                y = x
-                for c in l[2][:-1]:
-                    y = self._conv(c["name"], y)
+                y = self._conv_pair(l[2][0]["name"], l[2][1]["name"], x)
                 sc = self._conv(l[3]["name"], x) if l[3] else x
                 a = self.q["add"][l[1]]
                 out_off = tqp[a["out"]][1]

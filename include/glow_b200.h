@@ -510,6 +510,28 @@ int glowb200_channelwise_quantized_conv2d_add_i8(
     int32_t residual_pre, int32_t residual_post, int32_t residual_scale, int32_t splat,
     glowb200_stream_t stream);
 
+/* Two such convolutions, the second over the result of the first, which nothing else reads: bit-identical to the two
+ * calls.  The first's result lives in the workspace -- where the layers allow it, already in the padded layout that the
+ * second reads, so that no copy is made in between.  in_dims, mid_dims and out_dims are HOST arrays {N,H,W,C}; the
+ * layers' members are the arguments of the single call (arrays of shapes and activation arguments on the HOST). */
+typedef struct glowb200_conv_layer {
+  const int8_t *filter;
+  const int32_t *bias, *filter_offsets, *bias_offsets, *bias_pre, *bias_post, *bias_scale, *out_pre, *out_post, *out_scale;
+  const int32_t *filter_row_sums; /* may be NULL */
+  const int64_t *filter_dims, *kernels, *strides, *pads, *dilation;
+  int64_t group;
+  int32_t in_offset, out_offset, act_type;
+  const int32_t *act_args;
+  int flags;
+} glowb200_conv_layer;
+size_t glowb200_channelwise_quantized_conv2d_pair_workspace_bytes(
+    const int64_t *in_dims, const int64_t *mid_dims, const int64_t *out_dims, const glowb200_conv_layer *first,
+    const glowb200_conv_layer *second);
+int glowb200_channelwise_quantized_conv2d_pair_i8_i32(
+    int8_t *out, const int8_t *in, const int64_t *in_dims, const int64_t *mid_dims, const int64_t *out_dims,
+    const glowb200_conv_layer *first, const glowb200_conv_layer *second, void *workspace, size_t workspace_bytes,
+    int32_t *status, glowb200_stream_t stream);
+
 /* Convolution (2-D), int8 with int32 bias, one quantisation per tensor.
  * Replaces libjit_conv2d_i8_i32 (libjit_conv.cpp:496-510, body :49-147; scalars derived at
  * LLVMIRGen.cpp:2501-2599).  The reference's depthUnroll argument only blocks its loops and
