@@ -95,6 +95,25 @@ __device__ __forceinline__ uint32_t add_quant_word(uint32_t l, uint32_t r, const
 }
 #endif
 
+#ifdef __CUDACC__
+// x / d for 0 <= x < 2^31 with reciprocal = floor((2^32 - 1) / d): the estimate is the quotient or one less.
+__device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
+  const int q = (int)__umulhi((uint32_t)x, reciprocal);
+  return q + (x - q * d >= d ? 1 : 0);
+}
+// Walks x down a mixed radix: returns x % d and leaves x / d.
+struct Divisor {
+  int d;
+  uint32_t reciprocal;
+  __host__ __device__ explicit Divisor(int d) : d(d), reciprocal(d > 0 ? 0xffffffffu / (uint32_t)d : 0u) {}
+  __device__ __forceinline__ int rest(int &x) const {
+    const int q = fast_div(x, d, reciprocal), r = x - q * d;
+    x = q;
+    return r;
+  }
+};
+#endif
+
 // libjit_clip_i8 (libjit_defs.h:146-148).
 __host__ __device__ __forceinline__ int32_t clip_i8(int32_t v) {
   return v < -128 ? -128 : (v > 127 ? 127 : v);

@@ -24,31 +24,32 @@ unsigned grid_of(int64_t blocks, int per_sm) {
 }
 
 // one thread per 16-byte chunk of the im2col matrix (C a multiple of 16: a chunk never
-// straddles two taps)
+// straddles two taps).  64-bit divisions bound it first: every second pixel of 64 x 56 x 56 x 256 13 us, now 10.
+struct Im2colRadix {
+  Divisor row, pixel, width, height, taps;
+  Im2colRadix(const ConvGeom &g, int Kpad) : row(Kpad >> 4), pixel(g.C >> 4), width(g.OW), height(g.OH), taps(g.KW) {}
+};
 __global__ void __launch_bounds__(256) im2col_i8_vec_kernel(const int8_t *__restrict__ x, int8_t *__restrict__ a,
-                                                             const __grid_constant__ ConvGeom g, int Kpad, int pad_word) {
+                                                             const __grid_constant__ ConvGeom g, const __grid_constant__ Im2colRadix radix,
+                                                             int Kpad, int pad_word) {
   pdl_wait();
   pdl_launch_dependents();
-  const int chunks_per_row = Kpad >> 4;
-  const int64_t total = (int64_t)g.N * g.OH * g.OW * chunks_per_row;
-  const int c_chunks = g.C >> 4;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / chunks_per_row;
-    const int ch = (int)(i - row * chunks_per_row);
-    const int tap = ch / c_chunks, cc = ch - tap * c_chunks;
+  const int total = g.N * g.OH * g.OW * (Kpad >> 4), step = gridDim.x * blockDim.x;  // (below 2^31: the launcher's condition)
+  for (int64_t at = blockIdx.x * blockDim.x + threadIdx.x; at < total; at += step) {
+    const int i = (int)at;
+    int n = i, tap = radix.row.rest(n);
+    const int ow = radix.width.rest(n), oh = radix.height.rest(n), cc = radix.pixel.rest(tap);
     int4 v = make_int4(0, 0, 0, 0);
     if (tap < g.KH * g.KW) {
-      const int kh = tap / g.KW, kw = tap - kh * g.KW;
-      const int ow = (int)(row % g.OW);
-      const int64_t r2 = row / g.OW;
-      const int oh = (int)(r2 % g.OH), n = (int)(r2 / g.OH);
+      int kh = tap;
+      const int kw = radix.taps.rest(kh);
       const int ih = oh * g.SH - g.PT + kh * g.DH, iw = ow * g.SW - g.PL + kw * g.DW;
       if (ih >= 0 && iw >= 0 && ih < g.H && iw < g.W)
-        v = *reinterpret_cast<const int4 *>(x + (((int64_t)n * g.H + ih) * g.W + iw) * g.C + cc * 16);
+        v = __ldg(reinterpret_cast<const int4 *>(x + (((int64_t)n * g.H + ih) * g.W + iw) * g.C) + cc);
       else
         v = make_int4(pad_word, pad_word, pad_word, pad_word);
     }
-    *reinterpret_cast<int4 *>(a + row * Kpad + ch * 16) = v;
+    reinterpret_cast<int4 *>(a)[i] = v;
   }
 }
 
@@ -155,35 +156,66 @@ __global__ void __launch_bounds__(256) im2col_i8_rows_kernel(const int8_t *__res
 // of output pixel (n, oh, ow) is byte kw * C + c of window (n, oh + a, ow) of plane e, so the
 // convolution is a contraction whose left-hand rows are four windows of one plane, Y = OH + 3 rows
 // per image: 2 * 32 bytes per (y, ow) instead of KH * KW * C per output pixel, and no im2col matrix.
-// One thread per window; behind them `tail` zero windows (the four windows of the last rows reach that far)
-// and the filter re-laid to match: [OC, KH, KW, C] -> [OC, 2 planes, 4 rows a, 32 bytes], tap
-// (kh = 2a + e, kw, c) at byte kw * C + c of (e, a), everything else zero.
+// One thread per window, cut from the words of the image row that it lies across; behind them `tail` zero windows (the
+// four windows of the last rows reach that far) and the filter re-laid to match: [OC, KH, KW, C] -> [OC, 2 planes, 4 rows a,
+// 32 bytes], tap (kh = 2a + e, kw, c) at byte kw * C + c of (e, a), everything else zero.
+// What bounds it is the 53 MB that a batch of 64 images of 224 x 224 writes, and instructions beside it: 31 us with a
+// window's 21 bytes loaded one by one and 64-bit divisions, 23 by way of shared memory, now 19.
+struct WindowRadix {
+  Divisor width, height, images;
+  WindowRadix(const ConvGeom &g, int Y) : width(g.OW), height(Y), images(g.N) {}
+};
 __global__ void __launch_bounds__(256) row_windows_i8_kernel(const int8_t *__restrict__ x, int8_t *__restrict__ planes,
-                                                              const __grid_constant__ ConvGeom g, int Y, int64_t plane_bytes,
-                                                              int8_t pad, int tail, const int8_t *__restrict__ f,
+                                                              const __grid_constant__ ConvGeom g, const __grid_constant__ WindowRadix radix,
+                                                              int64_t plane_bytes, int8_t pad, int tail, const int8_t *__restrict__ f,
                                                               int8_t *__restrict__ fb) {
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t per_plane = (int64_t)g.N * Y * g.OW, windows = 2 * per_plane, total = windows + tail + (int64_t)g.OC * 8;
-  const int run = g.KW * g.C;
+  const int run = g.KW * g.C, row_bytes = g.W * g.C;
+  const int per_plane = g.N * radix.height.d * g.OW;
+  const int64_t windows = 2 * (int64_t)per_plane, total = windows + tail + (int64_t)g.OC * 8;
+  const uint32_t pad4 = 0x01010101u * (uint32_t)(uint8_t)pad;
+  const bool whole_words = ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)row_bytes) & 3) == 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
     int4 *dst;
     if (i < windows) {
-      const int e = (int)(i / per_plane);
-      int64_t r = i - e * per_plane;
-      const int ow = (int)(r % g.OW);
-      r /= g.OW;
-      const int y = (int)(r % Y), n = (int)(r / Y);
-      const int ih = 2 * y - g.PT + e, b0 = (2 * ow - g.PL) * g.C;  // first byte of the window in its image row
-      const bool row_in = ih >= 0 && ih < g.H;
-      const int8_t *src = x + ((int64_t)n * g.H + (row_in ? ih : 0)) * g.W * g.C;
-      for (int b = 0; b < run; b++) {
-        const int o = b0 + b;
-        const int8_t v = (row_in && o >= 0 && o < g.W * g.C) ? src[o] : pad;
-        w[b >> 2] |= (uint32_t)(uint8_t)v << (8 * (b & 3));
+      const int e = i >= per_plane ? 1 : 0, at = (int)(i - (e ? per_plane : 0));
+      int n = at;
+      const int ow = radix.width.rest(n), y = radix.height.rest(n);
+      const int ih = 2 * y - g.PT + e, first = (2 * ow - g.PL) * g.C, from = first & ~3;  // bytes of the image row
+      if (ih >= 0 && ih < g.H) {
+        const int8_t *src = x + ((int64_t)n * g.H + ih) * row_bytes;
+        uint32_t word[9];
+        if (whole_words) {  // (a word then lies inside the row or outside, none across its ends)
+#pragma unroll
+          for (int k = 0; k < 9; k++) {
+            word[k] = pad4;
+            if (4 * k < run + 3 && (unsigned)(from + 4 * k) < (unsigned)row_bytes) word[k] = __ldg(reinterpret_cast<const uint32_t *>(src + from) + k);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 9; k++) {
+            word[k] = pad4;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+              const int o = from + 4 * k + b;
+              if (o - first < run && o >= 0 && o < row_bytes) word[k] = (word[k] & ~(0xffu << (8 * b))) | (uint32_t)(uint8_t)src[o] << (8 * b);
+            }
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) w[k] = __funnelshift_r(word[k], word[k + 1], 8 * (first & 3));
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) w[k] = pad4;
       }
-      dst = reinterpret_cast<int4 *>(planes + e * plane_bytes + (i - e * per_plane) * 32);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int valid = run - 4 * k;  // bytes of the word that are taps
+        w[k] = valid <= 0 ? 0u : valid >= 4 ? w[k] : w[k] & ((1u << (8 * valid)) - 1u);
+      }
+      dst = reinterpret_cast<int4 *>(planes + e * plane_bytes + (int64_t)at * 32);
     } else if (i < windows + tail) {
       dst = reinterpret_cast<int4 *>(planes + 2 * plane_bytes + (i - windows) * 32);
     } else {
@@ -191,12 +223,15 @@ __global__ void __launch_bounds__(256) row_windows_i8_kernel(const int8_t *__res
       const int oc = (int)(r >> 3), e = (int)(r >> 2) & 1, kh = 2 * ((int)r & 3) + e;
       if (kh < g.KH) {
         const int8_t *src = f + ((int64_t)oc * g.KH + kh) * run;
-        for (int b = 0; b < run; b++) w[b >> 2] |= (uint32_t)(uint8_t)src[b] << (8 * (b & 3));
+#pragma unroll
+        for (int b = 0; b < 32; b++)
+          if (b < run) w[b >> 2] |= (uint32_t)(uint8_t)src[b] << (8 * (b & 3));
       }
       dst = reinterpret_cast<int4 *>(fb + r * 32);
     }
-    dst[0] = make_int4((int)w[0], (int)w[1], (int)w[2], (int)w[3]);
-    dst[1] = make_int4((int)w[4], (int)w[5], (int)w[6], (int)w[7]);
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
   }
 }
 
@@ -460,7 +495,7 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       int8_t *fb = reinterpret_cast<int8_t *>(ws + wp_bytes);
       const int tail = (int)((wp_bytes - 2 * plane_bytes) / 32);  // the four windows of the last rows reach past the second plane
       const int64_t items = 2 * rows + tail + (int64_t)g.OC * 8, blocks = (items + 255) / 256;
-      GLOWB200_CUDA_OK(launch_pdl(row_windows_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, planes, g, Y,
+      GLOWB200_CUDA_OK(launch_pdl(row_windows_i8_kernel, grid_of(blocks, 64), 256, 0, s, in, planes, g, WindowRadix(g, Y),
                                   plane_bytes, (int8_t)p.a_offset, tail, filter, fb));
       const int32_t *bs = filter_row_sums;  // (the zeros of the new layout do not change them)
       if (bs == nullptr) {
@@ -482,11 +517,11 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
   if (pl.need_im2col) {
     int8_t *abuf = reinterpret_cast<int8_t *>(ws);
     const int8_t pad = (int8_t)p.a_offset;
-    if ((g.C % 16) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+    if ((g.C % 16) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && pl.M * (pl.Kpad >> 4) < (1ll << 31)) {
       const int64_t chunks = pl.M * (pl.Kpad >> 4);
       const int64_t blocks = (chunks + 255) / 256;
       const uint32_t b = (uint8_t)pad;
-      GLOWB200_CUDA_OK(launch_pdl(im2col_i8_vec_kernel, grid_of(blocks, 64), 256, 0, s, in, abuf, g, pl.Kpad,
+      GLOWB200_CUDA_OK(launch_pdl(im2col_i8_vec_kernel, grid_of(blocks, 64), 256, 0, s, in, abuf, g, Im2colRadix(g, pl.Kpad), pl.Kpad,
                                   (int)(b | (b << 8) | (b << 16) | (b << 24))));
     } else if ((int64_t)g.KH * rows_pitch(g) <= 48 * 1024 && (int64_t)g.N * g.OH < (1ll << 31) && (pl.Kpad >> 4) <= 256 &&
                (reinterpret_cast<uintptr_t>(abuf) & 15) == 0) {

@@ -325,12 +325,6 @@ __device__ __forceinline__ bool barrier_and(bool mine) {
   return ok != 0;
 }
 
-// x / d for 0 <= x < 2^31 with reciprocal = floor((2^32 - 1) / d): the estimate is the quotient or one less.
-__device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
-  const int q = (int)__umulhi((uint32_t)x, reciprocal);
-  return q + (x - q * d >= d ? 1 : 0);
-}
-
 // The halo of a PaddedOut, and the next layer's filter in tap pairs: 16-byte pieces dealt to `threads` threads.
 __device__ void fill_padded(const PaddedOut &o, int8_t *out, int channels, int64_t thread, int64_t threads) {
   const int pieces = channels >> 4, side = o.wp - o.w;

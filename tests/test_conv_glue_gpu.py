@@ -205,3 +205,52 @@ def test_binary_muldiv_batched_add_bit_exact(oracle):
         st = ops.quantize_scale_offset_32to8(0.004 if sl.dtype == np.int32 else 1.3)
         np.testing.assert_array_equal(ops.batched_add_i8(t(batch), t(sl), -6, 4, 1, lt, st).cpu().numpy(),
                                       oracle.batched_add_i8(batch, sl, -6, 4, 1, lt, st))
+
+
+@pytest.mark.parametrize("channels", [1, 2, 3, 4])
+@pytest.mark.parametrize("scale,offset", [(0.05, 3), (0.0371, -128), (3e-39, 0), (1e3, 500)])
+def test_quantize_planes_next_to_ties(channels, scale, offset):
+    """Four pixels at a time by the reciprocal: every element the one that the division gives."""
+    rng = np.random.default_rng(channels)
+    f = (rng.standard_normal((2, channels, 6, 20)) * 40 * scale).astype(np.float32)
+    k = np.arange(-140, 140, dtype=np.float32)
+    ties = ((k + np.float32(.5)) * np.float32(scale)).astype(np.float32)
+    near = np.concatenate([ties, np.nextafter(ties, np.float32(-np.inf)), np.nextafter(ties, np.float32(np.inf)),
+                           np.float32([0, 1e30, -1e30, np.inf, -np.inf, 2000 * scale, -2000 * scale])]).astype(np.float32)
+    flat = f.reshape(-1)
+    flat[:] = np.resize(np.concatenate([near, flat]), flat.size) if flat.size < 2 * near.size else \
+        np.concatenate([near, flat[near.size:]])
+    two = ops.transpose(ops.element_quantize_i8(t(f), scale, offset), (0, 2, 3, 1))
+    assert torch.equal(ops.quantize_transpose_i8(t(f), (0, 2, 3, 1), scale, offset), two)
+
+
+@pytest.mark.parametrize("n,h,w,c,oc,k,p", [
+    (2, 20, 24, 3, 16, (7, 7), (3, 3, 3, 3)),     # image rows of whole words
+    (2, 21, 23, 3, 16, (7, 7), (3, 3, 3, 3)),     # rows that start anywhere
+    (1, 33, 150, 4, 16, (8, 8), (5, 6, 5, 6)),    # 32 bytes of taps, and windows beyond the row on both sides
+    (3, 9, 10, 1, 16, (3, 3), (1, 1, 1, 1)),
+    (1, 15, 14, 30, 16, (5, 1), (2, 0, 2, 0)),
+])
+def test_stem_windows(oracle, n, h, w, c, oc, k, p):
+    """(images enough that the few-row kernel leaves the layer to the row windows)"""
+    case = (n * 40, h, w, c, oc, k, (2, 2), p, 1, (1, 1), 1)
+    x = _conv_inputs(oracle, case, True)
+    pp = [t(a) for a in x["pp"]]
+    args = (t(x["inp"]), t(x["filt"]), t(x["bias"]), k, (2, 2), p, 1, (1, 1), 3, -7, t(x["fo"]), t(x["bo"]), pp[:3], pp[3:], 1, None)
+    want = ops.channelwise_quantized_conv2d(*args, flags=ops.FC_FORCE_ANY_SHAPE_KERNEL)
+    assert torch.equal(ops.channelwise_quantized_conv2d(*args, flags=ops.FC_WEIGHT_OFFSETS_ZERO), want)
+
+
+@pytest.mark.parametrize("c", [16, 48, 20])
+@pytest.mark.parametrize("k,s,p", [((3, 3), (2, 2), (1, 1, 1, 1)), ((3, 3), (1, 1), (4, 4, 4, 4)), ((2, 4), (3, 1), (1, 0, 1, 3)),
+                                   ((7, 7), (1, 1), (0, 0, 0, 0)), ((5, 6), (2, 3), (0, 0, 0, 0)), ((9, 9), (9, 9), (0, 0, 0, 0))])
+def test_pools_in_words(oracle, c, k, s, p):
+    """Windows that leave the image (wholly, for some), and windows inside it, whose rows eight lanes share."""
+    rng = np.random.default_rng(c + k[0])
+    x = rng.integers(-128, 128, (3, 13, 11, c)).astype(np.int8)
+    ohw = ops.conv_out_hw((13, 11), k, s, p)
+    np.testing.assert_array_equal(ops.max_pool_i8(t(x), k, s, p, -7).cpu().numpy(), oracle.max_pool_i8(x, ohw, k, s, p, -7))
+    for cip in (True, False):
+        tr = ops.quantize_scale_offset_32to8(np.float32(0.6) / np.float32(k[0] * k[1] if cip else 1))
+        np.testing.assert_array_equal(ops.avg_pool_i8(t(x), k, s, p, cip, 3, -4, tr).cpu().numpy(),
+                                      oracle.avg_pool_i8(x, ohw, k, s, p, cip, 3, -4, tr))
