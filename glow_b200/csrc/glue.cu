@@ -216,6 +216,10 @@ __global__ void __launch_bounds__(kThreads) dequantize_i8_kernel(float *__restri
 }
 
 struct PoolGeom { int N, H, W, C, OH, OW, KH, KW, SH, SW, PT, PL; };
+struct PoolRadix {
+  Divisor words, width, height;
+  PoolRadix(const PoolGeom &g, int words) : words(words), width(g.OW), height(g.OH) {}
+};  // of an output's index: pieces of a pixel, pixels of a row, rows
 
 // libjit_max_pool_generic<int8_t> (libjit.cpp:811-870): cells outside the image are skipped,
 // an empty window yields the default value (the output offset).
@@ -240,40 +244,59 @@ __global__ void __launch_bounds__(kThreads) max_pool_i8_kernel(const int8_t *__r
   }
 }
 
-// The same for 16 channels per thread (C a multiple of 16, 16-byte aligned tensors): four
-// byte-wise signed maxima per instruction.
+// The same for 16 channels per thread (C a multiple of 16, 16-byte aligned tensors).  A word's four bytes are the upper
+// halves of two pairs of 16-bit numbers -- itself, and itself moved up by a byte -- whose lower halves decide nothing
+// between different bytes; one instruction takes the maximum of a pair.  A window that reaches out of the image reads its
+// last row or column inside again.  K: the window's sides, 0 any.  64 x 112 x 112 x 64 to 56 x 56: 21 us with a branch
+// per tap, 64-bit divisions and byte-wise maxima, now 13.
+template <int K>
 __global__ void __launch_bounds__(kThreads) max_pool_i8_vec_kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out,
-                                                                   const __grid_constant__ PoolGeom g, int8_t def) {
+                                                                   const __grid_constant__ PoolGeom g,
+                                                                   const __grid_constant__ PoolRadix radix, int8_t def) {
   pdl_wait();
   pdl_launch_dependents();
   const int cc = g.C >> 4;
-  const int64_t total = (int64_t)g.N * g.OH * g.OW * cc;
-  const uint32_t lowest = 0x80808080u;  // four times -128
+  const int64_t total = (int64_t)g.N * g.OH * g.OW * cc;  // (below 2^31: the launcher's condition)
+  const int KH = K ? K : g.KH, KW = K ? K : g.KW;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % cc);
-    int64_t r = i / cc;
-    const int ow = (int)(r % g.OW);
-    r /= g.OW;
-    const int oh = (int)(r % g.OH), n = (int)(r / g.OH);
-    uint4 best = make_uint4(lowest, lowest, lowest, lowest);
-    bool any = false;
-    for (int kh = 0; kh < g.KH; kh++)
-      for (int kw = 0; kw < g.KW; kw++) {
-        const int ih = oh * g.SH - g.PT + kh, iw = ow * g.SW - g.PL + kw;
-        if (ih < 0 || iw < 0 || ih >= g.H || iw >= g.W) continue;
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(in + (((int64_t)n * g.H + ih) * g.W + iw) * g.C) + c);
-        best.x = __vmaxs4(best.x, v.x);
-        best.y = __vmaxs4(best.y, v.y);
-        best.z = __vmaxs4(best.z, v.z);
-        best.w = __vmaxs4(best.w, v.w);
-        any = true;
+    int n = (int)i;
+    const int c = radix.words.rest(n), ow = radix.width.rest(n), oh = radix.height.rest(n);
+    const int ih0 = oh * g.SH - g.PT, iw0 = ow * g.SW - g.PL;
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) hi[k] = lo[k] = 0x80008000u;
+    const uint4 *image = reinterpret_cast<const uint4 *>(in + (int64_t)n * g.H * g.W * g.C) + c;
+    const bool any = g.H > 0 && g.W > 0 && ih0 < g.H && iw0 < g.W && ih0 + KH > 0 && iw0 + KW > 0;
+    if (any) {
+#pragma unroll
+      for (int kh = 0; kh < KH; kh++) {
+        const int ih = min(max(ih0 + kh, 0), g.H - 1);
+#pragma unroll
+        for (int kw = 0; kw < KW; kw++) {
+          const int iw = min(max(iw0 + kw, 0), g.W - 1);
+          const uint4 v = __ldg(image + ((int64_t)ih * g.W + iw) * cc);
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            asm("max.s16x2 %0, %0, %1;" : "+r"(hi[k]) : "r"(w[k]));
+            asm("max.s16x2 %0, %0, %1;" : "+r"(lo[k]) : "r"(w[k] << 8));
+          }
+        }
       }
-    if (!any) {
-      const uint32_t d4 = 0x01010101u * (uint32_t)(uint8_t)def;
-      best = make_uint4(d4, d4, d4, d4);
     }
-    reinterpret_cast<uint4 *>(out)[i] = best;
+    uint32_t best[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) best[k] = any ? __byte_perm(lo[k], hi[k], 0x7351) : 0x01010101u * (uint32_t)(uint8_t)def;
+    reinterpret_cast<uint4 *>(out)[i] = make_uint4(best[0], best[1], best[2], best[3]);
   }
+}
+
+__device__ __forceinline__ int8_t avg_result(int32_t sum, int32_t area, int count_include_pads, int32_t out_off, const Triple &t) {
+  if (count_include_pads) return (int8_t)clip_i8(scale32(sum, t.pre, t.post, t.scale, out_off));
+  if (area == 0) return (int8_t)out_off;
+  // libjit_div_round_i32 (libjit_defs.h:238-244): round half away from zero
+  const int32_t s = scale32(sum, t.pre, t.post, t.scale, 0), rnd = area >> 1;
+  return (int8_t)clip_i8((s > 0 ? (s + rnd) / area : (s - rnd) / area) + out_off);
 }
 
 // libjit_avg_pool_i8 (libjit.cpp:2812-2897)
@@ -315,18 +338,51 @@ __global__ void __launch_bounds__(kThreads) avg_pool_i8_kernel(const int8_t *__r
         sum += (int32_t)in[(((int64_t)n * g.H + ih) * g.W + iw) * g.C + c] - in_off;
         area++;
       }
-    int32_t res;
-    if (count_include_pads) {
-      res = clip_i8(scale32(sum, t.pre, t.post, t.scale, out_off));
-    } else if (area == 0) {
-      res = out_off;
-    } else {
-      // libjit_div_round_i32 (libjit_defs.h:238-244): round half away from zero
-      const int32_t s = scale32(sum, t.pre, t.post, t.scale, 0);
-      const int32_t rnd = area >> 1;
-      res = clip_i8((s > 0 ? (s + rnd) / area : (s - rnd) / area) + out_off);
+    out[i] = avg_result(sum, area, count_include_pads, out_off, t);
+  }
+}
+
+// The same where every window lies inside the image and four channels make an aligned word (a global average pool): a
+// thread takes a word's channels and every P-th row of the window, P lanes add up.  With a byte and 49 loads per thread a
+// 7 x 7 x 2048 image took 12 us, a few blocks' chain of loads, now 5; 64 of them 11, now 8.
+template <int P>
+__global__ void __launch_bounds__(kThreads) avg_pool_i8_words_kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out,
+                                                                     const __grid_constant__ PoolGeom g,
+                                                                     const __grid_constant__ PoolRadix radix, int count_include_pads,
+                                                                     int32_t out_off, int32_t in_off, Triple t) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int words = g.C >> 2, part = threadIdx.x & (P - 1);
+  const int64_t total = (int64_t)g.N * g.OH * g.OW * words, groups = (int64_t)gridDim.x * (kThreads / P);
+  const int64_t rounds = (total + groups - 1) / groups;
+  for (int64_t k = 0; k < rounds; k++) {  // (whole warps: the lanes of an output add up)
+    const int64_t i = k * groups + (int64_t)blockIdx.x * (kThreads / P) + threadIdx.x / P;
+    const bool mine = i < total;
+    int32_t sum[4] = {0, 0, 0, 0};
+    if (mine) {
+      int n = (int)i;
+      const int c = radix.words.rest(n), ow = radix.width.rest(n), oh = radix.height.rest(n);
+      const uint32_t *p0 = reinterpret_cast<const uint32_t *>(in) + (((int64_t)n * g.H + oh * g.SH) * g.W + ow * g.SW) * words + c;
+      for (int kh = part; kh < g.KH; kh += P) {
+        const uint32_t *row = p0 + (int64_t)kh * g.W * words;
+#pragma unroll 8
+        for (int kw = 0; kw < g.KW; kw++) {
+          const int32_t v = (int32_t)__ldg(row + (int64_t)kw * words);
+#pragma unroll
+          for (int b = 0; b < 4; b++) sum[b] = __dp4a(v, 1 << (8 * b), sum[b]);
+        }
+      }
     }
-    out[i] = (int8_t)res;
+#pragma unroll
+    for (int d = 1; d < P; d <<= 1)
+#pragma unroll
+      for (int b = 0; b < 4; b++) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], d);
+    if (!mine || part != 0) continue;
+    const int32_t area = g.KH * g.KW;
+    uint32_t word = 0;
+#pragma unroll
+    for (int b = 0; b < 4; b++) word |= (uint32_t)(uint8_t)avg_result(sum[b] - area * in_off, area, count_include_pads, out_off, t) << (8 * b);
+    reinterpret_cast<uint32_t *>(out)[i] = word;
   }
 }
 
@@ -376,6 +432,56 @@ __global__ void __launch_bounds__(kThreads) transpose4_short_inner_kernel(const 
     const T *from = src + (int64_t)i0 * s0 + (int64_t)i1 * s1 + i2;
     TO *to = dst + i * d3;
     for (int c = 0; c < d3; c++) to[c] = f(from[(int64_t)c * s3]);
+  }
+}
+
+// The Quantize on its way from C <= 4 channel planes to NHWC, four pixels at a time: C loads of 16 bytes, one word per
+// channel of quotients, whose bytes are dealt out to C words of the result.  The quotient is x times the reciprocal; only
+// where that (its error is below 6e-4 within +- 2000) lies within 1e-3 of a tie does the division decide, so every element is
+// quantize_one's.  What bounds it is memory: 64 x 3 x 224 x 224 24 us with a pixel and three divisions per thread, now 9.
+template <int C>
+__global__ void __launch_bounds__(kThreads) quantize_planes_kernel(const float *__restrict__ src, int8_t *__restrict__ dst, int d0, int d1,
+                                                                   int d2, int s0, int s1, int s3, float scale, int32_t offset) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const unsigned fours = (unsigned)d2 >> 2, total = (unsigned)d0 * (unsigned)d1 * fours;
+  const float inverse = __fdiv_rn(1.0f, scale), shift = (float)offset;
+  constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: its sum with u has rint(u) in the low bits
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / fours, i2 = (i - r * fours) * 4, i0 = r / (unsigned)d1, i1 = r - i0 * (unsigned)d1;
+    const float *from = src + (int64_t)i0 * s0 + (int64_t)i1 * s1 + i2;
+    float x[C][4];
+#pragma unroll
+    for (int c = 0; c < C; c++) *reinterpret_cast<float4 *>(x[c]) = __ldg(reinterpret_cast<const float4 *>(from + (int64_t)c * s3));
+    uint32_t q[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      int32_t v[4];
+      bool sure = true;
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float u = __fadd_rn(__fmul_rn(x[c][e], inverse), shift), m = __fadd_rn(u, kMagic);
+        sure = sure && fabsf(u) < 2000.0f && fabsf(__fadd_rn(u, -__fadd_rn(m, -kMagic))) < 0.499f;
+        v[e] = __float_as_int(m) - __float_as_int(kMagic);
+      }
+      if (!sure) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = quantize_one(x[c][e], scale, offset);
+      }
+      asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(q[c]) : "r"(v[3]), "r"(v[2]), "r"(0));
+      asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(q[c]) : "r"(v[1]), "r"(v[0]), "r"(q[c]));
+    }
+    uint32_t *to = reinterpret_cast<uint32_t *>(dst + (size_t)i * 4 * C);
+#pragma unroll
+    for (int w = 0; w < C; w++) {
+      uint32_t word = 0;
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        const int k = 4 * w + b, pixel = k / C, c = k % C;
+        word |= ((q[c] >> (8 * pixel)) & 0xffu) << (8 * b);
+      }
+      to[w] = word;
+    }
   }
 }
 
@@ -539,8 +645,9 @@ extern "C" int glowb200_max_pool_i8(const int8_t *in, int8_t *out, const int64_t
   const int64_t total = (int64_t)g.N * g.OH * g.OW * g.C;
   if (total == 0) return GLOWB200_OK;
   GLOWB200_REQUIRE(in && out, "NULL tensor pointer");
-  if ((g.C & 15) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0)
-    GLOWB200_CUDA_OK(launch_pdl(max_pool_i8_vec_kernel, grid_for(total >> 4), kThreads, 0, GLOWB200_STREAM, in, out, g, (int8_t)out_offset));
+  if ((g.C & 15) == 0 && total >> 4 < (1ll << 31) && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0)
+    GLOWB200_CUDA_OK(launch_pdl(g.KH == 3 && g.KW == 3 ? max_pool_i8_vec_kernel<3> : max_pool_i8_vec_kernel<0>, grid_for(total >> 4), kThreads, 0, GLOWB200_STREAM, in, out, g,
+                                PoolRadix(g, g.C / 16), (int8_t)out_offset));
   else
     max_pool_i8_kernel<<<grid_for(total), kThreads, 0, GLOWB200_STREAM>>>(in, out, g, (int8_t)out_offset);
   GLOWB200_CUDA_OK(cudaGetLastError());
@@ -556,8 +663,21 @@ extern "C" int glowb200_avg_pool_i8(const int8_t *in, int8_t *out, const int64_t
   const int64_t total = (int64_t)g.N * g.OH * g.OW * g.C;
   if (total == 0) return GLOWB200_OK;
   GLOWB200_REQUIRE(in && out, "NULL tensor pointer");
+  const Triple scale{out_pre, out_post, out_scale};
+  if (g.PT == 0 && g.PL == 0 && (int64_t)(g.OH - 1) * g.SH + g.KH <= g.H && (int64_t)(g.OW - 1) * g.SW + g.KW <= g.W && g.C % 4 == 0 && total < (1ll << 31) &&
+      ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 3) == 0) {
+    // eight lanes to an output until the outputs alone fill the SMs
+    const int64_t words = total / 4;
+    auto with = [&](auto kernel, int lanes) {
+      return launch_pdl(kernel, grid_for(words * lanes), kThreads, 0, GLOWB200_STREAM, in, out, g, PoolRadix(g, g.C / 4),
+                        count_include_pads ? 1 : 0, out_offset, in_offset, scale);
+    };
+    if (g.KH >= 5 && words <= kB200Sms * 512) GLOWB200_CUDA_OK(with(avg_pool_i8_words_kernel<8>, 8));
+    else GLOWB200_CUDA_OK(with(avg_pool_i8_words_kernel<1>, 1));
+    return GLOWB200_OK;
+  }
   GLOWB200_CUDA_OK(launch_pdl(avg_pool_i8_kernel, grid_for(total), kThreads, 0, GLOWB200_STREAM, in, out, g, count_include_pads ? 1 : 0,
-                              out_offset, in_offset, Triple{out_pre, out_post, out_scale}));
+                              out_offset, in_offset, scale));
   GLOWB200_CUDA_OK(cudaGetLastError());
   return GLOWB200_OK;
 }
@@ -621,5 +741,13 @@ extern "C" int glowb200_quantize_transpose_i8(int8_t *dest, const float *src, co
   if (t.total == 0) return GLOWB200_OK;
   GLOWB200_REQUIRE(src && dest, "NULL tensor pointer");
   GLOWB200_REQUIRE(scale != 0.0f, "scale must not be zero");
+  if (t.d[3] <= 4 && t.st[2] == 1 && t.st[3] != 1 && ((t.d[2] | t.st[0] | t.st[1] | t.st[3]) & 3) == 0 &&
+      (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dest) & 3) == 0) {
+    auto kernel = t.d[3] == 1 ? quantize_planes_kernel<1> : t.d[3] == 2 ? quantize_planes_kernel<2> : t.d[3] == 3 ? quantize_planes_kernel<3>
+                                                                                                              : quantize_planes_kernel<4>;
+    GLOWB200_CUDA_OK(launch_pdl(kernel, grid_for(t.total / t.d[3] / 4), kThreads, 0, GLOWB200_STREAM, src, dest, t.d[0], t.d[1], t.d[2],
+                                t.st[0], t.st[1], t.st[3], scale, offset));
+    return GLOWB200_OK;
+  }
   return run_transpose(t, src, dest, QuantizeF{scale, offset}, GLOWB200_STREAM);
 }
