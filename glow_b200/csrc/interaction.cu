@@ -58,17 +58,21 @@ __global__ void __launch_bounds__(256) pairwise_dot_kernel(const float *__restri
 // the kernel above.  Every dot still is the sequential FMA chain over k = 0..D-1, so the bits are
 // the same.  Rows are padded by 4 floats (D + 4, an odd number of 16-byte units for D a multiple of 8) so that
 // the neighbouring rows a warp reads fall into different banks.
-// What bounds it is latency: both forms tried for many vectors -- this one, and 8 x 4 tiles over a transposed copy with
-// packed FMAs -- issue about one instruction every other cycle per scheduler (4096 samples of 65 x 128: 138 us;
-// smaller blocks or fewer registers per thread did not help).  Few vectors have few tiles -- 28 of 4 x 4 for 27
+// What bounds it, for many vectors, is the copying and the sums in turn: 45 us of one and 67 of the other for 4096 samples of
+// 65 x 128, where a multiply-add of three registers takes a scheduler 1.5 to 1.9 clocks.  Vectors come by asynchronous
+// copies, without a register on the way (133 -> 114 us), and more blocks fit an SM when they have no idle warps
+// (108).  Not better: 8 x 4 tiles over a transposed copy with packed multiply-adds (138), 6 x 6, 7 x 7 and 8 x 8 tiles of
+// several samples to a block (124 - 146), two buffers and a block that goes on (122 - 136).
+// Few vectors have few tiles -- 28 of 4 x 4 for 27
 // vectors, the rest of the block idle -- and go in 2 x 2 tiles with no more warps than those fill: 128 samples of
-// 27 x 64 5.4 -> 3.5 us, 4096 samples 35 -> 22, 2048 of 17 x 32 15.0 -> 5.4.
-template <int R>
-__global__ void __launch_bounds__(256, 4) pairwise_dot_tiled_kernel(const float *__restrict__ dense, int64_t ld_dense,
-                                                                 const float *__restrict__ pooled, int64_t ld_pooled,
-                                                                 int tables, int D, float *__restrict__ out_f,
-                                                                 int8_t *__restrict__ out_q, int64_t ld_out, float q_scale,
-                                                                 int32_t q_offset, int vec_in) {
+// 27 x 64 5.4 -> 3.3 us, 4096 samples 35 -> 21, 2048 of 17 x 32 15.0 -> 5.4.
+// The quantized result takes the reciprocal of its scale; next to a tie the division decides.
+template <int R, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) pairwise_dot_tiled_kernel(const float *__restrict__ dense, int64_t ld_dense,
+                                                                             const float *__restrict__ pooled, int64_t ld_pooled,
+                                                                             int tables, int D, float *__restrict__ out_f,
+                                                                             int8_t *__restrict__ out_q, int64_t ld_out, float q_scale,
+                                                                             int32_t q_offset, int vec_in) {
   pdl_wait();               // (launched as a programmatic dependent of the pooling kernel)
   pdl_launch_dependents();  // a contraction that follows may set up now (it waits for this kernel before its loads)
   extern __shared__ __align__(16) float v[];  // [R * ceil(n / R)][D + 4]; rows beyond n are zero
@@ -78,11 +82,14 @@ __global__ void __launch_bounds__(256, 4) pairwise_dot_tiled_kernel(const float 
     const int q = D >> 2;
     for (int i = threadIdx.x; i < nb * R * q; i += blockDim.x) {
       const int r = i / q, k = (i - r * q) * 4;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < n) x = r == 0 ? __ldg(reinterpret_cast<const float4 *>(dense + b * ld_dense + k))
-                            : __ldg(reinterpret_cast<const float4 *>(pooled + b * ld_pooled + (int64_t)(r - 1) * D + k));
-      *reinterpret_cast<float4 *>(v + r * pitch + k) = x;
+      if (r >= n)
+        *reinterpret_cast<float4 *>(v + r * pitch + k) = make_float4(0.f, 0.f, 0.f, 0.f);
+      else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(v + r * pitch + k)),
+                     "l"(r == 0 ? dense + b * ld_dense + k : pooled + b * ld_pooled + (int64_t)(r - 1) * D + k)
+                     : "memory");
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
     for (int i = threadIdx.x; i < nb * R * D; i += blockDim.x) {
       const int r = i / D, k = i - r * D;
@@ -90,11 +97,13 @@ __global__ void __launch_bounds__(256, 4) pairwise_dot_tiled_kernel(const float 
     }
   }
   __syncthreads();
+  const float inverse = __fdiv_rn(1.0f, q_scale), shift = (float)q_offset;
   auto emit = [&](int64_t col, float x) {
     if (out_q) {
-      const float t = __fadd_rn(__fdiv_rn(x, q_scale), (float)q_offset);
-      const float c = fminf(fmaxf(nearbyintf(t), -2147483648.0f), 2147483520.0f);
-      out_q[b * ld_out + col] = (int8_t)clip_i8((int32_t)c);
+      bool sure = true;
+      int32_t q = quantize_by_reciprocal(x, inverse, shift, sure);
+      if (!sure) q = (int32_t)fminf(fmaxf(nearbyintf(__fadd_rn(__fdiv_rn(x, q_scale), shift)), -2147483648.0f), 2147483520.0f);
+      out_q[b * ld_out + col] = (int8_t)clip_i8(q);
     } else {
       out_f[b * ld_out + col] = x;
     }
@@ -167,13 +176,16 @@ extern "C" int glowb200_pairwise_dot_interaction(const float *dense, int64_t ld_
   const int R = tiles_of(4) >= 80 ? 4 : 2;  // (66 tiles -- 41 vectors -- still gain from the smaller ones)
   const size_t tiled_smem = (size_t)((n + R - 1) / R * R) * (dim + 4) * sizeof(float);
   if ((dim % 4) == 0 && tiled_smem <= 200 * 1024) {
-    auto kernel = R == 4 ? pairwise_dot_tiled_kernel<4> : pairwise_dot_tiled_kernel<2>;
-    if (tiled_smem > 48 * 1024)
-      GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_smem));
     const int64_t warps = (tiles_of(R) + 31) / 32;
-    const unsigned threads = R == 4 ? 256 : 32 * (unsigned)(warps < 2 ? 2 : warps > 8 ? 8 : warps);
     const int vec_in = (reinterpret_cast<uintptr_t>(dense) % 16 == 0) && (ld_dense % 4 == 0) &&
                        (tables == 0 || (reinterpret_cast<uintptr_t>(pooled) % 16 == 0 && ld_pooled % 4 == 0));
+    // Blocks with no more threads than tiles once six of them to an SM fill it more than twice (4096 samples of 65 x 128: 108 us
+    // against 114); fewer samples are copied and summed faster by larger ones (512 samples: 18.4 against 27).
+    const bool many = R == 4 && tiles_of(4) <= 160 && batch >= 2 * 6 * (int64_t)sm_count();
+    auto kernel = many ? pairwise_dot_tiled_kernel<4, 160, 6> : R == 4 ? pairwise_dot_tiled_kernel<4, 256, 4> : pairwise_dot_tiled_kernel<2, 256, 4>;
+    const unsigned threads = many ? 160 : R == 4 ? 256 : 32 * (unsigned)(warps < 2 ? 2 : warps > 8 ? 8 : warps);
+    if (tiled_smem > 48 * 1024)
+      GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_smem));
     GLOWB200_CUDA_OK(launch_pdl(kernel, (unsigned)batch, threads, tiled_smem, cs, dense, ld_dense, pooled, ld_pooled,
                                 (int)tables, (int)dim, out_f32, out_i8, ld_out, quant_scale, quant_offset, vec_in));
     return GLOWB200_OK;

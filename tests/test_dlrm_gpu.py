@@ -150,3 +150,19 @@ def test_peer_rendezvous_kernel_and_its_bounded_wait():
     torch.cuda.synchronize()
     assert int(st.item()) == 0
     buf.release()
+
+
+@pytest.mark.parametrize("B,T,D", [(1776, 47, 8), (1777, 67, 4), (1775, 50, 8)])
+def test_interaction_of_many_samples(oracle, B, T, D):
+    """Launches on either side of the change of block size, quantized next to ties as well."""
+    rng = np.random.default_rng(T)
+    dense = (rng.integers(-6, 7, (B, D)) / 4).astype(np.float32)   # dots on a grid: many are halves of the scale
+    pooled = (rng.integers(-6, 7, (B, T, D)) / 4).astype(np.float32)
+    want = oracle.pairwise_dot_interaction(dense, pooled)
+    args = torch.from_numpy(dense).to(DEV), torch.from_numpy(pooled).to(DEV)
+    np.testing.assert_array_equal(ops.pairwise_dot_interaction(*args).cpu().numpy().view(np.uint32), want.view(np.uint32))
+    # (|dot| <= 2.25 * 8 = 18: at 1e-3 quotients reach 18000, beyond where the reciprocal is trusted, and stay inside
+    # int32, where the reference's conversion is defined)
+    for scale, offset in ((0.125, -7), (0.37, 100), (1e-3, 0)):
+        np.testing.assert_array_equal(ops.pairwise_dot_interaction(*args, quant=(scale, offset)).cpu().numpy(),
+                                      oracle.element_quantize_i8(want, scale, offset))
