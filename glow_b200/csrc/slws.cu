@@ -6,8 +6,8 @@
 //   * a "segments" kernel turns lengths (or offsets) into validated bag boundaries in the caller's
 //     workspace, one int64 array per table (tables of up to 2048 bags pooled with fp32 accumulation need none:
 //     their warps add up the lengths before their bags themselves);
-//   * fp32 accumulation over rows of a multiple of 8 columns is slws_run.cu's and, in launches where the longest
-//     bag decides, slws_spread.cu's;
+//   * fp32 accumulation over rows of a multiple of 8 columns is slws_run.cu's, in launches where the longest
+//     bag decides slws_spread.cu's and in those that fill the GPU with rows that suit it slws_stream.cu's;
 //   * fp16 accumulation, which the reference rounds at every step, is done exactly that way, step by
 //     step, by slws_gather_kernel below: a group of `lpr` lanes (a power of two, 1..32) per bag, each
 //     lane with P chunks of 8 columns, indices read coalesced and handed round by shuffles, kUnroll rows
@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(kGatherThreads, P == 4 ? 8 : 12) slws_gather_k
 
 // ------------------------------------------------------------------------------------------
 // Any-shape gather-pool: rows of any width and alignment (a column count that is not a
-// multiple of 8, a table that is not 8-byte aligned).  One warp per bag, byte loads, column
+// multiple of 8 -- uint8 rows of a multiple of 4 go to slws_stream.cu, which has these operations as well --, a
+// table that is not 8-byte aligned).  One warp per bag, byte loads, column
 // tiles of 128; the row-by-row arithmetic of the reference in its order, without FMA
 // contraction.  Correct for everything, fast for nothing -- real tables take the kernel above.
 // ------------------------------------------------------------------------------------------
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(256) slws_gather_any_kernel(const __grid_const
 struct GatherConfig {
   int kind, idx64, out16, acc16;
 };
-enum class Form { kAnyShape, kRuns, kFp16Steps };  // the any-shape kernel, slws_run.cu / slws_spread.cu, slws_gather_kernel
+enum class Form { kAnyShape, kRuns, kFp16Steps };  // the any-shape kernel, slws_run.cu / slws_spread.cu / slws_stream.cu, slws_gather_kernel
 
 template <int BITS, typename IdxT>
 cudaError_t launch_fp16_steps(SlwsLaunch L, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {
@@ -421,6 +422,16 @@ int plan(const GatherConfig &g, int64_t in_line, int64_t out_line, bool operands
   align = (int)((align | in_line) & -(align | in_line));
   align = align >= 8 ? 8 : align >= 4 ? 4 : 1;
   form = Form::kAnyShape;
+  // (the any-shape kernel takes 4.5 times as long for 100 columns as any other for 104; both give the reference's bits)
+  if (out_line % 8 == 4 && out_line > 36 && operands_fit && !g.acc16 && kind < 2) {
+    SlwsLaunch L{};
+    L.kind = kind;
+    L.in_line = (int32_t)in_line;
+    L.out_line = (int32_t)out_line;
+    L.single.data = reinterpret_cast<const void *>((uintptr_t)align);  // (as far as where rows start goes)
+    if (slws_stream_takes(L, align)) form = Form::kRuns;
+    return GLOWB200_OK;
+  }
   // (above 1024 columns, and for other widths, the any-shape kernel's operation order stays)
   if (out_line == 0 || out_line % 8 != 0 || out_line > 1024 || !operands_fit) return GLOWB200_OK;
   if (!g.acc16) form = Form::kRuns;

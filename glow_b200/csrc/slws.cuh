@@ -297,10 +297,13 @@ constexpr int64_t kInlineLengthsMax = 2048;
 constexpr int64_t kMostRows = INT32_MAX / 7 * 4ll;
 
 // Gather-pool with fp32 accumulation for rows of a multiple of 8 columns, any alignment (align: what
-// every row of every table starts on -- 8, 4 or 1 bytes): chooses between the two kernels (slws_spread.cu) by the
-// bags and, where the caller knows them, the rows of the launch (kRowsUnknown: it does not).
+// every row of every table starts on -- 8, 4 or 1 bytes), or any that slws_stream_takes: chooses between the three
+// kernels (slws_spread.cu) by the bags and, where the caller knows them, the rows of the launch (kRowsUnknown: it does not).
 constexpr int64_t kRowsUnknown = -1;
 cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, int64_t rows, cudaStream_t s);
+// slws_stream.cu: whether it can pool a launch's rows at all, and the launch.
+bool slws_stream_takes(const SlwsLaunch &L, int align);
+cudaError_t launch_slws_stream(const SlwsLaunch &L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s);
 cudaError_t launch_slws_run(SlwsLaunch L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s);
 
 }  // namespace glowb200

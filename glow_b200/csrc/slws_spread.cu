@@ -249,7 +249,12 @@ cudaError_t launch_slws_spread(const SlwsLaunch &L, SpreadShape c, int align, in
 }  // namespace
 
 // Which kernel pools a launch.  Rows of up to 256 columns at 4-byte boundaries; wider ones fill a warp in
-// slws_run.cu as well.
+// slws_run.cu as well.  Widths off the eights have slws_stream.cu alone.
+//   * slws_stream.cu takes the rows that suit it (see there for both sides of every line) from 24 bags per SM on of up to 64
+//     columns; of wider ones from 64 on, or, where the boundaries are known and with them the skewed tables, from 84 on (47 x 250
+//     41 against 33 us, 8 x 1000 of 20 rows 14.2 against 15.7; one table of 12,000 skewed bags 38 against 43).  Not bags of fewer than
+//     five rows on average, nor of twelve in launches of up to 150 bags per SM (64 x 250 of 10 rows 14.2 against 16.0).
+//     What follows is the rules for the others.
 //   * small launches take this one: up to the 12 bags per SM that are resident at once of rows of 32 columns, which leave
 //     half of the lanes idle here (2 x 211 skewed bags 16.9 -> 11.4 us); up to 24 of 64 columns (26 x 128 13.7 -> 11.7); up to 84 of
 //     wider rows, which occupy a warp per bag in either kernel (30 tables, 400 skewed 4-bit bags of 96 columns: 67 -> 50,
@@ -274,7 +279,10 @@ cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t n
     const int64_t slots = sms * kWarps * blocks_per_sm(four_bit ? 4 : 8, v, lanes, rows) * times;
     return SpreadShape{v, lanes, rows, (int)std::min<int64_t>(kMaxRun, std::max<int64_t>(32 / lanes, (total + slots - 1) / slots))};
   };
-  const int64_t small = sms * (columns <= 32 ? 12 : columns <= 64 ? 24 : 84);
+  if (columns % 8 != 0) return launch_slws_stream(L, align, max_segments, num_jobs, s);
+  const bool streams = columns > 32 && slws_stream_takes(L, align) && !(columns > 56 && columns <= 64 && (four_bit || !L.inline_lengths)) &&
+                       !(rows >= 0 && rows < total * (total <= sms * 150 ? 12 : 5));
+  const int64_t small = sms * (columns <= 32 ? 12 : columns <= 64 ? 24 : streams && L.inline_lengths ? 64 : 84);
   const bool short_bags = rows >= 0 && rows < total * 8, wide_bytes = !four_bit && columns > 128;
   if (align < 4 || columns > 256 || (wide_bytes && total <= sms * 32)) return launch_slws_run(L, align, max_segments, num_jobs, s);
   if (total <= small && !short_bags && !(columns <= 128 && total > sms * 12 && total <= sms * 16)) {
@@ -284,6 +292,7 @@ cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t n
                                            : shape(8, 32, four_bit && total <= sms * 12 ? 32 : 16, 1);
     return launch_slws_spread(L, c, align, max_segments, num_jobs, s);
   }
+  if (streams) return launch_slws_stream(L, align, max_segments, num_jobs, s);
   if (columns > 32 && max_segments > kInlineLengthsMax && total <= sms * 384 && (rows < 0 || rows >= 1 << 17))
     L.skip_from = four_bit || columns <= 64 ? 1 : 128;
   if (cudaError_t e = launch_slws_run(L, align, max_segments, num_jobs, s)) return e;

@@ -1,0 +1,113 @@
+"""The gather-pool that copies whole rows into shared memory, at its edges: rows at every alignment and the last of a
+table, bags round the 32 rows of a step, empty ones, runs cut anywhere, rows that are not there, widths that only it
+takes.  Every bag against the bits that the bag gives when it is pooled alone, by another kernel where there is one, and
+against float64."""
+import numpy as np
+import pytest
+import torch
+
+from glow_b200 import ops
+from test_slws_runs_gpu import DEV, EDGES, check, dev, make_table, pool, want_and_size, with_4bit_surplus
+
+pytestmark = pytest.mark.gpu
+
+
+def request_of(rng, rows, bags, kind, idt=np.int64):
+    lengths = rng.choice(EDGES[:24] + [40, 40, 90], bags).astype(np.int32)
+    n = int(lengths.sum())
+    idx = rng.integers(0, rows, n).astype(idt)
+    idx[rng.integers(0, n, n // 7)] = rows - 1   # the last row ends the table: its last piece is cut
+    return lengths, idx, rng.normal(0, 1, n).astype(np.float16 if kind & 1 else np.float32)
+
+
+def check_pooled(table, kind, dim, w, idx, lengths, got):
+    want, size = want_and_size(table, kind, dim, w, idx, lengths)
+    check(got.cpu().numpy(), want, with_4bit_surplus(size, table, kind, w, idx, lengths), 2e-3 if kind & 1 else 1e-5)
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 40), (0, 48), (0, 64), (0, 72), (0, 96), (0, 128), (1, 48), (1, 88), (1, 128),
+                                      (2, 40), (2, 56), (2, 96), (2, 128), (2, 136), (2, 256), (3, 48), (3, 104), (3, 192), (3, 256)])
+@pytest.mark.parametrize("bags,rows", [(10_000, 1), (20_000, 37), (37_000, 5000)])
+def test_single_tables(kind, dim, bags, rows):
+    """(above 2048 bags of 57..64 columns another kernel's: those go in tables of 2048 below)"""
+    rng = np.random.default_rng(bags + dim + kind)
+    table = make_table(kind, rows, dim, 5)
+    lengths, idx, w = request_of(rng, rows, bags, kind, np.int32 if kind & 1 else np.int64)
+    d = dev(table)
+    st = ops.new_status(DEV)
+    whole = pool(d, w, idx, lengths, kind, status=st)
+    assert int(st.item()) == 0
+    ends = np.cumsum(lengths)
+    for b in list(range(30)) + list(rng.integers(0, bags, 10)) + [bags - 1]:
+        e, l = int(ends[b]), int(lengths[b])
+        assert torch.equal(pool(d, w[e - l:e], idx[e - l:e], lengths[b:b + 1], kind)[0], whole[b])
+    few = 600
+    check_pooled(table, kind, dim, w[:ends[few - 1]], idx[:ends[few - 1]], lengths[:few], whole[:few])
+
+
+@pytest.mark.parametrize("kind,dim,shift", [(0, 96, 8), (0, 96, 4), (0, 100, 4), (1, 96, 12), (2, 96, 4), (3, 128, 4), (2, 240, 8)])
+def test_tables_at_any_four_bytes(kind, dim, shift):
+    rng = np.random.default_rng(shift)
+    table = make_table(kind, 900, dim, 5)
+    lengths, idx, w = request_of(rng, 900, 12_000, kind)
+    assert torch.equal(pool(dev(table, shift), w, idx, lengths, kind), pool(dev(table), w, idx, lengths, kind))
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("dim", [44, 60, 68, 100, 124])
+@pytest.mark.parametrize("bags", [1, 7, 300, 2049, 15_000])
+def test_widths_off_the_eights(oracle, kind, dim, bags):
+    """The operations of the any-shape kernel, which has them otherwise, in the reference's order: bit for bit."""
+    rng = np.random.default_rng(bags + dim)
+    table = make_table(kind, 700, dim, 9)
+    lengths, idx, w = request_of(rng, 700, bags, kind, np.int32)
+    lengths[0] = max(1, lengths[0])
+    n = int(lengths.sum())
+    idx, w = np.resize(idx, n) if idx.size else np.zeros(n, np.int32), np.resize(w, n) if w.size else np.ones(n, w.dtype)
+    d = dev(table)
+    whole = pool(d, w, idx, lengths, kind)
+    few = min(bags, 400)
+    e = int(lengths[:few].sum())
+    want = oracle.frwq_slws_interp(table, kind, w[:e], idx[:e], lengths[:few])
+    np.testing.assert_array_equal(whole[:few].cpu().numpy().view(np.uint8), want.view(np.uint8))
+    padded = ops.pad_fused_rows(d, kind, 256)
+    assert torch.equal(ops.fused_rowwise_quantized_sparse_lengths_weighted_sum(padded, dev(w), dev(idx), dev(lengths), kind, out_line=dim), whole)
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 64), (0, 128), (3, 128)])
+def test_rows_that_are_not_there(kind, dim):
+    """Indices outside the table, a table without rows, negative lengths and lengths beyond the indices."""
+    rng = np.random.default_rng(dim)
+    rows, bags, tables = 300, 1900, 8
+    table = make_table(kind, rows, dim, 5)
+    dt = np.float16 if kind & 1 else np.float32
+    lengths = rng.integers(0, 40, (tables, bags)).astype(np.int32)
+    idx = [rng.integers(0, rows, int(l.sum())) for l in lengths]
+    w = [rng.normal(0, 1, i.size).astype(dt) for i in idx]
+    bad = [i.copy() for i in idx]
+    for i in bad:
+        i[::11] = rows + 5
+        i[::17] = -3
+    d, out = dev(table), torch.empty((tables, bags, dim), dtype=torch.float16 if kind & 1 else torch.float32, device=DEV)
+    st = ops.new_status(DEV)
+
+    def run(indices, weights, lens, data=None):
+        b = ops.SlwsBatch(kind, table.shape[1], torch.int64, device=DEV)
+        b.bind([d if data is None else data] * tables, [dev(x) for x in weights], [dev(x) for x in indices], [dev(x) for x in lens], list(out))
+        b.run(st)
+        return out.clone()
+
+    with_bad = run(bad, w, lengths)
+    assert int(st.item()) == ops.STATUS_INDEX_OUT_OF_RANGE
+    st.zero_()
+    nothing = [np.where((i >= 0) & (i < rows), x, 0).astype(dt) for i, x in zip(bad, w)]
+    there = [np.where((i >= 0) & (i < rows), i, 0) for i in bad]
+    clean = run(there, nothing, lengths)
+    assert int(st.item()) == 0 and torch.equal(with_bad.float(), clean.float())   # (a zero sum may have either sign)
+    none = run(bad, w, lengths, d[:0])
+    assert int(st.item()) == ops.STATUS_INDEX_OUT_OF_RANGE and not none.any()
+    st.zero_()
+    odd = lengths.copy()
+    odd[:, 5], odd[:, -1] = -4, odd[:, -1] + 60
+    run(idx, w, odd)
+    assert int(st.item()) == (ops.STATUS_NEGATIVE_LENGTH | ops.STATUS_LENGTHS_OVERRUN)
