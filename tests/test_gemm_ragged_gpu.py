@@ -105,3 +105,15 @@ def test_workspaces_of_every_size(oracle, M, K, N, shift):
                                        status=status)
         np.testing.assert_array_equal(got.cpu().numpy(), want)
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("m,n", [(2048, 1000), (2049, 1024), (4096, 500), (4097, 512), (3136, 512), (9472, 256), (9473, 250)])
+def test_products_on_either_side_of_one_round_of_tiles(m, n):
+    """128-column tiles that all have an SM at once, and one more: the same integers as the loop the reference has."""
+    rng = np.random.default_rng(m)
+    k = 144
+    x, w = (torch.from_numpy(rng.integers(-128, 128, s, dtype=np.int8)).cuda() for s in ((m, k), (n, k)))
+    col = lambda lo, hi: torch.from_numpy(rng.integers(lo, hi + 1, n, dtype=np.int32)).cuda()
+    args = (x, w, col(-4000, 4000), col(0, 0), (col(0, 1), col(0, 9), col(1, 90)), (col(2, 3), col(15, 15), col(255, 510)), 3, -5, 0)
+    want = ops.rowwise_quantized_fc(*args, flags=ops.FC_WEIGHT_OFFSETS_ZERO | ops.FC_FORCE_ANY_SHAPE_KERNEL)
+    assert torch.equal(ops.rowwise_quantized_fc(*args, flags=ops.FC_WEIGHT_OFFSETS_ZERO), want)
