@@ -513,6 +513,21 @@ int run_conv(GemmParams p, const int8_t *in, const int8_t *filter, const ConvGeo
       return run_gemm_row_windows(p, planes, rows, g.OW, fb, bs, s);
     }
   }
+  // Every s-th pixel of an image whose sides are multiples of s: the contraction's loads take them from the input itself, whole
+  // lines of output pixels to a tile.  At least 96 of a tile's 128 rows have to be pixels (28 x 28 of 64 x 56 x 56 x 256 to 512
+  // channels, 112 rows to a tile: 10 + 15 us with a copy of the pixels, now 17).
+  if (pl.need_im2col && g.KH == 1 && g.KW == 1 && g.SH == g.SW && g.PT == 0 && g.PL == 0 && g.H == g.OH * g.SH && g.W == g.OW * g.SW &&
+      (flags & GLOWB200_FC_WEIGHT_OFFSETS_ZERO) && g.C % 16 == 0 && aligned && g.OW <= 128 && 128 / g.OW * g.OW >= 96) {
+    const int32_t *sums = filter_row_sums;
+    if (sums == nullptr) {
+      int32_t *bs = reinterpret_cast<int32_t *>(ws + pl.a_bytes + pl.f_bytes);
+      if (int rc = glowb200_i8_row_sums(filter, g.OC, g.C, bs, reinterpret_cast<glowb200_stream_t>(s))) return rc;
+      sums = bs;
+    }
+    p.K = g.C;
+    p.N = g.OC;
+    return run_gemm_strided(p, in, (int64_t)g.N * g.OH, g.OW, g.SW, g.W, filter, sums, s);
+  }
   const int8_t *a = in;
   if (pl.need_im2col) {
     int8_t *abuf = reinterpret_cast<int8_t *>(ws);

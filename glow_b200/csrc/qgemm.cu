@@ -124,6 +124,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+      : "memory");
+}
+
 // ---- CTA pairs (a cluster of two CTAs issuing one MMA over both SMs, cta_group::2) ----
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -454,7 +461,8 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   GEMM_TRACE(0, threadIdx.x == 0);
-  const int m_tiles = (p.M + kTileM - 1) / kTileM, n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
+  const int tile_rows = !PAIR && p.strided_lines ? p.strided_rows : kTileM;  // rows of a tile that are the product's
+  const int m_tiles = !PAIR && p.strided_lines ? (p.M + tile_rows - 1) / tile_rows : (p.M + kTileM - 1) / kTileM, n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int tiles = m_tiles * n_tiles;
   const int k_blocks = (p.K + kBlockK - 1) / kBlockK;
   // columns of one accumulator buffer: BLOCK_N rounded up to a power of two (240 -> 256)
@@ -499,7 +507,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       int it = 0;  // k-blocks issued so far, over all tiles of this CTA
       bool live = true;
       for (int t = walker; t < tiles && live; t += walkers) {
-        const int m0 = (t % m_tiles) * kTileM + (int)rank * kBlockM, n0 = (t / m_tiles) * BLOCK_N;
+        const int m0 = (t % m_tiles) * tile_rows + (int)rank * kBlockM, n0 = (t / m_tiles) * BLOCK_N;
         for (int kb = 0; kb < k_blocks; kb++, it++) {
           const int s = it % STAGES;
           if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag)) { live = false; break; }
@@ -512,8 +520,10 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             tma_load_2d_pair(b_dst, &map_b, kb * kBlockK, n0 + (int)rank * (BLOCK_N / 2), leader_full);
             continue;
           }
-          mbar_expect_tx(&full[s], S::kStageBytes);
-          if (p.conv_windows) {
+          mbar_expect_tx(&full[s], S::kBBytes + (uint32_t)tile_rows * kBlockK);
+          if (p.strided_lines) {
+            tma_load_3d(a_dst, &map_a, kb * kBlockK, 0, (t % m_tiles) * p.strided_lines, &full[s]);
+          } else if (p.conv_windows) {
             // four 128 x 32-byte sub-tiles: window a of plane kb of the 128 pixels, one per MMA k-step
             for (int a4 = 0; a4 < 4; a4++)
               tma_load_2d(a_dst + a4 * (kBlockM * 32), &map_a, 0, kb * p.conv_windows + m0 + a4 * p.conv_wp, &full[s]);
@@ -606,7 +616,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     int m_tile = walker % m_tiles, n_tile = walker / m_tiles;
     for (int t = walker; t < tiles; t += walkers, lt++) {
       for (; m_tile >= m_tiles; m_tile -= m_tiles) n_tile++;
-      const int m0 = m_tile * kTileM + (int)rank * kBlockM, n0 = n_tile * BLOCK_N;
+      const int m0 = m_tile * tile_rows + (int)rank * kBlockM, n0 = n_tile * BLOCK_N;
       m_tile += walkers;
       const int buf = lt & 1;
       // (1) per-column constants of this tile (the main loop of this or the next tile is running).
@@ -653,8 +663,8 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             if (folded) {
               reinterpret_cast<int2 *>(cols)[et] = make_int2(cp.c, cp.scale);
               reinterpret_cast<int32_t *>(cols)[2 * BLOCK_N + et] = pre;
-            } else {
-              cols[et] = cp;
+            } else {  // nothing to unpack: {c, scale, pre, post}
+              cols[et] = ColParams{cp.c, cp.scale, pre, post};
               col_rounding[et] = (int32_t)((1u << post) >> 1);
             }
           }
@@ -688,7 +698,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       GEMM_TRACE(4, lt == 0 && et == 0);
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * kAccCols;
       int out_index = row;  // row of the result this accumulator row becomes
-      bool row_ok = row < p.M;
+      bool row_ok = row < p.M && (PAIR || quarter * 32 + lane < tile_rows);
       if (p.conv_entries > 0 || p.conv_windows) {  // padded pixel -> (image, oh, ow); the halo rows are dropped
         const int img = fast_div(row, p.conv_hpwp, image_div), rem = row - img * p.conv_hpwp;
         const int oh = fast_div(rem, p.conv_wp, line_div), ow = rem - oh * p.conv_wp;
@@ -845,7 +855,7 @@ i8_gemm_requant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
                 for (int cc = 0; cc < 2; cc++) {
                   const int4 cp = *reinterpret_cast<const int4 *>(&cols[j + cc]);
-                  const int32_t pre = cp.z & 0xff, post = cp.z >> 8;
+                  const int32_t pre = kFolds ? cp.z : cp.z & 0xff, post = kFolds ? cp.w : cp.z >> 8;
 #pragma unroll
                   for (int i = 0; i < 4; i++) {
                     uint32_t v = acc[8 * (i >> 1) + 4 * g + 2 * (i & 1) + cc] + (uint32_t)cp.x;
@@ -1130,7 +1140,8 @@ int launch_tile_mode(const CUtensorMap &ma, const CUtensorMap &mb, const GemmPar
   // per device and cheap: set on every launch rather than tracked
   GLOWB200_CUDA_OK(cudaFuncSetAttribute(i8_gemm_requant_kernel<BLOCK_N, STAGES, MODE>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-  const int tiles = ((p.N + BLOCK_N - 1) / BLOCK_N) * ((p.M + kBlockM - 1) / kBlockM);
+  const int tile_rows = p.strided_lines ? p.strided_rows : kBlockM;
+  const int tiles = ((p.N + BLOCK_N - 1) / BLOCK_N) * ((p.M + tile_rows - 1) / tile_rows);
   const int sms = sm_count();
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(tiles < sms ? tiles : sms));
@@ -1292,6 +1303,29 @@ int run_gemm_shifted_rows(GemmParams p, const int8_t *padded, int64_t rows, int 
   if (p.k_corr == 0) p.k_corr = p.K;
   // C = 64: a 128-byte window over two neighbouring pixels, sliding by one pixel per row
   return launch_for_block_n(pick_tile(p.M, p.N, false), padded, (int)buffer_rows, C == 64 ? 128 : C, C, b, p, s);
+}
+
+int run_gemm_strided(GemmParams p, const int8_t *in, int64_t lines, int ow, int stride, int width, const int8_t *b, const int32_t *b_row_sums,
+                     cudaStream_t s) {
+  GLOWB200_REQUIRE(ow > 0 && ow <= kBlockM && lines * ow < (1ll << 31) && p.K % 16 == 0 && ptr16(in) && ptr16(b) && b_row_sums != nullptr,
+                   "strided convolution: unsupported shape");
+  p.M = (int)(lines * ow);
+  p.strided_lines = kBlockM / ow;
+  p.strided_rows = p.strided_lines * ow;
+  p.b_row_sums = b_row_sums;
+  p.a_row_sums = nullptr;
+  if (p.k_corr == 0) p.k_corr = p.K;
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return set_error(GLOWB200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  CUtensorMap ma;
+  cuuint64_t dims[3] = {(cuuint64_t)p.K, (cuuint64_t)ow, (cuuint64_t)lines};
+  cuuint64_t strides[2] = {(cuuint64_t)stride * p.K, (cuuint64_t)stride * width * p.K};
+  cuuint32_t box[3] = {(cuuint32_t)kBlockK, (cuuint32_t)ow, (cuuint32_t)p.strided_lines};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t *>(in), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(GLOWB200_ERR_CUDA, "cuTensorMapEncodeTiled (strided) failed with CUresult %d", (int)r);
+  return launch_for_block_n(pick_tile(p.M, p.N, false), nullptr, 0, 0, 0, b, p, s, &ma);
 }
 
 int run_gemm_row_windows(GemmParams p, const int8_t *planes, int64_t rows, int ow, const int8_t *b, const int32_t *b_row_sums,

@@ -65,6 +65,10 @@ struct GemmParams {
   // (n * Y + oh) * OW + ow of the product (conv_hpwp = Y * OW, conv_wp = OW); rows with oh >= conv_oh
   // are computed and dropped.
   int conv_windows;
+  // Strided pointwise convolution (strided_lines != 0): the left operand is every second (or third ...) pixel of the
+  // input, a 3-D map [lines of output pixels, OW, C] whose box is strided_lines of them; a tile has that many lines' pixels,
+  // strided_lines * OW <= 128 of its rows, and the rest are dropped.
+  int strided_lines, strided_rows;
   int conv_row_off[32];
   int conv_hpwp, conv_wp, conv_oh, conv_ow;
   int32_t u_b_offset, u_bias_pre, u_bias_post, u_bias_scale, u_out_pre, u_out_post, u_out_scale;
@@ -166,6 +170,11 @@ int run_prepare_operands(PrepParams p, cudaStream_t s);
 // buffer_rows: rows the padded buffer holds when the taps reach beyond `rows` (several planes); 0 = rows.
 int run_gemm_shifted_rows(GemmParams p, const int8_t *padded, int64_t rows, int C, const int8_t *b,
                           const int32_t *b_row_sums, cudaStream_t s, int64_t buffer_rows = 0);
+
+// A pointwise convolution of stride s over an input whose height and width are multiples of it, read in place: p.M output
+// pixels in `lines` lines of ow; p.K = channels (a multiple of 16).  No weight offsets.
+int run_gemm_strided(GemmParams p, const int8_t *in, int64_t lines, int ow, int stride, int width, const int8_t *b, const int32_t *b_row_sums,
+                     cudaStream_t s);
 
 // The row-window convolution: `planes` holds two planes of `rows` 32-byte windows each, back to back,
 // with 3 * ow + 1 readable windows behind the second; b is [N, 256] (plane, a, 32 bytes).

@@ -254,3 +254,27 @@ def test_pools_in_words(oracle, c, k, s, p):
         tr = ops.quantize_scale_offset_32to8(np.float32(0.6) / np.float32(k[0] * k[1] if cip else 1))
         np.testing.assert_array_equal(ops.avg_pool_i8(t(x), k, s, p, cip, 3, -4, tr).cpu().numpy(),
                                       oracle.avg_pool_i8(x, ohw, k, s, p, cip, 3, -4, tr))
+
+
+@pytest.mark.parametrize("n,hw,c,oc,s", [
+    (30, (56, 56), 64, 96, 2),     # 112 rows of a tile are pixels, the last tile cut
+    (41, (28, 28), 144, 64, 2),    # 126, channels that end within a k-block
+    (90, (14, 14), 256, 130, 2),   # ragged result rows
+    (70, (12, 24), 48, 64, 2),     # lines of 12
+    (9, (27, 126), 80, 72, 3),     # stride 3
+    (40, (57, 56), 64, 64, 2),     # an odd height: a copy of the pixels
+    (12, (40, 260), 64, 64, 2),    # lines longer than a tile: likewise
+    (11, (64, 154), 64, 64, 2),    # lines of 77, which leave too much of a tile
+])
+@pytest.mark.parametrize("act", [0, 1, 2])
+def test_strided_pointwise(n, hw, c, oc, s, act):
+    rng = np.random.default_rng(c + oc)
+    x, f = (t(rng.integers(-128, 128, sh, dtype=np.int8)) for sh in ((n, *hw, c), (oc, 1, 1, c)))
+    scales = rng.uniform(.002, .02, oc).astype(np.float32)
+    pp = [t(a) for a in ops.rowwise_requant_params(scales, .05, np.float32(.05) * scales, .2 * np.sqrt(c / 64))]
+    zero = torch.zeros(oc, dtype=torch.int32, device=DEV)
+    args = (x, f, t(rng.integers(-4000, 4000, oc, dtype=np.int32)), (1, 1), (s, s), (0,) * 4, 1, (1, 1), -20, 5, zero, zero, pp[:3], pp[3:],
+            act, [-30, 70] if act == 2 else None)
+    want = ops.channelwise_quantized_conv2d(*args, flags=ops.FC_FORCE_ANY_SHAPE_KERNEL)
+    for sums in (ops.i8_row_sums(f.view(oc, c)), None):
+        assert torch.equal(ops.channelwise_quantized_conv2d(*args, filter_row_sums=sums, flags=ops.FC_WEIGHT_OFFSETS_ZERO), want)
