@@ -32,11 +32,11 @@ sys.path.insert(0, ROOT)
 ROWS, DIM, BATCH = 1_000_000, 64, 1024
 IN_LINE = DIM + 8
 # DRAM bytes per gathered 72-byte row of the uint8 gather kernel: dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch of slws_run_kernel over 64 tables (2.10 M rows), from the
+# dram__bytes_write.sum of one launch of slws_stream_kernel over 64 tables (2.10 M rows), from the
 # ncu capture summarised in profiles/.  ncu cannot run inside the timed region, so `traffic` is
 # this figure x the rows of the timed launch (traffic is proportional to rows: every row is
-# fetched once, L2 hit rate 13 %).
-NCU_DRAM_BYTES_PER_ROW = 209.7
+# fetched once, L2 hit rate 16 %).
+NCU_DRAM_BYTES_PER_ROW = 208.9
 METRIC = "frwq_slws_hbm_gbps"
 UNIT = "GB/s"
 
@@ -1106,13 +1106,13 @@ def run_slws4_line(args):
                        "dim": D, "tables_per_gpu": T, "l2_policy": "tables far larger than L2, uniform indices"},
             "roofline": {"bound": "hbm", "achieved": per_gpu, "peak": peak, "unit": "GB/s", "frac": per_gpu / peak,
                          "peak_source": src,
-                         # DRAM bytes per launch: 198 B per row in the ncu capture of a smaller case of D=128
+                         # DRAM bytes per launch: 200 B per row in the ncu capture of a smaller case of D=128
                          # (profiles/), scaled by the rows of a launch; not captured for the other widths
-                         "traffic": 198.0 * float(np.mean([int(rq[3][-1]) for rq in reqs])) if D == 128 else None,
-                         "kernel": "slws_run_kernel<4,1,4,P,U>",
+                         "traffic": 200.0 * float(np.mean([int(rq[3][-1]) for rq in reqs])) if D == 128 else None,
+                         "kernel": "slws_stream_kernel<4,1,4,V>" if D > 64 else "slws_run_kernel<4,1,4,P,U>",
                          "rows_per_s": sum(int(reqs[i % R][3][-1]) for i in range(args.steps)) / (ms * 1e-3)},
-            # boundaries and pooling; few enough bags add the launch that would take skewed tables
-            "gpu_launches": (3 if D > 32 and T * B <= 384 * 148 else 2) * args.steps, "clocks": clocks}
+            # boundaries and pooling; 64 columns and few enough bags add the launch that would take skewed tables
+            "gpu_launches": (3 if D == 64 and T * B <= 384 * 148 else 2) * args.steps, "clocks": clocks}
         if world == 1 and not args.no_cpu_baseline:
             threads = os.cpu_count() or 1
             v, passes, dt = slws4_cpu_rate(D, min(args.cpu_seconds, 10.0), threads)
@@ -1478,7 +1478,7 @@ def run_slws4_sharded_line(args):
                        "dim": D, "tables": T, "l2_policy": "tables far larger than L2, uniform indices"},
             "roofline": {"bound": "hbm", "achieved": per_gpu, "peak": peak, "unit": "GB/s", "frac": per_gpu / peak,
                          "peak_source": src, "traffic": None,
-                         "kernel": "slws_run_kernel<4,1,4,P,U> over shards + sum_partials_kernel"},
+                         "kernel": "slws_run_kernel / slws_stream_kernel over shards + sum_partials_kernel"},
             "gpu_launches": 3 * args.steps, "clocks": clocks}))
     if world > 1:
         dist.destroy_process_group()
@@ -1806,7 +1806,7 @@ def main():
                          "nominal_peak": 8000.0, "frac_of_nominal": achieved / 8000.0,
                          # DRAM bytes per launch: bytes per gathered row from the ncu capture x the rows
                          "traffic": (None if args.row_bytes else NCU_DRAM_BYTES_PER_ROW * rows_per_launch),
-                         "kernel": "slws_run_kernel<8,0,8,2,4> (one launch: the warps add up the lengths themselves)",
+                         "kernel": "slws_stream_kernel<8,0,8,2> (one launch: the warps add up the lengths themselves)",
                          "launch_us": launch_us, "algorithmic_bytes_per_launch": moved / args.steps},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d // e2e_steps,
                     "d2h_bytes_per_step": d2h // e2e_steps, "steps": e2e_steps,
