@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(32, warps_per_sm(V)) slws_stream_kernel(const 
             if (number[k] >= 0) copy_piece_part(to + k * pitch, from(k), number[k] == last_row ? last_valid : 16);
         }
       }
+      __syncwarp();  // every lane has read its rows' numbers (the lanes do not leave the copies together): the next step's may come
       left -= kStep;
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };

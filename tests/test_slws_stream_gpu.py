@@ -111,3 +111,24 @@ def test_rows_that_are_not_there(kind, dim):
     odd[:, 5], odd[:, -1] = -4, odd[:, -1] + 60
     run(idx, w, odd)
     assert int(st.item()) == (ops.STATUS_NEGATIVE_LENGTH | ops.STATUS_LENGTHS_OVERRUN)
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 40), (0, 72), (0, 88), (0, 128), (2, 128), (2, 256), (3, 104)])
+@pytest.mark.parametrize("rows_of_a_bag", [33, 64, 65])
+def test_the_first_steps_of_a_run(kind, dim, rows_of_a_bag):
+    """The second step of a run is asked for right behind the first, by lanes that do not leave the first's copies together
+    (3 to 9 pieces to a row, so that 0 to 5 lanes copy none): each step of 32 rows has a number range of its own, and a row
+    fetched by the other step's number is not in the sums."""
+    rng = np.random.default_rng(dim + rows_of_a_bag)
+    rows, bags = 4096, 30_000
+    table = make_table(kind, rows, dim, 5)
+    lengths = np.full(bags, rows_of_a_bag, np.int32)
+    step = np.arange(rows_of_a_bag) // 32
+    idx = (rng.integers(0, rows // 4, (bags, rows_of_a_bag)) + step * (rows // 4)).reshape(-1)
+    w = rng.normal(0, 1, idx.size).astype(np.float16 if kind & 1 else np.float32)
+    got = pool(dev(table), w, idx, lengths, kind)
+    few = 300
+    check_pooled(table, kind, dim, w[:few * rows_of_a_bag], idx[:few * rows_of_a_bag], lengths[:few], got[:few])
+    for b in (0, 1, 17, bags - 1):
+        at = slice(b * rows_of_a_bag, (b + 1) * rows_of_a_bag)
+        assert torch.equal(pool(dev(table), w[at], idx[at], lengths[:1], kind)[0], got[b])
