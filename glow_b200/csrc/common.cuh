@@ -101,8 +101,11 @@ __device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
   const int q = (int)__umulhi((uint32_t)x, reciprocal);
   return q + (x - q * d >= d ? 1 : 0);
 }
-// nearbyintf(x / scale + offset) as an integer, by the reciprocal of the scale.  Its error is below 6e-4 within +- 2000;
-// next to a tie, and beyond, `sure` becomes false and the division has to decide (what rounds beyond int8 is clipped then).
+// nearbyintf(x / scale + offset) as an integer, by the reciprocal of the scale.  Where neither the sum nor the offset is beyond
+// +- 2000, the quotient is below 4000: the product's error of three halves of a unit in its last place (7.2e-4) and the roundings of
+// both sums (1.2e-4) stay below 1e-3.  Next to a tie, and beyond, `sure` becomes false and the division has to decide (what
+// rounds beyond int8 is clipped then).  `sure` starts as reciprocal_decides(offset).
+__device__ __forceinline__ bool reciprocal_decides(float offset) { return fabsf(offset) <= 2000.0f; }
 __device__ __forceinline__ int32_t quantize_by_reciprocal(float x, float inverse, float offset, bool &sure) {
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: its sum with u has rint(u) in the low bits
   const float u = __fadd_rn(__fmul_rn(x, inverse), offset), m = __fadd_rn(u, kMagic);

@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kThreads) transpose4_short_inner_kernel(const 
 
 // The Quantize on its way from C <= 4 channel planes to NHWC, four pixels at a time: C loads of 16 bytes, one word per
 // channel of quotients, whose bytes are dealt out to C words of the result.  The quotient is x times the reciprocal, next to a
-// tie the division decides: every element is quantize_one's.  What bounds it is memory: 64 x 3 x 224 x 224 24 us with a pixel and three divisions per thread, now 9.
+// tie, and for offsets far outside int8, the division decides: every element is quantize_one's.  What bounds it is memory: 64 x 3 x 224 x 224 24 us with a pixel and three divisions per thread, now 9.
 template <int C>
 __global__ void __launch_bounds__(kThreads) quantize_planes_kernel(const float *__restrict__ src, int8_t *__restrict__ dst, int d0, int d1,
                                                                    int d2, int s0, int s1, int s3, float scale, int32_t offset) {
@@ -445,6 +445,7 @@ __global__ void __launch_bounds__(kThreads) quantize_planes_kernel(const float *
   pdl_launch_dependents();
   const unsigned fours = (unsigned)d2 >> 2, total = (unsigned)d0 * (unsigned)d1 * fours;
   const float inverse = __fdiv_rn(1.0f, scale), shift = (float)offset;
+  const bool decides = reciprocal_decides(shift);
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const unsigned r = i / fours, i2 = (i - r * fours) * 4, i0 = r / (unsigned)d1, i1 = r - i0 * (unsigned)d1;
     const float *from = src + (int64_t)i0 * s0 + (int64_t)i1 * s1 + i2;
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(kThreads) quantize_planes_kernel(const float *
 #pragma unroll
     for (int c = 0; c < C; c++) {
       int32_t v[4];
-      bool sure = true;
+      bool sure = decides;
 #pragma unroll
       for (int e = 0; e < 4; e++) v[e] = quantize_by_reciprocal(x[c][e], inverse, shift, sure);
       if (!sure) {

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) pairwise_dot_kernel(const float *__restri
 // Few vectors have few tiles -- 28 of 4 x 4 for 27
 // vectors, the rest of the block idle -- and go in 2 x 2 tiles with no more warps than those fill: 128 samples of
 // 27 x 64 5.4 -> 3.3 us, 4096 samples 35 -> 21, 2048 of 17 x 32 15.0 -> 5.4.
-// The quantized result takes the reciprocal of its scale; next to a tie the division decides.
+// The quantized result takes the reciprocal of its scale; next to a tie, and for offsets far outside int8, the division decides.
 template <int R, int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) pairwise_dot_tiled_kernel(const float *__restrict__ dense, int64_t ld_dense,
                                                                              const float *__restrict__ pooled, int64_t ld_pooled,
@@ -98,9 +98,10 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) pairwise_dot_tiled_kernel(con
   }
   __syncthreads();
   const float inverse = __fdiv_rn(1.0f, q_scale), shift = (float)q_offset;
+  const bool decides = reciprocal_decides(shift);
   auto emit = [&](int64_t col, float x) {
     if (out_q) {
-      bool sure = true;
+      bool sure = decides;
       int32_t q = quantize_by_reciprocal(x, inverse, shift, sure);
       if (!sure) q = (int32_t)fminf(fmaxf(nearbyintf(__fadd_rn(__fdiv_rn(x, q_scale), shift)), -2147483648.0f), 2147483520.0f);
       out_q[b * ld_out + col] = (int8_t)clip_i8(q);

@@ -224,6 +224,22 @@ def test_quantize_planes_next_to_ties(channels, scale, offset):
     assert torch.equal(ops.quantize_transpose_i8(t(f), (0, 2, 3, 1), scale, offset), two)
 
 
+@pytest.mark.parametrize("scale,offset", [(0.0371, 1999), (0.0371, -2001), (0.0371, 20000), (0.0371, -20000), (1 / 3, 100_000), (7.3, -100_000),
+                                          (0.0371, 1 << 24), (0.05, -(2 ** 31 - 1))])
+def test_quantize_planes_of_large_offsets(oracle, scale, offset):
+    """The quotient is as large as the offset there, and its rounding as wide as the distance between results: the division's
+    all the same."""
+    rng = np.random.default_rng(abs(offset) % 1000)
+    k = np.arange(-200, 200) - float(offset)
+    near = ((k + .5) * scale).astype(np.float32)
+    x = np.concatenate([near, np.nextafter(near, np.float32(-np.inf)), np.nextafter(near, np.float32(np.inf)),
+                        ((rng.uniform(-140, 140, 200_000) - offset) * scale).astype(np.float32)])
+    x = np.resize(x, (1, 3, 100, 800)).astype(np.float32)
+    got = ops.quantize_transpose_i8(t(x), (0, 2, 3, 1), scale, offset)
+    np.testing.assert_array_equal(got.cpu().numpy(), oracle.element_quantize_i8(x, scale, offset).transpose(0, 2, 3, 1))
+    assert torch.equal(got, ops.transpose(ops.element_quantize_i8(t(x), scale, offset), (0, 2, 3, 1)))
+
+
 @pytest.mark.parametrize("n,h,w,c,oc,k,p", [
     (2, 20, 24, 3, 16, (7, 7), (3, 3, 3, 3)),     # image rows of whole words
     (2, 21, 23, 3, 16, (7, 7), (3, 3, 3, 3)),     # rows that start anywhere

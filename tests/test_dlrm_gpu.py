@@ -166,3 +166,19 @@ def test_interaction_of_many_samples(oracle, B, T, D):
     for scale, offset in ((0.125, -7), (0.37, 100), (1e-3, 0)):
         np.testing.assert_array_equal(ops.pairwise_dot_interaction(*args, quant=(scale, offset)).cpu().numpy(),
                                       oracle.element_quantize_i8(want, scale, offset))
+
+
+@pytest.mark.parametrize("T", [20, 64])
+@pytest.mark.parametrize("scale,offset", [(0.0371, -1999), (0.0371, -20_000), (1 / 3, -100_000)])
+def test_interaction_quantized_with_large_offsets(oracle, T, scale, offset):
+    """(dots round -scale * offset, whose results fill int8: the quotients are as large as the offset)"""
+    rng = np.random.default_rng(T)
+    B, size = 400, np.sqrt(-scale * offset)
+    v = np.zeros((B, T + 1, 4), np.float32)
+    v[..., 0] = size * (1 + rng.uniform(-60, 60, (B, T + 1)) / -offset)
+    v[..., 1:] = rng.uniform(-.01, .01, (B, T + 1, 3))
+    dense, pooled = np.ascontiguousarray(v[:, 0]), np.ascontiguousarray(v[:, 1:])
+    want = oracle.element_quantize_i8(oracle.pairwise_dot_interaction(dense, pooled), scale, offset)
+    got = ops.pairwise_dot_interaction(torch.from_numpy(dense).to(DEV), torch.from_numpy(pooled).to(DEV), quant=(scale, offset))
+    assert len(np.unique(want)) > 200
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
