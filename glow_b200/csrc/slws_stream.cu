@@ -91,7 +91,9 @@ __device__ __forceinline__ void pool_word_strict(uint32_t word, float scale, flo
 
 // V columns per lane.  STRICT: uint8 rows of a width that slws_gather_any_kernel pools else, by its operations: (q * scale + offset)
 // * w added up, each rounded on its own, as the reference's Interpreter has them (20 x 2000 of 100 columns 321 -> 76 us).
-template <int BITS, bool SO16, int ALIGN, int V, bool STRICT = false>
+// CUT: the table starts off 16 bytes, and the bytes in front of it, which row 0's first piece has, are not to be read.  (An
+// instance of its own: in all of them it cost 64 skewed tables of 4096 bags of 128 columns 546 -> 554 us.)
+template <int BITS, bool SO16, int ALIGN, int V, bool STRICT = false, bool CUT = false>
 __global__ void __launch_bounds__(32, warps_per_sm(V)) slws_stream_kernel(const __grid_constant__ SlwsLaunch p, int bags_per_warp, int chunks) {
   pdl_wait();
   pdl_launch_dependents();
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(32, warps_per_sm(V)) slws_stream_kernel(const 
       const float w = out16 ? __half2float(__ushort_as_half((unsigned short)(high ? word >> 16 : word))) : __uint_as_float(word);
       meta[stage * kStep + lane] = make_float2(w, __int_as_float(r < 0 ? -1 : (int)(((uint32_t)r * in_line + (uint32_t)data) & 15u)));
       numbers[lane] = r;
-      const bool plain = !__any_sync(kAllLanes, r < 0 || r == last_row);
+      const bool plain = !__any_sync(kAllLanes, r < 0 || r == last_row || (CUT && r == 0));
       __syncwarp();
       const uint32_t to = copy_to + stage * stage_bytes;
       const int32_t *number = numbers + copier;
@@ -196,8 +198,14 @@ __global__ void __launch_bounds__(32, warps_per_sm(V)) slws_stream_kernel(const 
           if (k + copier < kStep) copy_piece(to + k * pitch, from(k));
         } else {
           // (a row that is not there is not read: as row 0 it cost a launch of bags of one row 900 us, all warps at the same lines)
-          for (int k = 0; k + copier < kStep; k += per_copy)
-            if (number[k] >= 0) copy_piece_part(to + k * pitch, from(k), number[k] == last_row ? last_valid : 16);
+          for (int k = 0; k + copier < kStep; k += per_copy) {
+            if (CUT && piece == 0 && number[k] == 0) {  // (word by word)
+              for (int b = (int)data & 15; b < 16; b += 4)
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + k * pitch + b), "r"(__ldg(reinterpret_cast<const uint32_t *>(from(k) + b))) : "memory");
+            } else if (number[k] >= 0) {
+              copy_piece_part(to + k * pitch, from(k), number[k] == last_row ? last_valid : 16);
+            }
+          }
         }
       }
       __syncwarp();  // every lane has read its rows' numbers (the lanes do not leave the copies together): the next step's may come
@@ -296,13 +304,14 @@ __global__ void __launch_bounds__(32, warps_per_sm(V)) slws_stream_kernel(const 
 // Columns of a lane.
 int columns_of(const SlwsLaunch &L) { return L.out_line <= 64 ? 2 : L.out_line <= 128 ? 4 : 8; }
 
-template <int BITS, bool SO16, int ALIGN>
+template <int BITS, bool SO16, int ALIGN, bool CUT = false>
 cudaError_t launch_columns(const SlwsLaunch &L, int run, int chunks, dim3 grid, cudaStream_t s) {
-  auto kernel = columns_of(L) == 2 ? slws_stream_kernel<BITS, SO16, ALIGN, 2> : slws_stream_kernel<BITS, SO16, ALIGN, 4>;
+  auto kernel = columns_of(L) == 2 ? slws_stream_kernel<BITS, SO16, ALIGN, 2, false, CUT> : slws_stream_kernel<BITS, SO16, ALIGN, 4, false, CUT>;
   if constexpr (BITS == 8) {
-    if (L.out_line % 8 != 0) kernel = columns_of(L) == 2 ? slws_stream_kernel<BITS, SO16, ALIGN, 2, true> : slws_stream_kernel<BITS, SO16, ALIGN, 4, true>;
+    if (L.out_line % 8 != 0)
+      kernel = columns_of(L) == 2 ? slws_stream_kernel<BITS, SO16, ALIGN, 2, true, CUT> : slws_stream_kernel<BITS, SO16, ALIGN, 4, true, CUT>;
   } else {
-    if (columns_of(L) == 8) kernel = slws_stream_kernel<BITS, SO16, ALIGN, 8>;
+    if (columns_of(L) == 8) kernel = slws_stream_kernel<BITS, SO16, ALIGN, 8, false, CUT>;
   }
   return launch_pdl(kernel, grid, 32, warp_bytes(chunks), s, L, run, chunks);
 }
@@ -334,6 +343,14 @@ cudaError_t launch_slws_stream(const SlwsLaunch &L, int align, int64_t max_segme
   const int64_t round = std::max<int64_t>(1, (total + resident - 1) / resident);
   const int run = (int)(round <= 16 ? (round + 1) / (round <= 6 && round > 1 && !L.inline_lengths ? 3 : 2) : round <= 40 ? 6 : 12);
   const dim3 grid((unsigned)((max_segments + run - 1) / run), (unsigned)num_jobs);
+  if (!L.jobs && (reinterpret_cast<uintptr_t>(L.single.data) & 15) != 0) {
+    switch (L.kind) {
+      case GLOWB200_UINT8_FUSED: return launch_columns<8, false, 4, true>(L, run, chunks, grid, s);
+      case GLOWB200_UINT8_FUSED_FP16: return launch_columns<8, true, 4, true>(L, run, chunks, grid, s);
+      case GLOWB200_UINT4_FUSED: return launch_columns<4, false, 4, true>(L, run, chunks, grid, s);
+      default: return launch_columns<4, true, 4, true>(L, run, chunks, grid, s);
+    }
+  }
   switch (L.kind) {
     case GLOWB200_UINT8_FUSED: return align == 8 ? launch_columns<8, false, 8>(L, run, chunks, grid, s) : launch_columns<8, false, 4>(L, run, chunks, grid, s);
     case GLOWB200_UINT8_FUSED_FP16: return launch_columns<8, true, 4>(L, run, chunks, grid, s);

@@ -53,6 +53,18 @@ def test_tables_at_any_four_bytes(kind, dim, shift):
     assert torch.equal(pool(dev(table, shift), w, idx, lengths, kind), pool(dev(table), w, idx, lengths, kind))
 
 
+@pytest.mark.parametrize("rows", [1, 2, 40])
+@pytest.mark.parametrize("kind,dim", [(0, 40), (0, 96), (0, 100), (1, 128), (2, 96), (3, 128)])
+@pytest.mark.parametrize("shift", [4, 8, 12])
+def test_the_first_row_of_a_table_off_sixteen_bytes(kind, dim, rows, shift):
+    """Its first piece begins in front of the table, and what lies there is not read."""
+    rng = np.random.default_rng(rows + shift)
+    table = make_table(kind, rows, dim, 5)
+    lengths, idx, w = request_of(rng, rows, 13_000, kind)
+    idx[rng.integers(0, idx.size, idx.size // 5)] = 0
+    assert torch.equal(pool(dev(table, shift), w, idx, lengths, kind), pool(dev(table), w, idx, lengths, kind))
+
+
 @pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("dim", [44, 60, 68, 100, 124])
 @pytest.mark.parametrize("bags", [1, 7, 300, 2049, 15_000])
