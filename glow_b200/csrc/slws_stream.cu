@@ -36,8 +36,19 @@ constexpr int kStep = 32;     // rows of a step: lane l knows row l
 constexpr int kStages = 2;    // steps in shared memory: being added up, on its way
 // Warps on an SM, by the registers they are given: 64 or 96.
 constexpr int warps_per_sm(int v) { return v == 2 ? 32 : 20; }
-constexpr int kMostChunks = 18;  // of a row that slws_run.cu could pool as well; and of any
-constexpr int kMostChunksAlone = 32;
+// Pieces of a row that slws_run.cu could pool as well.  It reads the sectors that hold columns or the scale, and this kernel the
+// whole row: rows stored apart (ops.pad_fused_rows) are copied with the padding between.  Both in us at 8 x 4000 bags of
+// 40 rows / 16 x 2000 of 20 / one of 20,000 of 30, slws_run.cu -> this one: uint8 rows of 40 columns in 128 bytes 71 / 49 / 54 -> 65 / 43 / 54, in 192
+// 2 - 7 % slower, in 256 81 / 54 / 58 -> 97 / 63 / 69; 4-bit ones of 40 in 64 bytes 69 / 47 / 51 -> 65 / 43 / 52, in 112 0 / -4 / +4 %, in 256 81 / 54 / 58 ->
+// 103 / 66 / 71; uint8 ones of 96 in 160 bytes -5 / -6 / -3 %, in 192 -3 / -3 / +3 %, in 256 89 / 58 / 65 -> 97 / 63 / 69; 4-bit ones of 96 in 144 -6 / 0 / 0 %, in
+// 160 -4 / +3 / 0 %; 4-bit ones of 160 to 256 columns, and uint8 ones with halves (whose rows the other kernels read in
+// words), 2 - 8 % faster in 256 bytes still.
+int most_chunks(int kind, int columns) {
+  if (kind == GLOWB200_UINT8_FUSED_FP16 || columns > 128) return 18;
+  if (columns <= 64) return kind >= 2 ? 6 : columns <= 56 ? 8 : 7;
+  return kind >= 2 ? 9 : 10;
+}
+constexpr int kMostChunksAlone = 32;  // of any other row
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void copy_piece(uint32_t to, const uint8_t *from) {
@@ -328,7 +339,7 @@ int chunks_of(const SlwsLaunch &L) {
 bool slws_stream_takes(const SlwsLaunch &L, int align) {
   // (a row's pieces may reach 20 bytes into the next row)
   return align >= 4 && L.out_line % 4 == 0 && L.out_line <= (L.kind >= 2 ? 256 : 128) && L.in_line >= 32 &&
-         chunks_of(L) <= (L.out_line % 8 == 0 ? kMostChunks : kMostChunksAlone);
+         chunks_of(L) <= (L.out_line % 8 == 0 ? most_chunks(L.kind, L.out_line) : kMostChunksAlone);
 }
 
 cudaError_t launch_slws_stream(const SlwsLaunch &L, int align, int64_t max_segments, int64_t num_jobs, cudaStream_t s) {

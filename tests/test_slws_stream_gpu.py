@@ -65,6 +65,19 @@ def test_the_first_row_of_a_table_off_sixteen_bytes(kind, dim, rows, shift):
     assert torch.equal(pool(dev(table, shift), w, idx, lengths, kind), pool(dev(table), w, idx, lengths, kind))
 
 
+@pytest.mark.parametrize("kind,dim,strides", [(0, 40, (112, 128, 144, 256)), (0, 96, (144, 160, 176, 256)), (1, 96, (256, 288, 304)),
+                                              (2, 56, (96, 112, 256)), (2, 96, (144, 160, 256)), (3, 256, (256, 288, 304))])
+def test_rows_stored_apart(kind, dim, strides):
+    """Up to so many pieces to a row they are copied whole, padding and all; beyond, another kernel reads their columns."""
+    rng = np.random.default_rng(dim)
+    table = make_table(kind, 800, dim, 5)
+    lengths, idx, w = request_of(rng, 800, 13_000, kind)
+    want = pool(dev(table), w, idx, lengths, kind)
+    for stride in strides:
+        apart = ops.pad_fused_rows(dev(table), kind, stride)
+        assert torch.equal(pool(apart, w, idx, lengths, kind, out_line=dim), want)
+
+
 @pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("dim", [44, 60, 68, 100, 124])
 @pytest.mark.parametrize("bags", [1, 7, 300, 2049, 15_000])
