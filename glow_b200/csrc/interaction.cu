@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) pairwise_dot_kernel(const float *__restri
 // the neighbouring rows a warp reads fall into different banks.
 // What bounds it, for many vectors, is the copying and the sums in turn: 45 us of one and 67 of the other for 4096 samples of
 // 65 x 128, where a multiply-add of three registers takes a scheduler 1.5 to 1.9 clocks.  Vectors come by asynchronous
-// copies, without a register on the way (133 -> 114 us), and more blocks fit an SM when they have no idle warps
+// copies, without a register on the way (133 -> 114 us), and more blocks fit an SM when they are smaller
 // (108).  Not better: 8 x 4 tiles over a transposed copy with packed multiply-adds (138), 6 x 6, 7 x 7 and 8 x 8 tiles of
 // several samples to a block (124 - 146), two buffers and a block that goes on (122 - 136).
 // Few vectors have few tiles -- 28 of 4 x 4 for 27
@@ -180,9 +180,11 @@ extern "C" int glowb200_pairwise_dot_interaction(const float *dense, int64_t ld_
     const int64_t warps = (tiles_of(R) + 31) / 32;
     const int vec_in = (reinterpret_cast<uintptr_t>(dense) % 16 == 0) && (ld_dense % 4 == 0) &&
                        (tables == 0 || (reinterpret_cast<uintptr_t>(pooled) % 16 == 0 && ld_pooled % 4 == 0));
-    // Blocks with no more threads than tiles once six of them to an SM fill it more than twice (4096 samples of 65 x 128: 108 us
-    // against 114); fewer samples are copied and summed faster by larger ones (512 samples: 18.4 against 27).
-    const bool many = R == 4 && tiles_of(4) <= 160 && batch >= 2 * 6 * (int64_t)sm_count();
+    // Blocks of 160 threads once six of them to an SM -- where its shared memory holds six -- fill it more than twice (4096 samples of
+    // 65 x 128: 108 us against 114; of 49 x 64 51 against 53; 16,384 of 57 x 96 270 against 296); fewer samples are copied and summed faster by
+    // larger ones (512 samples: 18.4 against 27), and so are vectors of which fewer blocks fit (4096 of 65 x 160 143 us against 154, of
+    // 65 x 256 239 against 249).
+    const bool many = R == 4 && tiles_of(4) <= 160 && batch >= 2 * 6 * (int64_t)sm_count() && 6 * (tiled_smem + 1024) <= 228 * 1024;
     auto kernel = many ? pairwise_dot_tiled_kernel<4, 160, 6> : R == 4 ? pairwise_dot_tiled_kernel<4, 256, 4> : pairwise_dot_tiled_kernel<2, 256, 4>;
     const unsigned threads = many ? 160 : R == 4 ? 256 : 32 * (unsigned)(warps < 2 ? 2 : warps > 8 ? 8 : warps);
     if (tiled_smem > 48 * 1024)

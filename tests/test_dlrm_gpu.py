@@ -152,16 +152,24 @@ def test_peer_rendezvous_kernel_and_its_bounded_wait():
     buf.release()
 
 
-@pytest.mark.parametrize("B,T,D", [(1776, 47, 8), (1777, 67, 4), (1775, 50, 8)])
+@pytest.mark.parametrize("B,T,D", [
+    (1776, 47, 8),      # 78 tiles of 4 x 4: tiles of 2 x 2
+    (1776, 48, 8),      # 91: blocks of 160 threads
+    (1777, 67, 4),
+    (1775, 50, 8),      # a sample fewer: blocks of 256
+    (1777, 64, 128),    # 35.9 KB a block, six of which just fit an SM
+    (1777, 67, 200),    # 55 KB: too large for six
+    (1776, 68, 8),      # 171 tiles: blocks of 256
+])
 def test_interaction_of_many_samples(oracle, B, T, D):
-    """Launches on either side of the change of block size, quantized next to ties as well."""
+    """Launches on either side of the changes of tile and block size, quantized next to ties as well."""
     rng = np.random.default_rng(T)
     dense = (rng.integers(-6, 7, (B, D)) / 4).astype(np.float32)   # dots on a grid: many are halves of the scale
     pooled = (rng.integers(-6, 7, (B, T, D)) / 4).astype(np.float32)
     want = oracle.pairwise_dot_interaction(dense, pooled)
     args = torch.from_numpy(dense).to(DEV), torch.from_numpy(pooled).to(DEV)
     np.testing.assert_array_equal(ops.pairwise_dot_interaction(*args).cpu().numpy().view(np.uint32), want.view(np.uint32))
-    # (|dot| <= 2.25 * 8 = 18: at 1e-3 quotients reach 18000, beyond where the reciprocal is trusted, and stay inside
+    # (|dot| <= 2.25 * D: at 1e-3 quotients reach 9000 and more, beyond where the reciprocal is trusted, and stay inside
     # int32, where the reference's conversion is defined)
     for scale, offset in ((0.125, -7), (0.37, 100), (1e-3, 0)):
         np.testing.assert_array_equal(ops.pairwise_dot_interaction(*args, quant=(scale, offset)).cpu().numpy(),
