@@ -102,14 +102,14 @@ __device__ __forceinline__ int fast_div(int x, int d, uint32_t reciprocal) {
   return q + (x - q * d >= d ? 1 : 0);
 }
 // nearbyintf(x / scale + offset) as an integer, by the reciprocal of the scale.  Where neither the sum nor the offset is beyond
-// +- 2000, the quotient is below 4000: the product's error of three halves of a unit in its last place (7.2e-4) and the roundings of
-// both sums (1.2e-4) stay below 1e-3.  Next to a tie, and beyond, `sure` becomes false and the division has to decide (what
-// rounds beyond int8 is clipped then).  `sure` starts as reciprocal_decides(offset).
-__device__ __forceinline__ bool reciprocal_decides(float offset) { return fabsf(offset) <= 2000.0f; }
-__device__ __forceinline__ int32_t quantize_by_reciprocal(float x, float inverse, float offset, bool &sure) {
+// +- 2000, the quotient is below 4000: three roundings of a relative 2^-24 (of the reciprocal, the product and the division; 7.2e-4) and
+// those of both sums (1.2e-4) stay below 1e-3.  Next to a tie, and beyond, `sure` becomes false and the division has to decide (what
+// rounds beyond int8 is clipped then).  limit: reciprocal_limit(offset), beyond which no sum is sure.
+__host__ __device__ inline float reciprocal_limit(int32_t offset) { return offset >= -2000 && offset <= 2000 ? 2000.0f : 0.0f; }
+__device__ __forceinline__ int32_t quantize_by_reciprocal(float x, float inverse, float offset, float limit, bool &sure) {
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: its sum with u has rint(u) in the low bits
   const float u = __fadd_rn(__fmul_rn(x, inverse), offset), m = __fadd_rn(u, kMagic);
-  sure = sure && fabsf(u) < 2000.0f && fabsf(__fadd_rn(u, -__fadd_rn(m, -kMagic))) < 0.499f;
+  sure = sure && fabsf(u) < limit && fabsf(__fadd_rn(u, -__fadd_rn(m, -kMagic))) < 0.499f;
   return __float_as_int(m) - __float_as_int(kMagic);
 }
 // Walks x down a mixed radix: returns x % d and leaves x / d.

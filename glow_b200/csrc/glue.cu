@@ -440,12 +440,11 @@ __global__ void __launch_bounds__(kThreads) transpose4_short_inner_kernel(const 
 // tie, and for offsets far outside int8, the division decides: every element is quantize_one's.  What bounds it is memory: 64 x 3 x 224 x 224 24 us with a pixel and three divisions per thread, now 9.
 template <int C>
 __global__ void __launch_bounds__(kThreads) quantize_planes_kernel(const float *__restrict__ src, int8_t *__restrict__ dst, int d0, int d1,
-                                                                   int d2, int s0, int s1, int s3, float scale, int32_t offset) {
+                                                                   int d2, int s0, int s1, int s3, float scale, int32_t offset, float limit) {
   pdl_wait();
   pdl_launch_dependents();
   const unsigned fours = (unsigned)d2 >> 2, total = (unsigned)d0 * (unsigned)d1 * fours;
   const float inverse = __fdiv_rn(1.0f, scale), shift = (float)offset;
-  const bool decides = reciprocal_decides(shift);
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const unsigned r = i / fours, i2 = (i - r * fours) * 4, i0 = r / (unsigned)d1, i1 = r - i0 * (unsigned)d1;
     const float *from = src + (int64_t)i0 * s0 + (int64_t)i1 * s1 + i2;
@@ -456,9 +455,9 @@ __global__ void __launch_bounds__(kThreads) quantize_planes_kernel(const float *
 #pragma unroll
     for (int c = 0; c < C; c++) {
       int32_t v[4];
-      bool sure = decides;
+      bool sure = true;
 #pragma unroll
-      for (int e = 0; e < 4; e++) v[e] = quantize_by_reciprocal(x[c][e], inverse, shift, sure);
+      for (int e = 0; e < 4; e++) v[e] = quantize_by_reciprocal(x[c][e], inverse, shift, limit, sure);
       if (!sure) {
 #pragma unroll
         for (int e = 0; e < 4; e++) v[e] = quantize_one(x[c][e], scale, offset);
@@ -741,7 +740,7 @@ extern "C" int glowb200_quantize_transpose_i8(int8_t *dest, const float *src, co
     auto kernel = t.d[3] == 1 ? quantize_planes_kernel<1> : t.d[3] == 2 ? quantize_planes_kernel<2> : t.d[3] == 3 ? quantize_planes_kernel<3>
                                                                                                               : quantize_planes_kernel<4>;
     GLOWB200_CUDA_OK(launch_pdl(kernel, grid_for(t.total / t.d[3] / 4), kThreads, 0, GLOWB200_STREAM, src, dest, t.d[0], t.d[1], t.d[2],
-                                t.st[0], t.st[1], t.st[3], scale, offset));
+                                t.st[0], t.st[1], t.st[3], scale, offset, reciprocal_limit(offset)));
     return GLOWB200_OK;
   }
   return run_transpose(t, src, dest, QuantizeF{scale, offset}, GLOWB200_STREAM);

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) pairwise_dot_tiled_kernel(con
                                                                              const float *__restrict__ pooled, int64_t ld_pooled,
                                                                              int tables, int D, float *__restrict__ out_f,
                                                                              int8_t *__restrict__ out_q, int64_t ld_out, float q_scale,
-                                                                             int32_t q_offset, int vec_in) {
+                                                                             int32_t q_offset, float limit, int vec_in) {
   pdl_wait();               // (launched as a programmatic dependent of the pooling kernel)
   pdl_launch_dependents();  // a contraction that follows may set up now (it waits for this kernel before its loads)
   extern __shared__ __align__(16) float v[];  // [R * ceil(n / R)][D + 4]; rows beyond n are zero
@@ -98,11 +98,10 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) pairwise_dot_tiled_kernel(con
   }
   __syncthreads();
   const float inverse = __fdiv_rn(1.0f, q_scale), shift = (float)q_offset;
-  const bool decides = reciprocal_decides(shift);
   auto emit = [&](int64_t col, float x) {
     if (out_q) {
-      bool sure = decides;
-      int32_t q = quantize_by_reciprocal(x, inverse, shift, sure);
+      bool sure = true;
+      int32_t q = quantize_by_reciprocal(x, inverse, shift, limit, sure);
       if (!sure) q = (int32_t)fminf(fmaxf(nearbyintf(__fadd_rn(__fdiv_rn(x, q_scale), shift)), -2147483648.0f), 2147483520.0f);
       out_q[b * ld_out + col] = (int8_t)clip_i8(q);
     } else {
@@ -190,7 +189,7 @@ extern "C" int glowb200_pairwise_dot_interaction(const float *dense, int64_t ld_
     if (tiled_smem > 48 * 1024)
       GLOWB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_smem));
     GLOWB200_CUDA_OK(launch_pdl(kernel, (unsigned)batch, threads, tiled_smem, cs, dense, ld_dense, pooled, ld_pooled,
-                                (int)tables, (int)dim, out_f32, out_i8, ld_out, quant_scale, quant_offset, vec_in));
+                                (int)tables, (int)dim, out_f32, out_i8, ld_out, quant_scale, quant_offset, reciprocal_limit(quant_offset), vec_in));
     return GLOWB200_OK;
   }
   const size_t smem = (size_t)n * (dim + 1) * sizeof(float);
