@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(256) im2col_i8_rows_kernel(const int8_t *__res
 // What bounds it is the 53 MB that a batch of 64 images of 224 x 224 writes, and instructions beside it: 31 us with a
 // window's 21 bytes loaded one by one and 64-bit divisions, 23 by way of shared memory, now 19.
 struct WindowRadix {
-  Divisor width, height, images;
-  WindowRadix(const ConvGeom &g, int Y) : width(g.OW), height(Y), images(g.N) {}
+  Divisor width, height;
+  WindowRadix(const ConvGeom &g, int Y) : width(g.OW), height(Y) {}
 };
 __global__ void __launch_bounds__(256) row_windows_i8_kernel(const int8_t *__restrict__ x, int8_t *__restrict__ planes,
                                                               const __grid_constant__ ConvGeom g, const __grid_constant__ WindowRadix radix,

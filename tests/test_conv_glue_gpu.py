@@ -274,10 +274,13 @@ def test_pools_in_words(oracle, c, k, s, p):
 
 @pytest.mark.parametrize("n,hw,c,oc,s", [
     (30, (56, 56), 64, 96, 2),     # 112 rows of a tile are pixels, the last tile cut
-    (41, (28, 28), 144, 64, 2),    # 126, channels that end within a k-block
+    (41, (28, 28), 144, 64, 2),    # few rows: the few-row kernel
+    (44, (28, 28), 144, 64, 2),    # 126, channels that end within a k-block
     (90, (14, 14), 256, 130, 2),   # ragged result rows
-    (70, (12, 24), 48, 64, 2),     # lines of 12
-    (9, (27, 126), 80, 72, 3),     # stride 3
+    (70, (12, 24), 48, 64, 2),     # few rows
+    (120, (12, 24), 48, 64, 2),    # lines of 12
+    (9, (27, 126), 80, 72, 3),     # few rows
+    (22, (27, 126), 80, 72, 3),    # stride 3
     (40, (57, 56), 64, 64, 2),     # an odd height: a copy of the pixels
     (12, (40, 260), 64, 64, 2),    # lines longer than a tile: likewise
     (11, (64, 154), 64, 64, 2),    # lines of 77, which leave too much of a tile
