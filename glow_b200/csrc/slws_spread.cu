@@ -254,13 +254,6 @@ cudaError_t launch_slws_spread(const SlwsLaunch &L, SpreadShape c, int align, in
 //     columns; of wider ones from 64 on, or, where the boundaries are known and with them the skewed tables, from 84 on (47 x 250
 //     41 against 33 us, 8 x 1000 of 20 rows 14.2 against 15.7; one table of 12,000 skewed bags 38 against 43).  Not bags of fewer than
 //     five rows on average, nor of twelve in launches of up to 150 bags per SM (64 x 250 of 10 rows 14.2 against 16.0).
-//     Where the rows are unknown to the host: not rows of 57 to 64 columns, which fill slws_run.cu's groups and gain nothing with
-//     bags of 20 rows (16 x 2000 of them 45.1 against 43.0 us, 64 x 512 45.9 against 46.0) and lose with bags of one to three (64 x 512
-//     13.3 - 17.5 against 18.4 - 21.5).  Of other widths the bags of 20 rows gain 2 to 13 % (32 x 4096 of 96 columns 151 -> 132, of 40 115 -> 99),
-//     those of one to three between 25 % (32 x 4096 of 128 4-bit columns 50 -> 38) and -12 % (of 40 uint8 ones 34 -> 38).  In row shards, most
-//     of whose rows are elsewhere and take a place in a step all the same, not rows of 113 to 128 columns either (half to an eighth of the rows
-//     here, 2 M rows to a table: 32 x 4096 bags of 20 uint8 rows 147 - 128 against 154 - 140, 4 x 8192 of 64 4-bit ones 106 - 99
-//     against 116 - 110); narrower ones leave lanes of slws_run.cu's groups idle (64 x 512 of 96 columns 51 - 45 against 49 - 43).
 //     What follows is the rules for the others.
 //   * small launches take this one: up to the 12 bags per SM that are resident at once of rows of 32 columns, which leave
 //     half of the lanes idle here (2 x 211 skewed bags 16.9 -> 11.4 us); up to 24 of 64 columns (26 x 128 13.7 -> 11.7); up to 84 of
@@ -287,9 +280,8 @@ cudaError_t launch_slws(SlwsLaunch L, int align, int64_t max_segments, int64_t n
     return SpreadShape{v, lanes, rows, (int)std::min<int64_t>(kMaxRun, std::max<int64_t>(32 / lanes, (total + slots - 1) / slots))};
   };
   if (columns % 8 != 0) return launch_slws_stream(L, align, max_segments, num_jobs, s);
-  const bool whole_groups = (columns > 56 && columns <= 64 && (four_bit || !L.inline_lengths || rows < 0)) ||
-                            (columns > 112 && columns <= 128 && L.sharded);
-  const bool streams = columns > 32 && slws_stream_takes(L, align) && !whole_groups && !(rows >= 0 && rows < total * (total <= sms * 150 ? 12 : 5));
+  const bool streams = columns > 32 && slws_stream_takes(L, align) && !(columns > 56 && columns <= 64 && (four_bit || !L.inline_lengths)) &&
+                       !(rows >= 0 && rows < total * (total <= sms * 150 ? 12 : 5));
   const int64_t small = sms * (columns <= 32 ? 12 : columns <= 64 ? 24 : streams && L.inline_lengths ? 64 : 84);
   const bool short_bags = rows >= 0 && rows < total * 8, wide_bytes = !four_bit && columns > 128;
   if (align < 4 || columns > 256 || (wide_bytes && total <= sms * 32)) return launch_slws_run(L, align, max_segments, num_jobs, s);
