@@ -15,8 +15,8 @@
 // Here the groups of a warp are busy until its run of up to 32 bags is used up, and a step costs its
 // arithmetic (two instructions per column pair and row) plus what all groups share.  256 even tables of 64
 // columns, bound by the rate of random DRAM lines: 329 -> 310 us.  What is left to it beside slws_stream.cu:
-// rows of up to 32 columns, 4-bit ones of up to 64, uint8 ones of more than 128 (10 x 3000 even bags of 256
-// 114 us against 122), bags of a few rows, rows stored far apart, and the middle sizes that slws_spread.cu lists.
+// rows of up to 32 columns, 4-bit ones of less than 32 bytes or 57 to 64 columns, uint8 ones of more than 128 (10 x 3000 even bags
+// of 256 114 us against 122), bags of a few rows, rows stored far apart, and the middle sizes that slws_spread.cu lists.
 //
 // Memory.  U rows per group are requested before the first is consumed, and the indices of the group's next
 // step -- of its next bag, if this step ends one -- while they are on their way.  What decides is that none

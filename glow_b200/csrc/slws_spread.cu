@@ -254,6 +254,12 @@ cudaError_t launch_slws_spread(const SlwsLaunch &L, SpreadShape c, int align, in
 //     columns; of wider ones from 64 on, or, where the boundaries are known and with them the skewed tables, from 84 on (47 x 250
 //     41 against 33 us, 8 x 1000 of 20 rows 14.2 against 15.7; one table of 12,000 skewed bags 38 against 43).  Not bags of fewer than
 //     five rows on average, nor of twelve in launches of up to 150 bags per SM (64 x 250 of 10 rows 14.2 against 16.0).
+//     Where the host does not know the rows (the unsized entry points, row shards) bags of a few may be among them: 16 x 2000 even bags of one, three and
+//     ten rows of 64 columns 15 -> 21, 18 -> 23 and 31.5 -> 32.5 us, of 40 47 -> 46; but skewed ones of one to three on average 66 -> 40 and
+//     73 -> 44, of 20 98 -> 76.  The rows of a row shard that are elsewhere take a place in a step all the same, which the widths that leave no lanes of
+//     slws_run.cu's groups idle show (half, a quarter, an eighth of the rows here, 2 M to a table, 16 x 2000 bags of 40: 128 4-bit
+//     columns even 72 - 66 -> 76 - 71, skewed 194 - 187 -> 125 - 116; uint8 80 - 69 -> 79 - 71, 181 - 168 -> 134 - 122; of 96 columns 78 - 69 -> 73 - 66, 180 - 168 ->
+//     124 - 114).
 //     What follows is the rules for the others.
 //   * small launches take this one: up to the 12 bags per SM that are resident at once of rows of 32 columns, which leave
 //     half of the lanes idle here (2 x 211 skewed bags 16.9 -> 11.4 us); up to 24 of 64 columns (26 x 128 13.7 -> 11.7); up to 84 of

@@ -25,6 +25,10 @@
 // Not better, and not taken: 4-bit rows of 64 columns (40 x 2000 98 against 113), uint8 ones where the boundaries are known
 // (4 x 5000 even 22 against 25), uint8 rows of more than 128, of which shared memory holds too few (10 x 3000 even of 256 114
 // against 122), and bags of a row or two (32 x 4096 of 128 36 against 38).
+// Not better, and taken all the same, as the host knows neither the skew nor whether L2 holds the tables: even bags over small tables
+// (50,000 rows).  4 x 8192 of 64 rows of 128 4-bit columns 93 -> 101 (from memory, 10 M rows: 120 -> 101), of uint8 ones 95 -> 99, of 56 4-bit ones with
+// halves 75 -> 83 (1 M rows 89 -> 87, skewed 132 -> 116); 2 x 8192 of 16 rows of 40 columns 28 -> 34 (1 M rows 34 -> 34, skewed ones of
+// 56 4-bit columns 58 -> 50).
 #include <algorithm>
 
 #include "slws.cuh"
@@ -37,16 +41,21 @@ constexpr int kStages = 2;    // steps in shared memory: being added up, on its 
 // Warps on an SM, by the registers they are given: 64 or 96.
 constexpr int warps_per_sm(int v) { return v == 2 ? 32 : 20; }
 // Pieces of a row that slws_run.cu could pool as well.  It reads the sectors that hold columns or the scale, and this kernel the
-// whole row: rows stored apart (ops.pad_fused_rows) are copied with the padding between.  Both in us at 8 x 4000 bags of
-// 40 rows / 16 x 2000 of 20 / one of 20,000 of 30, slws_run.cu -> this one: uint8 rows of 40 columns in 128 bytes 71 / 49 / 54 -> 65 / 43 / 54, in 192
-// 2 - 7 % slower, in 256 81 / 54 / 58 -> 97 / 63 / 69; 4-bit ones of 40 in 64 bytes 69 / 47 / 51 -> 65 / 43 / 52, in 112 0 / -4 / +4 %, in 256 81 / 54 / 58 ->
-// 103 / 66 / 71; uint8 ones of 96 in 160 bytes -5 / -6 / -3 %, in 192 -3 / -3 / +3 %, in 256 89 / 58 / 65 -> 97 / 63 / 69; 4-bit ones of 96 in 144 -6 / 0 / 0 %, in
-// 160 -4 / +3 / 0 %; 4-bit ones of 160 to 256 columns, and uint8 ones with halves (whose rows the other kernels read in
-// words), 2 - 8 % faster in 256 bytes still.
+// whole row: rows stored apart (ops.pad_fused_rows) are copied with the padding between.  Even bags lose by that, skewed ones gain
+// as long as the rest of the launch gains more; the lines lie where the two are about equal.  This kernel's time over slws_run.cu's (with
+// slws_spread.cu), 8 x 4000 bags of 40 rows, 16 x 2000 of 20, one of 20,000 of 30 and 100 x 512 of 30, even; skewed:
+//   uint8, 40 columns in 160 bytes 1.02 1.00 1.04 1.00; 0.95 0.76 1.00 0.72, in 224 1.10 1.08 1.11 1.12; 1.03 0.88 1.01 0.82, in 256 1.20 1.14 1.14 1.17; 1.06 0.87 1.06 0.85
+//   uint8, 96 columns in 192 bytes 0.96 0.97 1.03 0.97; 0.85 0.68 0.85 0.66, in 256 1.10 1.08 1.05 1.09; 0.90 0.73 0.90 0.72
+//   4-bit, 48 columns in 128 bytes 0.98 0.96 1.04 0.95; 0.95 0.72 1.01 0.71, in 192 1.08 1.07 1.14 1.09; 1.04 0.84 1.00 0.80, in 256 1.25 1.21 1.17 1.24; 1.11 0.91 1.10 0.90
+//   4-bit, 96 columns in 192 bytes 0.98 1.02 1.03 1.04; 0.85 0.77 0.86 0.77, in 256 1.11 1.15 1.06 1.16; 0.91 0.82 0.91 0.84
+//   128 with halves in 192 bytes 1.01 1.04 1.04 1.07; 1.00 0.63 0.98 0.63, in 256 1.13 1.18 1.09 1.21; 1.07 0.67 1.07 0.68
+//   4-bit, 256 columns in 256 bytes 0.97 0.95 0.95 0.98; 0.82 0.56 0.91 0.67
+//   uint8 with halves, whose rows the other kernels read in words, 96 columns in 256 bytes 0.92 0.93 0.93 0.91; 0.90 0.53 0.90 0.52
+// 64 uint8 columns are padded to 128 bytes for launches that the rate of random lines bounds, and there it costs what the padding
+// gains: 256 x 1024 even bags of 32 rows 268 -> 301 us, skewed ones 439 -> 426 (in 112 bytes 358 -> 352, 539 -> 495).
 int most_chunks(int kind, int columns) {
-  if (kind == GLOWB200_UINT8_FUSED_FP16 || columns > 128) return 18;
-  if (columns <= 64) return kind >= 2 ? 6 : columns <= 56 ? 8 : 7;
-  return kind >= 2 ? 9 : 10;
+  if (kind == GLOWB200_UINT8_FUSED && columns <= 64) return columns <= 56 ? 14 : 7;
+  return kind >= 2 && columns <= 64 ? 12 : 18;
 }
 constexpr int kMostChunksAlone = 32;  // of any other row
 
