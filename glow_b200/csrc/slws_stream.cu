@@ -51,12 +51,9 @@ constexpr int warps_per_sm(int v) { return v == 2 ? 32 : 20; }
 //   128 with halves in 192 bytes 1.01 1.04 1.04 1.07; 1.00 0.63 0.98 0.63, in 256 1.13 1.18 1.09 1.21; 1.07 0.67 1.07 0.68
 //   4-bit, 256 columns in 256 bytes 0.97 0.95 0.95 0.98; 0.82 0.56 0.91 0.67
 //   uint8 with halves, whose rows the other kernels read in words, 96 columns in 256 bytes 0.92 0.93 0.93 0.91; 0.90 0.53 0.90 0.52
-// 64 uint8 columns are padded to 128 bytes for launches that the rate of random lines bounds, and there it costs what the padding
-// gains: 256 x 1024 even bags of 32 rows 268 -> 301 us, skewed ones 439 -> 426 (in 112 bytes 358 -> 352, 539 -> 495).
-int most_chunks(int kind, int columns) {
-  if (kind == GLOWB200_UINT8_FUSED && columns <= 64) return columns <= 56 ? 14 : 7;
-  return kind >= 2 && columns <= 64 ? 12 : 18;
-}
+//   uint8, 64 columns in 128 bytes (boundaries unknown) 256 x 1024 of 32, tables of 1 M rows 0.94, of 0.5 M 1.12; 0.97; 40 x 2000 of 20 1.17; 0.88, 100 x 512 0.97;
+//     0.77, in 192 16 x 2000 1.09; 1.01, 100 x 512 1.05; 0.84, in 256 1.22; 1.09, 1.18; 0.94
+int most_chunks(int kind, int columns) { return columns <= 64 && kind != GLOWB200_UINT8_FUSED_FP16 ? 12 : 18; }
 constexpr int kMostChunksAlone = 32;  // of any other row
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
