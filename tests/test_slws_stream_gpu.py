@@ -157,3 +157,62 @@ def test_the_first_steps_of_a_run(kind, dim, rows_of_a_bag):
     for b in (0, 1, 17, bags - 1):
         at = slice(b * rows_of_a_bag, (b + 1) * rows_of_a_bag)
         assert torch.equal(pool(dev(table), w[at], idx[at], lengths[:1], kind)[0], got[b])
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 96), (1, 96), (2, 96), (3, 128), (0, 100)])
+def test_weights_of_rows_that_are_not_there(kind, dim):
+    """A row that is not there adds nothing, whatever its weight: a NaN or an infinity of an index outside the table (or of
+    another shard's row) is in no sum, nor is what a lane beyond the end of a bag had in its register."""
+    rng = np.random.default_rng(dim + kind)
+    rows, bags = 500, 13_000
+    table = make_table(kind, rows, dim, 5)
+    d = dev(table)
+    dt = np.float16 if kind & 1 else np.float32
+    lengths = rng.integers(0, 75, bags).astype(np.int32)
+    n = int(lengths.sum())
+    idx, w = rng.integers(0, rows, n), rng.normal(0, 1, n).astype(dt)
+    out = rng.random(n) < 0.2
+    bad_i, bad_w, there, nothing = idx.copy(), w.copy(), idx.copy(), w.copy()
+    bad_i[out] = rng.choice([rows, rows + 9, -1], out.sum())
+    bad_w[out] = rng.choice(np.array([np.nan, np.inf, -np.inf, 1.0], dt), out.sum())
+    there[out], nothing[out] = 0, 0
+    st = ops.new_status(DEV)
+    got = pool(d, bad_w, bad_i, lengths, kind, status=st)
+    assert int(st.item()) == ops.STATUS_INDEX_OUT_OF_RANGE
+    want = pool(d, nothing, there, lengths, kind)
+    assert bool(torch.isfinite(want).all()) and torch.equal(got.float(), want.float())   # (a zero sum may have either sign)
+    few = 500   # and the kernel of small launches
+    few_n = int(lengths[:few].sum())
+    assert torch.equal(pool(d, bad_w[:few_n], bad_i[:few_n], lengths[:few], kind).float(), want[:few].float())
+    # offsets that go backwards: every bag is a stream of its own, and the rows behind its end have weights of before
+    mean = 37
+    begins = np.arange(bags + 1, dtype=np.int64) % 200 * mean
+    begins[1::2] += 40   # bags of 77 rows, and ones that end before they begin
+    weights = w[:begins.max() + 1].copy()
+    weights[rng.random(weights.size) < 0.002] = np.nan
+    out = ops.embedding_bag_byte_rowwise_offsets(d, dev(weights), dev(idx[:weights.size]), dev(begins), kind, has_end_offset=True, status=st)
+    for b in range(0, 400):
+        at, to = int(begins[b]), max(int(begins[b]), int(begins[b + 1]))
+        alone = pool(d, weights[at:to], idx[at:to], np.int32([to - at]), kind)[0]
+        assert torch.equal(torch.nan_to_num(out[b].float(), nan=1e30), torch.nan_to_num(alone.float(), nan=1e30)), b
+
+
+@pytest.mark.parametrize("kind,dim", [(0, 96), (2, 128)])
+def test_weights_of_other_shards_rows(kind, dim):
+    rng = np.random.default_rng(dim)
+    rows, bags, tables, shards = 300, 1900, 8, 4
+    table = make_table(kind, rows, dim, 5)
+    d = dev(table)
+    lengths = rng.integers(0, 60, (tables, bags)).astype(np.int32)
+    idx = [rng.integers(0, rows * shards, int(l.sum())) for l in lengths]
+    mine = [(i >= rows) & (i < 2 * rows) for i in idx]
+    w = [np.where(m, rng.normal(0, 1, m.size), np.inf).astype(np.float32) for m in mine]
+    out = torch.empty((tables, bags, dim), device=DEV)
+    st = ops.new_status(DEV)
+    b = ops.SlwsBatch(kind, table.shape[1], torch.int64, device=DEV)
+    b.bind([d] * tables, [dev(x) for x in w], [dev(x) for x in idx], [dev(x) for x in lengths], list(out), row_ranges=[(rows, rows * shards)] * tables)
+    b.run(st)
+    assert int(st.item()) == 0
+    for i in range(tables):
+        want = pool(d, np.where(mine[i], w[i], 0).astype(np.float32), np.where(mine[i], idx[i] - rows, 0), lengths[i], kind)
+        assert torch.equal(out[i], want)
