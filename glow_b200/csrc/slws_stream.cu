@@ -333,7 +333,8 @@ cudaError_t launch_columns(const SlwsLaunch &L, int run, int chunks, dim3 grid, 
   return launch_pdl(kernel, grid, 32, warp_bytes(chunks), s, L, run, chunks);
 }
 
-// 16-byte pieces that a row lies across at most, by what the rows start on.
+// 16-byte pieces that a row lies across at most, by what the rows start on (tables of a batch start on 16 bytes: the descriptors'
+// contract).
 int chunks_of(const SlwsLaunch &L) {
   const uintptr_t at = (L.jobs ? 0 : reinterpret_cast<uintptr_t>(L.single.data)) | (uintptr_t)L.in_line;
   const int start = (at & 15) == 0 ? 16 : (at & 7) == 0 ? 8 : 4;
